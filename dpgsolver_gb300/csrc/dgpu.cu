@@ -182,14 +182,16 @@ template <int D, int Q, int NV>
 size_t volume_smem_bytes()
 {
 	using S = TPShape<D, Q>;
-	return (sizeof(TPOps) + 7) / 8 * 8 + (size_t)S::E * (NV * S::N * 2 + D * NV * S::N) * sizeof(double);
+	return sizeof(TPOps) + (size_t)S::E * (TPSmem<D, Q, NV>::VOL * sizeof(double) +
+	                                       (TPSmem<D, Q, NV>::EXP + TPSmem<D, Q, NV>::AEXP) * sizeof(int));
 }
 
 template <int D, int Q, int NV>
 size_t lift_smem_bytes()
 {
 	using S = TPShape<D, Q>;
-	return (sizeof(TPOps) + 7) / 8 * 8 + (size_t)S::E * (3 * NV * S::N + 8) * sizeof(double);
+	return sizeof(TPOps) + (size_t)S::E * (TPSmem<D, Q, NV>::LIFT * sizeof(double) +
+	                                       TPSmem<D, Q, NV>::LEXP * sizeof(int));
 }
 
 template <int D, int Q, int NV>

@@ -152,7 +152,7 @@ __device__ __forceinline__ void num_flux_vjp_boundary(const TPParams& P, int b, 
 // ---------------------------------------------------------------------------------------------------------------
 template <int D, int Q, int NV, int PDE>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS)
-tp_adj_volume_kernel(const TPOps ops, const TPParams P, const AdjArgs A)
+tp_adj_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const AdjArgs A)
 {
 	using S = TPShape<D, Q>;
 	constexpr int N = S::N, NF = S::NF, E = S::E;
@@ -349,7 +349,7 @@ tp_adj_face_kernel(const TPParams P, const AdjArgs A)
 
 template <int D, int Q, int NV>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS)
-tp_adj_lift_kernel(const TPOps ops, const TPParams P, const AdjArgs A)
+tp_adj_lift_kernel(const __grid_constant__ TPOps ops, const TPParams P, const AdjArgs A)
 {
 	using S = TPShape<D, Q>;
 	constexpr int N = S::N, NF = S::NF, E = S::E;

@@ -1,0 +1,177 @@
+// Block fixed-point contractions: FP64-accurate short dot products on the integer pipe.
+//
+// Why. The FP64 pipe of GB300 retires one warp instruction per scheduler every 64 cycles (measured: DFMA 62, DADD and
+// DMUL 74 cycles at 1.92 GHz, conversions between double and integer or float 62, double to float 29), while a 32 x 32
+// -> 64 bit multiply-add (IMAD.WIDE) takes 2, an integer add 1, a shift or a logic operation 2. An operator entry times
+// a value as three wide multiply-adds is therefore ten times cheaper than one DFMA, as long as the operands' conversion
+// is shared by several products. The contractions of the residual (1D derivative, interpolation, traces, lifting)
+// are such products with constant operators.
+//
+// Representation. The values that enter one sum share a block exponent eb, the largest biased exponent among them
+// (taken over one element and one variable, so that an element's result does not depend on its neighbours in the
+// launch). A value v is held as the integer X = v 2^(1082 - eb), |X| < 2^60, rounded to a multiple of 4 and kept as
+// two limbs: h = X >> 32 (signed) and l = the next 30 bits (0 <= l < 2^30), X = h 2^32 + 4 l. An operator entry w is
+// W = w 2^s = h 2^32 + 4 l with l balanced (|l| <= 2^29). sum X W then needs h h, h l and l h products only:
+//   sum X W / 2^64 = a.h + a.m / 2^30,   a.h = sum hX hW,   a.m = sum (hW lX + lW hX).
+// s is chosen on the host so that sum |W| <= 2^63 over every sum an operator enters (and |W| < 2^62), which bounds
+// a.h by 2^59 and, for at most 32 terms, a.m by 2^62: neither accumulator can overflow.
+//
+// Accuracy. A value is rounded to 2^-59 of its block's largest magnitude, an operator entry to about 2^-60 of its
+// row sum, and the dropped l l products are below 2^-60 of the sum's bound (l of the operator is balanced, so
+// they have no bias): the sum is exact to a few 2^-59 of max |v| sum |w|, where FP64 arithmetic rounds every partial sum
+// to 2^-53. The result is rounded once to FP64, to nearest.
+//
+// States. A density or an energy far below its element's largest one would keep less than FP64's relative precision,
+// which the divisions by the density feel: an element whose densities or energies spread over more than kFixSpread
+// binary orders stays on the FP64 loops as well (fix_spread), so that each is held to 2^-54 relative.
+//
+// Range. Infinities, NaN, magnitudes of 2^824 and above and non-zero blocks below 2^-823 do not enter: fix_in_range
+// tells, and the caller keeps its FP64 loop for such an element, which propagates them as before. (A block of zeros and
+// denormals enters as zeros.)
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace dgpu {
+
+struct FixW {
+	int l, h;
+};
+
+struct FixAcc {
+	long long h, m;
+};
+
+constexpr int kFixMin = 200, kFixMax = 1846;   // biased block exponents that enter
+
+__device__ __forceinline__ int fix_exponent(double x)
+{
+	return (__double2hiint(x) >> 20) & 0x7ff;
+}
+constexpr int kFixSpread = 4;
+
+// Reduced by elem_max beside the exponents: the smallest exponent, as 2047 minus it.
+__device__ __forceinline__ int fix_low(double x) { return 2047 - fix_exponent(x); }
+__device__ __forceinline__ bool fix_spread(int eb, int low) { return eb - (2047 - low) <= kFixSpread; }
+__device__ __forceinline__ bool fix_in_range(int eb)
+{
+	return eb == 0 || (unsigned)(eb - kFixMin) <= (unsigned)(kFixMax - kFixMin);
+}
+__device__ __forceinline__ int fix_block(int eb) { return eb < kFixMin ? kFixMin : eb; }
+
+// x as limbs (.x = l, .y = h) at block exponent eb >= its own exponent.
+__device__ __forceinline__ int2 fix_pack(double x, int eb)
+{
+	const int hi = __double2hiint(x), lo = __double2loint(x);
+	const unsigned mh = (hi & 0x000fffff) | 0x00100000;
+	unsigned long long m = ((unsigned long long)__funnelshift_l(lo, mh, 7) << 32) | ((unsigned)lo << 7);
+	asm("shr.u64 %0, %0, %1;" : "+l"(m) : "r"(eb - ((hi >> 20) & 0x7ff)));   // clamps: 0 beyond 63
+	const long long s = hi >> 31;
+	const long long X = (long long)(m ^ (unsigned long long)s) + (2 - s);    // sign, and half of the last kept unit
+	return make_int2((int)((unsigned)X >> 2), (int)(X >> 32));
+}
+
+__device__ __forceinline__ void fix_mac(FixAcc& a, const FixW w, const int2 x)
+{
+	a.h += (long long)w.h * x.y;
+	a.m += (long long)w.h * x.x;
+	a.m += (long long)w.l * x.y;
+}
+
+// sum X W / 2^61: |result| <= 2^62.
+__device__ __forceinline__ long long fix_sum(const FixAcc& a) { return a.h * 8 + (a.m >> 27); }
+
+// Exponent that makes fix_sum a value: v = fix_sum 2^fix_scale for a block eb and an operator scaled by 2^s.
+__device__ __forceinline__ int fix_scale(int eb, int s) { return 61 - s + eb - 1082; }
+
+// r 2^e rounded to nearest, by integer operations (a conversion on the FP64 pipe costs twice as much); the result must
+// be a normal number, |r| < 2^63.
+__device__ __forceinline__ double fix_to_double(long long r, int e)
+{
+	const int sg = (int)(r >> 63);
+	unsigned long long u = ((unsigned long long)r ^ (long long)sg) - (long long)sg;
+	const int n = __clzll((long long)u);
+	u <<= (n - 1) & 63;                                   // leading bit at 62 (r = 0: u stays 0)
+	const unsigned long long q = (u + 0x200) >> 10;       // 53 bits, or 2^53 after a carry
+	int hi = (int)(q >> 32) + ((1085 - n + e) << 20);     // the leading bit adds one to the exponent field
+	hi = (hi & 0x7fffffff) | (sg & 0x80000000);
+	return u ? __hiloint2double(hi, (int)q) : 0.0;
+}
+
+// Limbs of an integer value |X| < 2^60 (a contraction's result that enters the next one).
+__device__ __forceinline__ int2 fix_limbs(long long X)
+{
+	X += 2;
+	return make_int2((int)((unsigned)X >> 2), (int)(X >> 32));
+}
+
+// Per-element maxima of K non-negative integers over the threads of each element (N consecutive threads per element,
+// e = threadIdx.x / N), into sx[e * stride + k]. sx must be zero before (a barrier in between), and the caller
+// synchronises before reading. All threads of the CTA must call it.
+template <int N, int K>
+__device__ __forceinline__ void elem_max(const int (&x)[K], int e, bool active, int* sx, int stride)
+{
+	const int lane = threadIdx.x & 31;
+	if constexpr (N == 4 || N == 8 || N == 16) {   // elements aligned inside a warp
+#pragma unroll
+		for (int k = 0; k < K; ++k) {
+			int r = x[k];
+#pragma unroll
+			for (int o = N / 2; o > 0; o >>= 1)
+				r = max(r, __shfl_xor_sync(0xffffffffu, r, o));
+			if (active && lane % N == 0)
+				sx[e * stride + k] = r;
+		}
+	} else if constexpr (N < 32) {   // up to five elements in a warp: segmented maxima towards each one's first lane
+		const int node = threadIdx.x - e * N;
+#pragma unroll
+		for (int k = 0; k < K; ++k) {
+			int r = x[k];
+#pragma unroll
+			for (int o = 1; o < N; o *= 2) {
+				const int t = __shfl_down_sync(0xffffffffu, r, o);
+				if (node + o < N && lane + o < 32)
+					r = max(r, t);
+			}
+			if (active && (node == 0 || lane == 0))
+				atomicMax(sx + e * stride + k, r);
+		}
+	} else {
+		const int w0 = (threadIdx.x & ~31);
+		const int e0 = w0 / N, e1 = (N % 32 == 0) ? e0 : (w0 + 31) / N;
+		for (int s = e0; s <= e1; ++s)
+#pragma unroll
+			for (int k = 0; k < K; ++k) {
+				const int r = __reduce_max_sync(0xffffffffu, (active && e == s) ? x[k] : 0);
+				if (lane == 0 && r > 0)
+					atomicMax(sx + s * stride + k, r);
+			}
+	}
+}
+
+// One 1D pass along `dir` of limb blocks: out[var][node] = sum_m M[a(node)][m] in[var][a -> m], rescaled to limbs.
+// sum |W| <= 2^62 for these operators, so |out| < 2^60 at a block exponent raised by 62 - s.
+template <int D, int Q, int NV>
+__device__ __forceinline__ void fix_pass(const int2* __restrict__ in, int2* __restrict__ out, const FixW (*M)[5], int dir,
+                                         int node)
+{
+	constexpr int N = (D == 2 ? Q * Q : Q * Q * Q);
+	const int stride = (dir == 0 ? 1 : (dir == 1 ? Q : Q * Q));
+	const int a = (dir == 0 ? node % Q : (dir == 1 ? (node / Q) % Q : node / (Q * Q)));
+	const int base = node - a * stride;
+	FixW w[Q];
+#pragma unroll
+	for (int m = 0; m < Q; ++m)
+		w[m] = M[a][m];
+#pragma unroll
+	for (int v = 0; v < NV; ++v) {
+		FixAcc s = {0, 0};
+#pragma unroll
+		for (int m = 0; m < Q; ++m)
+			fix_mac(s, w[m], in[v * N + base + m * stride]);
+		out[v * N + node] = fix_limbs(s.h * 4 + (s.m >> 28));
+	}
+}
+
+}  // namespace dgpu

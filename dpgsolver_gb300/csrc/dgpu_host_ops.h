@@ -194,6 +194,72 @@ inline void gauss_lobatto_nodes(int q, double* x)
 		x[q / 2] = 0.0;
 }
 
+// Scale of a fixed-point operator (dgpu_fix.cuh): the largest s with sum 2^s <= 2^bits and max 2^s < 2^62, where sum
+// bounds sum |w| over every sum the operator enters and max its entries.
+inline int fix_shift(double sum, double mx, int bits)
+{
+	if (!(sum > 0.0) || !(sum < 1e30))
+		return 0;
+	int a, b;
+	frexp(sum * (1.0 + 1e-9), &a);   // sum < 2^a
+	frexp(mx, &b);
+	return a - bits > b - 61 ? bits - a : 61 - b;
+}
+
+inline FixW fix_entry(double w, int s)
+{
+	const long long W = 4 * llrint(ldexp(w, s - 2));
+	FixW f;
+	f.h = (int)((W + (1ll << 31)) >> 32);
+	f.l = (int)((W - f.h * (1ll << 32)) / 4);
+	return f;
+}
+
+// The fixed-point operators of TPOps from its FP64 ones.
+inline void derive_fix_ops(int q, int d, TPOps* o)
+{
+	double sD = 0.0, mD = 0.0, sT = 0.0, sU = 0.0, mL = 0.0, sB = 0.0, mB = 0.0, sI = 0.0, mI = 0.0;
+	for (int a = 0; a < q; ++a) {
+		double rD = 0.0, rB = 0.0, rI = 0.0;
+		for (int m = 0; m < q; ++m) {
+			rD += fabs(o->Dgl[m][a]);
+			rB += fabs(o->B[a][m]);
+			rI += fabs(o->Binv[a][m]);
+			mD = fmax(mD, fabs(o->Dgl[m][a]));
+			mB = fmax(mB, fabs(o->B[a][m]));
+			mI = fmax(mI, fabs(o->Binv[a][m]));
+		}
+		sD = fmax(sD, d * rD);
+		sB = fmax(sB, rB);
+		sI = fmax(sI, rI);
+		sU = fmax(sU, 1.0 + d * (fabs(o->lb[0][a]) + fabs(o->lb[1][a])));
+		mL = fmax(mL, fmax(fabs(o->lb[0][a]), fabs(o->lb[1][a])));
+	}
+	for (int s = 0; s < 2; ++s) {
+		double r = 0.0;
+		for (int m = 0; m < q; ++m)
+			r += fabs(o->lb[s][m]);
+		sT = fmax(sT, r);
+	}
+	o->sD = fix_shift(sD, mD, 63);
+	o->sT = fix_shift(sT, mL, 63);
+	o->sU = fix_shift(sU, fmax(mL, 1.0), 63);
+	o->sB = fix_shift(sB, mB, 62);
+	o->sBinv = fix_shift(sI, mI, 62);
+	for (int a = 0; a < q; ++a)
+		for (int m = 0; m < q; ++m) {
+			o->fD[a][m] = fix_entry(o->Dgl[m][a], o->sD);
+			o->fB[a][m] = fix_entry(o->B[a][m], o->sB);
+			o->fBinv[a][m] = fix_entry(o->Binv[a][m], o->sBinv);
+		}
+	for (int s = 0; s < 2; ++s)
+		for (int m = 0; m < q; ++m) {
+			o->fT[s][m] = fix_entry(o->lb[s][m], o->sT);
+			o->fU[s][m] = fix_entry(o->lb[s][m], o->sU);
+		}
+	o->fOne = fix_entry(1.0, o->sU);
+}
+
 // B, B^-1, Dgl, l_gl(+-1), Bezier maps, positivity constants, transposes: see TPOps.
 inline bool derive_tp_ops(const dgpu_tp_operators* ops, int d, TPOps* out)
 {
@@ -244,6 +310,7 @@ inline bool derive_tp_ops(const dgpu_tp_operators* ops, int d, TPOps* out)
 			out->BT[a][m] = out->B[m][a];
 			out->BinvT[a][m] = out->Binv[m][a];
 		}
+	derive_fix_ops(q, d, out);
 	return true;
 }
 

@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(256) jac_scatter_kernel(const double* __restri
 // scale_rhs_by_m_inv_std, solve_dg.c:265-272, is M times the explicit right-hand side).
 template <int D, int Q, int NV>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS)
-tp_mass_kernel(const TPOps ops, const TPParams P, const double* __restrict__ in, double* __restrict__ out)
+tp_mass_kernel(const __grid_constant__ TPOps ops, const TPParams P, const double* __restrict__ in, double* __restrict__ out)
 {
 	using S = TPShape<D, Q>;
 	constexpr int N = S::N, E = S::E;

@@ -18,7 +18,7 @@ namespace dgpu {
 // contraction and the traces of each. Per element: 2 x (su, st, sf) in shared memory.
 template <int D, int Q, int NV, int PDE>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS)
-tp_jvp_volume_kernel(const TPOps ops, const TPParams P, const TPParams Pd, const double* __restrict__ u,
+tp_jvp_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const TPParams Pd, const double* __restrict__ u,
                      const double* __restrict__ du)
 {
 	using S = TPShape<D, Q>;

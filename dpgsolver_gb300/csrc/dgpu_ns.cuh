@@ -49,7 +49,7 @@ __device__ __forceinline__ int face_node_of(int node, int nd)
 
 // lambda(t) of every face side at its own nodes (setup).
 template <int D, int Q>
-__global__ void __launch_bounds__(256) tp_ns_lambda_kernel(const TPOps ops, const TPParams P, double* lam)
+__global__ void __launch_bounds__(256) tp_ns_lambda_kernel(const __grid_constant__ TPOps ops, const TPParams P, double* lam)
 {
 	using S = TPShape<D, Q>;
 	constexpr int NF = S::NF, N = S::N;
@@ -116,7 +116,7 @@ __device__ __forceinline__ void ns_element_gradient(const TPOps* sops, const TPP
 
 template <int D, int Q, int NV, bool GLL_IN>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS)
-tp_ns_grad_kernel(const TPOps ops, const TPParams P, const double* __restrict__ u)
+tp_ns_grad_kernel(const __grid_constant__ TPOps ops, const TPParams P, const double* __restrict__ u)
 {
 	using S = TPShape<D, Q>;
 	constexpr int N = S::N, NF = S::NF, E = S::E, PER_E = NsSmem<D, Q, NV>::PER_E;
@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(128) tp_ns_jvp_face_kernel(const TPParams P, c
 
 template <int D, int Q, int NV, bool GLL_IN>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS)
-tp_ns_volume_kernel(const TPOps ops, const TPParams P, const double* __restrict__ u)
+tp_ns_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const double* __restrict__ u)
 {
 	using S = TPShape<D, Q>;
 	constexpr int N = S::N, NF = S::NF, E = S::E, PER_E = NsSmem<D, Q, NV>::PER_E;
@@ -485,7 +485,7 @@ struct NsJvpSmem {
 
 template <int D, int Q, int NV>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS)
-tp_ns_jvp_volume_kernel(const TPOps ops, const TPParams P, const TPParams Pd, const double* __restrict__ u,
+tp_ns_jvp_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const TPParams Pd, const double* __restrict__ u,
                         const double* __restrict__ du)
 {
 	using S = TPShape<D, Q>;

@@ -82,7 +82,7 @@ struct NsAdjSmem {
 
 template <int D, int Q, int NV>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS)
-tp_ns_adj_volume_kernel(const TPOps ops, const TPParams P, const AdjArgs A, const NsAdjArgs B)
+tp_ns_adj_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const AdjArgs A, const NsAdjArgs B)
 {
 	using S = TPShape<D, Q>;
 	constexpr int N = S::N, NF = S::NF, E = S::E, PER_E = NsAdjSmem<D, Q, NV>::PER_E;
@@ -312,7 +312,7 @@ tp_ns_adj_face_kernel(const TPParams P, const AdjArgs A, const NsAdjArgs B)
 // ubar = V^T ugbar. Per element (doubles): h (D blocks), sa, sb, sc.
 template <int D, int Q, int NV>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS)
-tp_ns_adj_lift_kernel(const TPOps ops, const TPParams P, const AdjArgs A, const NsAdjArgs B)
+tp_ns_adj_lift_kernel(const __grid_constant__ TPOps ops, const TPParams P, const AdjArgs A, const NsAdjArgs B)
 {
 	using S = TPShape<D, Q>;
 	constexpr int N = S::N, NF = S::NF, E = S::E, PER_E = NsAdjSmem<D, Q, NV>::PER_E;

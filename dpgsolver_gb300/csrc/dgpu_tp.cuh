@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "dgpu_fix.cuh"
 #include "dgpu_physics.cuh"
 
 namespace dgpu {
@@ -42,6 +43,14 @@ struct TPOps {
 	double BSg[kQMax][kQMax];   // B ccBS0:   Bezier coefficients -> GL nodal values
 	double BT[kQMax][kQMax];    // B^T    (adjoint: V^T)
 	double BinvT[kQMax][kQMax]; // Binv^T (adjoint: V^-T)
+	// Fixed-point forms (dgpu_fix.cuh) and their scales: W = w 2^s
+	FixW fD[kQMax][kQMax];      // Dgl^T: fD[a][m] = Dgl[m][a], summed over the D directions
+	FixW fT[2][kQMax];          // lb as the trace operator
+	FixW fU[2][kQMax];          // lb as the lifting operator, summed over the 2D faces and fOne
+	FixW fOne;                  // the volume term's weight 1 in that sum
+	FixW fB[kQMax][kQMax];      // B and B^-1 as 1D passes (sum |W| <= 2^62)
+	FixW fBinv[kQMax][kQMax];
+	int sD, sT, sU, sB, sBinv, pad_;
 	float SBf[kQMax][kQMax];    // SBg rounded to FP32 (positivity pre-filter)
 	float pos_err;              // |FP32 Bezier coefficient - exact| <= pos_err * max_i |x_i| (per variable)
 };
@@ -164,11 +173,17 @@ __device__ __forceinline__ unsigned long long abs_bits(double x)
 	return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
 }
 
-// Copies the operator set into shared memory; the caller synchronises before use.
+// Copies the operator set (a __grid_constant__ kernel parameter) into shared memory; the caller synchronises before use.
+// The loads go through the parameter's generic address: indexed by thread, the constant port would serve the 32 addresses
+// of a warp one after the other.
 __device__ __forceinline__ void load_ops(TPOps* sops, const TPOps& ops)
 {
-	for (int i = threadIdx.x; i < (int)(sizeof(TPOps) / 8); i += blockDim.x)
-		reinterpret_cast<double*>(sops)[i] = reinterpret_cast<const double*>(&ops)[i];
+	const double* src = reinterpret_cast<const double*>(&ops);
+	for (int i = threadIdx.x; i < (int)(sizeof(TPOps) / 8); i += blockDim.x) {
+		double x;
+		asm volatile("ld.f64 %0, [%1];" : "=d"(x) : "l"(src + i));
+		reinterpret_cast<double*>(sops)[i] = x;
+	}
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -179,129 +194,313 @@ template <int D, int Q, int NV>
 struct TPSmem {
 	static constexpr int N = TPShape<D, Q>::N;
 	static constexpr int VOL = NV * N * 2 + D * NV * N;   // su, st, sf
-	static constexpr int LIFT = 3 * NV * N + 8;           // sa, sb, sc, per-element scalars
+	static constexpr int NFT = 2 * D * TPShape<D, Q>::NF;  // face nodes of the element
+	static constexpr int LIFT = 3 * NV * N;               // sa, sb, sc (at first the face terms: NV NFT <= 3 NV N)
+	// block exponents (ints) per element, kept apart:
+	static constexpr int AEXP = NV + (NV > 1 ? 2 : 0);    // of a change of basis: one per variable, spreads of rho and E
+	static constexpr int EXP = AEXP + NV;                 // of the volume term: state, spreads, fluxes
+	static constexpr int LEXP = 2 * AEXP + 2 * NV;        // of the lift: faces, FP32 scales, two changes of basis
 };
 
-// Volume term of the CTA's E elements; per element PER_E doubles at base (su, st, sf at the start).
-template <int D, int Q, int NV, int PDE, bool GLL_IN, int PER_E>
-__device__ __forceinline__ void tp_volume_body(const TPOps* sops, const TPParams& P, const double* __restrict__ u,
-                                               int v0, int n_here, double* base)
+// Node index of face node t of local face lf with coordinate 0 along the face's normal direction, and the stride
+// along it (tangential coordinates in ascending direction order).
+template <int D, int Q>
+__device__ __forceinline__ void tp_face_line(int lf, int t, int& base, int& stride)
 {
-	using S = TPShape<D, Q>;
-	constexpr int N = S::N, NF = S::NF;
-	const int tid = threadIdx.x;
-	for (int i = tid; i < n_here * NV * N; i += blockDim.x) {   // coalesced: contiguous element blocks
-		const int e = i / (NV * N), r = i % (NV * N);
-		const double x = u[(size_t)v0 * NV * N + i];
-		base[e * PER_E + r] = x;
-		if (GLL_IN && P.keep_coef)
-			P.keep_coef[(size_t)v0 * NV * N + i] = x;
+	const int nd = lf >> 1;
+	if (D == 2) {
+		stride = (nd == 0 ? 1 : Q);
+		base = (nd == 0 ? t * Q : t);
+	} else {
+		const int t0 = t % Q, t1 = t / Q;
+		stride = (nd == 0 ? 1 : (nd == 1 ? Q : Q * Q));
+		base = (nd == 0 ? t0 * Q + t1 * Q * Q : (nd == 1 ? t0 + t1 * Q * Q : t0 + t1 * Q));
+	}
+}
+
+// Face node index on local face lf of the line through node.
+template <int D, int Q>
+__device__ __forceinline__ int tp_face_node(int lf, int node)
+{
+	const int nd = lf >> 1;
+	if (D == 2)
+		return nd == 0 ? node_coord<Q>(node, 1) : node_coord<Q>(node, 0);
+	const int c0 = node_coord<Q>(node, 0), c1 = node_coord<Q>(node, 1), c2 = node_coord<Q>(node, 2);
+	return nd == 0 ? c1 + Q * c2 : (nd == 1 ? c0 + Q * c2 : c0 + Q * c1);
+}
+
+// Contravariant flux of W at a node with the w-weighted metric terms g.
+template <int D, int NV, int PDE>
+__device__ __forceinline__ void tp_flux(const TPParams& P, const double* W, const double* g, double (*fr)[NV])
+{
+	if constexpr (PDE == kEuler) {
+		euler_flux_ref<D>(W, g, fr);
+	} else {
+		// advection: f_i = b_i u ; fr_j = sum_i g[j][i] b_i u
+#pragma unroll
+		for (int j = 0; j < D; ++j) {
+			double gb = 0.0;
+#pragma unroll
+			for (int i = 0; i < D; ++i)
+				gb += g[j * D + i] * P.b_adv[i];
+			fr[j][0] = gb * W[0];
+		}
+	}
+}
+
+// tp_pass along the direction of the given stride, not unrolled (the rare FP64 path beside the fixed-point one).
+template <int Q, int NV>
+__device__ __noinline__ void tp_pass_rolled(const double* in, double* out, const double (*M)[kQMax], int node,
+                                            int stride, int N)
+{
+	const int a = (node / stride) % Q;
+#pragma unroll 1
+	for (int k = 0; k < NV; ++k) {
+		const double* x = in + k * N + node - a * stride;
+		double s = 0.0;
+#pragma unroll 1
+		for (int m = 0; m < Q; ++m)
+			s += M[a][m] * x[m * stride];
+		out[k * N + node] = s;
+	}
+}
+
+// M (x) .. (x) M applied to the CTA's elements in block fixed point (FP64 passes for an element out of range): x holds
+// the node's values on entry and exit; buf and tmp NV N words per element, sx AEXP zeroed ints per element. STATE: x is
+// a conserved state (fix_spread). All threads of the CTA must call it; buf is free again after the next barrier.
+template <int D, int Q, int NV, bool STATE>
+__device__ __forceinline__ void tp_apply_fix(double* x, double* buf, double* tmp, const FixW (*F)[kQMax], int sF,
+                                             const double (*M)[kQMax], int e, int node, bool active, int* sx)
+{
+	constexpr int N = TPShape<D, Q>::N, XE = TPSmem<D, Q, NV>::AEXP, K = STATE ? XE : NV;
+	int eb[K];
+#pragma unroll
+	for (int k = 0; k < NV; ++k)
+		eb[k] = active ? fix_exponent(x[k]) : 0;
+	if constexpr (K > NV) {
+		eb[NV] = active ? fix_low(x[0]) : 0;
+		eb[NV + 1] = active ? fix_low(x[NV - 1]) : 0;
+	}
+	elem_max<N, K>(eb, e, active, sx, XE);
+	__syncthreads();
+	bool ok = true;
+	if (active) {
+		if constexpr (K > NV)
+			ok = fix_spread(sx[e * XE], sx[e * XE + NV]) && fix_spread(sx[e * XE + NV - 1], sx[e * XE + NV + 1]);
+#pragma unroll
+		for (int k = 0; k < NV; ++k) {
+			ok = ok && fix_in_range(sx[e * XE + k]);
+			eb[k] = fix_block(sx[e * XE + k]);
+		}
+#pragma unroll
+		for (int k = 0; k < NV; ++k) {
+			if (ok)
+				reinterpret_cast<int2*>(buf)[k * N + node] = fix_pack(x[k], eb[k]);
+			else
+				buf[k * N + node] = x[k];
+		}
 	}
 	__syncthreads();
+	double *src = buf, *dst = tmp;
+#pragma unroll
+	for (int dir = 0; dir < D - 1; ++dir) {
+		if (active) {
+			if (ok)
+				fix_pass<D, Q, NV>(reinterpret_cast<int2*>(src), reinterpret_cast<int2*>(dst), F, dir, node);
+			else   // Inf, NaN, huge values or a spread state: FP64 for this element
+				tp_pass_rolled<Q, NV>(src, dst, M, node, dir == 0 ? 1 : Q, N);
+		}
+		__syncthreads();
+		double* t = src;
+		src = dst;
+		dst = t;
+	}
+	constexpr int stride = (D == 2 ? Q : Q * Q);
+	if (active) {
+		if (ok) {
+			const int a = node / stride, base = node % stride;
+			FixW w[Q];
+#pragma unroll
+			for (int m = 0; m < Q; ++m)
+				w[m] = F[a][m];
+#pragma unroll
+			for (int k = 0; k < NV; ++k) {
+				FixAcc s = {0, 0};
+#pragma unroll
+				for (int m = 0; m < Q; ++m)
+					fix_mac(s, w[m], reinterpret_cast<const int2*>(src)[k * N + base + m * stride]);
+				x[k] = fix_to_double(fix_sum(s), fix_scale(eb[k] + (D - 1) * (62 - sF), sF));
+			}
+		} else {
+			tp_pass_rolled<Q, NV>(src, dst, M, node, stride, N);
+#pragma unroll
+			for (int k = 0; k < NV; ++k)
+				x[k] = dst[k * N + node];
+		}
+	}
+}
 
+// Volume term of the CTA's E elements; per element PER_E doubles at base (su, st, sf at the start), sx the block
+// exponents. The flux is FP64; the derivative and the traces contract in block fixed point (dgpu_fix.cuh): 90 of the
+// 138 FP64 operations per node at q = 4 leave the FP64 pipe, which bounds the kernel.
+template <int D, int Q, int NV, int PDE, bool GLL_IN, int PER_E>
+__device__ __forceinline__ void tp_volume_body(const TPOps* sops, const TPParams& P, const double* __restrict__ u,
+                                               int v0, int n_here, double* base, int* sx)
+{
+	using S = TPShape<D, Q>;
+	constexpr int N = S::N, NF = S::NF, XE = TPSmem<D, Q, NV>::EXP, AE = TPSmem<D, Q, NV>::AEXP;
+	const int tid = threadIdx.x;
 	const int e = tid / N, node = tid % N;
 	const bool active = e < n_here;
+	const int v = v0 + e;
 	double* su = base + e * PER_E;
 	double* st = su + NV * N;
 	double* sf = st + NV * N;
-
-	if (GLL_IN) {
-		// ug = V u: passes su -> st (-> sf) -> ... ; copy into su so the traces and flux read one buffer
-		tp_apply<D, Q, NV>(su, st, sf, sops->B, node, active);
-		if (active)
-#pragma unroll
-			for (int k = 0; k < NV; ++k) {
-				su[k * N + node] = st[k * N + node];
-				if (P.keep_gl)
-					P.keep_gl[((size_t)(v0 + e) * NV + k) * N + node] = st[k * N + node];
-			}
-		__syncthreads();
-	}
-
-	const int v = v0 + e;
-	if (active) {
-		double W[NV];
+	double W[NV];
+	if (active)
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
-			W[k] = su[k * N + node];
+			W[k] = u[((size_t)v * NV + k) * N + node];
+	for (int i = tid; i < S::E * XE + (GLL_IN ? S::E * AE : 0); i += blockDim.x)
+		sx[i] = 0;
+	__syncthreads();
+	if (GLL_IN) {
+		if (active && P.keep_coef)
+#pragma unroll
+			for (int k = 0; k < NV; ++k)
+				P.keep_coef[((size_t)v * NV + k) * N + node] = W[k];
+		tp_apply_fix<D, Q, NV, true>(W, su, st, sops->fB, sops->sB, sops->B, e, node, active, sx + S::E * XE);   // V u
+		if (active && P.keep_gl)
+#pragma unroll
+			for (int k = 0; k < NV; ++k)
+				P.keep_gl[((size_t)v * NV + k) * N + node] = W[k];
+	}
+
+	double fr[D][NV];
+	int eb[XE];
+#pragma unroll
+	for (int k = 0; k < XE; ++k)
+		eb[k] = 0;
+	if (active) {
 		double g[D * D];
 #pragma unroll
 		for (int c = 0; c < D * D; ++c)
 			g[c] = P.gmet[((size_t)v * D * D + c) * N + node];
-		if constexpr (PDE == kEuler) {
-			double fr[D][D + 2];
-			euler_flux_ref<D>(W, g, fr);
+		tp_flux<D, NV, PDE>(P, W, g, fr);
+#pragma unroll
+		for (int k = 0; k < NV; ++k) {
+			eb[k] = fix_exponent(W[k]);
+			int m = 0;
 #pragma unroll
 			for (int j = 0; j < D; ++j)
+				m = max(m, fix_exponent(fr[j][k]));
+			eb[AE + k] = m;
+		}
+		if constexpr (AE > NV) {
+			eb[NV] = fix_low(W[0]);
+			eb[NV + 1] = fix_low(W[NV - 1]);
+		}
+	}
+	elem_max<N, XE>(eb, e, active, sx, XE);
+	__syncthreads();
+	bool ok = true;
+	if (active) {
+		if constexpr (AE > NV)
+			ok = fix_spread(sx[e * XE], sx[e * XE + NV]) && fix_spread(sx[e * XE + NV - 1], sx[e * XE + NV + 1]);
 #pragma unroll
-				for (int k = 0; k < NV; ++k)
-					sf[(j * NV + k) * N + node] = fr[j][k];
+		for (int k = 0; k < NV; ++k) {
+			ok = ok && fix_in_range(sx[e * XE + k]) && fix_in_range(sx[e * XE + AE + k]);
+			eb[k] = fix_block(sx[e * XE + k]);
+			eb[AE + k] = fix_block(sx[e * XE + AE + k]);
+		}
+		if (ok) {
+			int2* xu = reinterpret_cast<int2*>(su);
+			int2* xf = reinterpret_cast<int2*>(sf);
+#pragma unroll
+			for (int k = 0; k < NV; ++k) {
+				xu[k * N + node] = fix_pack(W[k], eb[k]);
+#pragma unroll
+				for (int j = 0; j < D; ++j)
+					xf[(j * NV + k) * N + node] = fix_pack(fr[j][k], eb[AE + k]);
+			}
 		} else {
-			// advection: f_i = b_i u ; fr_j = sum_i g[j][i] b_i u
 #pragma unroll
-			for (int j = 0; j < D; ++j) {
-				double gb = 0.0;
+			for (int k = 0; k < NV; ++k) {
+				su[k * N + node] = W[k];
 #pragma unroll
-				for (int i = 0; i < D; ++i)
-					gb += g[j * D + i] * P.b_adv[i];
-				sf[j * N + node] = gb * W[0];
+				for (int j = 0; j < D; ++j)
+					sf[(j * NV + k) * N + node] = fr[j][k];
 			}
 		}
 	}
 	__syncthreads();
+	if (!active)
+		return;
 
-	if (active) {
-		// volume term in GL space: sum_j Dgl_j^T (w fr_j)
-		double acc[NV];
+	// volume term in GL space: sum_j Dgl_j^T (w fr_j)
+	if (ok) {
+		const int2* xf = reinterpret_cast<const int2*>(sf);
+		FixAcc acc[NV];
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
-			acc[k] = 0.0;
+			acc[k] = {0, 0};
 #pragma unroll
 		for (int j = 0; j < D; ++j) {
 			const int stride = (j == 0 ? 1 : (j == 1 ? Q : Q * Q));
 			const int a = node_coord<Q>(node, j);
 			const int b0 = node - a * stride;
-			double w[Q];
 #pragma unroll
-			for (int m = 0; m < Q; ++m)
-				w[m] = sops->Dgl[m][a];
+			for (int m = 0; m < Q; ++m) {
+				const FixW w = sops->fD[a][m];
 #pragma unroll
-			for (int k = 0; k < NV; ++k) {
-				const double* f = sf + (j * NV + k) * N + b0;
-#pragma unroll
-				for (int m = 0; m < Q; ++m)
-					acc[k] += w[m] * f[m * stride];
+				for (int k = 0; k < NV; ++k)
+					fix_mac(acc[k], w, xf[(j * NV + k) * N + b0 + m * stride]);
 			}
 		}
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
-			P.vol_gl[((size_t)v * NV + k) * N + node] = acc[k];
+			P.vol_gl[((size_t)v * NV + k) * N + node] = fix_to_double(fix_sum(acc[k]), fix_scale(eb[AE + k], sops->sD));
+	} else {
+#pragma unroll 1
+		for (int k = 0; k < NV; ++k) {
+			double acc = 0.0;
+#pragma unroll 1
+			for (int j = 0; j < D; ++j) {
+				const int stride = (j == 0 ? 1 : (j == 1 ? Q : Q * Q));
+				const int a = (node / stride) % Q;
+				const double* f = sf + (j * NV + k) * N + node - a * stride;
+				for (int m = 0; m < Q; ++m)
+					acc += sops->Dgl[m][a] * f[m * stride];
+			}
+			P.vol_gl[((size_t)v * NV + k) * N + node] = acc;
+		}
+	}
 
-		// traces of ug on the 2D local faces
-		for (int it = node; it < 2 * D * NF; it += N) {
-			const int lf = it / NF, t = it % NF;
-			const int nd = lf >> 1, side = lf & 1;
-			int t0, t1;
-			if (D == 2) {
-				t0 = t; t1 = 0;
-			} else {
-				t0 = t % Q; t1 = t / Q;
-			}
-			// node index with coordinate m along nd and tangential (t0, t1) in ascending direction order
-			int stride_n, base_n;
-			if (D == 2) {
-				stride_n = (nd == 0 ? 1 : Q);
-				base_n = (nd == 0 ? t0 * Q : t0);
-			} else {
-				stride_n = (nd == 0 ? 1 : (nd == 1 ? Q : Q * Q));
-				base_n = (nd == 0 ? t0 * Q + t1 * Q * Q : (nd == 1 ? t0 + t1 * Q * Q : t0 + t1 * Q));
-			}
-			const int fs = P.vol_face[(size_t)v * 2 * D + lf];
-			double* dst = P.traces + (size_t)fs * NV * NF;
+	// traces of ug on the 2D local faces
+	for (int it = node; it < 2 * D * NF; it += N) {
+		const int lf = it / NF, t = it % NF, side = lf & 1;
+		int stride_n, base_n;
+		tp_face_line<D, Q>(lf, t, base_n, stride_n);
+		const int fs = P.vol_face[(size_t)v * 2 * D + lf];
+		double* dst = P.traces + (size_t)fs * NV * NF;
+		if (ok) {
+			const int2* xu = reinterpret_cast<const int2*>(su) + base_n;
+			FixW w[Q];
+#pragma unroll
+			for (int m = 0; m < Q; ++m)
+				w[m] = sops->fT[side][m];
 #pragma unroll
 			for (int k = 0; k < NV; ++k) {
-				double s = 0.0;
+				FixAcc s = {0, 0};
 #pragma unroll
+				for (int m = 0; m < Q; ++m)
+					fix_mac(s, w[m], xu[k * N + m * stride_n]);
+				dst[k * NF + t] = fix_to_double(fix_sum(s), fix_scale(eb[k], sops->sT));
+			}
+		} else {
+#pragma unroll 1
+			for (int k = 0; k < NV; ++k) {
+				double s = 0.0;
 				for (int m = 0; m < Q; ++m)
 					s += sops->lb[side][m] * su[k * N + base_n + m * stride_n];
 				dst[k * NF + t] = s;
@@ -312,7 +511,7 @@ __device__ __forceinline__ void tp_volume_body(const TPOps* sops, const TPParams
 
 template <int D, int Q, int NV, int PDE, bool GLL_IN>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS)
-tp_volume_kernel(const TPOps ops, const TPParams P, const double* __restrict__ u)
+tp_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const double* __restrict__ u)
 {
 	using S = TPShape<D, Q>;
 	extern __shared__ double smem[];
@@ -321,8 +520,10 @@ tp_volume_kernel(const TPOps ops, const TPParams P, const double* __restrict__ u
 	const int v0 = blockIdx.x * S::E;
 	if (blockIdx.x == 0 && threadIdx.x == 0 && P.max_bits)
 		*P.max_bits = 0ull;
-	tp_volume_body<D, Q, NV, PDE, GLL_IN, TPSmem<D, Q, NV>::VOL>(sops, P, u, v0, min(S::E, P.n_vol - v0),
-	                                                                   smem + sizeof(TPOps) / 8);
+	double* base = smem + sizeof(TPOps) / 8;
+	constexpr int VOL = TPSmem<D, Q, NV>::VOL;
+	tp_volume_body<D, Q, NV, PDE, GLL_IN, VOL>(sops, P, u, v0, min(S::E, P.n_vol - v0), base,
+	                                           reinterpret_cast<int*>(base + S::E * VOL));
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -493,7 +694,7 @@ __device__ __noinline__ bool tp_positivity_exact(const double (*toB)[kQMax], con
 // element PER_E doubles at base.
 template <int D, int Q, int NV, int MODE, int PER_E>
 __device__ __forceinline__ void tp_lift_body(const TPOps* sops, const TPParams& P, const RkArgs& rk, int v0,
-                                             int n_here, double* base)
+                                             int n_here, double* base, int* sx)
 {
 	using S = TPShape<D, Q>;
 	constexpr int N = S::N, NF = S::NF;
@@ -504,36 +705,95 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, const TPParams& 
 	double* sa = base + e * PER_E;
 	double* sb = sa + NV * N;
 	double* sc = sb + NV * N;
-	int* sscale = reinterpret_cast<int*>(sc + NV * N);   // NV ints (FP32 scales) + spare
-	if (active && node < 8)
-		reinterpret_cast<double*>(sscale)[node] = 0.0;
-	__syncthreads();  // the lift below reads sops->lb written by other warps
-
-	double Rg[NV];  // GL-space residual R_gl of this node
+	constexpr int NFT = TPSmem<D, Q, NV>::NFT, NR = (NFT + N - 1) / N;
+	constexpr int AE = TPSmem<D, Q, NV>::AEXP;
+	const int* sscale = sx + S::E * NV + e * NV;   // FP32 scales of the positivity pre-filter
+	for (int i = tid; i < S::E * TPSmem<D, Q, NV>::LEXP; i += blockDim.x)
+		sx[i] = 0;
+	double fv[NR][NV], Rg[NV];   // the face terms this thread stages; GL-space residual R_gl of this node
+	int eb[NV];
+#pragma unroll
+	for (int k = 0; k < NV; ++k)
+		eb[k] = 0;
 	if (active) {
 #pragma unroll
-		for (int k = 0; k < NV; ++k)
+		for (int k = 0; k < NV; ++k) {
 			Rg[k] = P.vol_gl[((size_t)v * NV + k) * N + node];
+			eb[k] = fix_exponent(Rg[k]);
+		}
 #pragma unroll
-		for (int lf = 0; lf < 2 * D; ++lf) {
+		for (int r = 0; r < NR; ++r) {
+			const int it = node + r * N;
+			if (it >= NFT)
+				break;
+			const int lf = it / NF, t = it % NF;
 			const int fs = P.vol_face[(size_t)v * 2 * D + lf];
 			const int f = fs >> 1, s = fs & 1;
-			const int nd = lf >> 1;
-			const int a = node_coord<Q>(node, nd);
-			int t;
-			if (D == 2) {
-				t = (nd == 0 ? node_coord<Q>(node, 1) : node_coord<Q>(node, 0));
-			} else {
-				const int c0 = node_coord<Q>(node, 0), c1 = node_coord<Q>(node, 1), c2 = node_coord<Q>(node, 2);
-				t = (nd == 0 ? c1 + Q * c2 : (nd == 1 ? c0 + Q * c2 : c0 + Q * c1));
-			}
 			const int idx = (s == 1 && P.nc_inv) ? P.nc_inv[(size_t)f * NF + t] : t;
-			// side 0: rhs -= E^T nnf ; side 1: rhs -= E^T (-nnf)   (compute_face_rlhs_T.c:297-310)
-			const double l = (s == 0 ? -1.0 : 1.0) * sops->lb[lf & 1][a];
 			const double* src = P.nnf + (size_t)f * NV * NF;
 #pragma unroll
+			for (int k = 0; k < NV; ++k) {
+				// side 0: rhs -= E^T nnf ; side 1: rhs -= E^T (-nnf)   (compute_face_rlhs_T.c:297-310)
+				const double x = src[k * NF + idx];
+				fv[r][k] = s == 0 ? -x : x;
+				eb[k] = max(eb[k], fix_exponent(x));
+			}
+		}
+	}
+	__syncthreads();   // sx is zero; the lift below reads sops written by other warps
+	elem_max<N, NV>(eb, e, active, sx, NV);
+	__syncthreads();
+	bool ok = true;
+	if (active) {
+#pragma unroll
+		for (int k = 0; k < NV; ++k) {
+			ok = ok && fix_in_range(sx[e * NV + k]);
+			eb[k] = fix_block(sx[e * NV + k]);
+		}
+#pragma unroll
+		for (int r = 0; r < NR; ++r) {
+			const int it = node + r * N;
+			if (it >= NFT)
+				break;
+#pragma unroll
 			for (int k = 0; k < NV; ++k)
-				Rg[k] += l * src[k * NF + idx];
+				if (ok)
+					reinterpret_cast<int2*>(sa)[k * NFT + it] = fix_pack(fv[r][k], eb[k]);
+				else
+					sa[k * NFT + it] = fv[r][k];
+		}
+	}
+	__syncthreads();
+
+	if (active) {
+		if (ok) {
+			FixAcc acc[NV];
+			const FixW one = sops->fOne;
+#pragma unroll
+			for (int k = 0; k < NV; ++k) {
+				const int2 x = fix_pack(Rg[k], eb[k]);
+				acc[k] = {(long long)one.h * x.y, (long long)one.h * x.x};   // the weight 1 has no low limb
+			}
+#pragma unroll
+			for (int lf = 0; lf < 2 * D; ++lf) {
+				const FixW w = sops->fU[lf & 1][node_coord<Q>(node, lf >> 1)];
+				const int2* x = reinterpret_cast<const int2*>(sa) + lf * NF + tp_face_node<D, Q>(lf, node);
+#pragma unroll
+				for (int k = 0; k < NV; ++k)
+					fix_mac(acc[k], w, x[k * NFT]);
+			}
+#pragma unroll
+			for (int k = 0; k < NV; ++k)
+				Rg[k] = fix_to_double(fix_sum(acc[k]), fix_scale(eb[k], sops->sU));
+		} else {
+#pragma unroll 1
+			for (int lf = 0; lf < 2 * D; ++lf) {
+				const double l = sops->lb[lf & 1][node_coord<Q>(node, lf >> 1)];
+				const double* x = sa + lf * NF + tp_face_node<D, Q>(lf, node);
+#pragma unroll
+				for (int k = 0; k < NV; ++k)
+					Rg[k] += l * x[k * NFT];
+			}
 		}
 		const double iw = P.inv_wJ[(size_t)v * N + node];
 #pragma unroll
@@ -544,22 +804,21 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, const TPParams& 
 			for (int k = 0; k < NV; ++k)
 				Rg[k] += P.source[((size_t)v * NV + k) * N + node];
 	}
+	__syncthreads();   // the face terms are read; sa, sb, sc are reused
 
 	const bool need_coef = (MODE == kModeRhs) || ((MODE == kModeRkGl || MODE == kModeRkGlOut) && rk.want_max);
 	unsigned long long mx = 0ull;
 	double R[NV];
 	if (MODE != kModeRkGlNoMax && need_coef) {
 		// R = V^-1 R_gl (GLL coefficients): D passes of Binv
-		if (active)
 #pragma unroll
-			for (int k = 0; k < NV; ++k)
-				sa[k * N + node] = Rg[k];
-		__syncthreads();
-		tp_apply<D, Q, NV>(sa, sb, sc, sops->Binv, node, active);
+		for (int k = 0; k < NV; ++k)
+			R[k] = Rg[k];
+		tp_apply_fix<D, Q, NV, false>(R, sa, sb, sops->fBinv, sops->sBinv, sops->Binv, e, node, active,
+		                              sx + 2 * S::E * NV);
 		if (active) {
 #pragma unroll
 			for (int k = 0; k < NV; ++k) {
-				R[k] = sb[k * N + node];
 				const unsigned long long bits = abs_bits(R[k]);
 				mx = bits > mx ? bits : mx;
 			}
@@ -612,14 +871,15 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, const TPParams& 
 			float* xf = reinterpret_cast<float*>(sa);
 			float* tf = xf + NV * N;
 			float* tmpf = reinterpret_cast<float*>(sc);
-			if (active) {
+			int sb32[NV];
 #pragma unroll
-				for (int k = 0; k < NV; ++k) {
-					const float x = (float)snew[k];
+			for (int k = 0; k < NV; ++k) {
+				const float x = active ? (float)snew[k] : 0.f;
+				if (active)
 					xf[k * N + node] = x;
-					atomicMax(&sscale[k], __float_as_int(fabsf(x)));
-				}
+				sb32[k] = __float_as_int(fabsf(x));
 			}
+			elem_max<N, NV>(sb32, e, active, sx + S::E * NV, NV);
 			__syncthreads();
 			tp_apply<D, Q, NV>(xf, tf, tmpf, sops->SBf, node, active);
 			bool safe = true;
@@ -668,19 +928,15 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, const TPParams& 
 		if constexpr (MODE == kModeRkGlOut) {
 			// the new state's GLL coefficients: V^-1 of the GL values (D passes of Binv)
 			__syncthreads();   // sa/sb/sc are free again
-			if (active)
-#pragma unroll
-				for (int k = 0; k < NV; ++k)
-					sa[k * N + node] = snew[k];
-			__syncthreads();
-			tp_apply<D, Q, NV>(sa, sb, sc, sops->Binv, node, active);
+			tp_apply_fix<D, Q, NV, true>(snew, sa, sb, sops->fBinv, sops->sBinv, sops->Binv, e, node, active,
+			                             sx + S::E * (2 * NV + AE));
 			if (active)
 #pragma unroll
 				for (int k = 0; k < NV; ++k) {
 					const size_t o = ((size_t)v * NV + k) * N + node;
-					rk.out_coef[o] = sb[k * N + node];
+					rk.out_coef[o] = snew[k];
 					if (rk.out_host)
-						rk.out_host[o] = sb[k * N + node];
+						rk.out_host[o] = snew[k];
 				}
 		}
 	}
@@ -692,15 +948,17 @@ struct LiftOccupancy { static constexpr int value = (MODE == kModeRkGlNoMax) ? 4
 
 template <int D, int Q, int NV, int MODE>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS, LiftOccupancy<MODE>::value)
-tp_lift_kernel(const TPOps ops, const TPParams P, const RkArgs rk)
+tp_lift_kernel(const __grid_constant__ TPOps ops, const TPParams P, const RkArgs rk)
 {
 	using S = TPShape<D, Q>;
 	extern __shared__ double smem[];
 	TPOps* sops = reinterpret_cast<TPOps*>(smem);
 	load_ops(sops, ops);
 	const int v0 = blockIdx.x * S::E;
-	tp_lift_body<D, Q, NV, MODE, TPSmem<D, Q, NV>::LIFT>(sops, P, rk, v0, min(S::E, P.n_vol - v0),
-	                                                            smem + sizeof(TPOps) / 8);
+	constexpr int LIFT = TPSmem<D, Q, NV>::LIFT;
+	double* base = smem + sizeof(TPOps) / 8;
+	tp_lift_body<D, Q, NV, MODE, LIFT>(sops, P, rk, v0, min(S::E, P.n_vol - v0), base,
+	                                   reinterpret_cast<int*>(base + S::E * LIFT));
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -710,7 +968,7 @@ tp_lift_kernel(const TPOps ops, const TPParams P, const RkArgs rk)
 // state between a caller's pinned host buffer and the device and changes its basis.
 template <int D, int Q, int NV, bool TO_GL>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS)
-tp_convert_kernel(const TPOps ops, int n_vol, const double* __restrict__ in, double* __restrict__ out,
+tp_convert_kernel(const __grid_constant__ TPOps ops, int n_vol, const double* __restrict__ in, double* __restrict__ out,
                   double* __restrict__ in_copy, double* __restrict__ out_copy)
 {
 	using S = TPShape<D, Q>;
@@ -718,32 +976,33 @@ tp_convert_kernel(const TPOps ops, int n_vol, const double* __restrict__ in, dou
 	extern __shared__ double smem[];
 	TPOps* sops = reinterpret_cast<TPOps*>(smem);
 	double* base = smem + sizeof(TPOps) / 8;
-	constexpr int PER_E = 3 * NV * N;
+	constexpr int PER_E = 2 * NV * N;
+	int* sx = reinterpret_cast<int*>(base + E * PER_E);
 	const int tid = threadIdx.x;
 	load_ops(sops, ops);
 	const int v0 = blockIdx.x * E;
-	const int n_here = min(E, n_vol - v0);
-	for (int i = tid; i < n_here * NV * N; i += blockDim.x) {
-		const int e = i / (NV * N), r = i % (NV * N);
-		const double x = in[(size_t)v0 * NV * N + i];
-		base[e * PER_E + r] = x;
-		if (in_copy)
-			in_copy[(size_t)v0 * NV * N + i] = x;
-	}
-	__syncthreads();
 	const int e = tid / N, node = tid % N;
-	const bool active = e < n_here;
-	double* sa = base + e * PER_E;
-	double* sb = sa + NV * N;
-	double* sc = sb + NV * N;
-	tp_apply<D, Q, NV>(sa, sb, sc, TO_GL ? sops->B : sops->Binv, node, active);
+	const bool active = e < min(E, n_vol - v0);
+	double x[NV];
+	const size_t o = (size_t)(v0 + e) * NV * N + node;
 	if (active)
 #pragma unroll
 		for (int k = 0; k < NV; ++k) {
-			const size_t o = ((size_t)(v0 + e) * NV + k) * N + node;
-			out[o] = sb[k * N + node];
+			x[k] = in[o + (size_t)k * N];
+			if (in_copy)
+				in_copy[o + (size_t)k * N] = x[k];
+		}
+	for (int i = tid; i < E * TPSmem<D, Q, NV>::AEXP; i += blockDim.x)
+		sx[i] = 0;
+	__syncthreads();
+	tp_apply_fix<D, Q, NV, true>(x, base + e * PER_E, base + e * PER_E + NV * N, TO_GL ? sops->fB : sops->fBinv,
+	                       TO_GL ? sops->sB : sops->sBinv, TO_GL ? sops->B : sops->Binv, e, node, active, sx);
+	if (active)
+#pragma unroll
+		for (int k = 0; k < NV; ++k) {
+			out[o + (size_t)k * N] = x[k];
 			if (out_copy)
-				out_copy[o] = sb[k * N + node];
+				out_copy[o + (size_t)k * N] = x[k];
 		}
 }
 

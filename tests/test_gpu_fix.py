@@ -1,0 +1,69 @@
+"""Block fixed-point contractions (csrc/dgpu_fix.cuh) at the edges of their range, against the CPU oracle.
+
+The fixed-point sums are exact to a few 2^-59 of their largest term, below FP64's own rounding, so the tolerance is the
+1e-12 of the other parity tests; a state outside the range takes the FP64 loops and meets the same tolerance.
+"""
+import numpy as np
+import pytest
+
+import oracle
+from dpgsolver_gb300.host import problem as P
+
+pytestmark = pytest.mark.gpu
+
+
+def _residual(prob, sol):
+    from dpgsolver_gb300.solver import Simulation
+    with Simulation(prob) as sim:
+        sim.upload_state(sol)
+        back = sim.sol_coef
+        sim.compute_rhs()
+        return sim.rhs, back
+
+
+@pytest.mark.parametrize("p", [1, 2, 3, 4])
+@pytest.mark.parametrize("power", [-1000, -830, -818, 0, 818, 830, 990])
+def test_scaled_advection(gpu_lib, p, power):
+    """The linear residual scales exactly with the state, inside, at and beyond the ends of the block range."""
+    prob = P.advection_2d(5, p)
+    r0, _ = oracle.Oracle(prob).compute_rhs(prob.sol)
+    r, back = _residual(prob, np.ldexp(prob.sol, power))
+    assert np.array_equal(back, np.ldexp(prob.sol, power))
+    r = np.ldexp(r, -power)
+    assert np.max(np.abs(r - r0)) <= 1e-12 * np.max(np.abs(r0))
+
+
+@pytest.mark.parametrize("d,p", [(2, 1), (2, 3), (3, 2), (3, 3), (3, 4)])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_non_finite_values_stay_in_their_elements(gpu_lib, d, p, bad):
+    """A NaN or Inf reaches the elements that the dense operators carry it to, and no other element changes a bit."""
+    prob = P.euler_vortex_2d(5, p) if d == 2 else P.euler_hex_3d(4, p)
+    r0, _ = _residual(prob, prob.sol)
+    sol = prob.sol.copy()
+    sol[7, 0, 1] = bad
+    with np.errstate(all="ignore"):
+        ref, _ = oracle.Oracle(prob).compute_rhs(sol)
+    r, _ = _residual(prob, sol)
+    hit = np.any(~np.isfinite(ref), axis=(1, 2))
+    assert 1 <= hit.sum() < prob.n_volumes
+    assert np.array_equal(np.any(~np.isfinite(r), axis=(1, 2)), hit)
+    assert np.array_equal(r[~hit], r0[~hit])
+
+
+@pytest.mark.parametrize("d,p", [(2, 2), (3, 2), (3, 3)])
+@pytest.mark.parametrize("scale", [2.0 ** -3, 2.0 ** -12, 1e-9])
+def test_density_spread(gpu_lib, d, p, scale):
+    """One node of an element at a fraction of its density (velocity and pressure kept): the residual on either side of
+    the spread rule."""
+    prob = P.euler_vortex_2d(5, p) if d == 2 else P.euler_hex_3d(3, p)
+    sol = prob.sol.copy()
+    n = prob.ops.n_vs // 2
+    sol[4, 0, n] *= scale
+    sol[4, 1:1 + d, n] *= scale
+    ref, _ = oracle.Oracle(prob).compute_rhs(sol)
+    r, back = _residual(prob, sol)
+    assert np.array_equal(back, sol)
+    # the flux divides by densities down to scale: its rounding errors scale with the largest value at hand
+    ok = np.isfinite(ref)
+    assert np.array_equal(np.isfinite(r), ok)
+    assert np.max(np.abs(np.where(ok, r - ref, 0.0))) <= 1e-12 * max(1.0, 1e-3 / scale) * np.max(np.abs(ref[ok]))
