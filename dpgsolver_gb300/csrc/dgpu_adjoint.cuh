@@ -30,7 +30,7 @@ __device__ __forceinline__ void euler_flux_ref_vjp(const double* W, const double
                                                    double* Wbar)
 {
 	const double rho = W[0], E = W[D + 1];
-	const double rho_inv = 1.0 / rho;
+	const double rho_inv = recip(rho);
 	double u[D], U[D];
 	double V2 = 0.0;
 #pragma unroll
@@ -423,7 +423,7 @@ tp_objective_kernel(const TPParams P, const int* __restrict__ faces, int n_obj, 
 	const double* tL = P.traces + (size_t)(2 * f) * NV * NF;
 	const double sc = P.fgeo[((size_t)f * (D + 1) + D) * NF + i];
 	const double rho = tL[i], E = tL[(D + 1) * NF + i];
-	const double rho_inv = 1.0 / rho;
+	const double rho_inv = recip(rho);
 	double V2 = 0.0, u[D];
 #pragma unroll
 	for (int k = 0; k < D; ++k) {

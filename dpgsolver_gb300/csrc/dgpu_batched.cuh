@@ -113,8 +113,11 @@ template <int D, int Q, int NV>
 struct BSmem {
 	static constexpr int N = TPShape<D, Q>::N;
 	static constexpr int NFQ = TPShape<D, Q>::NF;
-	static constexpr int VOL = NV * N * 2 + D * NV * N + 2 * D * NV * NFQ;   // su, st, sf, own-order traces
-	static constexpr int LIFT = 3 * NV * N + 8 + 2 * D * NV * NFQ;           // sa, sb, sc, scalars, face terms
+	static constexpr int VX = NV * N * 2 + D * NV * N + 2 * D * NV * NFQ;    // su, st, sf, own-order traces
+	static constexpr int LX = 3 * NV * N + 2 * D * NV * NFQ;                 // sa, sb, sc, face terms
+	// then the block exponents (ints) of dgpu_fix.cuh
+	static constexpr int VOL = VX + (TPSmem<D, Q, NV>::EXP + TPSmem<D, Q, NV>::AEXP + 1) / 2;
+	static constexpr int LIFT = LX + (TPSmem<D, Q, NV>::LEXP + 1) / 2;
 };
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -125,109 +128,59 @@ __device__ void bvol_body(const BParams& P, const BatchOps* sops, const BGroup& 
                           const double* __restrict__ u, double* base)
 {
 	constexpr int N = TPShape<D, Q>::N, NFQ = TPShape<D, Q>::NF;
-	constexpr int PER_E = BSmem<D, Q, NV>::VOL;
+	constexpr int PER_E = BSmem<D, Q, NV>::VOL, XE = TPSmem<D, Q, NV>::EXP, AE = TPSmem<D, Q, NV>::AEXP;
 	const int tid = threadIdx.x;
 	const int n_here = min(E, G.n_vol - e0);
-	const double* ublk = u + G.state_off + (long long)e0 * NV * N;
-	for (int i = tid; i < n_here * NV * N; i += blockDim.x) {
-		const int e = i / (NV * N), r = i % (NV * N);
-		base[e * PER_E + r] = ublk[i];
-	}
-	__syncthreads();
 	const int e = tid / N, node = tid % N;
 	const bool active = e < n_here;
 	double* su = base + e * PER_E;
 	double* st = su + NV * N;
 	double* sf = st + NV * N;
 	double* str = sf + D * NV * N;   // [lf][NV][NFQ]
-	if (GLL_IN) {
-		tp_apply<D, Q, NV>(su, st, sf, sops->t.B, node, active);
-		if (active)
-#pragma unroll
-			for (int k = 0; k < NV; ++k)
-				su[k * N + node] = st[k * N + node];
-		__syncthreads();
-	}
-	const long long v = G.elem0 + e0 + e;   // group-sorted element index
+	int* sx = reinterpret_cast<int*>(base + BSmem<D, Q, NV>::VX);   // element 0's block exponents, 2 PER_E ints apart
+	double W[NV];
 	if (active) {
-		double W[NV];
+		const double* ublk = u + G.state_off + (long long)(e0 + e) * NV * N + node;
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
-			W[k] = su[k * N + node];
+			W[k] = ublk[k * N];
+		for (int i = node; i < XE + AE; i += N)
+			sx[e * 2 * PER_E + i] = 0;
+	}
+	__syncthreads();
+	if (GLL_IN)
+		tp_apply_fix<D, Q, NV, true>(W, su, st, sops->t.fB, sops->t.sB, sops->t.B, e, node, active, sx + XE, 2 * PER_E);
+	const long long v = G.elem0 + e0 + e;   // group-sorted element index
+	double fr[D][NV];
+	if (active) {
 		double g[D * D];
 		const double* gm = P.gmet + G.gmet_off + (long long)(e0 + e) * D * D * N;
 #pragma unroll
 		for (int c = 0; c < D * D; ++c)
 			g[c] = gm[c * N + node];
-		if constexpr (PDE == kEuler) {
-			double fr[D][D + 2];
-			euler_flux_ref<D>(W, g, fr);
-#pragma unroll
-			for (int j = 0; j < D; ++j)
-#pragma unroll
-				for (int k = 0; k < NV; ++k)
-					sf[(j * NV + k) * N + node] = fr[j][k];
-		} else {
-#pragma unroll
-			for (int j = 0; j < D; ++j) {
-				double gb = 0.0;
-#pragma unroll
-				for (int i = 0; i < D; ++i)
-					gb += g[j * D + i] * P.b_adv[i];
-				sf[j * N + node] = gb * W[0];
-			}
-		}
+		tp_flux<D, NV, PDE>(P.b_adv, W, g, fr);
+	}
+	int eb[2 * NV];
+	const bool ok = tp_stage_volume<D, Q, NV>(W, fr, e, node, active, su, sf, sx, 2 * PER_E, eb);
+	if (active) {
 		// traces at this element's own GL points, all faces, into shared memory
+		double out[NV];
 		for (int it = node; it < 2 * D * NFQ; it += N) {
 			const int lf = it / NFQ, t = it % NFQ;
-			const int nd = lf >> 1, side = lf & 1;
-			const int t0 = (D == 2 ? t : t % Q), t1 = (D == 2 ? 0 : t / Q);
-			int stride_n, base_n;
-			if (D == 2) {
-				stride_n = (nd == 0 ? 1 : Q);
-				base_n = (nd == 0 ? t0 * Q : t0);
-			} else {
-				stride_n = (nd == 0 ? 1 : (nd == 1 ? Q : Q * Q));
-				base_n = (nd == 0 ? t0 * Q + t1 * Q * Q : (nd == 1 ? t0 + t1 * Q * Q : t0 + t1 * Q));
-			}
+			tp_trace<D, Q, NV>(&sops->t, su, eb, ok, lf, t, out);
 #pragma unroll
-			for (int k = 0; k < NV; ++k) {
-				double s = 0.0;
-#pragma unroll
-				for (int m = 0; m < Q; ++m)
-					s += sops->t.lb[side][m] * su[k * N + base_n + m * stride_n];
-				str[(lf * NV + k) * NFQ + t] = s;
-			}
+			for (int k = 0; k < NV; ++k)
+				str[(lf * NV + k) * NFQ + t] = out[k];
 		}
-	}
-	__syncthreads();
-	if (active) {
 		// volume term in GL space
-		double acc[NV];
-#pragma unroll
-		for (int k = 0; k < NV; ++k)
-			acc[k] = 0.0;
-#pragma unroll
-		for (int j = 0; j < D; ++j) {
-			const int stride = (j == 0 ? 1 : (j == 1 ? Q : Q * Q));
-			const int a = node_coord<Q>(node, j);
-			const int b0 = node - a * stride;
-			double w[Q];
-#pragma unroll
-			for (int m = 0; m < Q; ++m)
-				w[m] = sops->t.Dgl[m][a];
-#pragma unroll
-			for (int k = 0; k < NV; ++k) {
-				const double* f = sf + (j * NV + k) * N + b0;
-#pragma unroll
-				for (int m = 0; m < Q; ++m)
-					acc[k] += w[m] * f[m * stride];
-			}
-		}
+		tp_derivative<D, Q, NV>(&sops->t, sf, eb, ok, node, out);
 		double* vg = P.vol_gl + G.state_off + (long long)(e0 + e) * NV * N;
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
-			vg[k * N + node] = acc[k];
+			vg[k * N + node] = out[k];
+	}
+	__syncthreads();
+	if (active) {
 		// traces at each face's order: copy (q_f == Q) or tangential interpolation Q -> q_f. In 3D the
 		// interpolation is separable: a thread takes one (variable, i0) column, contracts the first tangential
 		// direction once per b (Q^2 FMAs) and reuses the Q partial sums for all q_f outputs i1.
@@ -351,12 +304,14 @@ __device__ void blift_body(const BParams& P, const BatchOps* sops, const BGroup&
 	double* sa = base + e * PER_E;
 	double* sb = sa + NV * N;
 	double* sc = sb + NV * N;
-	int* sscale = reinterpret_cast<int*>(sc + NV * N);
-	double* sg = sc + NV * N + 8;        // [lf][NV][NFQ]: E_lf^T-side face terms at this element's points
+	double* sg = sc + NV * N;            // [lf][NV][NFQ]: E_lf^T-side face terms at this element's points
+	constexpr int AE = TPSmem<D, Q, NV>::AEXP, SX = 2 * PER_E;
+	int* sx = reinterpret_cast<int*>(base + BSmem<D, Q, NV>::LX);   // element 0's block exponents, SX ints apart
+	const int* sscale = sx + e * SX + NV;   // FP32 scales of the positivity pre-filter
 	const long long v = G.elem0 + e0 + e;
-	if (active && node < 8)
-		reinterpret_cast<double*>(sscale)[node] = 0.0;
 	if (active) {
+		for (int i = node; i < TPSmem<D, Q, NV>::LEXP; i += N)
+			sx[e * SX + i] = 0;
 		// face terms at the element's own points: copy (q_f == Q) or transposed interpolation q_f -> Q
 		// (separable in 3D: a thread takes one (variable, a) column, contracts i0 for every i1 once and reuses
 		// the q_f partial sums for all Q outputs b).
@@ -416,54 +371,50 @@ __device__ void blift_body(const BParams& P, const BatchOps* sops, const BGroup&
 	}
 	__syncthreads();
 
-	double Rg[NV];
+	constexpr int NFT = TPSmem<D, Q, NV>::NFT, NR = (NFT + N - 1) / N;
+	double fv[NR][NV], Rg[NV];
 	if (active) {
 		const double* vg = P.vol_gl + G.state_off + (long long)(e0 + e) * NV * N;
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
 			Rg[k] = vg[k * N + node];
 #pragma unroll
-		for (int lf = 0; lf < 2 * D; ++lf) {
-			const int nd = lf >> 1;
-			const int a = node_coord<Q>(node, nd);
-			int t;
-			if (D == 2) {
-				t = (nd == 0 ? node_coord<Q>(node, 1) : node_coord<Q>(node, 0));
-			} else {
-				const int c0 = node_coord<Q>(node, 0), c1 = node_coord<Q>(node, 1), c2 = node_coord<Q>(node, 2);
-				t = (nd == 0 ? c1 + Q * c2 : (nd == 1 ? c0 + Q * c2 : c0 + Q * c1));
-			}
-			const double l = sops->t.lb[lf & 1][a];
+		for (int r = 0; r < NR; ++r) {
+			const int it = node + r * N;
+			if (it >= NFT)
+				break;
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
-				Rg[k] += l * sg[(lf * NV + k) * NFQ + t];
+				fv[r][k] = sg[((it / NFQ) * NV + k) * NFQ + it % NFQ];
 		}
+	}
+	tp_lift_sum<D, Q, NV>(&sops->t, fv, Rg, e, node, active, sa, sx, SX);
+	if (active) {
 		const double iw = P.inv_wJ[G.wj_off + (long long)(e0 + e) * N + node];
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
-			Rg[k] *= iw;
+			Rg[k] = mul(Rg[k], iw);
 		if (P.source) {
 			const double* sv = P.source + G.state_off + (long long)(e0 + e) * NV * N + node;
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
-				Rg[k] += sv[(long long)k * N];
+				Rg[k] = add(Rg[k], sv[(long long)k * N]);
 		}
 	}
+	__syncthreads();   // the face terms are read; sa, sb, sc are reused
 
 	const bool need_coef = (MODE == kModeRhs) || (MODE != kModeRkGlNoMax && rk.want_max);
 	unsigned long long mx = 0ull;
 	double R[NV];
 	if (need_coef) {
-		if (active)
 #pragma unroll
-			for (int k = 0; k < NV; ++k)
-				sa[k * N + node] = Rg[k];
-		__syncthreads();
-		tp_apply<D, Q, NV>(sa, sb, sc, sops->t.Binv, node, active);
+		for (int k = 0; k < NV; ++k)
+			R[k] = Rg[k];
+		tp_apply_fix<D, Q, NV, false>(R, sa, sb, sops->t.fBinv, sops->t.sBinv, sops->t.Binv, e, node, active,
+		                              sx + 2 * NV, SX);
 		if (active) {
 #pragma unroll
 			for (int k = 0; k < NV; ++k) {
-				R[k] = sb[k * N + node];
 				const unsigned long long bits = abs_bits(R[k]);
 				mx = bits > mx ? bits : mx;
 			}
@@ -489,14 +440,9 @@ __device__ void blift_body(const BParams& P, const BatchOps* sops, const BGroup&
 #pragma unroll
 			for (int k = 0; k < NV; ++k) {
 				const double s = rk.u[so + (long long)k * N];
-				if (rk.stage == 0) {
+				if (rk.stage == 0)
 					rk.u0[so + (long long)k * N] = s;
-					snew[k] = s + rk.dt * Rg[k];
-				} else if (rk.stage == 1) {
-					snew[k] = (1.0 / 4.0) * (3.0 * rk.u0[so + (long long)k * N] + s + rk.dt * Rg[k]);
-				} else {
-					snew[k] = (1.0 / 3.0) * (rk.u0[so + (long long)k * N] + 2.0 * s + 2.0 * rk.dt * Rg[k]);
-				}
+				snew[k] = rk_update(rk.stage, s, rk.stage == 0 ? s : rk.u0[so + (long long)k * N], rk.dt, Rg[k]);
 			}
 		}
 		if (rk.positivity) {
@@ -508,14 +454,15 @@ __device__ void blift_body(const BParams& P, const BatchOps* sops, const BGroup&
 			float* xf = reinterpret_cast<float*>(sa);
 			float* tf = xf + NV * N;
 			float* tmpf = reinterpret_cast<float*>(sc);
-			if (active) {
+			int sb32[NV];
 #pragma unroll
-				for (int k = 0; k < NV; ++k) {
-					const float x = (float)snew[k];
+			for (int k = 0; k < NV; ++k) {
+				const float x = active ? (float)snew[k] : 0.f;
+				if (active)
 					xf[k * N + node] = x;
-					atomicMax(&sscale[k], __float_as_int(fabsf(x)));
-				}
+				sb32[k] = __float_as_int(fabsf(x));
 			}
+			elem_max<N, NV>(sb32, e, active, sx + NV, SX);
 			__syncthreads();
 			tp_apply<D, Q, NV>(xf, tf, tmpf, sops->t.SBf, node, active);
 			bool safe = true;
@@ -607,25 +554,29 @@ __global__ void __launch_bounds__(256) bconvert_group_kernel(const BParams P, in
 	double* base = smem + sizeof(BatchOps) / 8;
 	const BGroup G = P.groups[g];
 	load_batch_ops(sops, &P.ops[g]);
-	constexpr int N = TPShape<D, Q>::N;
-	constexpr int PER_E = 3 * NV * N;
-	const int E = G.E, e0 = blockIdx.x * E, n_here = min(E, G.n_vol - e0);
-	const double* src = in + G.state_off + (long long)e0 * NV * N;
-	for (int i = threadIdx.x; i < n_here * NV * N; i += blockDim.x) {
-		const int e = i / (NV * N), r = i % (NV * N);
-		base[e * PER_E + r] = src[i];
+	constexpr int N = TPShape<D, Q>::N, AE = TPSmem<D, Q, NV>::AEXP;
+	constexpr int PER_E = 3 * NV * N;   // two buffers, then the block exponents
+	const int E = G.E, e0 = blockIdx.x * E;
+	const int e = threadIdx.x / N, node = threadIdx.x % N;
+	const bool active = e < min(E, G.n_vol - e0);
+	int* sx = reinterpret_cast<int*>(base + 2 * NV * N);
+	const long long o = G.state_off + (long long)(e0 + e) * NV * N + node;
+	double x[NV];
+	if (active) {
+#pragma unroll
+		for (int k = 0; k < NV; ++k)
+			x[k] = in[o + k * N];
+		for (int i = node; i < AE; i += N)
+			sx[e * 2 * PER_E + i] = 0;
 	}
 	__syncthreads();
-	const int e = threadIdx.x / N, node = threadIdx.x % N;
-	const bool active = e < n_here;
-	double* sa = base + e * PER_E;
-	double* sb = sa + NV * N;
-	double* sc = sb + NV * N;
-	tp_apply<D, Q, NV>(sa, sb, sc, TO_GL ? sops->t.B : sops->t.Binv, node, active);
+	tp_apply_fix<D, Q, NV, true>(x, base + e * PER_E, base + e * PER_E + NV * N, TO_GL ? sops->t.fB : sops->t.fBinv,
+	                             TO_GL ? sops->t.sB : sops->t.sBinv, TO_GL ? sops->t.B : sops->t.Binv, e, node, active,
+	                             sx, 2 * PER_E);
 	if (active)
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
-			out[G.state_off + (long long)(e0 + e) * NV * N + (long long)k * N + node] = sb[k * N + node];
+			out[o + k * N] = x[k];
 }
 
 }  // namespace dgpu

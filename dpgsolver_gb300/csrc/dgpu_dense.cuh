@@ -477,14 +477,9 @@ __device__ void dlift_body(const BParams& P, const DGroup& G, int e0, int E, con
 		} else {
 			const double s = rk.u[o];
 			double sn;
-			if (rk.stage == 0) {
+			if (rk.stage == 0)
 				rk.u0[o] = s;
-				sn = s + rk.dt * R;
-			} else if (rk.stage == 1) {
-				sn = (1.0 / 4.0) * (3.0 * rk.u0[o] + s + rk.dt * R);
-			} else {
-				sn = (1.0 / 3.0) * (rk.u0[o] + 2.0 * s + 2.0 * rk.dt * R);
-			}
+			sn = rk_update(rk.stage, s, rk.stage == 0 ? s : rk.u0[o], rk.dt, R);
 			rk.u[o] = sn;
 			smem[e * PER_E + NV * nvs + rem] = sn;   // kept for the positivity check
 		}
@@ -609,7 +604,7 @@ __device__ __noinline__ void dlift_tile(const BParams& P, const DGroup& G, int e
 }
 
 template <int D, int NV, int PDE, bool GLL_IN>
-__global__ void __launch_bounds__(256) bvol_fused_kernel(const BParams P, const BTile* tiles, int n_tiles,
+__global__ void __launch_bounds__(256, 2) bvol_fused_kernel(const BParams P, const BTile* tiles, int n_tiles,
                                                            const double* __restrict__ u)
 {
 	extern __shared__ double smem[];

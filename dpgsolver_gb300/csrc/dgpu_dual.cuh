@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include "dgpu_fix.cuh"
+
 namespace dgpu {
 
 template <int K>
@@ -67,7 +69,7 @@ template <int K>
 __device__ __forceinline__ Dual<K> operator/(const Dual<K>& a, const Dual<K>& b)
 {
 	Dual<K> r;
-	const double inv = 1.0 / b.v;
+	const double inv = fix_rcp(b.v);
 	r.v = a.v * inv;
 #pragma unroll
 	for (int k = 0; k < K; ++k)
@@ -123,11 +125,11 @@ __device__ __forceinline__ bool operator>(const Dual<K>& a, double b) { return a
 // sqrt with the derivative 1/(2 sqrt(x)); at x = 0 the derivative is taken as 0 (the one-sided subgradient of
 // |V| = sqrt(V^2) at rest), where the exact derivative does not exist.
 template <int K>
-__device__ __forceinline__ Dual<K> sqrt(const Dual<K>& a)
+__device__ __forceinline__ Dual<K> root(const Dual<K>& a)
 {
 	Dual<K> r;
-	r.v = ::sqrt(a.v);
-	const double s = (r.v > 0.0 ? 0.5 / r.v : 0.0);
+	r.v = fix_sqrt(a.v);
+	const double s = (r.v > 0.0 ? 0.5 * fix_rcp(r.v) : 0.0);
 #pragma unroll
 	for (int k = 0; k < K; ++k)
 		r.d[k] = a.d[k] * s;
@@ -145,6 +147,18 @@ __device__ __forceinline__ Dual<K> pow(const Dual<K>& a, double b)
 	Dual<K> r;
 	r.v = ::pow(a.v, b);
 	const double s = b * r.v / a.v;
+#pragma unroll
+	for (int k = 0; k < K; ++k)
+		r.d[k] = a.d[k] * s;
+	return r;
+}
+
+template <int K>
+__device__ __forceinline__ Dual<K> recip(const Dual<K>& a)
+{
+	Dual<K> r;
+	r.v = fix_rcp(a.v);
+	const double s = -(r.v * r.v);
 #pragma unroll
 	for (int k = 0; k < K; ++k)
 		r.d[k] = a.d[k] * s;

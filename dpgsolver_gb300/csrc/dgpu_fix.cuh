@@ -174,4 +174,71 @@ __device__ __forceinline__ void fix_pass(const int2* __restrict__ in, int2* __re
 	}
 }
 
+// ---------------------------------------------------------------------------------------------------------------
+// Reciprocal, square root and magnitude comparison of doubles on the integer pipe
+// ---------------------------------------------------------------------------------------------------------------
+// 1/x and sqrt(x) in FP64 arithmetic take 8 to 10 operations of 64 cycles; a comparison takes one. Newton's iteration
+// (Newton-Raphson for 1/x, the binomial series of sqrt(s0^2 + r) for the root) on integers, started from the FP32
+// approximations of the special function unit, needs about 50 to 70 cycles. Residuals are formed exactly, the result
+// carries an error of a few 2^-60 before its single rounding to nearest (at most 0.508 and 0.501 ulp over 2^30 random
+// arguments each, powers of two exact). Zeros, denormals, Inf, NaN, negative roots and reciprocals
+// that would be denormal take the FP64 operation.
+__device__ __forceinline__ double fix_rcp(double x)
+{
+	const int hi = __double2hiint(x), lo = __double2loint(x);
+	const int ex = (hi >> 20) & 0x7ff;
+	if ((unsigned)(ex - 1) >= 2044u)   // 0, denormal, Inf, NaN, or a denormal result
+		return 1.0 / x;
+	const float f = __int_as_float((__funnelshift_l(lo, hi, 3) & 0x007fffff) | 0x3f800000);   // [1, 2)
+	float y;
+	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(f));
+	const unsigned M = (min(__float_as_uint(y), 0x3f7fffffu) & 0x007fffff) | 0x00800000;      // y 2^24
+	const unsigned dh = (hi & 0x000fffff) | 0x00100000;                                        // 1.m 2^52
+	// e = 1 - d y in units of 2^-76, exactly: |e| < 2^54, so the low 64 bits suffice
+	const long long e = -(long long)((unsigned long long)(unsigned)lo * M + ((unsigned long long)(dh * M) << 32));
+	const int eh = (int)(e >> 32);
+	// y (1 + e + e^2) in units of 2^-60
+	const long long t = (long long)eh * (int)M + (long long)(((unsigned long long)(unsigned)e * M) >> 32);
+	const unsigned sq = (unsigned)(((long long)eh * eh) >> 20);
+	const unsigned long long R = ((unsigned long long)M << 36) + (t >> 8) + __umulhi(sq, M);
+	const unsigned long long q = (R + 64) >> 7;   // 53 bits, leading bit 52 (or 2^53)
+	const int rh = (int)(q >> 32) + ((2044 - ex) << 20);
+	return __hiloint2double(rh | (hi & 0x80000000), (int)q);
+}
+
+__device__ __forceinline__ double fix_sqrt(double x)
+{
+	const int hi = __double2hiint(x), lo = __double2loint(x);
+	const int ex = hi >> 20;   // negative for a negative argument
+	if ((unsigned)(ex - 1) >= 2046u)
+		return ::sqrt(x);
+	const int t = (ex + 1) & 1;   // x = f 4^k, f = 1.m 2^t in [1, 4)
+	const float f = __int_as_float((__funnelshift_l(lo, hi, 3) & 0x007fffff) | (0x3f800000 + (t << 23)));
+	float y;
+	asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(f));
+	const unsigned M = (min(__float_as_uint(y), 0x3f7fffffu) & 0x007fffff) | 0x00800000;      // y 2^24, y in (1/2, 1]
+	const unsigned mh = (hi & 0x000fffff) | 0x00100000;
+	const unsigned long long X =
+		((((unsigned long long)mh) << 32) | (unsigned)lo) << (8 + t);                            // f 2^60
+	const unsigned S0 = (unsigned)(((unsigned long long)(unsigned)(X >> 32) * M) >> 22);         // s0 = f y, 2^30
+	const long long r = (long long)(X - (unsigned long long)S0 * S0);                           // f - s0^2, 2^60
+	const int d = (int)(((1ll << 54) - (long long)((unsigned long long)S0 * M)) >> 4);           // 1 - s0 y, 2^50
+	// u = r y / 2 in units of 2^-62, then sqrt(f) = s0 + u + u (d - u y / 2) + ...
+	const long long u = (long long)(((unsigned long long)(unsigned)r * M) >> 23) + (((r >> 32) * (int)M) << 9);
+	const int U = (int)(u >> 12);                                                               // 2^50
+	const int z = d - (int)(((long long)U * (int)M) >> 25);
+	const long long v = ((long long)U * z) >> 38;
+	const unsigned long long q = (((unsigned long long)S0 << 32) + u + v + 512) >> 10;
+	const int rh = (int)(q >> 32) + ((((ex - 1023 - t) >> 1) + 1022) << 20);
+	return __hiloint2double(rh, (int)q);
+}
+
+// |a| < |b|, false when either is NaN.
+__device__ __forceinline__ bool abs_less(double a, double b)
+{
+	const unsigned long long ua = (unsigned long long)__double_as_longlong(a) & 0x7fffffffffffffffull;
+	const unsigned long long ub = (unsigned long long)__double_as_longlong(b) & 0x7fffffffffffffffull;
+	return ua < ub && ub <= 0x7ff0000000000000ull;
+}
+
 }  // namespace dgpu

@@ -16,7 +16,11 @@ namespace dgpu {
 
 using ::fabs;
 using ::pow;
-using ::sqrt;
+
+// 1/x, sqrt(x) and the comparison of magnitudes of the flux routines' scalar type: doubles on the integer pipe
+// (dgpu_fix.cuh), Dual in dgpu_dual.cuh.
+__device__ __forceinline__ double recip(double x) { return fix_rcp(x); }
+__device__ __forceinline__ double root(double x) { return fix_sqrt(x); }
 
 constexpr double kGamma = 1.4;          // definitions_physics.h:23
 constexpr double kGm1 = 0.4;            // definitions_physics.h:24
@@ -41,6 +45,50 @@ __device__ __forceinline__ T max_abs_real(const T& a, const T& b)
 	return (c < 0.0 ? -c : c);
 }
 
+// Products and sums with their rounding written out, so that every kernel a flux routine is inlined into (the launch
+// forms of a batched mesh among them) rounds alike: mad is one fused operation, mul and add are never fused.
+template <typename A, typename B, typename C>
+__device__ __forceinline__ C mad(A a, B b, const C& c)
+{
+	return a * b + c;
+}
+__device__ __forceinline__ double mad(double a, double b, double c) { return __fma_rn(a, b, c); }
+template <typename A, typename B>
+__device__ __forceinline__ auto mul(A a, B b)
+{
+	return a * b;
+}
+__device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+template <typename T>
+__device__ __forceinline__ T add(const T& a, const T& b)
+{
+	return a + b;
+}
+__device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
+template <typename T>
+__device__ __forceinline__ T sub(const T& a, const T& b)
+{
+	return a - b;
+}
+__device__ __forceinline__ double sub(double a, double b) { return __dadd_rn(a, -b); }
+
+__device__ __forceinline__ double min_abs_real(double a, double b) { return fabs(abs_less(a, b) ? a : b); }
+__device__ __forceinline__ double max_abs_real(double a, double b) { return fabs(abs_less(b, a) ? a : b); }
+
+// |a|, and the larger of two non-negative values (a NaN in a gives b).
+template <typename T>
+__device__ __forceinline__ T abs_real(const T& a)
+{
+	return a > 0.0 ? a : -a;
+}
+__device__ __forceinline__ double abs_real(double a) { return fabs(a); }
+template <typename T>
+__device__ __forceinline__ T larger(const T& a, const T& b)
+{
+	return a > b ? a : b;
+}
+__device__ __forceinline__ double larger(double a, double b) { return abs_less(b, a) ? a : b; }
+
 // Contravariant volume flux at one cubature node for the Euler equations:
 //   fr_j[eq] = sum_i g[j*D+i] f_i[eq]
 // with f the physical flux of compute_Flux_T_euler / compute_Flux_euler_0 (flux_euler_T.c:71-143, 259-298)
@@ -52,25 +100,25 @@ template <int D, typename T = double>
 __device__ __forceinline__ void euler_flux_ref(const T* W, const double* g, T (*fr)[D + 2])
 {
 	const T rho = W[0], E = W[D + 1];
-	const T rho_inv = 1.0 / rho;
-	T m2 = 0.0;
+	const T rho_inv = recip(rho);
+	T m2 = mul(W[1], W[1]);
 #pragma unroll
-	for (int k = 0; k < D; ++k)
-		m2 += W[1 + k] * W[1 + k];
-	const T p = kGm1 * (E - 0.5 * (m2 * rho_inv));
-	const T Ep = E + p;
+	for (int k = 1; k < D; ++k)
+		m2 = mad(W[1 + k], W[1 + k], m2);
+	const T p = mul(kGm1, mad(-0.5, mul(m2, rho_inv), E));
+	const T Ep = add(E, p);
 #pragma unroll
 	for (int j = 0; j < D; ++j) {
-		T M = 0.0;
+		T M = mul(g[j * D], W[1]);
 #pragma unroll
-		for (int i = 0; i < D; ++i)
-			M += g[j * D + i] * W[1 + i];
-		const T U = M * rho_inv;
+		for (int i = 1; i < D; ++i)
+			M = mad(g[j * D + i], W[1 + i], M);
+		const T U = mul(M, rho_inv);
 		fr[j][0] = M;
 #pragma unroll
 		for (int m = 0; m < D; ++m)
-			fr[j][1 + m] = W[1 + m] * U + p * g[j * D + m];
-		fr[j][D + 1] = Ep * U;
+			fr[j][1 + m] = mad(W[1 + m], U, mul(p, g[j * D + m]));
+		fr[j][D + 1] = mul(Ep, U);
 	}
 }
 
@@ -79,18 +127,18 @@ __device__ __forceinline__ void euler_flux_ref(const T* W, const double* g, T (*
 template <int D, typename T>
 __device__ __forceinline__ void euler_side_lf(const T* W, const double* n, T& mn, T& Vn, T& p, T& lam)
 {
-	const T rho_inv = 1.0 / W[0];
-	T m2 = 0.0;
-	mn = 0.0;
+	const T rho_inv = recip(W[0]);
+	T m2 = mul(W[1], W[1]);
+	mn = mul(n[0], W[1]);
 #pragma unroll
-	for (int k = 0; k < D; ++k) {
-		m2 += W[1 + k] * W[1 + k];
-		mn += n[k] * W[1 + k];
+	for (int k = 1; k < D; ++k) {
+		m2 = mad(W[1 + k], W[1 + k], m2);
+		mn = mad(n[k], W[1 + k], mn);
 	}
-	const T q = m2 * rho_inv;   // rho |V|^2
-	Vn = mn * rho_inv;
-	p = kGm1 * (W[D + 1] - 0.5 * q);
-	lam = sqrt(q * rho_inv) + sqrt(kGamma * p * rho_inv);
+	const T q = mul(m2, rho_inv);   // rho |V|^2
+	Vn = mul(mn, rho_inv);
+	p = mul(kGm1, mad(-0.5, q, W[D + 1]));
+	lam = add(root(mul(q, rho_inv)), root(mul(mul(kGamma, p), rho_inv)));
 }
 
 // Lax-Friedrichs (compute_Numerical_Flux_T_euler_lax_friedrichs, numerical_flux_euler_T.c:60-327):
@@ -105,14 +153,16 @@ __device__ __forceinline__ void num_flux_lax_friedrichs(const T* WL, const T* WR
 	T mnL, VnL, pL, lamL, mnR, VnR, pR, lamR;
 	euler_side_lf<D>(WL, n, mnL, VnL, pL, lamL);
 	euler_side_lf<D>(WR, n, mnR, VnR, pR, lamR);
-	const T maxV = (lamL > lamR ? lamL : lamR);
+	const T maxV = larger(lamL, lamR);
 	const double h = 0.5 * scale;
-	const T pLR = pL + pR;
-	nF[0] = h * ((mnL + mnR) + maxV * (WL[0] - WR[0]));
+	const T pLR = add(pL, pR);
+	nF[0] = mul(h, mad(maxV, sub(WL[0], WR[0]), add(mnL, mnR)));
 #pragma unroll
 	for (int k = 0; k < D; ++k)
-		nF[1 + k] = h * ((WL[1 + k] * VnL + WR[1 + k] * VnR + pLR * n[k]) + maxV * (WL[1 + k] - WR[1 + k]));
-	nF[D + 1] = h * (((WL[D + 1] + pL) * VnL + (WR[D + 1] + pR) * VnR) + maxV * (WL[D + 1] - WR[D + 1]));
+		nF[1 + k] = mul(h, mad(maxV, sub(WL[1 + k], WR[1 + k]),
+		                       mad(WL[1 + k], VnL, mad(WR[1 + k], VnR, mul(pLR, n[k])))));
+	nF[D + 1] = mul(h, mad(maxV, sub(WL[D + 1], WR[D + 1]),
+	                       mad(add(WL[D + 1], pL), VnL, mul(add(WR[D + 1], pR), VnR))));
 }
 
 // Roe-Pike with the entropy fix of Qu et al. 2015 (compute_Numerical_Flux_T_euler_roe_pike,
@@ -121,51 +171,51 @@ template <int D, typename T = double>
 __device__ __forceinline__ void num_flux_roe_pike(const T* WL, const T* WR, const double* n, T* nF)
 {
 	const T rhoL = WL[0], rhoR = WR[0], EL = WL[D + 1], ER = WR[D + 1];
-	const T rhoL_inv = 1.0 / rhoL, rhoR_inv = 1.0 / rhoR;
-	T uL[D], uR[D];
-	T V2L = 0.0, V2R = 0.0, VnL = 0.0, VnR = 0.0;
+	const T rhoL_inv = recip(rhoL), rhoR_inv = recip(rhoR);
+	T uL[D], uR[D], V2L, V2R, VnL, VnR;
 #pragma unroll
 	for (int k = 0; k < D; ++k) {
-		uL[k] = WL[1 + k] * rhoL_inv;
-		uR[k] = WR[1 + k] * rhoR_inv;
-		V2L += uL[k] * uL[k];
-		V2R += uR[k] * uR[k];
-		VnL += n[k] * uL[k];
-		VnR += n[k] * uR[k];
+		uL[k] = mul(WL[1 + k], rhoL_inv);
+		uR[k] = mul(WR[1 + k], rhoR_inv);
+		V2L = k ? mad(uL[k], uL[k], V2L) : mul(uL[k], uL[k]);
+		V2R = k ? mad(uR[k], uR[k], V2R) : mul(uR[k], uR[k]);
+		VnL = k ? mad(n[k], uL[k], VnL) : mul(n[k], uL[k]);
+		VnR = k ? mad(n[k], uR[k], VnR) : mul(n[k], uR[k]);
 	}
-	const T pL = kGm1 * (EL - 0.5 * rhoL * V2L), HL = (EL + pL) * rhoL_inv;
-	const T pR = kGm1 * (ER - 0.5 * rhoR * V2R), HR = (ER + pR) * rhoR_inv;
+	const T pL = mul(kGm1, mad(mul(-0.5, rhoL), V2L, EL)), HL = mul(add(EL, pL), rhoL_inv);
+	const T pR = mul(kGm1, mad(mul(-0.5, rhoR), V2R, ER)), HR = mul(add(ER, pR), rhoR_inv);
 
 	// Roe averages (divisions by r + 1 through one reciprocal)
-	const T r = sqrt(rhoR * rhoL_inv), rP1_inv = 1.0 / (r + 1.0), rho = r * rhoL;
-	T u[D];
-	T Vn = 0.0, V2 = 0.0;
+	const T r = root(mul(rhoR, rhoL_inv)), rP1_inv = recip(add(r, T(1.0))), rho = mul(r, rhoL);
+	T u[D], Vn, V2;
 #pragma unroll
 	for (int k = 0; k < D; ++k) {
-		u[k] = (r * uR[k] + uL[k]) * rP1_inv;
-		Vn += n[k] * u[k];
-		V2 += u[k] * u[k];
+		u[k] = mul(mad(r, uR[k], uL[k]), rP1_inv);
+		Vn = k ? mad(n[k], u[k], Vn) : mul(n[k], u[k]);
+		V2 = k ? mad(u[k], u[k], V2) : mul(u[k], u[k]);
 	}
-	const T H = (r * HR + HL) * rP1_inv, c2 = kGm1 * (H - 0.5 * V2), c = sqrt(c2), c_inv = 1.0 / c;
+	const T H = mul(mad(r, HR, HL), rP1_inv), c2 = mul(kGm1, mad(-0.5, V2, H)), c = root(c2), c_inv = recip(c);
 
-	const T l1 = min_abs_real(VnL - c, Vn - c), l5 = max_abs_real(VnR + c, Vn + c);
-	const T l234 = (Vn > 0.0 ? Vn : -Vn);
+	const T l1 = min_abs_real(sub(VnL, c), sub(Vn, c)), l5 = max_abs_real(add(VnR, c), add(Vn, c));
+	const T l234 = abs_real(Vn);
 
-	const T drho = rhoR - rhoL, dE = ER - EL, dp = pR - pL, dVn = VnR - VnL;
-	const T lc1 = 0.5 * (l5 + l1) - l234, lc2 = 0.5 * (l5 - l1);
-	const T disInter1 = (lc1 * dp * c_inv + lc2 * rho * dVn) * c_inv;
-	const T disInter2 = lc1 * rho * dVn + lc2 * dp * c_inv;
+	const T drho = sub(rhoR, rhoL), dE = sub(ER, EL), dp = sub(pR, pL), dVn = sub(VnR, VnL);
+	const T lc1 = mad(0.5, add(l5, l1), -l234), lc2 = mul(0.5, sub(l5, l1));
+	const T lc1_dp = mul(mul(lc1, dp), c_inv), lc2_dp = mul(mul(lc2, dp), c_inv);
+	const T disInter1 = mul(mad(mul(lc2, rho), dVn, lc1_dp), c_inv);
+	const T disInter2 = mad(mul(lc1, rho), dVn, lc2_dp);
 
-	const T rhoVnL = rhoL * VnL, rhoVnR = rhoR * VnR, pLR = pL + pR;
-	nF[0] = 0.5 * ((rhoVnL + rhoVnR) - (l234 * drho + disInter1));
+	const T rhoVnL = mul(rhoL, VnL), rhoVnR = mul(rhoR, VnR), pLR = add(pL, pR);
+	nF[0] = mul(0.5, sub(add(rhoVnL, rhoVnR), mad(l234, drho, disInter1)));
 #pragma unroll
 	for (int k = 0; k < D; ++k) {
-		const T drhou = WR[1 + k] - WL[1 + k];
-		const T nFk = rhoVnL * uL[k] + rhoVnR * uR[k] + n[k] * pLR;
-		const T disk = l234 * drhou + disInter1 * u[k] + disInter2 * n[k];
-		nF[1 + k] = 0.5 * (nFk - disk);
+		const T drhou = sub(WR[1 + k], WL[1 + k]);
+		const T nFk = mad(rhoVnL, uL[k], mad(rhoVnR, uR[k], mul(n[k], pLR)));
+		const T disk = mad(l234, drhou, mad(disInter1, u[k], mul(disInter2, n[k])));
+		nF[1 + k] = mul(0.5, sub(nFk, disk));
 	}
-	nF[D + 1] = 0.5 * ((VnL * (EL + pL) + VnR * (ER + pR)) - (l234 * dE + disInter1 * H + disInter2 * Vn));
+	nF[D + 1] = mul(0.5, sub(mad(VnL, add(EL, pL), mul(VnR, add(ER, pR))),
+	                         mad(l234, dE, mad(disInter1, H, mul(disInter2, Vn)))));
 }
 
 // Upwind advection flux (compute_Numerical_Flux_T_advection_upwind, numerical_flux_advection_T.c:39-75).
@@ -233,7 +283,7 @@ __device__ __forceinline__ void euler_boundary_state(int bc, const T* WL, const 
 {
 	constexpr int NV = D + 2;
 	if (bc == kBcBackPressure || bc == kBcTotalTP) {
-		const T rho_l = WL[0], rho_l_inv = 1.0 / rho_l;
+		const T rho_l = WL[0], rho_l_inv = recip(rho_l);
 		T u_l[D], V2_l = 0.0, Vn_l = 0.0;
 #pragma unroll
 		for (int k = 0; k < D; ++k) {
@@ -244,7 +294,7 @@ __device__ __forceinline__ void euler_boundary_state(int bc, const T* WL, const 
 		const T p_l = kGm1 * (WL[D + 1] - 0.5 * rho_l * V2_l);
 		const T c2_l = kGamma * p_l * rho_l_inv;
 		if (bc == kBcBackPressure) {
-			if (!(sqrt(V2_l) < sqrt(c2_l))) {
+			if (!(root(V2_l) < root(c2_l))) {
 #pragma unroll
 				for (int k = 0; k < NV; ++k)
 					WR[k] = WL[k];
@@ -259,10 +309,10 @@ __device__ __forceinline__ void euler_boundary_state(int bc, const T* WL, const 
 			return;
 		}
 		const T H_l = (WL[D + 1] + p_l) * rho_l_inv;
-		const T R_l = Vn_l + (2.0 / kGm1) * sqrt(c2_l);
+		const T R_l = Vn_l + (2.0 / kGm1) * root(c2_l);
 		constexpr double aQ = 1.0 + 2.0 / kGm1;
 		const T bQ = -2.0 * R_l, cQ = 0.5 * kGm1 * (R_l * R_l - 2.0 * H_l);
-		const T t1 = bQ * (-0.5 / aQ), t2 = sqrt(bQ * bQ - 4.0 * aQ * cQ) * (0.5 / aQ);
+		const T t1 = bQ * (-0.5 / aQ), t2 = root(bQ * bQ - 4.0 * aQ * cQ) * (0.5 / aQ);
 		const T cM = t1 - t2, cP = t1 + t2;
 		const T c = (cM > cP ? cM : cP);
 		const T Vn = R_l - (2.0 / kGm1) * c;
@@ -306,7 +356,7 @@ __device__ __forceinline__ void euler_boundary_state(int bc, const T* WL, const 
 		return;
 	}
 	// Riemann: primitive variables of both sides
-	const T rho_l = WL[0], rho_l_inv = 1.0 / rho_l;
+	const T rho_l = WL[0], rho_l_inv = recip(rho_l);
 	T u_l[D], V2_l = 0.0, Vn_l = 0.0;
 #pragma unroll
 	for (int k = 0; k < D; ++k) {
@@ -324,8 +374,8 @@ __device__ __forceinline__ void euler_boundary_state(int bc, const T* WL, const 
 		Vn_r += n[k] * u_r[k];
 	}
 	const double p_r = kGm1 * (ext[D + 1] - 0.5 * rho_r * V2_r);
-	const T c_l = sqrt(kGamma * p_l * rho_l_inv);
-	const double c_r = ::sqrt(kGamma * p_r / rho_r);
+	const T c_l = root(kGamma * p_l * rho_l_inv);
+	const double c_r = root(kGamma * p_r / rho_r);
 	const T R_l = Vn_l + (2.0 / kGm1) * c_l;   // outgoing
 	const T R_r = Vn_r - (2.0 / kGm1) * c_r;   // incoming
 	const T Vn = 0.5 * (R_l + R_r), cc = 0.25 * kGm1 * (R_l - R_r);
@@ -401,7 +451,7 @@ struct NsPhys {
 template <int D, typename T>
 __device__ __forceinline__ void ns_viscous_sub(const T* W, const T (*G)[D + 2], const NsPhys& ph, T (*F)[D + 2])
 {
-	const T rho = W[0], E = W[D + 1], rho_inv = 1.0 / rho;
+	const T rho = W[0], E = W[D + 1], rho_inv = recip(rho);
 	T u[D], du[D][D], V2 = 0.0;
 #pragma unroll
 	for (int k = 0; k < D; ++k) {
@@ -416,7 +466,7 @@ __device__ __forceinline__ void ns_viscous_sub(const T* W, const T (*G)[D + 2], 
 	T mu = ph.mu;
 	if (ph.viscosity == kViscositySutherland) {
 		const T p = kGm1 * (E - 0.5 * rho * V2), Tt = p / (rho * ph.r_s);
-		mu = 0.08 * ph.mu / (1.0 + 112.0 / Tt) * sqrt(Tt);
+		mu = 0.08 * ph.mu / (1.0 + 112.0 / Tt) * root(Tt);
 	}
 	T div = 0.0;
 #pragma unroll

@@ -231,7 +231,7 @@ __device__ __forceinline__ int tp_face_node(int lf, int node)
 
 // Contravariant flux of W at a node with the w-weighted metric terms g.
 template <int D, int NV, int PDE>
-__device__ __forceinline__ void tp_flux(const TPParams& P, const double* W, const double* g, double (*fr)[NV])
+__device__ __forceinline__ void tp_flux(const double* b_adv, const double* W, const double* g, double (*fr)[NV])
 {
 	if constexpr (PDE == kEuler) {
 		euler_flux_ref<D>(W, g, fr);
@@ -242,8 +242,8 @@ __device__ __forceinline__ void tp_flux(const TPParams& P, const double* W, cons
 			double gb = 0.0;
 #pragma unroll
 			for (int i = 0; i < D; ++i)
-				gb += g[j * D + i] * P.b_adv[i];
-			fr[j][0] = gb * W[0];
+				gb = fma(g[j * D + i], b_adv[i], gb);
+			fr[j][0] = mul(gb, W[0]);
 		}
 	}
 }
@@ -260,19 +260,20 @@ __device__ __noinline__ void tp_pass_rolled(const double* in, double* out, const
 		double s = 0.0;
 #pragma unroll 1
 		for (int m = 0; m < Q; ++m)
-			s += M[a][m] * x[m * stride];
+			s = fma(M[a][m], x[m * stride], s);
 		out[k * N + node] = s;
 	}
 }
 
 // M (x) .. (x) M applied to the CTA's elements in block fixed point (FP64 passes for an element out of range): x holds
-// the node's values on entry and exit; buf and tmp NV N words per element, sx AEXP zeroed ints per element. STATE: x is
+// the node's values on entry and exit; buf and tmp NV N words per element, sx AEXP zeroed ints per element, stride_x ints apart. STATE: x is
 // a conserved state (fix_spread). All threads of the CTA must call it; buf is free again after the next barrier.
 template <int D, int Q, int NV, bool STATE>
 __device__ __forceinline__ void tp_apply_fix(double* x, double* buf, double* tmp, const FixW (*F)[kQMax], int sF,
-                                             const double (*M)[kQMax], int e, int node, bool active, int* sx)
+                                             const double (*M)[kQMax], int e, int node, bool active, int* sx,
+                                             int stride_x)
 {
-	constexpr int N = TPShape<D, Q>::N, XE = TPSmem<D, Q, NV>::AEXP, K = STATE ? XE : NV;
+	constexpr int N = TPShape<D, Q>::N, K = STATE ? TPSmem<D, Q, NV>::AEXP : NV;
 	int eb[K];
 #pragma unroll
 	for (int k = 0; k < NV; ++k)
@@ -281,16 +282,17 @@ __device__ __forceinline__ void tp_apply_fix(double* x, double* buf, double* tmp
 		eb[NV] = active ? fix_low(x[0]) : 0;
 		eb[NV + 1] = active ? fix_low(x[NV - 1]) : 0;
 	}
-	elem_max<N, K>(eb, e, active, sx, XE);
+	elem_max<N, K>(eb, e, active, sx, stride_x);
 	__syncthreads();
 	bool ok = true;
 	if (active) {
+		const int* se = sx + e * stride_x;
 		if constexpr (K > NV)
-			ok = fix_spread(sx[e * XE], sx[e * XE + NV]) && fix_spread(sx[e * XE + NV - 1], sx[e * XE + NV + 1]);
+			ok = fix_spread(se[0], se[NV]) && fix_spread(se[NV - 1], se[NV + 1]);
 #pragma unroll
 		for (int k = 0; k < NV; ++k) {
-			ok = ok && fix_in_range(sx[e * XE + k]);
-			eb[k] = fix_block(sx[e * XE + k]);
+			ok = ok && fix_in_range(se[k]);
+			eb[k] = fix_block(se[k]);
 		}
 #pragma unroll
 		for (int k = 0; k < NV; ++k) {
@@ -340,6 +342,240 @@ __device__ __forceinline__ void tp_apply_fix(double* x, double* buf, double* tmp
 	}
 }
 
+// The contractions of the volume term, shared by the uniform and the batched kernels: the node's state W and fluxes fr
+// are staged in su (NV N words) and sf (D NV N words) of its element, in block fixed point when the element is in range
+// (the return value), as doubles otherwise; eb receives the element's block exponents. sx: EXP zeroed ints per element,
+// `stride` ints apart. All threads of the CTA must call it; synchronises before it returns.
+template <int D, int Q, int NV>
+__device__ __forceinline__ bool tp_stage_volume(const double* W, const double (*fr)[NV], int e, int node, bool active,
+                                                double* su, double* sf, int* sx, int stride, int* eb)
+{
+	constexpr int N = TPShape<D, Q>::N, XE = TPSmem<D, Q, NV>::EXP, AE = TPSmem<D, Q, NV>::AEXP;
+	int x[XE];
+#pragma unroll
+	for (int k = 0; k < XE; ++k)
+		x[k] = 0;
+	if (active) {
+#pragma unroll
+		for (int k = 0; k < NV; ++k) {
+			x[k] = fix_exponent(W[k]);
+			int m = 0;
+#pragma unroll
+			for (int j = 0; j < D; ++j)
+				m = max(m, fix_exponent(fr[j][k]));
+			x[AE + k] = m;
+		}
+		if constexpr (AE > NV) {
+			x[NV] = fix_low(W[0]);
+			x[NV + 1] = fix_low(W[NV - 1]);
+		}
+	}
+	elem_max<N, XE>(x, e, active, sx, stride);
+	__syncthreads();
+	bool ok = true;
+	if (active) {
+		const int* se = sx + e * stride;
+		if constexpr (AE > NV)
+			ok = fix_spread(se[0], se[NV]) && fix_spread(se[NV - 1], se[NV + 1]);
+#pragma unroll
+		for (int k = 0; k < NV; ++k) {
+			ok = ok && fix_in_range(se[k]) && fix_in_range(se[AE + k]);
+			eb[k] = fix_block(se[k]);
+			eb[NV + k] = fix_block(se[AE + k]);
+		}
+		if (ok) {
+			int2* xu = reinterpret_cast<int2*>(su);
+			int2* xf = reinterpret_cast<int2*>(sf);
+#pragma unroll
+			for (int k = 0; k < NV; ++k) {
+				xu[k * N + node] = fix_pack(W[k], eb[k]);
+#pragma unroll
+				for (int j = 0; j < D; ++j)
+					xf[(j * NV + k) * N + node] = fix_pack(fr[j][k], eb[NV + k]);
+			}
+		} else {
+#pragma unroll
+			for (int k = 0; k < NV; ++k) {
+				su[k * N + node] = W[k];
+#pragma unroll
+				for (int j = 0; j < D; ++j)
+					sf[(j * NV + k) * N + node] = fr[j][k];
+			}
+		}
+	}
+	__syncthreads();
+	return ok;
+}
+
+// out[k] = sum_j Dgl_j^T (w fr_j) at the node.
+template <int D, int Q, int NV>
+__device__ __forceinline__ void tp_derivative(const TPOps* sops, const double* sf, const int* eb, bool ok, int node,
+                                              double* out)
+{
+	constexpr int N = TPShape<D, Q>::N;
+	if (ok) {
+		const int2* xf = reinterpret_cast<const int2*>(sf);
+		FixAcc acc[NV];
+#pragma unroll
+		for (int k = 0; k < NV; ++k)
+			acc[k] = {0, 0};
+#pragma unroll
+		for (int j = 0; j < D; ++j) {
+			const int stride = (j == 0 ? 1 : (j == 1 ? Q : Q * Q));
+			const int a = node_coord<Q>(node, j);
+			const int b0 = node - a * stride;
+#pragma unroll
+			for (int m = 0; m < Q; ++m) {
+				const FixW w = sops->fD[a][m];
+#pragma unroll
+				for (int k = 0; k < NV; ++k)
+					fix_mac(acc[k], w, xf[(j * NV + k) * N + b0 + m * stride]);
+			}
+		}
+#pragma unroll
+		for (int k = 0; k < NV; ++k)
+			out[k] = fix_to_double(fix_sum(acc[k]), fix_scale(eb[NV + k], sops->sD));
+	} else {
+#pragma unroll
+		for (int k = 0; k < NV; ++k)
+			out[k] = 0.0;
+#pragma unroll 1
+		for (int j = 0; j < D; ++j) {
+			const int stride = (j == 0 ? 1 : (j == 1 ? Q : Q * Q));
+			const int a = (node / stride) % Q;
+			const double* f = sf + j * NV * N + node - a * stride;
+#pragma unroll 1
+			for (int m = 0; m < Q; ++m)
+#pragma unroll
+				for (int k = 0; k < NV; ++k)
+					out[k] = fma(sops->Dgl[m][a], f[k * N + m * stride], out[k]);
+		}
+	}
+}
+
+// out[k] = the trace of the staged state at node t of local face lf.
+template <int D, int Q, int NV>
+__device__ __forceinline__ void tp_trace(const TPOps* sops, const double* su, const int* eb, bool ok, int lf, int t,
+                                         double* out)
+{
+	constexpr int N = TPShape<D, Q>::N;
+	int stride, base;
+	tp_face_line<D, Q>(lf, t, base, stride);
+	if (ok) {
+		const int2* xu = reinterpret_cast<const int2*>(su) + base;
+		FixW w[Q];
+#pragma unroll
+		for (int m = 0; m < Q; ++m)
+			w[m] = sops->fT[lf & 1][m];
+#pragma unroll
+		for (int k = 0; k < NV; ++k) {
+			FixAcc s = {0, 0};
+#pragma unroll
+			for (int m = 0; m < Q; ++m)
+				fix_mac(s, w[m], xu[k * N + m * stride]);
+			out[k] = fix_to_double(fix_sum(s), fix_scale(eb[k], sops->sT));
+		}
+	} else {
+#pragma unroll
+		for (int k = 0; k < NV; ++k)
+			out[k] = 0.0;
+#pragma unroll 1
+		for (int m = 0; m < Q; ++m)
+#pragma unroll
+			for (int k = 0; k < NV; ++k)
+				out[k] = fma(sops->lb[lf & 1][m], su[k * N + base + m * stride], out[k]);
+	}
+}
+
+// The lifting, shared likewise: fv holds the signed face terms of the element's face nodes node + r N (node index
+// lf NF + t), Rg the node's volume term; Rg becomes volume term + sum over the faces of E_lf^T (face terms). sa: NV NFT
+// words of the element, sx: NV zeroed ints per element. All threads of the CTA must call it; sa must not be written
+// before the next barrier.
+template <int D, int Q, int NV>
+__device__ __forceinline__ void tp_lift_sum(const TPOps* sops, const double (*fv)[NV], double* Rg, int e, int node,
+                                            bool active, double* sa, int* sx, int stride)
+{
+	constexpr int N = TPShape<D, Q>::N, NF = TPShape<D, Q>::NF, NFT = TPSmem<D, Q, NV>::NFT, NR = (NFT + N - 1) / N;
+	int eb[NV];
+#pragma unroll
+	for (int k = 0; k < NV; ++k)
+		eb[k] = 0;
+	if (active) {
+#pragma unroll
+		for (int k = 0; k < NV; ++k) {
+			eb[k] = fix_exponent(Rg[k]);
+#pragma unroll
+			for (int r = 0; r < NR; ++r)
+				if (node + r * N < NFT)
+					eb[k] = max(eb[k], fix_exponent(fv[r][k]));
+		}
+	}
+	elem_max<N, NV>(eb, e, active, sx, stride);
+	__syncthreads();
+	bool ok = true;
+	if (active) {
+#pragma unroll
+		for (int k = 0; k < NV; ++k) {
+			ok = ok && fix_in_range(sx[e * stride + k]);
+			eb[k] = fix_block(sx[e * stride + k]);
+		}
+#pragma unroll
+		for (int r = 0; r < NR; ++r) {
+			const int it = node + r * N;
+			if (it >= NFT)
+				break;
+#pragma unroll
+			for (int k = 0; k < NV; ++k)
+				if (ok)
+					reinterpret_cast<int2*>(sa)[k * NFT + it] = fix_pack(fv[r][k], eb[k]);
+				else
+					sa[k * NFT + it] = fv[r][k];
+		}
+	}
+	__syncthreads();
+	if (!active)
+		return;
+	if (ok) {
+		FixAcc acc[NV];
+		const FixW one = sops->fOne;
+#pragma unroll
+		for (int k = 0; k < NV; ++k) {
+			const int2 x = fix_pack(Rg[k], eb[k]);
+			acc[k] = {(long long)one.h * x.y, (long long)one.h * x.x};   // the weight 1 has no low limb
+		}
+#pragma unroll
+		for (int lf = 0; lf < 2 * D; ++lf) {
+			const FixW w = sops->fU[lf & 1][node_coord<Q>(node, lf >> 1)];
+			const int2* x = reinterpret_cast<const int2*>(sa) + lf * NF + tp_face_node<D, Q>(lf, node);
+#pragma unroll
+			for (int k = 0; k < NV; ++k)
+				fix_mac(acc[k], w, x[k * NFT]);
+		}
+#pragma unroll
+		for (int k = 0; k < NV; ++k)
+			Rg[k] = fix_to_double(fix_sum(acc[k]), fix_scale(eb[k], sops->sU));
+	} else {
+#pragma unroll 1
+		for (int lf = 0; lf < 2 * D; ++lf) {
+			const double l = sops->lb[lf & 1][node_coord<Q>(node, lf >> 1)];
+			const double* x = sa + lf * NF + tp_face_node<D, Q>(lf, node);
+#pragma unroll
+			for (int k = 0; k < NV; ++k)
+				Rg[k] = fma(l, x[k * NFT], Rg[k]);
+		}
+	}
+}
+
+// One SSP-RK3 stage of a value (solve_explicit.c:277-295), rounding written out.
+__device__ __forceinline__ double rk_update(int stage, double s, double s0, double dt, double R)
+{
+	if (stage == 0)
+		return mad(dt, R, s);
+	if (stage == 1)
+		return mul(0.25, mad(dt, R, mad(3.0, s0, s)));
+	return mul(1.0 / 3.0, mad(2.0, mad(dt, R, s), s0));
+}
+
 // Volume term of the CTA's E elements; per element PER_E doubles at base (su, st, sf at the start), sx the block
 // exponents. The flux is FP64; the derivative and the traces contract in block fixed point (dgpu_fix.cuh): 90 of the
 // 138 FP64 operations per node at q = 4 leave the FP64 pipe, which bounds the kernel.
@@ -369,7 +605,7 @@ __device__ __forceinline__ void tp_volume_body(const TPOps* sops, const TPParams
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
 				P.keep_coef[((size_t)v * NV + k) * N + node] = W[k];
-		tp_apply_fix<D, Q, NV, true>(W, su, st, sops->fB, sops->sB, sops->B, e, node, active, sx + S::E * XE);   // V u
+		tp_apply_fix<D, Q, NV, true>(W, su, st, sops->fB, sops->sB, sops->B, e, node, active, sx + S::E * XE, AE);   // V u
 		if (active && P.keep_gl)
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
@@ -377,135 +613,31 @@ __device__ __forceinline__ void tp_volume_body(const TPOps* sops, const TPParams
 	}
 
 	double fr[D][NV];
-	int eb[XE];
-#pragma unroll
-	for (int k = 0; k < XE; ++k)
-		eb[k] = 0;
 	if (active) {
 		double g[D * D];
 #pragma unroll
 		for (int c = 0; c < D * D; ++c)
 			g[c] = P.gmet[((size_t)v * D * D + c) * N + node];
-		tp_flux<D, NV, PDE>(P, W, g, fr);
-#pragma unroll
-		for (int k = 0; k < NV; ++k) {
-			eb[k] = fix_exponent(W[k]);
-			int m = 0;
-#pragma unroll
-			for (int j = 0; j < D; ++j)
-				m = max(m, fix_exponent(fr[j][k]));
-			eb[AE + k] = m;
-		}
-		if constexpr (AE > NV) {
-			eb[NV] = fix_low(W[0]);
-			eb[NV + 1] = fix_low(W[NV - 1]);
-		}
+		tp_flux<D, NV, PDE>(P.b_adv, W, g, fr);
 	}
-	elem_max<N, XE>(eb, e, active, sx, XE);
-	__syncthreads();
-	bool ok = true;
-	if (active) {
-		if constexpr (AE > NV)
-			ok = fix_spread(sx[e * XE], sx[e * XE + NV]) && fix_spread(sx[e * XE + NV - 1], sx[e * XE + NV + 1]);
-#pragma unroll
-		for (int k = 0; k < NV; ++k) {
-			ok = ok && fix_in_range(sx[e * XE + k]) && fix_in_range(sx[e * XE + AE + k]);
-			eb[k] = fix_block(sx[e * XE + k]);
-			eb[AE + k] = fix_block(sx[e * XE + AE + k]);
-		}
-		if (ok) {
-			int2* xu = reinterpret_cast<int2*>(su);
-			int2* xf = reinterpret_cast<int2*>(sf);
-#pragma unroll
-			for (int k = 0; k < NV; ++k) {
-				xu[k * N + node] = fix_pack(W[k], eb[k]);
-#pragma unroll
-				for (int j = 0; j < D; ++j)
-					xf[(j * NV + k) * N + node] = fix_pack(fr[j][k], eb[AE + k]);
-			}
-		} else {
-#pragma unroll
-			for (int k = 0; k < NV; ++k) {
-				su[k * N + node] = W[k];
-#pragma unroll
-				for (int j = 0; j < D; ++j)
-					sf[(j * NV + k) * N + node] = fr[j][k];
-			}
-		}
-	}
-	__syncthreads();
+	int eb[2 * NV];
+	const bool ok = tp_stage_volume<D, Q, NV>(W, fr, e, node, active, su, sf, sx, XE, eb);
 	if (!active)
 		return;
-
-	// volume term in GL space: sum_j Dgl_j^T (w fr_j)
-	if (ok) {
-		const int2* xf = reinterpret_cast<const int2*>(sf);
-		FixAcc acc[NV];
+	double out[NV];
+	tp_derivative<D, Q, NV>(sops, sf, eb, ok, node, out);
 #pragma unroll
-		for (int k = 0; k < NV; ++k)
-			acc[k] = {0, 0};
-#pragma unroll
-		for (int j = 0; j < D; ++j) {
-			const int stride = (j == 0 ? 1 : (j == 1 ? Q : Q * Q));
-			const int a = node_coord<Q>(node, j);
-			const int b0 = node - a * stride;
-#pragma unroll
-			for (int m = 0; m < Q; ++m) {
-				const FixW w = sops->fD[a][m];
-#pragma unroll
-				for (int k = 0; k < NV; ++k)
-					fix_mac(acc[k], w, xf[(j * NV + k) * N + b0 + m * stride]);
-			}
-		}
-#pragma unroll
-		for (int k = 0; k < NV; ++k)
-			P.vol_gl[((size_t)v * NV + k) * N + node] = fix_to_double(fix_sum(acc[k]), fix_scale(eb[AE + k], sops->sD));
-	} else {
-#pragma unroll 1
-		for (int k = 0; k < NV; ++k) {
-			double acc = 0.0;
-#pragma unroll 1
-			for (int j = 0; j < D; ++j) {
-				const int stride = (j == 0 ? 1 : (j == 1 ? Q : Q * Q));
-				const int a = (node / stride) % Q;
-				const double* f = sf + (j * NV + k) * N + node - a * stride;
-				for (int m = 0; m < Q; ++m)
-					acc += sops->Dgl[m][a] * f[m * stride];
-			}
-			P.vol_gl[((size_t)v * NV + k) * N + node] = acc;
-		}
-	}
-
+	for (int k = 0; k < NV; ++k)
+		P.vol_gl[((size_t)v * NV + k) * N + node] = out[k];
 	// traces of ug on the 2D local faces
 	for (int it = node; it < 2 * D * NF; it += N) {
-		const int lf = it / NF, t = it % NF, side = lf & 1;
-		int stride_n, base_n;
-		tp_face_line<D, Q>(lf, t, base_n, stride_n);
+		const int lf = it / NF, t = it % NF;
 		const int fs = P.vol_face[(size_t)v * 2 * D + lf];
 		double* dst = P.traces + (size_t)fs * NV * NF;
-		if (ok) {
-			const int2* xu = reinterpret_cast<const int2*>(su) + base_n;
-			FixW w[Q];
+		tp_trace<D, Q, NV>(sops, su, eb, ok, lf, t, out);
 #pragma unroll
-			for (int m = 0; m < Q; ++m)
-				w[m] = sops->fT[side][m];
-#pragma unroll
-			for (int k = 0; k < NV; ++k) {
-				FixAcc s = {0, 0};
-#pragma unroll
-				for (int m = 0; m < Q; ++m)
-					fix_mac(s, w[m], xu[k * N + m * stride_n]);
-				dst[k * NF + t] = fix_to_double(fix_sum(s), fix_scale(eb[k], sops->sT));
-			}
-		} else {
-#pragma unroll 1
-			for (int k = 0; k < NV; ++k) {
-				double s = 0.0;
-				for (int m = 0; m < Q; ++m)
-					s += sops->lb[side][m] * su[k * N + base_n + m * stride_n];
-				dst[k * NF + t] = s;
-			}
-		}
+		for (int k = 0; k < NV; ++k)
+			dst[k * NF + t] = out[k];
 	}
 }
 
@@ -711,16 +843,10 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, const TPParams& 
 	for (int i = tid; i < S::E * TPSmem<D, Q, NV>::LEXP; i += blockDim.x)
 		sx[i] = 0;
 	double fv[NR][NV], Rg[NV];   // the face terms this thread stages; GL-space residual R_gl of this node
-	int eb[NV];
-#pragma unroll
-	for (int k = 0; k < NV; ++k)
-		eb[k] = 0;
 	if (active) {
 #pragma unroll
-		for (int k = 0; k < NV; ++k) {
+		for (int k = 0; k < NV; ++k)
 			Rg[k] = P.vol_gl[((size_t)v * NV + k) * N + node];
-			eb[k] = fix_exponent(Rg[k]);
-		}
 #pragma unroll
 		for (int r = 0; r < NR; ++r) {
 			const int it = node + r * N;
@@ -736,73 +862,20 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, const TPParams& 
 				// side 0: rhs -= E^T nnf ; side 1: rhs -= E^T (-nnf)   (compute_face_rlhs_T.c:297-310)
 				const double x = src[k * NF + idx];
 				fv[r][k] = s == 0 ? -x : x;
-				eb[k] = max(eb[k], fix_exponent(x));
 			}
 		}
 	}
-	__syncthreads();   // sx is zero; the lift below reads sops written by other warps
-	elem_max<N, NV>(eb, e, active, sx, NV);
-	__syncthreads();
-	bool ok = true;
+	__syncthreads();   // sx is zero; sops is written by other warps
+	tp_lift_sum<D, Q, NV>(sops, fv, Rg, e, node, active, sa, sx, NV);
 	if (active) {
-#pragma unroll
-		for (int k = 0; k < NV; ++k) {
-			ok = ok && fix_in_range(sx[e * NV + k]);
-			eb[k] = fix_block(sx[e * NV + k]);
-		}
-#pragma unroll
-		for (int r = 0; r < NR; ++r) {
-			const int it = node + r * N;
-			if (it >= NFT)
-				break;
-#pragma unroll
-			for (int k = 0; k < NV; ++k)
-				if (ok)
-					reinterpret_cast<int2*>(sa)[k * NFT + it] = fix_pack(fv[r][k], eb[k]);
-				else
-					sa[k * NFT + it] = fv[r][k];
-		}
-	}
-	__syncthreads();
-
-	if (active) {
-		if (ok) {
-			FixAcc acc[NV];
-			const FixW one = sops->fOne;
-#pragma unroll
-			for (int k = 0; k < NV; ++k) {
-				const int2 x = fix_pack(Rg[k], eb[k]);
-				acc[k] = {(long long)one.h * x.y, (long long)one.h * x.x};   // the weight 1 has no low limb
-			}
-#pragma unroll
-			for (int lf = 0; lf < 2 * D; ++lf) {
-				const FixW w = sops->fU[lf & 1][node_coord<Q>(node, lf >> 1)];
-				const int2* x = reinterpret_cast<const int2*>(sa) + lf * NF + tp_face_node<D, Q>(lf, node);
-#pragma unroll
-				for (int k = 0; k < NV; ++k)
-					fix_mac(acc[k], w, x[k * NFT]);
-			}
-#pragma unroll
-			for (int k = 0; k < NV; ++k)
-				Rg[k] = fix_to_double(fix_sum(acc[k]), fix_scale(eb[k], sops->sU));
-		} else {
-#pragma unroll 1
-			for (int lf = 0; lf < 2 * D; ++lf) {
-				const double l = sops->lb[lf & 1][node_coord<Q>(node, lf >> 1)];
-				const double* x = sa + lf * NF + tp_face_node<D, Q>(lf, node);
-#pragma unroll
-				for (int k = 0; k < NV; ++k)
-					Rg[k] += l * x[k * NFT];
-			}
-		}
 		const double iw = P.inv_wJ[(size_t)v * N + node];
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
-			Rg[k] *= iw;
+			Rg[k] = mul(Rg[k], iw);
 		if (P.source)
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
-				Rg[k] += P.source[((size_t)v * NV + k) * N + node];
+				Rg[k] = add(Rg[k], P.source[((size_t)v * NV + k) * N + node]);
 	}
 	__syncthreads();   // the face terms are read; sa, sb, sc are reused
 
@@ -815,7 +888,7 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, const TPParams& 
 		for (int k = 0; k < NV; ++k)
 			R[k] = Rg[k];
 		tp_apply_fix<D, Q, NV, false>(R, sa, sb, sops->fBinv, sops->sBinv, sops->Binv, e, node, active,
-		                              sx + 2 * S::E * NV);
+		                              sx + 2 * S::E * NV, AE);
 		if (active) {
 #pragma unroll
 			for (int k = 0; k < NV; ++k) {
@@ -849,16 +922,9 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, const TPParams& 
 #pragma unroll
 			for (int k = 0; k < NV; ++k) {
 				const double s = rk.u[o + (size_t)k * N];
-				if (rk.stage == 0) {
+				if (rk.stage == 0)
 					rk.u0[o + (size_t)k * N] = s;
-					snew[k] = s + rk.dt * Rg[k];
-				} else if (rk.stage == 1) {
-					const double sp = rk.u0[o + (size_t)k * N];
-					snew[k] = (1.0 / 4.0) * (3.0 * sp + s + rk.dt * Rg[k]);
-				} else {
-					const double sp = rk.u0[o + (size_t)k * N];
-					snew[k] = (1.0 / 3.0) * (sp + 2.0 * s + 2.0 * rk.dt * Rg[k]);
-				}
+				snew[k] = rk_update(rk.stage, s, rk.stage == 0 ? s : rk.u0[o + (size_t)k * N], rk.dt, Rg[k]);
 			}
 		}
 		if (rk.positivity) {
@@ -929,7 +995,7 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, const TPParams& 
 			// the new state's GLL coefficients: V^-1 of the GL values (D passes of Binv)
 			__syncthreads();   // sa/sb/sc are free again
 			tp_apply_fix<D, Q, NV, true>(snew, sa, sb, sops->fBinv, sops->sBinv, sops->Binv, e, node, active,
-			                             sx + S::E * (2 * NV + AE));
+			                             sx + S::E * (2 * NV + AE), AE);
 			if (active)
 #pragma unroll
 				for (int k = 0; k < NV; ++k) {
@@ -996,7 +1062,8 @@ tp_convert_kernel(const __grid_constant__ TPOps ops, int n_vol, const double* __
 		sx[i] = 0;
 	__syncthreads();
 	tp_apply_fix<D, Q, NV, true>(x, base + e * PER_E, base + e * PER_E + NV * N, TO_GL ? sops->fB : sops->fBinv,
-	                       TO_GL ? sops->sB : sops->sBinv, TO_GL ? sops->B : sops->Binv, e, node, active, sx);
+	                       TO_GL ? sops->sB : sops->sBinv, TO_GL ? sops->B : sops->Binv, e, node, active, sx,
+	                             TPSmem<D, Q, NV>::AEXP);
 	if (active)
 #pragma unroll
 		for (int k = 0; k < NV; ++k) {
