@@ -782,6 +782,24 @@ void set_group_E(dgpu_batch* c, int g, int E)
 		c->hgroups[c->gl[g].idx].E = E;
 }
 
+// Elements per CTA of the per-group kernels. A large group fills its CTAs (256 nodes); a group too small to give every
+// SM two of those is split further, down to a warp of a QUAD/HEX group or one dense volume: its kernels are chains
+// of dependent steps, so idle SMs cost more than half-empty CTAs.
+void default_tiles(dgpu_batch* c)
+{
+	for (int g = 0; g < c->n_all; ++g) {
+		const int n_vol = c->group_n_vol(g);
+		int E = c->gl[g].E_max, N = 32;
+		if (!c->gl[g].dense) {
+			const int q = c->hgroups[c->gl[g].idx].q;
+			N = c->d == 2 ? q * q : q * q * q;
+		}
+		while (E > 1 && n_vol < E * 2 * 152 && (E / 2) * N >= 32)
+			E /= 2;
+		set_group_E(c, g, E);
+	}
+}
+
 int type_faces(int t)
 {
 	return t == DGPU_TRI ? 3 : (t == DGPU_TET ? 4 : (t == DGPU_HEX ? 6 : (t == DGPU_QUAD ? 4 : 5)));
@@ -793,6 +811,118 @@ struct GroupIn {
 	const dgpu_tp_operators* tp;
 	const dgpu_dense_operators* dn;
 };
+
+template <typename T>
+cudaError_t upload_vec(T** dst, const std::vector<T>& src);
+
+// Uploads an operator in fixed point, entry (i, j) of `rows` x `cols` row-major from w, transposed or not.
+cudaError_t upload_fix(dgpu_batch* c, const double* w, int rows, int cols, bool transposed, int s, const FixW** out)
+{
+	std::vector<FixW> x((size_t)rows * cols);
+	for (int i = 0; i < rows; ++i)
+		for (int j = 0; j < cols; ++j)
+			x[transposed ? (size_t)j * rows + i : (size_t)i * cols + j] = fix_entry(w[(size_t)i * cols + j], s);
+	FixW* d = nullptr;
+	const cudaError_t e = upload_vec(&d, x);
+	if (e == cudaSuccess) {
+		c->dense_bufs.push_back(d);
+		*out = d;
+	}
+	return e;
+}
+
+// Largest row sum of |w| (column sum when by_col), and largest entry.
+double abs_sum(const double* w, int rows, int cols, bool by_col, double* mx)
+{
+	std::vector<double> s(by_col ? cols : rows, 0.0);
+	for (int i = 0; i < rows; ++i)
+		for (int j = 0; j < cols; ++j) {
+			const double a = fabs(w[(size_t)i * cols + j]);
+			s[by_col ? j : i] += a;
+			*mx = std::max(*mx, a);
+		}
+	return *std::max_element(s.begin(), s.end());
+}
+
+// Scale of an operator of fix_dot: |W| < 2^61 and sum |W| <= 2^66.
+int dense_shift(double sum, double mx) { return fix_shift(sum, 2.0 * mx, 66); }
+
+// The fixed-point operators of a dense group (dgpu_fix.cuh), each at the largest scale its sums allow.
+cudaError_t upload_fix_ops(dgpu_batch* c, const dgpu_dense_operators* op, int d, const std::vector<double>& Minv,
+                           const std::vector<double>& fops, const std::vector<long long>& foff, DGroup* G)
+{
+	const int nvs = op->n_vs, nvc = op->n_vc;
+	cudaError_t e;
+	double m = 0.0;
+	G->s_cv0 = dense_shift(abs_sum(op->cv0_vs_vc, nvc, nvs, false, &m), m);
+	if ((e = upload_fix(c, op->cv0_vs_vc, nvc, nvs, true, G->s_cv0, &G->xcv0)))
+		return e;
+	m = 0.0;
+	G->s_cv1 = dense_shift(abs_sum(op->cv1_vs_vc, d * nvc, nvs, true, &m), m);
+	if ((e = upload_fix(c, op->cv1_vs_vc, d * nvc, nvs, false, G->s_cv1, &G->xcv1)))
+		return e;
+	m = 0.0;
+	G->s_minv = dense_shift(abs_sum(Minv.data(), nvs, nvs, false, &m), m);
+	if ((e = upload_fix(c, Minv.data(), nvs, nvs, true, G->s_minv, &G->xminv)))
+		return e;
+	// face operators: one scale for the traces (rows) and the lifting (columns, every face's largest)
+	double mf = 0.0, trace = 0.0, lift = 0.0;
+	for (int lf = 0; lf < op->n_lf; ++lf) {
+		double col = 0.0;
+		for (int o = 0; o < op->n_ord; ++o)
+			for (int pf = 1; pf < kQMax; ++pf) {
+				const int k = (lf * op->n_ord + o) * kQMax + pf;
+				if (!op->cv0_vs_fc[k] || op->n_fc[k] < 1)
+					continue;
+				trace = std::max(trace, abs_sum(op->cv0_vs_fc[k], op->n_fc[k], nvs, false, &mf));
+				col = std::max(col, abs_sum(op->cv0_vs_fc[k], op->n_fc[k], nvs, true, &mf));
+			}
+		lift += col;
+	}
+	G->s_f = dense_shift(std::max(trace, lift), mf);
+	std::vector<FixW> xT(fops.size()), xL(fops.size());
+	for (int lf = 0; lf < op->n_lf; ++lf)
+		for (int o = 0; o < op->n_ord; ++o)
+			for (int pf = 1; pf < kQMax; ++pf) {
+				const long long off = foff[(lf * op->n_ord + o) * (kQMax + 1) + pf + 1];
+				const int n = op->n_fc[(lf * op->n_ord + o) * kQMax + pf];
+				if (off < 0)
+					continue;
+				for (int i = 0; i < n; ++i)
+					for (int a = 0; a < nvs; ++a) {
+						const FixW w = fix_entry(fops[off + (size_t)i * nvs + a], G->s_f);
+						xL[off + (size_t)i * nvs + a] = w;
+						xT[off + (size_t)a * n + i] = w;
+					}
+			}
+	FixW *dT = nullptr, *dL = nullptr;
+	if ((e = upload_vec(&dT, xT)))
+		return e;
+	c->dense_bufs.push_back(dT);
+	if ((e = upload_vec(&dL, xL)))
+		return e;
+	c->dense_bufs.push_back(dL);
+	G->xfT = dT;
+	G->xfL = dL;
+	if (!G->prism)
+		return cudaSuccess;
+	const int ntc = G->n_tvc, ntv = G->n_tvs, nlc = G->n_lvc, nlv = G->n_lvs;
+	double mt = 0.0, ml = 0.0, mt1 = 0.0, ml1 = 0.0;
+	const double t0 = std::max(abs_sum(op->tri_cv0, ntc, ntv, false, &mt), abs_sum(op->tri_cv0, ntc, ntv, true, &mt));
+	const double l0 = std::max(abs_sum(op->line_cv0, nlc, nlv, false, &ml), abs_sum(op->line_cv0, nlc, nlv, true, &ml));
+	G->s_t0 = fix_shift(t0, mt, 62);
+	G->s_l0 = fix_shift(l0, ml, 62);
+	// the last sum takes tri1 products of the x and y parts at s_t1 and line1 products of the z part at s_t1 + s_l0 - s_t0
+	const double r = ldexp(1.0, G->s_l0 - G->s_t0);
+	const double t1 = abs_sum(op->tri_cv1, 2 * ntc, ntv, true, &mt1), l1 = abs_sum(op->line_cv1, nlc, nlv, true, &ml1);
+	G->s_t1 = dense_shift(t1 + r * l1, std::max(mt1, r * ml1));
+	if ((e = upload_fix(c, op->tri_cv0, ntc, ntv, false, G->s_t0, &G->xt0)) ||
+	    (e = upload_fix(c, op->tri_cv0, ntc, ntv, true, G->s_t0, &G->xt0T)) ||
+	    (e = upload_fix(c, op->tri_cv1, 2 * ntc, ntv, false, G->s_t1, &G->xt1)) ||
+	    (e = upload_fix(c, op->line_cv0, nlc, nlv, false, G->s_l0, &G->xl0)))
+		return e;
+	return upload_fix(c, op->line_cv1, nlc, nlv, false, G->s_t1 + G->s_l0 - G->s_t0, &G->xl1);
+}
 
 dgpu_status create_impl(const dgpu_physics* phys, const std::vector<GroupIn>& gin, const int* vol_group,
                         const dgpu_mesh* mesh, const int* face_ord, dgpu_batch** out)
@@ -943,7 +1073,11 @@ dgpu_status create_impl(const dgpu_physics* phys, const std::vector<GroupIn>& gi
 			G.n_lf = op->n_lf;
 			G.n_ord = op->n_ord;
 			G.vol_per_e = DSmem::vol(nv, G.n_vs, G.n_vc);
-			G.lift_per_e = DSmem::lift(nv, G.n_vs);
+			G.nff_max = 1;
+			for (int k = 0; k < op->n_lf * op->n_ord * kQMax; ++k)
+				if (op->cv0_vs_fc[k])
+					G.nff_max = std::max(G.nff_max, op->n_fc[k]);
+			G.lift_per_e = DSmem::lift(nv, G.n_vs, G.n_lf, G.nff_max);
 			if (op->elem_type == DGPU_WEDGE && op->tri_cv0 && op->tri_cv1 && op->line_cv0 && op->line_cv1) {
 				const int ntv = op->n_tri_vs, ntc = op->n_tri_vc, nlv = op->n_line_vs, nlc = op->n_line_vc;
 				if (ntv < 1 || ntc < 1 || nlv < 1 || nlc < 1 || ntv * nlv != op->n_vs || ntc * nlc != op->n_vc)
@@ -971,18 +1105,20 @@ dgpu_status create_impl(const dgpu_physics* phys, const std::vector<GroupIn>& gi
 							}
 				if (!(diff <= 1e-12 * scale))
 					return reject(DGPU_ERR_INVALID_ARGUMENT, "the WEDGE factors do not reproduce the dense operators");
-				G.prism = 1;
+				// longer factors (no cubature in use has them) run as dense operators
+				G.prism = std::max(std::max(ntv, ntc), std::max(nlv, nlc)) <= 32 ? 1 : 0;
 				G.n_tvs = ntv;
 				G.n_tvc = ntc;
 				G.n_lvs = nlv;
 				G.n_lvc = nlc;
-				G.vol_per_e += DSmem::prism_tmp(nv, ntv, ntc, nlv, nlc);
+				if (G.prism)
+					G.vol_per_e += DSmem::prism_tmp(nv, ntv, ntc, nlv, nlc);
 			}
 			G.E = std::max(1, 256 / op->n_vc);
-			while (G.E > 1 && (size_t)G.E * G.vol_per_e * 8 > 96 * 1024)
+			while (G.E > 1 && (size_t)G.E * std::max(G.vol_per_e, G.lift_per_e) * 8 > 96 * 1024)
 				G.E /= 2;
 			G.E_fused = G.E;
-			if ((size_t)G.vol_per_e * 8 > 200 * 1024)
+			if ((size_t)std::max(G.vol_per_e, G.lift_per_e) * 8 > 200 * 1024)
 				return reject(DGPU_ERR_UNSUPPORTED, "dense operator set too large for one volume per CTA");
 		}
 	}
@@ -1401,6 +1537,7 @@ dgpu_status create_impl(const dgpu_physics* phys, const std::vector<GroupIn>& gi
 			G.ccSB0f = d_sbf;
 			G.pos_err = (float)(2.0 * (nvs + 2) * ldexp(1.0, -23) * row_max);
 		}
+		B_TRY(upload_fix_ops(c, op, d, Minv, fops, foff, &G));
 		G.cv0 = d_cv0;
 		G.cv1 = d_cv1;
 		G.minv = d_minv;
@@ -1445,9 +1582,11 @@ dgpu_status create_impl(const dgpu_physics* phys, const std::vector<GroupIn>& gi
 		B_TRY(upload_vec(&c->d_fext, fext));
 	}
 	B_TRY(bind(c));
-	if (c->navier_stokes)   // bind set every group's E_ns
-		B_TRY(cudaMemcpy(c->d_groups, c->hgroups.data(), c->hgroups.size() * sizeof(BGroup), cudaMemcpyHostToDevice));
 #undef B_TRY
+	default_tiles(c);
+	const dgpu_status ts = upload_group_tiles(c);   // bind set every group's E_ns
+	if (ts != DGPU_OK)
+		return reject(ts, c->err);
 	*out = c;
 	return DGPU_OK;
 }

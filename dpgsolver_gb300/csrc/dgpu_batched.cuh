@@ -60,6 +60,15 @@ struct DGroup {
 	const double* ccBS0;        // n_vs x n_vs: Bezier -> coefficients
 	const float* ccSB0f;        // ccSB0 in FP32 (the limiter's pre-filter)
 	float pos_err;              // bound on |b_fp32 - b| / max |s| of the pre-filter's Bezier coefficients
+	// Fixed-point forms (dgpu_fix.cuh), W = w 2^s, in the order the kernels' lanes read them:
+	const FixW* xcv0;           // [n_vs][n_vc], s_cv0
+	const FixW* xcv1;           // [D][n_vc][n_vs], s_cv1 (summed over j and r)
+	const FixW* xfT;            // face operators as trace operators: per table entry [n_vs][n_fc], s_f
+	const FixW* xfL;            // ... as lifting operators: [n_fc][n_vs], s_f (summed over the faces)
+	const FixW* xminv;          // [a][m], s_minv
+	const FixW *xt0, *xt0T, *xt1, *xl0, *xl1;   // WEDGE factors: tri0 [rt][t] and [t][rt], tri1, line0, line1
+	int s_cv0, s_cv1, s_f, s_minv, s_t0, s_l0, s_t1;   // s_l1 = s_t1 + s_l0 - s_t0 (one sum)
+	int nff_max;                // face nodes of the group's largest face
 };
 
 struct BParams {

@@ -12,6 +12,10 @@
 // One CTA handles E volumes of one group; every phase maps one thread to one output row of one volume (all
 // variables per thread), reading the operators through the L1 cache (they are shared by every CTA of the group)
 // and the volume's state and fluxes from shared memory. The state stays in coefficient space between stages.
+//
+// The contractions run in block fixed point (dgpu_fix.cuh): as FP64 sums they were chains of 35 to 400 operations of 64
+// cycles each, which bounded these kernels at every size. The blocks are one volume's values of one variable. A volume
+// whose blocks leave the fixed-point range (Inf, NaN, huge values) takes FP64 loops in the same phases.
 #pragma once
 
 #include "dgpu_batched.cuh"
@@ -19,40 +23,138 @@
 namespace dgpu {
 
 struct DSmem {
-	// doubles per element: state (NV n_vs), fluxes (D NV n_vc) and, for a factorised WEDGE, the partial sums of
-	// the sum-factorised contractions; the lift keeps its rhs (NV n_vs)
-	static __host__ __device__ int vol(int nv, int n_vs, int n_vc) { return nv * n_vs + 3 * nv * n_vc; }
+	// doubles per element: state (NV n_vs), fluxes (D NV n_vc), for a factorised WEDGE the partial sums of the
+	// sum-factorised contractions (factors of at most 32 terms, for fix_line's accumulators), and two sets of block exponents; the lift keeps the face terms, its rhs and the state
+	static __host__ __device__ int vol(int nv, int n_vs, int n_vc) { return nv * n_vs + 3 * nv * n_vc + nv + 1; }
 	static __host__ __device__ int prism_tmp(int nv, int n_tvs, int n_tvc, int n_lvs, int n_lvc)
 	{
 		return nv * (2 * n_lvs * n_tvc + n_lvc * n_tvs);
 	}
-	static __host__ __device__ int lift(int nv, int n_vs) { return 2 * nv * n_vs + 2; }
+	static __host__ __device__ int lift_faces(int nv, int n_lf, int nff_max) { return nv * n_lf * nff_max; }
+	static __host__ __device__ int lift(int nv, int n_vs, int n_lf, int nff_max)
+	{
+		return 2 * nv * n_vs + 2 + lift_faces(nv, n_lf, nff_max) + nv + 1;
+	}
 };
 
-// Traces of the CTA's volumes (state in shared memory) at each face's canonical nodes.
+// ---- blocks: len values of each of NV variables, contiguous per variable, at doubles `off` of an element ----
+// Their largest exponents into the element's ints at double xo, from int `slot`; one warp per (element, variable).
 template <int NV>
-__device__ void dtraces(const BParams& P, const DGroup& G, int e0, int n_here, const double* smem, int PER_E)
+__device__ __forceinline__ void blk_max(double* smem, int PER_E, int n_here, int off, int len, int xo, int slot)
 {
-	const int nvs = G.n_vs;
-	for (int it = threadIdx.x; it < n_here * G.n_lf * kQMax * kQMax; it += blockDim.x) {
-		const int i = it % (kQMax * kQMax), el = it / (kQMax * kQMax), lf = el % G.n_lf, e = el / G.n_lf;
+	const int lane = threadIdx.x & 31;
+	for (int p = threadIdx.x >> 5; p < n_here * NV; p += blockDim.x >> 5) {
+		const int e = p / NV, k = p % NV;
+		const double* x = smem + e * PER_E + off + k * len;
+		int m = 0;
+		for (int i = lane; i < len; i += 32)
+			m = max(m, fix_exponent(x[i]));
+		m = __reduce_max_sync(0xffffffffu, m);
+		if (lane == 0)
+			reinterpret_cast<int*>(smem + e * PER_E + xo)[slot + k] = m;
+	}
+}
+
+template <int NV>
+__device__ __forceinline__ bool blk_ok(const double* smem, int PER_E, int e, int xo, int slot)
+{
+	const int* x = reinterpret_cast<const int*>(smem + e * PER_E + xo) + slot;
+	bool ok = true;
+#pragma unroll
+	for (int k = 0; k < NV; ++k)
+		ok = ok && fix_in_range(x[k]);
+	return ok;
+}
+
+// The values packed in place, for the elements in range.
+template <int NV>
+__device__ __forceinline__ void blk_pack(double* smem, int PER_E, int n_here, int off, int len, int xo, int slot)
+{
+	const int lane = threadIdx.x & 31;
+	for (int p = threadIdx.x >> 5; p < n_here * NV; p += blockDim.x >> 5) {
+		const int e = p / NV, k = p % NV;
+		if (!blk_ok<NV>(smem, PER_E, e, xo, slot))
+			continue;
+		const int eb = fix_block(reinterpret_cast<const int*>(smem + e * PER_E + xo)[slot + k]);
+		double* x = smem + e * PER_E + off + k * len;
+		for (int i = lane; i < len; i += 32)
+			reinterpret_cast<int2*>(x)[i] = fix_pack(x[i], eb);
+	}
+}
+
+__device__ __forceinline__ FixW ldg_fix(const FixW* p)
+{
+	const int2 w = __ldg(reinterpret_cast<const int2*>(p));
+	return FixW{w.x, w.y};
+}
+
+// acc[k] += sum_i op[i so] x[k len + i sx], i < n: sums of any length. Their operators are scaled to |W| < 2^61 and
+// sum |W| <= 2^66 (a row of hundreds of terms scaled by its sum alone would keep too few bits of each entry); the low
+// accumulator is folded into the high one every 16 products, exactly, which keeps it below 2^63, and leaves
+// 0 <= m < 2^30.
+template <int NV>
+__device__ __forceinline__ void fix_dot(FixAcc* acc, const FixW* op, int so, const int2* x, int len, int sx, int n)
+{
+	for (int i0 = 0; i0 < n; i0 += 16) {
+		const int i1 = min(n, i0 + 16);
+#pragma unroll 4
+		for (int i = i0; i < i1; ++i) {
+			const FixW w = ldg_fix(op + (long long)i * so);
+#pragma unroll
+			for (int k = 0; k < NV; ++k)
+				fix_mac(acc[k], w, x[k * len + i * sx]);
+		}
+#pragma unroll
+		for (int k = 0; k < NV; ++k) {
+			acc[k].h += acc[k].m >> 30;
+			acc[k].m &= (1ll << 30) - 1;
+		}
+	}
+}
+
+// The value of a folded sum (block eb, operator scale s).
+__device__ __forceinline__ double fix_dot_value(const FixAcc& a, int eb, int s)
+{
+	const bool big = (unsigned long long)(a.h + (1ll << 58)) >> 59;   // |a.h| >= 2^58: its own unit is fine enough
+	const long long r = big ? a.h : a.h * 8 + (a.m >> 27);
+	return fix_to_double(r, fix_scale(eb, s) + (big ? 3 : 0));
+}
+
+// Traces of the CTA's volumes (state in shared memory at 0) at each face's canonical nodes.
+template <int NV>
+__device__ void dtraces(const BParams& P, const DGroup& G, int e0, int n_here, const double* smem, int PER_E, int xo)
+{
+	const int nvs = G.n_vs, nfm = G.nff_max;
+	for (int it = threadIdx.x; it < n_here * G.n_lf * nfm; it += blockDim.x) {
+		const int i = it % nfm, el = it / nfm, lf = el % G.n_lf, e = el / G.n_lf;
 		const long long v = G.elem0 + e0 + e;
 		const int4 fd = P.elf[v * kMaxLf + lf];
 		const long long fb = P.fbase[fd.x];
 		const int nff = (int)(P.fbase[fd.x + 1] - fb);
 		if (i >= nff)
 			continue;
-		const double* op = G.fops + G.fop_off[(lf * G.n_ord + fd.w) * (kQMax + 1) + fd.z] + (long long)i * nvs;
+		const long long o = G.fop_off[(lf * G.n_ord + fd.w) * (kQMax + 1) + fd.z];
 		const double* su = smem + e * PER_E;
 		double W[NV];
-#pragma unroll
-		for (int k = 0; k < NV; ++k)
-			W[k] = 0.0;
-		for (int m = 0; m < nvs; ++m) {
-			const double c = __ldg(op + m);
+		if (blk_ok<NV>(smem, PER_E, e, xo, 0)) {
+			FixAcc acc[NV];
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
-				W[k] += c * su[k * nvs + m];
+				acc[k] = {0, 0};
+			fix_dot<NV>(acc, G.xfT + o + i, nff, reinterpret_cast<const int2*>(su), nvs, 1, nvs);
+			const int* eb = reinterpret_cast<const int*>(su + xo);
+#pragma unroll
+			for (int k = 0; k < NV; ++k)
+				W[k] = fix_dot_value(acc[k], fix_block(eb[k]), G.s_f);
+		} else {
+			const double* op = G.fops + o + (long long)i * nvs;
+#pragma unroll 1
+			for (int k = 0; k < NV; ++k) {
+				double s = 0.0;
+				for (int m = 0; m < nvs; ++m)
+					s = fma(__ldg(op + m), su[k * nvs + m], s);
+				W[k] = s;
+			}
 		}
 		double* dst = P.traces + 2 * NV * fb + (long long)fd.y * NV * nff;
 #pragma unroll
@@ -61,107 +163,145 @@ __device__ void dtraces(const BParams& P, const DGroup& G, int e0, int n_here, c
 	}
 }
 
+// The w-weighted contravariant flux of W at cubature node r of an element, into its flux block [k][j][r] (doubles).
+template <int D, int NV, int PDE>
+__device__ __forceinline__ void dflux(const BParams& P, const DGroup& G, int elem, int r, const double* W, double* sf)
+{
+	const int nvc = G.n_vc;
+	double g[D * D], fr[D][NV];
+	const double* gm = P.gmet + G.gmet_off + (long long)elem * D * D * nvc;
+#pragma unroll
+	for (int c = 0; c < D * D; ++c)
+		g[c] = gm[c * nvc + r];
+	tp_flux<D, NV, PDE>(P.b_adv, W, g, fr);
+#pragma unroll
+	for (int j = 0; j < D; ++j)
+#pragma unroll
+		for (int k = 0; k < NV; ++k)
+			sf[(k * D + j) * nvc + r] = fr[j][k];
+}
+
+// One output of a sum-factorised WEDGE pass as limbs at the pass's block exponent: sum |W| <= 2^62.
+__device__ __forceinline__ int2 fix_line(const FixW* op, int so, const int2* x, int sx, int n)
+{
+	FixAcc a = {0, 0};
+#pragma unroll 4
+	for (int i = 0; i < n; ++i)
+		fix_mac(a, ldg_fix(op + i * so), x[i * sx]);
+	return fix_limbs(a.h * 4 + (a.m >> 28));
+}
+
 // Sum-factorised volume term of a WEDGE volume whose operators are Kronecker products of TRI and LINE factors
 // (basis index c * n_tvs + t, node index rz * n_tvc + rt): s_vc in two passes (TRI, then LINE), the flux, then
-// sum_j cv1_j^T (w fr_j) as LINE then TRI passes for x and y and TRI then LINE for z. Fills sf and vol_gl.
+// sum_j cv1_j^T (w fr_j) as LINE then TRI passes for x and y and TRI then LINE for z. Elements in range only.
 template <int D, int NV, int PDE>
-__device__ void dvol_prism_phases(const BParams& P, const DGroup& G, int e0, int n_here, double* smem, int PER_E)
+__device__ void dvol_prism_phases(const BParams& P, const DGroup& G, int e0, int n_here, double* smem, int PER_E, int xo)
 {
 	const int nvs = G.n_vs, nvc = G.n_vc, ntv = G.n_tvs, ntc = G.n_tvc, nlv = G.n_lvs, nlc = G.n_lvc;
-	const double* __restrict__ T0 = G.tri0;
-	const double* __restrict__ T1 = G.tri1;
-	const double* __restrict__ L0 = G.line0;
-	const double* __restrict__ L1 = G.line1;
+	const int so = NV * nvs, to = so + D * NV * nvc;   // flux block, partial sums
 	// 1a: v[k][c][rt] = sum_t T0[rt][t] s[k][c][t]
 	for (int it = threadIdx.x; it < n_here * NV * nlv * ntc; it += blockDim.x) {
 		const int e = it / (NV * nlv * ntc), rem = it % (NV * nlv * ntc);
 		const int k = rem / (nlv * ntc), c = (rem / ntc) % nlv, rt = rem % ntc;
-		const double* su = smem + e * PER_E + k * nvs + c * ntv;
-		const double* row = T0 + (long long)rt * ntv;
-		double acc = 0.0;
-		for (int t = 0; t < ntv; ++t)
-			acc += __ldg(row + t) * su[t];
-		smem[e * PER_E + NV * nvs + 3 * NV * nvc + rem] = acc;
+		const int2* su = reinterpret_cast<const int2*>(smem + e * PER_E) + k * nvs + c * ntv;
+		if (blk_ok<NV>(smem, PER_E, e, xo, 0))
+			reinterpret_cast<int2*>(smem + e * PER_E + to)[rem] = fix_line(G.xt0T + rt, ntc, su, 1, ntv);
 	}
 	__syncthreads();
 	// 1b: W[k] at (rz, rt) = sum_c L0[rz][c] v[k][c][rt]; the flux there
 	for (int it = threadIdx.x; it < n_here * nvc; it += blockDim.x) {
 		const int e = it / nvc, r = it % nvc, rz = r / ntc, rt = r % ntc;
-		const double* v = smem + e * PER_E + NV * nvs + 3 * NV * nvc;
-		double* sf = smem + e * PER_E + NV * nvs;
+		if (!blk_ok<NV>(smem, PER_E, e, xo, 0))
+			continue;
+		const int2* v = reinterpret_cast<const int2*>(smem + e * PER_E + to) + rt;
+		const int* eb = reinterpret_cast<const int*>(smem + e * PER_E + xo);
 		double W[NV];
 #pragma unroll
 		for (int k = 0; k < NV; ++k) {
-			double acc = 0.0;
+			FixAcc a = {0, 0};
 			for (int c = 0; c < nlv; ++c)
-				acc += __ldg(L0 + rz * nlv + c) * v[(k * nlv + c) * ntc + rt];
-			W[k] = acc;
+				fix_mac(a, ldg_fix(G.xl0 + rz * nlv + c), v[(k * nlv + c) * ntc]);
+			W[k] = fix_to_double(fix_sum(a), fix_scale(fix_block(eb[k]) + 62 - G.s_t0, G.s_l0));
 		}
-		double g[D * D];
-		const double* gm = P.gmet + G.gmet_off + (long long)(e0 + e) * D * D * nvc;
-#pragma unroll
-		for (int cc = 0; cc < D * D; ++cc)
-			g[cc] = gm[cc * nvc + r];
-		if constexpr (PDE == kEuler) {
-			double fr[D][D + 2];
-			euler_flux_ref<D>(W, g, fr);
-#pragma unroll
-			for (int j = 0; j < D; ++j)
-#pragma unroll
-				for (int k = 0; k < NV; ++k)
-					sf[(j * NV + k) * nvc + r] = fr[j][k];
-		} else {
-#pragma unroll
-			for (int j = 0; j < D; ++j) {
-				double gb = 0.0;
-#pragma unroll
-				for (int i = 0; i < D; ++i)
-					gb += g[j * D + i] * P.b_adv[i];
-				sf[j * nvc + r] = gb * W[0];
-			}
-		}
+		dflux<D, NV, PDE>(P, G, e0 + e, r, W, smem + e * PER_E + so);
 	}
+	__syncthreads();
+	blk_max<NV>(smem, PER_E, n_here, so, D * nvc, xo, NV);
+	__syncthreads();
+	blk_pack<NV>(smem, PER_E, n_here, so, D * nvc, xo, NV);
 	__syncthreads();
 	// 2a: gx, gy[k][c][rt] = sum_rz L0[rz][c] f_x,y[k][rz][rt];  h[k][rz][t] = sum_rt T0[rt][t] f_z[k][rz][rt]
 	const int gsz = NV * nlv * ntc;
 	for (int it = threadIdx.x; it < n_here * gsz; it += blockDim.x) {
 		const int e = it / gsz, rem = it % gsz;
 		const int k = rem / (nlv * ntc), c = (rem / ntc) % nlv, rt = rem % ntc;
-		const double* sf = smem + e * PER_E + NV * nvs;
-		double* tmp = smem + e * PER_E + NV * nvs + 3 * NV * nvc;
-		double ax = 0.0, ay = 0.0;
-		for (int rz = 0; rz < nlc; ++rz) {
-			const double l = __ldg(L0 + rz * nlv + c);
-			ax += l * sf[(0 * NV + k) * nvc + rz * ntc + rt];
-			ay += l * sf[(1 * NV + k) * nvc + rz * ntc + rt];
-		}
-		tmp[rem] = ax;
-		tmp[gsz + rem] = ay;
+		if (!blk_ok<NV>(smem, PER_E, e, xo, NV))
+			continue;
+		const int2* f = reinterpret_cast<const int2*>(smem + e * PER_E + so) + k * D * nvc + rt;
+		int2* tmp = reinterpret_cast<int2*>(smem + e * PER_E + to);
+		tmp[rem] = fix_line(G.xl0 + c, nlv, f, ntc, nlc);
+		tmp[gsz + rem] = fix_line(G.xl0 + c, nlv, f + nvc, ntc, nlc);
 	}
 	const int hsz = NV * nlc * ntv;
 	for (int it = threadIdx.x; it < n_here * hsz; it += blockDim.x) {
 		const int e = it / hsz, rem = it % hsz;
 		const int k = rem / (nlc * ntv), rz = (rem / ntv) % nlc, t = rem % ntv;
-		const double* fz = smem + e * PER_E + NV * nvs + (2 * NV + k) * nvc + rz * ntc;
-		double* h = smem + e * PER_E + NV * nvs + 3 * NV * nvc + 2 * gsz;
-		double acc = 0.0;
-		for (int rt = 0; rt < ntc; ++rt)
-			acc += __ldg(T0 + (long long)rt * ntv + t) * fz[rt];
-		h[rem] = acc;
+		if (!blk_ok<NV>(smem, PER_E, e, xo, NV))
+			continue;
+		const int2* fz = reinterpret_cast<const int2*>(smem + e * PER_E + so) + (k * D + 2) * nvc + rz * ntc;
+		reinterpret_cast<int2*>(smem + e * PER_E + to)[2 * gsz + rem] = fix_line(G.xt0 + t, ntv, fz, 1, ntc);
 	}
 	__syncthreads();
 	// 2b: vol[k][c][t] = sum_rt (T1x[rt][t] gx[k][c][rt] + T1y[rt][t] gy[k][c][rt]) + sum_rz L1[rz][c] h[k][rz][t]
 	for (int it = threadIdx.x; it < n_here * NV * nvs; it += blockDim.x) {
 		const int e = it / (NV * nvs), rem = it % (NV * nvs), k = rem / nvs, c = (rem % nvs) / ntv, t = rem % ntv;
-		const double* tmp = smem + e * PER_E + NV * nvs + 3 * NV * nvc;
-		const double* gx = tmp + (k * nlv + c) * ntc;
-		const double* gy = gx + gsz;
-		const double* h = tmp + 2 * gsz + k * nlc * ntv + t;
+		if (!blk_ok<NV>(smem, PER_E, e, xo, NV) || !blk_ok<NV>(smem, PER_E, e, xo, 0))
+			continue;
+		const int2* tmp = reinterpret_cast<const int2*>(smem + e * PER_E + to);
+		const int2* gx = tmp + (k * nlv + c) * ntc;
+		FixAcc a = {0, 0};
+		fix_dot<1>(&a, G.xt1 + t, ntv, gx, 0, 1, ntc);
+		fix_dot<1>(&a, G.xt1 + (long long)ntc * ntv + t, ntv, gx + gsz, 0, 1, ntc);
+		fix_dot<1>(&a, G.xl1 + c, nlv, tmp + 2 * gsz + k * nlc * ntv + t, 0, ntv, nlc);
+		const int eb = fix_block(reinterpret_cast<const int*>(smem + e * PER_E + xo)[NV + k]);
+		P.vol_gl[G.state_off + (long long)(e0 + e) * NV * nvs + rem] =
+			fix_dot_value(a, eb + 62 - G.s_l0, G.s_t1);
+	}
+}
+
+// The volume term of the elements that are out of range, in FP64 (dense operators; the state is read from memory and
+// the fluxes go through the element's flux block).
+template <int D, int NV, int PDE>
+__device__ __noinline__ void dvol_fp64(const BParams& P, const DGroup& G, int e0, int n_here,
+                                       const double* __restrict__ ublk, double* smem, int PER_E, int xo)
+{
+	const int nvs = G.n_vs, nvc = G.n_vc, so = NV * nvs;
+	__syncthreads();
+	for (int it = threadIdx.x; it < n_here * nvc; it += blockDim.x) {
+		const int e = it / nvc, r = it % nvc;
+		if (blk_ok<NV>(smem, PER_E, e, xo, 0) && blk_ok<NV>(smem, PER_E, e, xo, NV))
+			continue;
+		const double* row = G.cv0 + (long long)r * nvs;
+		double W[NV];
+#pragma unroll 1
+		for (int k = 0; k < NV; ++k) {
+			const double* su = ublk + ((long long)e * NV + k) * nvs;
+			double s = 0.0;
+			for (int m = 0; m < nvs; ++m)
+				s = fma(__ldg(row + m), su[m], s);
+			W[k] = s;
+		}
+		dflux<D, NV, PDE>(P, G, e0 + e, r, W, smem + e * PER_E + so);
+	}
+	__syncthreads();
+	for (int it = threadIdx.x; it < n_here * NV * nvs; it += blockDim.x) {
+		const int e = it / (NV * nvs), rem = it % (NV * nvs), k = rem / nvs, m = rem % nvs;
+		if (blk_ok<NV>(smem, PER_E, e, xo, 0) && blk_ok<NV>(smem, PER_E, e, xo, NV))
+			continue;
+		const double* f = smem + e * PER_E + so + k * D * nvc;
 		double acc = 0.0;
-		for (int rt = 0; rt < ntc; ++rt)
-			acc += __ldg(T1 + (long long)rt * ntv + t) * gx[rt] + __ldg(T1 + (long long)(ntc + rt) * ntv + t) * gy[rt];
-		for (int rz = 0; rz < nlc; ++rz)
-			acc += __ldg(L1 + rz * nlv + c) * h[rz * ntv];
+		for (int jr = 0; jr < D * nvc; ++jr)
+			acc = fma(__ldg(G.cv1 + (long long)jr * nvs + m), f[jr], acc);
 		P.vol_gl[G.state_off + (long long)(e0 + e) * NV * nvs + rem] = acc;
 	}
 }
@@ -174,7 +314,7 @@ __device__ void dvol_body(const BParams& P, const DGroup& G, int e0, int E, cons
                           double* smem)
 {
 	const int nvs = G.n_vs, nvc = G.n_vc;
-	const int PER_E = G.vol_per_e;
+	const int PER_E = G.vol_per_e, xo = PER_E - NV - 1, so = NV * nvs;
 	const int n_here = min(E, G.n_vol - e0);
 	const double* ublk = u + G.state_off + (long long)e0 * NV * nvs;
 	for (int i = threadIdx.x; i < n_here * NV * nvs; i += blockDim.x) {
@@ -182,71 +322,60 @@ __device__ void dvol_body(const BParams& P, const DGroup& G, int e0, int E, cons
 		smem[e * PER_E + r] = ublk[i];
 	}
 	__syncthreads();
+	blk_max<NV>(smem, PER_E, n_here, 0, nvs, xo, 0);
+	__syncthreads();
+	blk_pack<NV>(smem, PER_E, n_here, 0, nvs, xo, 0);
+	__syncthreads();
 	if (G.prism) {
-		dvol_prism_phases<D, NV, PDE>(P, G, e0, n_here, smem, PER_E);
-		dtraces<NV>(P, G, e0, n_here, smem, PER_E);
-		__syncthreads();   // shared memory is reused by the next tile
-		return;
-	}
-	const double* __restrict__ cv0 = G.cv0;
-	// phase 1: state at the cubature nodes, contravariant flux, w-weighted (w is folded into the metrics)
-	for (int it = threadIdx.x; it < n_here * nvc; it += blockDim.x) {
-		const int e = it / nvc, r = it % nvc;
-		const double* su = smem + e * PER_E;
-		double* sf = smem + e * PER_E + NV * nvs;   // [j][k][r]
-		double W[NV];
-#pragma unroll
-		for (int k = 0; k < NV; ++k)
-			W[k] = 0.0;
-		const double* row = cv0 + (long long)r * nvs;
-		for (int m = 0; m < nvs; ++m) {
-			const double c = __ldg(row + m);
+		dvol_prism_phases<D, NV, PDE>(P, G, e0, n_here, smem, PER_E, xo);
+	} else {
+		// phase 1: state at the cubature nodes, contravariant flux, w-weighted (w is folded into the metrics)
+		for (int it = threadIdx.x; it < n_here * nvc; it += blockDim.x) {
+			const int e = it / nvc, r = it % nvc;
+			if (!blk_ok<NV>(smem, PER_E, e, xo, 0))
+				continue;
+			const int* eb = reinterpret_cast<const int*>(smem + e * PER_E + xo);
+			FixAcc acc[NV];
+			double W[NV];
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
-				W[k] += c * su[k * nvs + m];
+				acc[k] = {0, 0};
+			fix_dot<NV>(acc, G.xcv0 + r, nvc, reinterpret_cast<const int2*>(smem + e * PER_E), nvs, 1, nvs);
+#pragma unroll
+			for (int k = 0; k < NV; ++k)
+				W[k] = fix_dot_value(acc[k], fix_block(eb[k]), G.s_cv0);
+			dflux<D, NV, PDE>(P, G, e0 + e, r, W, smem + e * PER_E + so);
 		}
-		double g[D * D];
-		const double* gm = P.gmet + G.gmet_off + (long long)(e0 + e) * D * D * nvc;
+		__syncthreads();
+		blk_max<NV>(smem, PER_E, n_here, so, D * nvc, xo, NV);
+		__syncthreads();
+		blk_pack<NV>(smem, PER_E, n_here, so, D * nvc, xo, NV);
+		__syncthreads();
+		// phase 2: rhs_vol[k][m] = sum_j sum_r cv1_j[r][m] sf[k][j][r]
+		for (int it = threadIdx.x; it < n_here * nvs; it += blockDim.x) {
+			const int e = it / nvs, m = it % nvs;
+			if (!blk_ok<NV>(smem, PER_E, e, xo, NV))
+				continue;
+			const int* eb = reinterpret_cast<const int*>(smem + e * PER_E + xo) + NV;
+			FixAcc acc[NV];
 #pragma unroll
-		for (int c = 0; c < D * D; ++c)
-			g[c] = gm[c * nvc + r];
-		if constexpr (PDE == kEuler) {
-			double fr[D][D + 2];
-			euler_flux_ref<D>(W, g, fr);
+			for (int k = 0; k < NV; ++k)
+				acc[k] = {0, 0};
+			fix_dot<NV>(acc, G.xcv1 + m, nvs, reinterpret_cast<const int2*>(smem + e * PER_E + so), D * nvc, 1, D * nvc);
+			double* out = P.vol_gl + G.state_off + (long long)(e0 + e) * NV * nvs + m;
 #pragma unroll
-			for (int j = 0; j < D; ++j)
-#pragma unroll
-				for (int k = 0; k < NV; ++k)
-					sf[(j * NV + k) * nvc + r] = fr[j][k];
-		} else {
-#pragma unroll
-			for (int j = 0; j < D; ++j) {
-				double gb = 0.0;
-#pragma unroll
-				for (int i = 0; i < D; ++i)
-					gb += g[j * D + i] * P.b_adv[i];
-				sf[j * nvc + r] = gb * W[0];
-			}
+			for (int k = 0; k < NV; ++k)
+				out[k * nvs] = fix_dot_value(acc[k], fix_block(eb[k]), G.s_cv1);
 		}
 	}
-	__syncthreads();
-	// phase 2: rhs_vol[k][m] = sum_j sum_r cv1_j[r][m] sf[j][k][r]
-	const double* __restrict__ cv1 = G.cv1;
-	for (int it = threadIdx.x; it < n_here * NV * nvs; it += blockDim.x) {
-		const int e = it / (NV * nvs), rem = it % (NV * nvs), k = rem / nvs, m = rem % nvs;
-		const double* sf = smem + e * PER_E + NV * nvs;
-		double acc = 0.0;
-#pragma unroll
-		for (int j = 0; j < D; ++j) {
-			const double* col = cv1 + (long long)j * nvc * nvs + m;
-			const double* f = sf + (j * NV + k) * nvc;
-			for (int r = 0; r < nvc; ++r)
-				acc += __ldg(col + (long long)r * nvs) * f[r];
-		}
-		P.vol_gl[G.state_off + (long long)(e0 + e) * NV * nvs + k * nvs + m] = acc;
+	dtraces<NV>(P, G, e0, n_here, smem, PER_E, xo);
+	bool bad = false;
+	for (int e = threadIdx.x; e < n_here; e += blockDim.x)
+		bad = bad || !blk_ok<NV>(smem, PER_E, e, xo, 0) || !blk_ok<NV>(smem, PER_E, e, xo, NV);
+	if (__syncthreads_or(bad)) {   // also: shared memory is reused by the next tile
+		dvol_fp64<D, NV, PDE>(P, G, e0, n_here, ublk, smem, PER_E, xo);
+		__syncthreads();
 	}
-	dtraces<NV>(P, G, e0, n_here, smem, PER_E);
-	__syncthreads();   // shared memory is reused by the next tile
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -274,15 +403,19 @@ __device__ void dense_positivity(const BParams& P, const DGroup& G, int e0, int 
 		const int e = it / (NV * nvs), rem = it % (NV * nvs);
 		reinterpret_cast<float*>(smem + e * PER_E + NV)[rem] = (float)smem[e * PER_E + NV * nvs + rem];
 	}
-	for (int it = threadIdx.x; it < n_here * NV; it += blockDim.x) {   // one thread per (volume, variable)
-		const int e = it / NV, k = it % NV;
+	for (int p = threadIdx.x >> 5; p < n_here * NV; p += blockDim.x >> 5) {   // one warp per (volume, variable)
+		const int e = p / NV, k = p % NV, lane = threadIdx.x & 31;
 		const double* sv = smem + e * PER_E + NV * nvs + k * nvs;
-		double mx = 0.0;
-		for (int a = 0; a < nvs; ++a)
-			mx = fmax(mx, fabs(sv[a]));
-		smem[e * PER_E + k] = mx;
-		if (k == 0)
-			smem[e * PER_E + 2 * NV * nvs + 1] = 0.0;   // unsafe flag
+		// the largest |s|'s high word, and the next one up: a bound of it within 2^-20 (NaN fails the tests below)
+		int mx = 0;
+		for (int a = lane; a < nvs; a += 32)
+			mx = max(mx, __double2hiint(sv[a]) & 0x7fffffff);
+		mx = __reduce_max_sync(0xffffffffu, mx);
+		if (lane == 0) {
+			smem[e * PER_E + k] = __hiloint2double(mx + 1, 0);
+			if (k == 0)
+				smem[e * PER_E + 2 * NV * nvs + 1] = 0.0;   // unsafe flag
+		}
 	}
 	__syncthreads();
 	for (int it = threadIdx.x; it < n_here * nvs; it += blockDim.x) {
@@ -418,55 +551,109 @@ __device__ void dense_positivity(const BParams& P, const DGroup& G, int e0, int 
 template <int NV, int MODE>
 __device__ void dlift_body(const BParams& P, const DGroup& G, int e0, int E, const RkArgs& rk, double* smem)
 {
-	const int nvs = G.n_vs;
-	const int PER_E = G.lift_per_e;
+	const int nvs = G.n_vs, nfm = G.nff_max, nft = G.n_lf * nfm;
+	const int PER_E = G.lift_per_e, fo = 2 * NV * nvs + 2, xo = PER_E - NV - 1;   // face terms, block exponents
 	const int n_here = min(E, G.n_vol - e0);
-	// phase 1: rhs = vol - sum_lf sgn cv0_fc^T nnf
-	for (int it = threadIdx.x; it < n_here * NV * nvs; it += blockDim.x) {
-		const int e = it / (NV * nvs), rem = it % (NV * nvs), k = rem / nvs, m = rem % nvs;
-		const long long v = G.elem0 + e0 + e;
-		double acc = P.vol_gl[G.state_off + (long long)(e0 + e) * NV * nvs + rem];
-		if (P.source)   // cv0^T diag(w J) s
-			acc += P.source[G.state_off + (long long)(e0 + e) * NV * nvs + rem];
-		for (int lf = 0; lf < G.n_lf; ++lf) {
+	const int lane = threadIdx.x & 31;
+	// phase 1: rhs = vol - sum_lf sgn cv0_fc^T nnf. The signed face terms of one variable (side 0: rhs -= ; side 1:
+	// rhs -= (-nnf)) make a block; the volume term (with the source's cv0^T diag(w J) s), whose high modes are far larger
+	// than a face term, is added in FP64.
+	for (int p = threadIdx.x >> 5; p < n_here * NV; p += blockDim.x >> 5) {
+		const int e = p / NV, k = p % NV;
+		const long long v = G.elem0 + e0 + e, so = G.state_off + (long long)(e0 + e) * NV * nvs + k * nvs;
+		double* x = smem + e * PER_E + fo + k * nft;
+		double* r = smem + e * PER_E + k * nvs;
+		int m = 0;
+		for (int i = lane; i < nvs; i += 32)
+			r[i] = P.source ? add(P.vol_gl[so + i], P.source[so + i]) : P.vol_gl[so + i];
+		for (int it = lane; it < nft; it += 32) {
+			const int lf = it / nfm, i = it % nfm;
 			const int4 fd = P.elf[v * kMaxLf + lf];
 			const long long fb = P.fbase[fd.x];
 			const int nff = (int)(P.fbase[fd.x + 1] - fb);
-			const double* op = G.fops + G.fop_off[(lf * G.n_ord + fd.w) * (kQMax + 1) + fd.z] + m;
-			const double* src = P.nnf + NV * fb + (long long)k * nff;
-			// side 1 reads the face flux (side 0's node order) at its own nodes through the inverse permutation
-			const int* ci = (fd.y == 1 && P.nc_inv) ? P.nc_inv + fb : nullptr;
-			double s = 0.0;
-			for (int i = 0; i < nff; ++i)
-				s += __ldg(op + (long long)i * nvs) * src[ci ? ci[i] : i];
-			acc += (fd.y == 0 ? -s : s);   // side 0: rhs -= ; side 1: rhs -= (-nnf)
+			double t = 0.0;
+			if (i < nff) {
+				// side 1 reads the face flux (side 0's node order) at its own nodes through the inverse permutation
+				t = P.nnf[NV * fb + (long long)k * nff + ((fd.y == 1 && P.nc_inv) ? P.nc_inv[fb + i] : i)];
+				t = fd.y == 0 ? -t : t;
+			}
+			x[it] = t;
+			m = max(m, fix_exponent(t));
 		}
-		smem[e * PER_E + rem] = acc;
+		m = __reduce_max_sync(0xffffffffu, m);
+		if (lane == 0)
+			reinterpret_cast<int*>(smem + e * PER_E + xo)[k] = m;
 	}
 	__syncthreads();
-	// phase 2: R = M_ref^-1 rhs / J, then the stage
-	const double* __restrict__ minv = G.minv;
+	blk_pack<NV>(smem, PER_E, n_here, fo, nft, xo, 0);
+	__syncthreads();
+	for (int it = threadIdx.x; it < n_here * nvs; it += blockDim.x) {
+		const int e = it / nvs, m = it % nvs;
+		const long long v = G.elem0 + e0 + e;
+		double* r = smem + e * PER_E + m;
+		if (blk_ok<NV>(smem, PER_E, e, xo, 0)) {
+			const int* eb = reinterpret_cast<const int*>(smem + e * PER_E + xo);
+			FixAcc acc[NV];
+#pragma unroll
+			for (int k = 0; k < NV; ++k)
+				acc[k] = {0, 0};
+			for (int lf = 0; lf < G.n_lf; ++lf) {
+				const int4 fd = P.elf[v * kMaxLf + lf];
+				const int nff = (int)(P.fbase[fd.x + 1] - P.fbase[fd.x]);
+				fix_dot<NV>(acc, G.xfL + G.fop_off[(lf * G.n_ord + fd.w) * (kQMax + 1) + fd.z] + m, nvs,
+				            reinterpret_cast<const int2*>(smem + e * PER_E + fo) + lf * nfm, nft, 1, nff);
+			}
+#pragma unroll
+			for (int k = 0; k < NV; ++k)
+				r[k * nvs] = add(r[k * nvs], fix_dot_value(acc[k], fix_block(eb[k]), G.s_f));
+		} else {
+#pragma unroll 1
+			for (int k = 0; k < NV; ++k) {
+				double acc = r[k * nvs];
+				for (int lf = 0; lf < G.n_lf; ++lf) {
+					const int4 fd = P.elf[v * kMaxLf + lf];
+					const int nff = (int)(P.fbase[fd.x + 1] - P.fbase[fd.x]);
+					const double* op = G.fops + G.fop_off[(lf * G.n_ord + fd.w) * (kQMax + 1) + fd.z] + m;
+					const double* x = smem + e * PER_E + fo + k * nft + lf * nfm;
+					for (int i = 0; i < nff; ++i)
+						acc = fma(__ldg(op + (long long)i * nvs), x[i], acc);
+				}
+				r[k * nvs] = acc;
+			}
+		}
+	}
+	__syncthreads();
+	// phase 2: R = M^-1 rhs, then the stage: 1/J alone for an orthonormal basis, a product with M_ref^-1 before it
+	// otherwise (in fixed point, on the rhs packed in place), each volume's own M^-1 in a curved group
+	const bool dense_m = !G.minv_vol && !G.minv_identity;
+	if (dense_m) {
+		blk_max<NV>(smem, PER_E, n_here, 0, nvs, xo, NV);
+		__syncthreads();
+		blk_pack<NV>(smem, PER_E, n_here, 0, nvs, xo, NV);
+		__syncthreads();
+	}
 	unsigned long long mx = 0ull;
 	for (int it = threadIdx.x; it < n_here * NV * nvs; it += blockDim.x) {
 		const int e = it / (NV * nvs), rem = it % (NV * nvs), k = rem / nvs, m = rem % nvs;
 		const double* sr = smem + e * PER_E + k * nvs;
 		double R;
-		if (G.minv_vol) {   // curved volumes: the volume's own M^-1
-			const double* row = G.minv_vol + ((long long)(e0 + e) * nvs + m) * nvs;
-			R = 0.0;
-			for (int a = 0; a < nvs; ++a)
-				R += __ldg(row + a) * sr[a];
-		} else {
-			if (G.minv_identity) {
+		if (!dense_m || !blk_ok<NV>(smem, PER_E, e, xo, NV)) {
+			if (G.minv_identity && !G.minv_vol) {
 				R = sr[m];
 			} else {
-				const double* row = minv + (long long)m * nvs;
+				const double* row = G.minv_vol ? G.minv_vol + ((long long)(e0 + e) * nvs + m) * nvs
+				                               : G.minv + (long long)m * nvs;
 				R = 0.0;
 				for (int a = 0; a < nvs; ++a)
-					R += __ldg(row + a) * sr[a];
+					R = fma(__ldg(row + a), sr[a], R);
 			}
-			R *= G.inv_J[e0 + e];
+		} else {
+			FixAcc acc = {0, 0};
+			fix_dot<1>(&acc, G.xminv + m, nvs, reinterpret_cast<const int2*>(sr), 0, 1, nvs);
+			R = fix_dot_value(acc, fix_block(reinterpret_cast<const int*>(smem + e * PER_E + xo)[NV + k]), G.s_minv);
 		}
+		if (!G.minv_vol)
+			R = mul(R, G.inv_J[e0 + e]);
 		const long long o = G.state_off + (long long)(e0 + e) * NV * nvs + rem;
 		if (MODE == kModeRhs || rk.want_max) {
 			const unsigned long long bits = abs_bits(R);

@@ -10,14 +10,14 @@
 // Representation. The values that enter one sum share a block exponent eb, the largest biased exponent among them
 // (taken over one element and one variable, so that an element's result does not depend on its neighbours in the
 // launch). A value v is held as the integer X = v 2^(1082 - eb), |X| < 2^60, rounded to a multiple of 4 and kept as
-// two limbs: h = X >> 32 (signed) and l = the next 30 bits (0 <= l < 2^30), X = h 2^32 + 4 l. An operator entry w is
-// W = w 2^s = h 2^32 + 4 l with l balanced (|l| <= 2^29). sum X W then needs h h, h l and l h products only:
+// two limbs, X = h 2^32 + 4 l with l balanced (|l| <= 2^29). An operator entry w is W = w 2^s = h 2^32 + 4 l likewise.
+// sum X W then needs h h, h l and l h products only:
 //   sum X W / 2^64 = a.h + a.m / 2^30,   a.h = sum hX hW,   a.m = sum (hW lX + lW hX).
 // s is chosen on the host so that sum |W| <= 2^63 over every sum an operator enters (and |W| < 2^62), which bounds
 // a.h by 2^59 and, for at most 32 terms, a.m by 2^62: neither accumulator can overflow.
 //
 // Accuracy. A value is rounded to 2^-59 of its block's largest magnitude, an operator entry to about 2^-60 of its
-// row sum, and the dropped l l products are below 2^-60 of the sum's bound (l of the operator is balanced, so
+// row sum, and the dropped l l products are below 2^-60 of the sum's bound (both l are balanced, so
 // they have no bias): the sum is exact to a few 2^-59 of max |v| sum |w|, where FP64 arithmetic rounds every partial sum
 // to 2^-53. The result is rounded once to FP64, to nearest.
 //
@@ -60,6 +60,12 @@ __device__ __forceinline__ bool fix_in_range(int eb)
 }
 __device__ __forceinline__ int fix_block(int eb) { return eb < kFixMin ? kFixMin : eb; }
 
+// Limbs of an integer: l from the low word taken as signed, h with the carry that makes up for it.
+__device__ __forceinline__ int2 fix_split(long long X)
+{
+	return make_int2((int)X >> 2, (int)((X + 0x80000000ll) >> 32));
+}
+
 // x as limbs (.x = l, .y = h) at block exponent eb >= its own exponent.
 __device__ __forceinline__ int2 fix_pack(double x, int eb)
 {
@@ -69,7 +75,7 @@ __device__ __forceinline__ int2 fix_pack(double x, int eb)
 	asm("shr.u64 %0, %0, %1;" : "+l"(m) : "r"(eb - ((hi >> 20) & 0x7ff)));   // clamps: 0 beyond 63
 	const long long s = hi >> 31;
 	const long long X = (long long)(m ^ (unsigned long long)s) + (2 - s);    // sign, and half of the last kept unit
-	return make_int2((int)((unsigned)X >> 2), (int)(X >> 32));
+	return fix_split(X);
 }
 
 __device__ __forceinline__ void fix_mac(FixAcc& a, const FixW w, const int2 x)
@@ -102,8 +108,7 @@ __device__ __forceinline__ double fix_to_double(long long r, int e)
 // Limbs of an integer value |X| < 2^60 (a contraction's result that enters the next one).
 __device__ __forceinline__ int2 fix_limbs(long long X)
 {
-	X += 2;
-	return make_int2((int)((unsigned)X >> 2), (int)(X >> 32));
+	return fix_split(X + 2);
 }
 
 // Per-element maxima of K non-negative integers over the threads of each element (N consecutive threads per element,
