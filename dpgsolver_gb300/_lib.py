@@ -15,6 +15,7 @@ REPO_DIR = os.path.dirname(PKG_DIR)
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libdgpu.so")
 SOURCES = ["dgpu.cu", "dgpu_batched.cu", "dgpu_mesh_io.cpp"]
+PARTS = {"dgpu.cu": 6, "dgpu_batched.cu": 5}   # compilations per source (DGPU_PART): host code, then kernels by case
 HEADERS = ["dgpu_ns.cuh", "dgpu_geometry.cuh", "dgpu_jacobian.cuh", "dgpu_tp.cuh", "dgpu_fix.cuh", "dgpu_physics.cuh", "dgpu_dual.cuh", "dgpu_adjoint.cuh", "dgpu_batched.cuh",
            "dgpu_batched_ns.cuh", "dgpu_ns_adjoint.cuh", "dgpu_dense.cuh", "dgpu_jvp.cuh", "dgpu_host_ops.h"]
 NVCC_FLAGS = ["-std=c++17", "-O3", "-gencode", "arch=compute_103a,code=sm_103a", "-lineinfo",
@@ -54,12 +55,14 @@ def build(force: bool = False, verbose: bool = False) -> str:
 def _build_locked(verbose: bool) -> str:
     objs, procs = [], []
     for src in SOURCES:   # translation units compile in parallel, then one link
-        obj = os.path.join(BUILD_DIR, os.path.splitext(src)[0] + ".o")
-        cmd = [nvcc_path()] + NVCC_FLAGS + ["-c", "-o", obj, os.path.join(CSRC, src)]
-        if verbose:
-            print(" ".join(cmd))
-        procs.append((cmd, subprocess.Popen(cmd)))
-        objs.append(obj)
+        for part in range(PARTS.get(src, 1)):
+            obj = os.path.join(BUILD_DIR, f"{os.path.splitext(src)[0]}_{part}.o")
+            define = [f"-DDGPU_PART={part}"] if src in PARTS else []
+            cmd = [nvcc_path()] + NVCC_FLAGS + define + ["-c", "-o", obj, os.path.join(CSRC, src)]
+            if verbose:
+                print(" ".join(cmd))
+            procs.append((cmd, subprocess.Popen(cmd)))
+            objs.append(obj)
     for cmd, pr in procs:
         if pr.wait() != 0:
             raise subprocess.CalledProcessError(pr.returncode, cmd)

@@ -25,17 +25,26 @@
 
 using namespace dgpu;
 
-namespace {
-
-thread_local std::string g_create_error;
-
+namespace dgpu {
 
 struct KernelTimer {
 	const char* name;
 	cudaEvent_t start, stop;
 };
 
-}  // namespace
+}  // namespace dgpu
+
+// The kernels are many instantiations: this file is compiled once for the host code (DGPU_PART 0) and once per part,
+// each of which defines one of the functions below, that set a context's launchers.
+#ifndef DGPU_PART
+#error "compile with -DDGPU_PART=0..5"
+#endif
+struct dgpu_ctx;
+cudaError_t dgpu_bind_2d(dgpu_ctx* c);                  // part 1: every PDE
+cudaError_t dgpu_bind_3d_advection_roe(dgpu_ctx* c);    // part 2: advection, Euler with Roe-Pike
+cudaError_t dgpu_bind_3d_lf(dgpu_ctx* c);               // part 3: Euler with Lax-Friedrichs
+cudaError_t dgpu_bind_3d_ns_roe(dgpu_ctx* c);           // part 4: Navier-Stokes on top of Euler
+cudaError_t dgpu_bind_3d_ns_lf(dgpu_ctx* c);            // part 5
 
 struct dgpu_ctx {
 	// problem
@@ -155,7 +164,9 @@ struct dgpu_ctx {
 
 namespace {
 
-dgpu_status fail(dgpu_ctx* c, dgpu_status st, const std::string& msg)
+thread_local std::string g_create_error;
+
+[[maybe_unused]] dgpu_status fail(dgpu_ctx* c, dgpu_status st, const std::string& msg)
 {
 	if (c)
 		c->err = msg;
@@ -164,7 +175,7 @@ dgpu_status fail(dgpu_ctx* c, dgpu_status st, const std::string& msg)
 	return st;
 }
 
-dgpu_status cuda_fail(dgpu_ctx* c, cudaError_t e, const char* what)
+[[maybe_unused]] dgpu_status cuda_fail(dgpu_ctx* c, cudaError_t e, const char* what)
 {
 	std::string m = std::string(what) + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")";
 	return fail(c, DGPU_ERR_CUDA, m);
@@ -208,7 +219,7 @@ size_t convert_smem_bytes()
 	return (sizeof(TPOps) + 7) / 8 * 8 + (size_t)S::E * (3 * NV * S::N) * sizeof(double);
 }
 
-void record_start(dgpu_ctx* c, const char* name)
+[[maybe_unused]] void record_start(dgpu_ctx* c, const char* name)
 {
 	if (!c->timing)
 		return;
@@ -220,7 +231,7 @@ void record_start(dgpu_ctx* c, const char* name)
 	c->timers.push_back(t);
 }
 
-void record_stop(dgpu_ctx* c)
+[[maybe_unused]] void record_stop(dgpu_ctx* c)
 {
 	if (!c->timing)
 		return;
@@ -645,22 +656,19 @@ cudaError_t launch_ns_adjoint_t(dgpu_ctx* c, const double* u, const double* rbar
 	return cudaGetLastError();
 }
 
-cudaError_t launch_nothing(dgpu_ctx*) { return cudaSuccess; }
+[[maybe_unused]] cudaError_t launch_nothing(dgpu_ctx*) { return cudaSuccess; }
 
 template <int D, int Q, int FLUX>
 cudaError_t bind_ns(dgpu_ctx* c)
 {
 	constexpr int NV = D + 2;
-	cudaError_t e = bind<D, Q, NV, kEuler, FLUX>(c);   // lift, convert, positivity: as for Euler
+	cudaError_t e;   // the Euler launchers are set: lift, convert, positivity stay
 	c->launch_volume_in = nullptr;   // the fused host step is Euler / advection only
 	c->launch_lift_out = nullptr;
-	if (e != cudaSuccess)
-		return e;
 	c->launch_volume = launch_ns_t<D, Q, FLUX, true>;
 	c->launch_volume_gl = launch_ns_t<D, Q, FLUX, false>;
 	c->launch_face = launch_nothing;
 	c->launch_adjoint = launch_ns_adjoint_t<D, Q, FLUX>;
-	c->launch_objective = launch_objective_t<D, Q, NV>;
 	c->launch_jvp = launch_ns_jvp_t<D, Q, FLUX, true>;
 	c->launch_jvp_tangent = launch_ns_jvp_t<D, Q, FLUX, false>;
 	const cudaFuncAttribute smem = cudaFuncAttributeMaxDynamicSharedMemorySize;
@@ -678,28 +686,71 @@ cudaError_t bind_ns(dgpu_ctx* c)
 	return cudaSuccess;
 }
 
-template <int D, int Q>
-cudaError_t bind_pde(dgpu_ctx* c)
-{
-	if (c->pde == DGPU_PDE_NAVIER_STOKES)
-		return c->flux == DGPU_NUM_FLUX_ROE_PIKE ? bind_ns<D, Q, kRoePike>(c) : bind_ns<D, Q, kLaxFriedrichs>(c);
-	if (c->pde == DGPU_PDE_ADVECTION)
-		return bind<D, Q, 1, kAdvection, kUpwind>(c);
-	if (c->flux == DGPU_NUM_FLUX_ROE_PIKE)
-		return bind<D, Q, D + 2, kEuler, kRoePike>(c);
-	return bind<D, Q, D + 2, kEuler, kLaxFriedrichs>(c);
-}
-
-template <int D>
-cudaError_t bind_q(dgpu_ctx* c)
-{
-	switch (c->q) {
-	case 2: return bind_pde<D, 2>(c);
-	case 3: return bind_pde<D, 3>(c);
-	case 4: return bind_pde<D, 4>(c);
-	case 5: return bind_pde<D, 5>(c);
-	default: return cudaErrorInvalidValue;
+// f<Q> for the context's order.
+#define DGPU_FOR_Q(c, f)                       \
+	switch ((c)->q) {                          \
+	case 2: return f<2>(c);                    \
+	case 3: return f<3>(c);                    \
+	case 4: return f<4>(c);                    \
+	case 5: return f<5>(c);                    \
+	default: return cudaErrorInvalidValue;     \
 	}
+
+#if DGPU_PART == 1
+template <int Q>
+cudaError_t bind_2d(dgpu_ctx* c)
+{
+	if (c->pde == DGPU_PDE_ADVECTION)
+		return bind<2, Q, 1, kAdvection, kUpwind>(c);
+	const bool roe = c->flux == DGPU_NUM_FLUX_ROE_PIKE;
+	const cudaError_t e = roe ? bind<2, Q, 4, kEuler, kRoePike>(c) : bind<2, Q, 4, kEuler, kLaxFriedrichs>(c);
+	if (e != cudaSuccess || c->pde != DGPU_PDE_NAVIER_STOKES)
+		return e;
+	return roe ? bind_ns<2, Q, kRoePike>(c) : bind_ns<2, Q, kLaxFriedrichs>(c);
+}
+#elif DGPU_PART == 2
+template <int Q>
+cudaError_t bind_3d_advection_roe(dgpu_ctx* c)
+{
+	return c->pde == DGPU_PDE_ADVECTION ? bind<3, Q, 1, kAdvection, kUpwind>(c) : bind<3, Q, 5, kEuler, kRoePike>(c);
+}
+#elif DGPU_PART == 3
+template <int Q>
+cudaError_t bind_3d_lf(dgpu_ctx* c) { return bind<3, Q, 5, kEuler, kLaxFriedrichs>(c); }
+#elif DGPU_PART == 4
+template <int Q>
+cudaError_t bind_3d_ns_roe(dgpu_ctx* c) { return bind_ns<3, Q, kRoePike>(c); }
+#elif DGPU_PART == 5
+template <int Q>
+cudaError_t bind_3d_ns_lf(dgpu_ctx* c) { return bind_ns<3, Q, kLaxFriedrichs>(c); }
+#endif
+
+}  // namespace
+
+#if DGPU_PART == 1
+cudaError_t dgpu_bind_2d(dgpu_ctx* c) { DGPU_FOR_Q(c, bind_2d) }
+#elif DGPU_PART == 2
+cudaError_t dgpu_bind_3d_advection_roe(dgpu_ctx* c) { DGPU_FOR_Q(c, bind_3d_advection_roe) }
+#elif DGPU_PART == 3
+cudaError_t dgpu_bind_3d_lf(dgpu_ctx* c) { DGPU_FOR_Q(c, bind_3d_lf) }
+#elif DGPU_PART == 4
+cudaError_t dgpu_bind_3d_ns_roe(dgpu_ctx* c) { DGPU_FOR_Q(c, bind_3d_ns_roe) }
+#elif DGPU_PART == 5
+cudaError_t dgpu_bind_3d_ns_lf(dgpu_ctx* c) { DGPU_FOR_Q(c, bind_3d_ns_lf) }
+#else   // the host code, to the end of the file
+
+namespace {
+
+// Sets the launchers of the context's dimension, order, PDE and flux.
+cudaError_t bind_context(dgpu_ctx* c)
+{
+	if (c->d == 2)
+		return dgpu_bind_2d(c);
+	const bool lf = c->pde != DGPU_PDE_ADVECTION && c->flux != DGPU_NUM_FLUX_ROE_PIKE;
+	const cudaError_t e = lf ? dgpu_bind_3d_lf(c) : dgpu_bind_3d_advection_roe(c);
+	if (e != cudaSuccess || c->pde != DGPU_PDE_NAVIER_STOKES)
+		return e;
+	return lf ? dgpu_bind_3d_ns_lf(c) : dgpu_bind_3d_ns_roe(c);
 }
 
 // Drops the captured step graphs (they hold the kernels' parameters by value: a stream or a buffer that changes makes
@@ -1287,7 +1338,7 @@ dgpu_status dgpu_create(const dgpu_physics* phys, const dgpu_tp_operators* ops, 
 		DG_TRY(cudaGetLastError());
 		DG_TRY(cudaStreamSynchronize(c->stream));
 	}
-	cudaError_t be = (d == 2 ? bind_q<2>(c) : bind_q<3>(c));
+	cudaError_t be = bind_context(c);
 	if (be != cudaSuccess) {
 		std::string m_ = std::string("kernel set-up: ") + cudaGetErrorString(be);
 		free_all(c);
@@ -1962,28 +2013,8 @@ extern "C" dgpu_status dgpu_compute_rhs_noalloc(const dgpu_physics* phys, const 
 	c.n_face = d_mesh->n_faces;
 	for (int k = 0; k < 3; ++k)
 		c.b_adv[k] = phys->b_adv[k];
-	memset(&c.ops, 0, sizeof c.ops);
-	double Bm[kQMax * kQMax], Bi[kQMax * kQMax];
-	for (int i = 0; i < q * q; ++i)
-		Bm[i] = ops->cv0_vs_vc[i];
-	if (!host_invert_small(q, Bm, Bi))
+	if (!derive_tp_ops(ops, d, &c.ops))
 		return fail(nullptr, DGPU_ERR_INVALID_ARGUMENT, "cv0_vs_vc is singular");
-	for (int a = 0; a < q; ++a)
-		for (int m = 0; m < q; ++m) {
-			c.ops.B[a][m] = Bm[a * q + m];
-			c.ops.Binv[a][m] = Bi[a * q + m];
-			double s = 0.0;
-			for (int k = 0; k < q; ++k)
-				s += ops->cv1_vs_vc[a * q + k] * Bi[k * q + m];
-			c.ops.Dgl[a][m] = s;
-		}
-	for (int s = 0; s < 2; ++s)
-		for (int m = 0; m < q; ++m) {
-			double acc = 0.0;
-			for (int k = 0; k < q; ++k)
-				acc += ops->cv0_vs_fc[s * q + k] * Bi[k * q + m];
-			c.ops.lb[s][m] = acc;
-		}
 	NoallocWeights W;
 	memset(&W, 0, sizeof W);
 	for (int n = 0; n < N; ++n) {
@@ -2042,7 +2073,7 @@ extern "C" dgpu_status dgpu_compute_rhs_noalloc(const dgpu_physics* phys, const 
 		            "bad mesh: a face index, local face, permutation or jacobian_det_vc is out of range");
 
 	// the residual kernels of dgpu_compute_rhs, unchanged, on the scratch views
-	DGPU_CUDA(nullptr, d == 2 ? bind_q<2>(&c) : bind_q<3>(&c));
+	DGPU_CUDA(nullptr, bind_context(&c));
 	DGPU_CUDA(nullptr, c.launch_volume(&c));
 	DGPU_CUDA(nullptr, c.launch_face(&c));
 	DGPU_CUDA(nullptr, c.launch_lift_rhs(&c));
@@ -2804,3 +2835,5 @@ extern "C" dgpu_status dgpu_set_source(dgpu_ctx* c, const double* source_vc)
 	DGPU_CUDA(c, cudaStreamSynchronize(c->stream));
 	return DGPU_OK;
 }
+
+#endif   // DGPU_PART == 0

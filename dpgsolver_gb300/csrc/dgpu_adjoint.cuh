@@ -442,7 +442,7 @@ tp_objective_kernel(const TPParams P, const int* __restrict__ faces, int n_obj, 
 }
 
 // out = a x + b y + c z (z may be null), elementwise over n doubles.
-__global__ void __launch_bounds__(256)
+static __global__ void __launch_bounds__(256)
 lincomb_kernel(size_t n, double a, const double* x, double b, const double* y, double c, const double* z,
                double* out)
 {

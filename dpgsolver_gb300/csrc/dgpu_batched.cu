@@ -22,9 +22,18 @@
 
 using namespace dgpu;
 
-namespace {
+// Compiled once for the host code (DGPU_PART 0) and once per part, each of which defines one of the functions below, that
+// set a context's launchers.
+#ifndef DGPU_PART
+#error "compile with -DDGPU_PART=0..4"
+#endif
+cudaError_t dgpu_batch_bind_2d(dgpu_batch* c);                  // part 1: every PDE
+cudaError_t dgpu_batch_bind_3d_advection_roe(dgpu_batch* c);    // part 2: advection, Euler with Roe-Pike
+cudaError_t dgpu_batch_bind_3d_lf(dgpu_batch* c);               // part 3: Euler with Lax-Friedrichs
+cudaError_t dgpu_batch_bind_3d_ns(dgpu_batch* c);               // part 4: Navier-Stokes on top of Euler
 
-thread_local std::string g_batch_error;
+namespace dgpu {
+
 constexpr int kBranches = 16;   // streams of the branch form
 
 struct GroupLaunch {
@@ -39,7 +48,7 @@ struct GroupLaunch {
 	int idx = 0;        // index among the TP or among the dense groups
 };
 
-}  // namespace
+}  // namespace dgpu
 
 struct dgpu_batch {
 	int d = 0, nv = 0, pde = 0, flux = 0, positivity = 0;
@@ -152,7 +161,9 @@ struct dgpu_batch {
 
 namespace {
 
-dgpu_status bfail(dgpu_batch* c, dgpu_status st, const std::string& m)
+thread_local std::string g_batch_error;
+
+[[maybe_unused]] dgpu_status bfail(dgpu_batch* c, dgpu_status st, const std::string& m)
 {
 	if (c)
 		c->err = m;
@@ -174,12 +185,13 @@ template <int D, int Q, int NV>
 size_t blift_smem(int E) { return sizeof(BatchOps) + (size_t)E * BSmem<D, Q, NV>::LIFT * sizeof(double); }
 template <int D, int Q, int NV>
 size_t bconv_smem(int E) { return sizeof(BatchOps) + (size_t)E * 3 * NV * TPShape<D, Q>::N * sizeof(double); }
-size_t dvol_smem(int, const DGroup& G, int E) { return (size_t)E * G.vol_per_e * sizeof(double); }
-size_t dlift_smem(int, const DGroup& G, int E) { return (size_t)E * G.lift_per_e * sizeof(double); }
+[[maybe_unused]] size_t dvol_smem(int, const DGroup& G, int E) { return (size_t)E * G.vol_per_e * sizeof(double); }
+[[maybe_unused]] size_t dlift_smem(int, const DGroup& G, int E) { return (size_t)E * G.lift_per_e * sizeof(double); }
 
-int threads_for(int E, int N) { return ((E * N + 31) / 32) * 32; }
+// Whole warps, and at least four: the faces' interpolation between orders takes every thread of the CTA.
+[[maybe_unused]] int threads_for(int E, int N) { return std::max(((E * N + 31) / 32) * 32, 128); }
 
-RkArgs rk_args(const dgpu_batch* c, double dt, int stage, int want_max)
+[[maybe_unused]] RkArgs rk_args(const dgpu_batch* c, double dt, int stage, int want_max)
 {
 	RkArgs rk;
 	rk.u = c->ug;
@@ -278,7 +290,7 @@ cudaError_t launch_dlift(dgpu_batch* c, int g, int mode, double dt, int stage, i
 }
 
 // the RK state of a dense group is its coefficient vector: u <-> ug is a copy of the group's range
-cudaError_t copy_dense(dgpu_batch* c, int g, bool to_gl)
+[[maybe_unused]] cudaError_t copy_dense(dgpu_batch* c, int g, bool to_gl)
 {
 	const DGroup& G = c->hdgroups[c->gl[g].idx];
 	if (G.n_vol == 0)
@@ -588,30 +600,42 @@ cudaError_t bind_ns(dgpu_batch* c)
 	return cudaSuccess;
 }
 
+}  // namespace
+
+#if DGPU_PART == 1
+cudaError_t dgpu_batch_bind_2d(dgpu_batch* c)
+{
+	if (c->pde == DGPU_PDE_ADVECTION)
+		return bind_all<2, 1, kAdvection, kUpwind>(c);
+	const bool roe = c->flux == DGPU_NUM_FLUX_ROE_PIKE;
+	const cudaError_t e = roe ? bind_all<2, 4, kEuler, kRoePike>(c) : bind_all<2, 4, kEuler, kLaxFriedrichs>(c);
+	if (e != cudaSuccess || !c->navier_stokes)   // Navier-Stokes: the lift and conversion kernels are the Euler ones
+		return e;
+	return roe ? bind_ns<2, kRoePike>(c) : bind_ns<2, kLaxFriedrichs>(c);
+}
+#elif DGPU_PART == 2
+cudaError_t dgpu_batch_bind_3d_advection_roe(dgpu_batch* c)
+{
+	return c->pde == DGPU_PDE_ADVECTION ? bind_all<3, 1, kAdvection, kUpwind>(c) : bind_all<3, 5, kEuler, kRoePike>(c);
+}
+#elif DGPU_PART == 3
+cudaError_t dgpu_batch_bind_3d_lf(dgpu_batch* c) { return bind_all<3, 5, kEuler, kLaxFriedrichs>(c); }
+#elif DGPU_PART == 4
+cudaError_t dgpu_batch_bind_3d_ns(dgpu_batch* c)
+{
+	return c->flux == DGPU_NUM_FLUX_ROE_PIKE ? bind_ns<3, kRoePike>(c) : bind_ns<3, kLaxFriedrichs>(c);
+}
+#else   // the host code, to the end of the file
+
+namespace {
+
 cudaError_t bind(dgpu_batch* c)
 {
-	if (c->navier_stokes) {   // the lift and conversion kernels are the Euler ones
-		cudaError_t e;
-		if (c->d == 2)
-			e = c->flux == DGPU_NUM_FLUX_ROE_PIKE ? bind_all<2, 4, kEuler, kRoePike>(c)
-			                                      : bind_all<2, 4, kEuler, kLaxFriedrichs>(c);
-		else
-			e = c->flux == DGPU_NUM_FLUX_ROE_PIKE ? bind_all<3, 5, kEuler, kRoePike>(c)
-			                                      : bind_all<3, 5, kEuler, kLaxFriedrichs>(c);
-		if (e != cudaSuccess)
-			return e;
-		if (c->d == 2)
-			return c->flux == DGPU_NUM_FLUX_ROE_PIKE ? bind_ns<2, kRoePike>(c) : bind_ns<2, kLaxFriedrichs>(c);
-		return c->flux == DGPU_NUM_FLUX_ROE_PIKE ? bind_ns<3, kRoePike>(c) : bind_ns<3, kLaxFriedrichs>(c);
-	}
-	if (c->d == 2) {
-		if (c->pde == DGPU_PDE_ADVECTION) return bind_all<2, 1, kAdvection, kUpwind>(c);
-		if (c->flux == DGPU_NUM_FLUX_ROE_PIKE) return bind_all<2, 4, kEuler, kRoePike>(c);
-		return bind_all<2, 4, kEuler, kLaxFriedrichs>(c);
-	}
-	if (c->pde == DGPU_PDE_ADVECTION) return bind_all<3, 1, kAdvection, kUpwind>(c);
-	if (c->flux == DGPU_NUM_FLUX_ROE_PIKE) return bind_all<3, 5, kEuler, kRoePike>(c);
-	return bind_all<3, 5, kEuler, kLaxFriedrichs>(c);
+	if (c->d == 2)
+		return dgpu_batch_bind_2d(c);
+	const bool lf = c->pde != DGPU_PDE_ADVECTION && c->flux != DGPU_NUM_FLUX_ROE_PIKE;
+	const cudaError_t e = lf ? dgpu_batch_bind_3d_lf(c) : dgpu_batch_bind_3d_advection_roe(c);
+	return e != cudaSuccess || !c->navier_stokes ? e : dgpu_batch_bind_3d_ns(c);
 }
 
 void drop_graphs(dgpu_batch* c)
@@ -1030,6 +1054,26 @@ dgpu_status create_impl(const dgpu_physics* phys, const std::vector<GroupIn>& gi
 				for (int i = 0; i < qf; ++i)
 					for (int a = 0; a < q; ++a)
 						c->hops[t].Iup[qf][i][a] = lagrange_value(xq, q, a, xf[i]);
+				// rows (interpolation) and columns (its transpose) of one scale
+				double sum = 0.0, mx = 0.0;
+				for (int i = 0; i < qf; ++i) {
+					double r = 0.0;
+					for (int a = 0; a < q; ++a) {
+						r += fabs(c->hops[t].Iup[qf][i][a]);
+						mx = std::max(mx, fabs(c->hops[t].Iup[qf][i][a]));
+					}
+					sum = std::max(sum, r);
+				}
+				for (int a = 0; a < q; ++a) {
+					double r = 0.0;
+					for (int i = 0; i < qf; ++i)
+						r += fabs(c->hops[t].Iup[qf][i][a]);
+					sum = std::max(sum, r);
+				}
+				c->hops[t].sI[qf] = fix_shift(sum, mx, 62);
+				for (int i = 0; i < qf; ++i)
+					for (int a = 0; a < q; ++a)
+						c->hops[t].fI[qf][i][a] = fix_entry(c->hops[t].Iup[qf][i][a], c->hops[t].sI[qf]);
 			}
 			c->hgroups[t].q = q;
 			const int N = (d == 2 ? q * q : q * q * q);
@@ -2013,3 +2057,5 @@ dgpu_status dgpu_batch_positivity_corrections(dgpu_batch* c, long long* n)
 }
 
 }  // extern "C"
+
+#endif   // DGPU_PART == 0

@@ -21,6 +21,8 @@ constexpr int kMaxOrd = 8;      // face orientations (QUAD faces)
 struct BatchOps {
 	TPOps t;
 	double Iup[kQMax + 1][kQMax][kQMax];   // Iup[qf][i][a]: GL(q) Lagrange a at GL(qf) node i, qf >= q
+	FixW fI[kQMax + 1][kQMax][kQMax];      // Iup in fixed point (dgpu_fix.cuh), as a 1D pass in both directions
+	int sI[kQMax + 3];                     // its scales
 };
 static_assert(sizeof(BatchOps) % 8 == 0, "BatchOps is copied to shared memory as doubles");
 
@@ -124,10 +126,27 @@ struct BSmem {
 	static constexpr int NFQ = TPShape<D, Q>::NF;
 	static constexpr int VX = NV * N * 2 + D * NV * N + 2 * D * NV * NFQ;    // su, st, sf, own-order traces
 	static constexpr int LX = 3 * NV * N + 2 * D * NV * NFQ;                 // sa, sb, sc, face terms
-	// then the block exponents (ints) of dgpu_fix.cuh
-	static constexpr int VOL = VX + (TPSmem<D, Q, NV>::EXP + TPSmem<D, Q, NV>::AEXP + 1) / 2;
-	static constexpr int LIFT = LX + (TPSmem<D, Q, NV>::LEXP + 1) / 2;
+	// then the element's faces (bface_table) and the block exponents (ints) of dgpu_fix.cuh
+	static constexpr int VOL = VX + 6 * D + (TPSmem<D, Q, NV>::EXP + TPSmem<D, Q, NV>::AEXP + 1) / 2;
+	static constexpr int LIFT = LX + 6 * D + (TPSmem<D, Q, NV>::LEXP + 1) / 2;
 };
+
+// The faces of a QUAD/HEX element, read once into shared memory (2D entries).
+struct BFace {
+	long long base;   // first face node
+	int side, qf, pad[2];
+};
+static_assert(sizeof(BFace) == 24, "three doubles per face");
+
+__device__ __forceinline__ void bface_table(const BParams& P, long long v, int n, int node, int N, BFace* t)
+{
+	for (int lf = node; lf < n; lf += N) {
+		const int4 fd = P.elf[v * kMaxLf + lf];
+		t[lf].base = P.fbase[fd.x];
+		t[lf].side = fd.y;
+		t[lf].qf = fd.z;
+	}
+}
 
 // ---------------------------------------------------------------------------------------------------------------
 // Volume term + traces at each face's order
@@ -146,7 +165,8 @@ __device__ void bvol_body(const BParams& P, const BatchOps* sops, const BGroup& 
 	double* st = su + NV * N;
 	double* sf = st + NV * N;
 	double* str = sf + D * NV * N;   // [lf][NV][NFQ]
-	int* sx = reinterpret_cast<int*>(base + BSmem<D, Q, NV>::VX);   // element 0's block exponents, 2 PER_E ints apart
+	BFace* tab = reinterpret_cast<BFace*>(su + BSmem<D, Q, NV>::VX);
+	int* sx = reinterpret_cast<int*>(base + BSmem<D, Q, NV>::VX + 6 * D);   // element 0's exponents, 2 PER_E ints apart
 	double W[NV];
 	if (active) {
 		const double* ublk = u + G.state_off + (long long)(e0 + e) * NV * N + node;
@@ -155,11 +175,11 @@ __device__ void bvol_body(const BParams& P, const BatchOps* sops, const BGroup& 
 			W[k] = ublk[k * N];
 		for (int i = node; i < XE + AE; i += N)
 			sx[e * 2 * PER_E + i] = 0;
+		bface_table(P, G.elem0 + e0 + e, 2 * D, node, N, tab);
 	}
 	__syncthreads();
 	if (GLL_IN)
 		tp_apply_fix<D, Q, NV, true>(W, su, st, sops->t.fB, sops->t.sB, sops->t.B, e, node, active, sx + XE, 2 * PER_E);
-	const long long v = G.elem0 + e0 + e;   // group-sorted element index
 	double fr[D][NV];
 	if (active) {
 		double g[D * D];
@@ -172,14 +192,35 @@ __device__ void bvol_body(const BParams& P, const BatchOps* sops, const BGroup& 
 	int eb[2 * NV];
 	const bool ok = tp_stage_volume<D, Q, NV>(W, fr, e, node, active, su, sf, sx, 2 * PER_E, eb);
 	if (active) {
-		// traces at this element's own GL points, all faces, into shared memory
+		// traces at this element's own GL points: written out where the face has them (q_f == Q), kept as limbs (or as
+		// doubles out of range) where the face's order is higher
 		double out[NV];
 		for (int it = node; it < 2 * D * NFQ; it += N) {
 			const int lf = it / NFQ, t = it % NFQ;
-			tp_trace<D, Q, NV>(&sops->t, su, eb, ok, lf, t, out);
+			if (tab[lf].qf == Q) {
+				tp_trace<D, Q, NV>(&sops->t, su, eb, ok, lf, t, out);
+				double* dst = P.traces + 2 * NV * tab[lf].base + (long long)tab[lf].side * NV * NFQ;
 #pragma unroll
-			for (int k = 0; k < NV; ++k)
-				str[(lf * NV + k) * NFQ + t] = out[k];
+				for (int k = 0; k < NV; ++k)
+					dst[k * NFQ + t] = out[k];
+			} else if (ok) {
+				int stride, b0;
+				tp_face_line<D, Q>(lf, t, b0, stride);
+				const int2* xu = reinterpret_cast<const int2*>(su) + b0;
+#pragma unroll
+				for (int k = 0; k < NV; ++k) {
+					FixAcc s = {0, 0};
+#pragma unroll
+					for (int m = 0; m < Q; ++m)
+						fix_mac(s, sops->t.fT[lf & 1][m], xu[k * N + m * stride]);
+					reinterpret_cast<int2*>(str)[(lf * NV + k) * NFQ + t] = fix_limbs(s.h * 4 + (s.m >> 28));
+				}
+			} else {
+				tp_trace<D, Q, NV>(&sops->t, su, eb, ok, lf, t, out);
+#pragma unroll
+				for (int k = 0; k < NV; ++k)
+					str[(lf * NV + k) * NFQ + t] = out[k];
+			}
 		}
 		// volume term in GL space
 		tp_derivative<D, Q, NV>(&sops->t, sf, eb, ok, node, out);
@@ -188,52 +229,65 @@ __device__ void bvol_body(const BParams& P, const BatchOps* sops, const BGroup& 
 		for (int k = 0; k < NV; ++k)
 			vg[k * N + node] = out[k];
 	}
+	if (active && node == 0)
+		sx[e * 2 * PER_E + XE] = ok;   // for the threads of the CTA that interpolate this element's traces
 	__syncthreads();
-	if (active) {
-		// traces at each face's order: copy (q_f == Q) or tangential interpolation Q -> q_f. In 3D the
-		// interpolation is separable: a thread takes one (variable, i0) column, contracts the first tangential
-		// direction once per b (Q^2 FMAs) and reuses the Q partial sums for all q_f outputs i1.
-		const int4* ef = P.elf + v * kMaxLf;
-		for (int lf = 0; lf < 2 * D; ++lf) {
-			const int4 fd = ef[lf];
-			const int qf = fd.z;
-			const int nff = (D == 2 ? qf : qf * qf);
-			double* dst = P.traces + 2 * NV * P.fbase[fd.x] + (long long)fd.y * NV * nff;
-			const double* src = str + lf * NV * NFQ;
-			if (qf == Q) {
-				for (int it = node; it < NV * nff; it += N)
-					dst[it] = src[it];
+	{
+		// the traces of the higher-order faces: tangential interpolation Q -> q_f, separable in 3D. A thread takes one
+		// (element, face, variable, i0) column, contracts the first tangential direction once per b and reuses the Q
+		// partial sums for all q_f outputs i1. In fixed point, the block exponent rising by each pass's 62 - s.
+		constexpr int NI = 2 * D * NV * kQMax;
+		for (int t = tid; t < n_here * NI; t += blockDim.x) {
+			const int e = t / NI, it = t % NI;
+			const double* str = base + e * PER_E + 2 * NV * N + D * NV * N;
+			const BFace* tab = reinterpret_cast<const BFace*>(base + e * PER_E + BSmem<D, Q, NV>::VX);
+			const int lf = it / (NV * kQMax), k = it / kQMax % NV, i0 = it % kQMax, qf = tab[lf].qf;
+			if (qf == Q || i0 >= qf)
 				continue;
-			}
-			const double(*I)[kQMax] = sops->Iup[qf];
-			if (D == 2) {
-				for (int it = node; it < NV * qf; it += N) {
-					const int k = it / qf, i = it % qf;
-					double s = 0.0;
+			const bool ok = sx[e * 2 * PER_E + XE] != 0;
+			const int nff = (D == 2 ? qf : qf * qf);
+			double* dst = P.traces + 2 * NV * tab[lf].base + (long long)tab[lf].side * NV * nff + k * nff + i0;
+			if (ok) {
+				const int2* src = reinterpret_cast<const int2*>(str) + (lf * NV + k) * NFQ;
+				const FixW* I0 = sops->fI[qf][i0];
+				const int sI = sops->sI[qf];
+				const int e1 = fix_block(sx[e * 2 * PER_E + k]) + 62 - sops->t.sT;
+				if (D == 2) {
+					FixAcc s = {0, 0};
 #pragma unroll
 					for (int a = 0; a < Q; ++a)
-						s += I[i][a] * src[k * NFQ + a];
-					dst[k * qf + i] = s;
-				}
-			} else {
-				for (int it = node; it < NV * qf; it += N) {
-					const int k = it / qf, i0 = it % qf;
-					double r[Q];
+						fix_mac(s, I0[a], src[a]);
+					dst[0] = fix_to_double(fix_sum(s), fix_scale(e1, sI));
+				} else {
+					int2 r[Q];
 #pragma unroll
 					for (int b = 0; b < Q; ++b) {
-						double acc = 0.0;
+						FixAcc s = {0, 0};
 #pragma unroll
 						for (int a = 0; a < Q; ++a)
-							acc += I[i0][a] * src[k * NFQ + a + Q * b];
-						r[b] = acc;
+							fix_mac(s, I0[a], src[a + Q * b]);
+						r[b] = fix_limbs(s.h * 4 + (s.m >> 28));
 					}
 					for (int i1 = 0; i1 < qf; ++i1) {
-						double s = 0.0;
+						FixAcc s = {0, 0};
 #pragma unroll
 						for (int b = 0; b < Q; ++b)
-							s += I[i1][b] * r[b];
-						dst[k * nff + i0 + qf * i1] = s;
+							fix_mac(s, sops->fI[qf][i1][b], r[b]);
+						dst[qf * i1] = fix_to_double(fix_sum(s), fix_scale(e1 + 62 - sI, sI));
 					}
+				}
+			} else {
+				const double* src = str + (lf * NV + k) * NFQ;
+				const double(*I)[kQMax] = sops->Iup[qf];
+				for (int i1 = 0; i1 < (D == 2 ? 1 : qf); ++i1) {
+					double s = 0.0;
+					for (int b = 0; b < (D == 2 ? 1 : Q); ++b) {
+						double r = 0.0;
+						for (int a = 0; a < Q; ++a)
+							r = fma(I[i0][a], src[a + Q * b], r);
+						s = D == 2 ? r : fma(I[i1][b], r, s);
+					}
+					dst[qf * i1] = s;
 				}
 			}
 		}
@@ -314,66 +368,98 @@ __device__ void blift_body(const BParams& P, const BatchOps* sops, const BGroup&
 	double* sb = sa + NV * N;
 	double* sc = sb + NV * N;
 	double* sg = sc + NV * N;            // [lf][NV][NFQ]: E_lf^T-side face terms at this element's points
-	constexpr int AE = TPSmem<D, Q, NV>::AEXP, SX = 2 * PER_E;
-	int* sx = reinterpret_cast<int*>(base + BSmem<D, Q, NV>::LX);   // element 0's block exponents, SX ints apart
+	constexpr int SX = 2 * PER_E;
+	BFace* tab = reinterpret_cast<BFace*>(sa + BSmem<D, Q, NV>::LX);
+	int* sx = reinterpret_cast<int*>(base + BSmem<D, Q, NV>::LX + 6 * D);   // element 0's block exponents, SX ints apart
 	const int* sscale = sx + e * SX + NV;   // FP32 scales of the positivity pre-filter
-	const long long v = G.elem0 + e0 + e;
 	if (active) {
 		for (int i = node; i < TPSmem<D, Q, NV>::LEXP; i += N)
 			sx[e * SX + i] = 0;
-		// face terms at the element's own points: copy (q_f == Q) or transposed interpolation q_f -> Q
-		// (separable in 3D: a thread takes one (variable, a) column, contracts i0 for every i1 once and reuses
-		// the q_f partial sums for all Q outputs b).
-		const int4* ef = P.elf + v * kMaxLf;
-		for (int lf = 0; lf < 2 * D; ++lf) {
-			const int4 fd = ef[lf];
-			const int qf = fd.z;
-			const int nff = (D == 2 ? qf : qf * qf);
-			const long long fb = P.fbase[fd.x];
-			const double* src = P.nnf + NV * fb;
-			const double sgn = (fd.y == 0 ? -1.0 : 1.0);   // side 0: rhs -= ; side 1: rhs -= (-nnf)
+		bface_table(P, G.elem0 + e0 + e, 2 * D, node, N, tab);
+	}
+	__syncthreads();
+	{
+		// face terms at the element's own points: copy (q_f == Q) or transposed interpolation q_f -> Q (separable in 3D).
+		// A thread takes one (element, face, variable, a) column: the face's values of the variable are one block; it
+		// contracts i0 for every i1 and reuses the q_f partial sums for all Q outputs b.
+		constexpr int NI = 2 * D * NV * Q;
+		for (int t = tid; t < n_here * NI; t += blockDim.x) {
+			const int e = t / NI, it = t % NI;
+			double* sg = base + e * PER_E + 3 * NV * N;
+			const BFace* tab = reinterpret_cast<const BFace*>(base + e * PER_E + BSmem<D, Q, NV>::LX);
+			const int lf = it / (NV * Q), k = it / Q % NV, a = it % Q;
+			const int qf = tab[lf].qf, nff = (D == 2 ? qf : qf * qf);
+			const long long fb = tab[lf].base;
+			const double* src = P.nnf + NV * fb + k * nff;
+			const bool flip = tab[lf].side == 0;   // side 0: rhs -= ; side 1: rhs -= (-nnf)
 			// side 1 reads the face flux (side 0's node order) at its own nodes through the inverse permutation
-			const int* ci = (fd.y == 1 && P.nc_inv) ? P.nc_inv + fb : nullptr;
-			double* out = sg + lf * NV * NFQ;
+			const int* ci = (!flip && P.nc_inv) ? P.nc_inv + fb : nullptr;
+			double* out = sg + (lf * NV + k) * NFQ + a;
 			if (qf == Q) {
-				for (int it = node; it < NV * NFQ; it += N) {
-					const int k = it / NFQ, i = it % NFQ;
-					out[it] = sgn * src[k * NFQ + (ci ? ci[i] : i)];
+#pragma unroll
+				for (int b = 0; b < (D == 2 ? 1 : Q); ++b) {
+					const int i = a + Q * b;
+					const double x = src[ci ? ci[i] : i];
+					out[Q * b] = flip ? -x : x;
 				}
 				continue;
 			}
-			const double(*I)[kQMax] = sops->Iup[qf];
-			if (D == 2) {
-				for (int it = node; it < NV * Q; it += N) {
-					const int k = it / Q, t = it % Q;
-					double s = 0.0;
-					for (int i = 0; i < qf; ++i)
-						s += I[i][t] * src[k * qf + (ci ? ci[i] : i)];
-					out[k * NFQ + t] = sgn * s;
-				}
-			} else {
-				for (int it = node; it < NV * Q; it += N) {
-					const int k = it / Q, a = it % Q;
-					double r[kQMax];
+			constexpr int N1 = (D == 2 ? 1 : kQMax);
+			// the block exponent first (high words, all loads in flight), the values row by row after it
+			int xe = 0;
 #pragma unroll
-					for (int i1 = 0; i1 < kQMax; ++i1) {
-						double acc = 0.0;
-						if (i1 < qf)
-							for (int i0 = 0; i0 < qf; ++i0) {
-								const int i = i0 + qf * i1;
-								acc += I[i0][a] * src[k * nff + (ci ? ci[i] : i)];
-							}
-						r[i1] = acc;
+			for (int i1 = 0; i1 < N1; ++i1)
+#pragma unroll
+				for (int i0 = 0; i0 < kQMax; ++i0) {
+					const int i = i0 + qf * i1;
+					if (i0 < qf && (D == 2 || i1 < qf))
+						xe = max(xe, (reinterpret_cast<const int*>(src)[2 * (ci ? ci[i] : i) + 1] >> 20) & 0x7ff);
+				}
+			if (fix_in_range(xe)) {
+				const int eb = fix_block(xe), sI = sops->sI[qf];
+				int2 r[N1];
+#pragma unroll
+				for (int i1 = 0; i1 < N1; ++i1) {
+					double x[kQMax];
+#pragma unroll
+					for (int i0 = 0; i0 < kQMax; ++i0) {
+						const int i = i0 + qf * i1;
+						x[i0] = (i0 < qf && (D == 2 || i1 < qf)) ? src[ci ? ci[i] : i] : 0.0;
 					}
+					FixAcc s = {0, 0};
+#pragma unroll
+					for (int i0 = 0; i0 < kQMax; ++i0)
+						fix_mac(s, sops->fI[qf][i0][a], fix_pack(x[i0], eb));   // entries beyond q_f are zero
+					if (D == 2) {
+						const double t = fix_to_double(fix_sum(s), fix_scale(eb, sI));
+						out[0] = flip ? -t : t;
+					}
+					r[i1] = fix_limbs(s.h * 4 + (s.m >> 28));
+				}
+				if (D == 3) {
 #pragma unroll
 					for (int bb = 0; bb < Q; ++bb) {
-						double s = 0.0;
+						FixAcc s = {0, 0};
 #pragma unroll
-						for (int i1 = 0; i1 < kQMax; ++i1)
-							if (i1 < qf)
-								s += I[i1][bb] * r[i1];
-						out[k * NFQ + a + Q * bb] = sgn * s;
+						for (int i1 = 0; i1 < N1; ++i1)
+							fix_mac(s, sops->fI[qf][i1][bb], r[i1]);
+						const double t = fix_to_double(fix_sum(s), fix_scale(eb + 62 - sI, sI));
+						out[Q * bb] = flip ? -t : t;
 					}
+				}
+			} else {
+#pragma unroll 1
+				for (int bb = 0; bb < (D == 2 ? 1 : Q); ++bb) {
+					double s = 0.0;
+					for (int i1 = 0; i1 < (D == 2 ? 1 : qf); ++i1) {
+						double r = 0.0;
+						for (int i0 = 0; i0 < qf; ++i0) {
+							const int i = i0 + qf * i1;
+							r = fma(sops->Iup[qf][i0][a], src[ci ? ci[i] : i], r);
+						}
+						s = D == 2 ? r : fma(sops->Iup[qf][i1][bb], r, s);
+					}
+					out[Q * bb] = flip ? -s : s;
 				}
 			}
 		}

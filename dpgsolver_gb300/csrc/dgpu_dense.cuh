@@ -55,27 +55,30 @@ __device__ __forceinline__ void blk_max(double* smem, int PER_E, int n_here, int
 	}
 }
 
+// Whether all of the element's blocks of the set are in range, as blk_pack left it.
 template <int NV>
 __device__ __forceinline__ bool blk_ok(const double* smem, int PER_E, int e, int xo, int slot)
 {
-	const int* x = reinterpret_cast<const int*>(smem + e * PER_E + xo) + slot;
-	bool ok = true;
-#pragma unroll
-	for (int k = 0; k < NV; ++k)
-		ok = ok && fix_in_range(x[k]);
-	return ok;
+	return reinterpret_cast<const int*>(smem + e * PER_E + xo)[2 * NV + (slot ? 1 : 0)] != 0;
 }
 
-// The values packed in place, for the elements in range.
+// The values packed in place, for the elements in range, and the flags of blk_ok.
 template <int NV>
 __device__ __forceinline__ void blk_pack(double* smem, int PER_E, int n_here, int off, int len, int xo, int slot)
 {
 	const int lane = threadIdx.x & 31;
 	for (int p = threadIdx.x >> 5; p < n_here * NV; p += blockDim.x >> 5) {
 		const int e = p / NV, k = p % NV;
-		if (!blk_ok<NV>(smem, PER_E, e, xo, slot))
+		int* xe = reinterpret_cast<int*>(smem + e * PER_E + xo);
+		bool ok = true;
+#pragma unroll
+		for (int j = 0; j < NV; ++j)
+			ok = ok && fix_in_range(xe[slot + j]);
+		if (k == 0 && lane == 0)
+			xe[2 * NV + (slot ? 1 : 0)] = ok;
+		if (!ok)
 			continue;
-		const int eb = fix_block(reinterpret_cast<const int*>(smem + e * PER_E + xo)[slot + k]);
+		const int eb = fix_block(xe[slot + k]);
 		double* x = smem + e * PER_E + off + k * len;
 		for (int i = lane; i < len; i += 32)
 			reinterpret_cast<int2*>(x)[i] = fix_pack(x[i], eb);
@@ -92,13 +95,16 @@ __device__ __forceinline__ FixW ldg_fix(const FixW* p)
 // sum |W| <= 2^66 (a row of hundreds of terms scaled by its sum alone would keep too few bits of each entry); the low
 // accumulator is folded into the high one every 16 products, exactly, which keeps it below 2^63, and leaves
 // 0 <= m < 2^30.
+// The terms are dealt to `split` lanes, of which this one is the part-th; fix_join adds the lanes' sums up (integers, so
+// the result does not depend on the split).
 template <int NV>
-__device__ __forceinline__ void fix_dot(FixAcc* acc, const FixW* op, int so, const int2* x, int len, int sx, int n)
+__device__ __forceinline__ void fix_dot(FixAcc* acc, const FixW* op, int so, const int2* x, int len, int sx, int n,
+                                        int part = 0, int split = 1)
 {
-	for (int i0 = 0; i0 < n; i0 += 16) {
-		const int i1 = min(n, i0 + 16);
+	for (int i0 = part; i0 < n; i0 += 16 * split) {
+		const int i1 = min(n, i0 + 16 * split);
 #pragma unroll 4
-		for (int i = i0; i < i1; ++i) {
+		for (int i = i0; i < i1; i += split) {
 			const FixW w = ldg_fix(op + (long long)i * so);
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
@@ -110,6 +116,34 @@ __device__ __forceinline__ void fix_dot(FixAcc* acc, const FixW* op, int so, con
 			acc[k].m &= (1ll << 30) - 1;
 		}
 	}
+}
+
+// Lanes of one output: split consecutive ones (a power of two). All lanes of the warp must call it.
+template <int NV>
+__device__ __forceinline__ void fix_join(FixAcc* acc, int split)
+{
+	for (int o = split >> 1; o > 0; o >>= 1)
+#pragma unroll
+		for (int k = 0; k < NV; ++k) {
+			acc[k].h += __shfl_xor_sync(0xffffffffu, acc[k].h, o);
+			acc[k].m += __shfl_xor_sync(0xffffffffu, acc[k].m, o);
+		}
+	if (split > 1)
+#pragma unroll
+		for (int k = 0; k < NV; ++k) {
+			acc[k].h += acc[k].m >> 30;
+			acc[k].m &= (1ll << 30) - 1;
+		}
+}
+
+// Lanes per output for n outputs of `terms` products each, on a CTA of 256 threads: as many as the idle threads allow while
+// a lane keeps 8 products.
+__device__ __forceinline__ int fix_split_for(int n, int terms)
+{
+	int sp = 1;
+	while (sp < 8 && n * sp * 2 <= 256 && terms >= 16 * sp)
+		sp *= 2;
+	return sp;
 }
 
 // The value of a folded sum (block eb, operator scale s).
@@ -124,24 +158,29 @@ __device__ __forceinline__ double fix_dot_value(const FixAcc& a, int eb, int s)
 template <int NV>
 __device__ void dtraces(const BParams& P, const DGroup& G, int e0, int n_here, const double* smem, int PER_E, int xo)
 {
-	const int nvs = G.n_vs, nfm = G.nff_max;
-	for (int it = threadIdx.x; it < n_here * G.n_lf * nfm; it += blockDim.x) {
-		const int i = it % nfm, el = it / nfm, lf = el % G.n_lf, e = el / G.n_lf;
+	const int nvs = G.n_vs, nfm = G.nff_max, n = n_here * G.n_lf * nfm, sp = fix_split_for(n, nvs);
+	for (int t0 = threadIdx.x & ~31; t0 < n * sp; t0 += blockDim.x) {   // whole warps: fix_join is a warp operation
+		const int t = t0 + (threadIdx.x & 31), it = t / sp;
+		const int i = it % nfm, el = it / nfm, lf = el % G.n_lf, e = min(el / G.n_lf, n_here - 1);
 		const long long v = G.elem0 + e0 + e;
 		const int4 fd = P.elf[v * kMaxLf + lf];
 		const long long fb = P.fbase[fd.x];
 		const int nff = (int)(P.fbase[fd.x + 1] - fb);
-		if (i >= nff)
-			continue;
+		const bool here = it < n && i < nff;
 		const long long o = G.fop_off[(lf * G.n_ord + fd.w) * (kQMax + 1) + fd.z];
 		const double* su = smem + e * PER_E;
+		const bool ok = blk_ok<NV>(smem, PER_E, e, xo, 0);
 		double W[NV];
-		if (blk_ok<NV>(smem, PER_E, e, xo, 0)) {
-			FixAcc acc[NV];
+		FixAcc acc[NV];
 #pragma unroll
-			for (int k = 0; k < NV; ++k)
-				acc[k] = {0, 0};
-			fix_dot<NV>(acc, G.xfT + o + i, nff, reinterpret_cast<const int2*>(su), nvs, 1, nvs);
+		for (int k = 0; k < NV; ++k)
+			acc[k] = {0, 0};
+		if (here && ok)
+			fix_dot<NV>(acc, G.xfT + o + i, nff, reinterpret_cast<const int2*>(su), nvs, 1, nvs, t % sp, sp);
+		fix_join<NV>(acc, sp);
+		if (!here || t % sp)
+			continue;
+		if (ok) {
 			const int* eb = reinterpret_cast<const int*>(su + xo);
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
@@ -330,17 +369,21 @@ __device__ void dvol_body(const BParams& P, const DGroup& G, int e0, int E, cons
 		dvol_prism_phases<D, NV, PDE>(P, G, e0, n_here, smem, PER_E, xo);
 	} else {
 		// phase 1: state at the cubature nodes, contravariant flux, w-weighted (w is folded into the metrics)
-		for (int it = threadIdx.x; it < n_here * nvc; it += blockDim.x) {
-			const int e = it / nvc, r = it % nvc;
-			if (!blk_ok<NV>(smem, PER_E, e, xo, 0))
-				continue;
-			const int* eb = reinterpret_cast<const int*>(smem + e * PER_E + xo);
+		const int n1 = n_here * nvc, s1 = fix_split_for(n1, nvs);
+		for (int t0 = threadIdx.x & ~31; t0 < n1 * s1; t0 += blockDim.x) {
+			const int t = t0 + (threadIdx.x & 31), it = min(t / s1, n1 - 1), e = it / nvc, r = it % nvc;
+			const bool ok = blk_ok<NV>(smem, PER_E, e, xo, 0);
 			FixAcc acc[NV];
 			double W[NV];
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
 				acc[k] = {0, 0};
-			fix_dot<NV>(acc, G.xcv0 + r, nvc, reinterpret_cast<const int2*>(smem + e * PER_E), nvs, 1, nvs);
+			if (ok)
+				fix_dot<NV>(acc, G.xcv0 + r, nvc, reinterpret_cast<const int2*>(smem + e * PER_E), nvs, 1, nvs, t % s1, s1);
+			fix_join<NV>(acc, s1);
+			if (!ok || t % s1 || t >= n1 * s1)
+				continue;
+			const int* eb = reinterpret_cast<const int*>(smem + e * PER_E + xo);
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
 				W[k] = fix_dot_value(acc[k], fix_block(eb[k]), G.s_cv0);
@@ -352,16 +395,21 @@ __device__ void dvol_body(const BParams& P, const DGroup& G, int e0, int E, cons
 		blk_pack<NV>(smem, PER_E, n_here, so, D * nvc, xo, NV);
 		__syncthreads();
 		// phase 2: rhs_vol[k][m] = sum_j sum_r cv1_j[r][m] sf[k][j][r]
-		for (int it = threadIdx.x; it < n_here * nvs; it += blockDim.x) {
-			const int e = it / nvs, m = it % nvs;
-			if (!blk_ok<NV>(smem, PER_E, e, xo, NV))
-				continue;
-			const int* eb = reinterpret_cast<const int*>(smem + e * PER_E + xo) + NV;
+		const int n2 = n_here * nvs, s2 = fix_split_for(n2, D * nvc);
+		for (int t0 = threadIdx.x & ~31; t0 < n2 * s2; t0 += blockDim.x) {
+			const int t = t0 + (threadIdx.x & 31), it = min(t / s2, n2 - 1), e = it / nvs, m = it % nvs;
+			const bool ok = blk_ok<NV>(smem, PER_E, e, xo, NV);
 			FixAcc acc[NV];
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
 				acc[k] = {0, 0};
-			fix_dot<NV>(acc, G.xcv1 + m, nvs, reinterpret_cast<const int2*>(smem + e * PER_E + so), D * nvc, 1, D * nvc);
+			if (ok)
+				fix_dot<NV>(acc, G.xcv1 + m, nvs, reinterpret_cast<const int2*>(smem + e * PER_E + so), D * nvc, 1, D * nvc,
+				            t % s2, s2);
+			fix_join<NV>(acc, s2);
+			if (!ok || t % s2 || t >= n2 * s2)
+				continue;
+			const int* eb = reinterpret_cast<const int*>(smem + e * PER_E + xo) + NV;
 			double* out = P.vol_gl + G.state_off + (long long)(e0 + e) * NV * nvs + m;
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
@@ -587,22 +635,28 @@ __device__ void dlift_body(const BParams& P, const DGroup& G, int e0, int E, con
 	__syncthreads();
 	blk_pack<NV>(smem, PER_E, n_here, fo, nft, xo, 0);
 	__syncthreads();
-	for (int it = threadIdx.x; it < n_here * nvs; it += blockDim.x) {
-		const int e = it / nvs, m = it % nvs;
+	const int n1 = n_here * nvs, s1 = fix_split_for(n1, nfm);
+	for (int t0 = threadIdx.x & ~31; t0 < n1 * s1; t0 += blockDim.x) {   // whole warps: fix_join is a warp operation
+		const int t = t0 + (threadIdx.x & 31), it = min(t / s1, n1 - 1), e = it / nvs, m = it % nvs;
 		const long long v = G.elem0 + e0 + e;
 		double* r = smem + e * PER_E + m;
-		if (blk_ok<NV>(smem, PER_E, e, xo, 0)) {
-			const int* eb = reinterpret_cast<const int*>(smem + e * PER_E + xo);
-			FixAcc acc[NV];
+		const bool ok = blk_ok<NV>(smem, PER_E, e, xo, 0);
+		FixAcc acc[NV];
 #pragma unroll
-			for (int k = 0; k < NV; ++k)
-				acc[k] = {0, 0};
+		for (int k = 0; k < NV; ++k)
+			acc[k] = {0, 0};
+		if (ok)
 			for (int lf = 0; lf < G.n_lf; ++lf) {
 				const int4 fd = P.elf[v * kMaxLf + lf];
 				const int nff = (int)(P.fbase[fd.x + 1] - P.fbase[fd.x]);
 				fix_dot<NV>(acc, G.xfL + G.fop_off[(lf * G.n_ord + fd.w) * (kQMax + 1) + fd.z] + m, nvs,
-				            reinterpret_cast<const int2*>(smem + e * PER_E + fo) + lf * nfm, nft, 1, nff);
+				            reinterpret_cast<const int2*>(smem + e * PER_E + fo) + lf * nfm, nft, 1, nff, t % s1, s1);
 			}
+		fix_join<NV>(acc, s1);
+		if (t % s1 || t >= n1 * s1)
+			continue;
+		if (ok) {
+			const int* eb = reinterpret_cast<const int*>(smem + e * PER_E + xo);
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
 				r[k * nvs] = add(r[k * nvs], fix_dot_value(acc[k], fix_block(eb[k]), G.s_f));
@@ -698,7 +752,7 @@ __host__ __device__ inline size_t dense_minv_smem(int nvs) { return (size_t)(2 *
 // volume_solver_T.c:115-145) formed in shared memory, then inverted by Gauss-Jordan elimination. M is symmetric
 // positive definite, so the pivots (Schur complements) are positive and no row exchange is needed.
 // cv0: n_vc x n_vs; wJ: per volume n_vc values w_n J_n; minv: per volume n_vs x n_vs row-major.
-__global__ void __launch_bounds__(128) dense_minv_kernel(const double* __restrict__ cv0,
+static __global__ void __launch_bounds__(128) dense_minv_kernel(const double* __restrict__ cv0,
                                                          const double* __restrict__ wJ, int nvs, int nvc,
                                                          int n_vol, double* __restrict__ minv)
 {
@@ -741,7 +795,7 @@ __global__ void __launch_bounds__(128) dense_minv_kernel(const double* __restric
 }
 
 template <int D, int NV, int PDE>
-__global__ void __launch_bounds__(256) dvol_group_kernel(const BParams P, int g, const double* __restrict__ u)
+__global__ void __launch_bounds__(256, 2) dvol_group_kernel(const BParams P, int g, const double* __restrict__ u)
 {
 	extern __shared__ double smem[];
 	const DGroup G = P.dgroups[g];
@@ -751,7 +805,7 @@ __global__ void __launch_bounds__(256) dvol_group_kernel(const BParams P, int g,
 }
 
 template <int NV, int MODE>
-__global__ void __launch_bounds__(256) dlift_group_kernel(const BParams P, int g, const RkArgs rk)
+__global__ void __launch_bounds__(256, 2) dlift_group_kernel(const BParams P, int g, const RkArgs rk)
 {
 	extern __shared__ double smem[];
 	const DGroup G = P.dgroups[g];

@@ -78,7 +78,7 @@ __device__ __forceinline__ void geo_pass(const double* in, double* out, const in
 // Shared memory of geo_volume_kernel, in doubles: X, Jm, mvm, V, dV, mvc, Jc and two pass temporaries.
 constexpr int kGeoSmem = (3 + 9 + 9 + 3 + 9 + 9 + 9) * kGeoNodes + 2 * 9 * kGeoNodes;
 
-__global__ void __launch_bounds__(128) geo_volume_kernel(const GeoOps G, int n_vol, const double* __restrict__ geom_coef,
+static __global__ void __launch_bounds__(128) geo_volume_kernel(const GeoOps G, int n_vol, const double* __restrict__ geom_coef,
                                                         GeoOut out)
 {
 	extern __shared__ double sm[];
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(128) geo_volume_kernel(const GeoOps G, int n_v
 
 // One thread per face cubature node: side 0's vm metric terms and coordinates at the node, the normal and the face
 // Jacobian.
-__global__ void __launch_bounds__(128) geo_face_kernel(const GeoOps G, int n_face, const int* __restrict__ face_vol,
+static __global__ void __launch_bounds__(128) geo_face_kernel(const GeoOps G, int n_face, const int* __restrict__ face_vol,
                                                       const int* __restrict__ face_lf,
                                                       const double* __restrict__ geom_coef, GeoOut out)
 {
@@ -295,7 +295,7 @@ struct BlendArgs {
 	double* geom_coef;       // [v][c][node]
 };
 
-__global__ void __launch_bounds__(128) blend_quad_kernel(const BlendArgs A)
+static __global__ void __launch_bounds__(128) blend_quad_kernel(const BlendArgs A)
 {
 	const int v = blockIdx.x * blockDim.x + threadIdx.x;
 	if (v >= A.n_vol)

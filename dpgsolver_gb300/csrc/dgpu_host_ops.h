@@ -218,11 +218,12 @@ inline FixW fix_entry(double w, int s)
 // The fixed-point operators of TPOps from its FP64 ones.
 inline void derive_fix_ops(int q, int d, TPOps* o)
 {
-	double sD = 0.0, mD = 0.0, sT = 0.0, sU = 0.0, mL = 0.0, sB = 0.0, mB = 0.0, sI = 0.0, mI = 0.0;
+	double sD = 0.0, sG = 0.0, mD = 0.0, sT = 0.0, sU = 0.0, mL = 0.0, sB = 0.0, mB = 0.0, sI = 0.0, mI = 0.0;
 	for (int a = 0; a < q; ++a) {
-		double rD = 0.0, rB = 0.0, rI = 0.0;
+		double rD = 0.0, rG = 0.0, rB = 0.0, rI = 0.0;
 		for (int m = 0; m < q; ++m) {
 			rD += fabs(o->Dgl[m][a]);
+			rG += fabs(o->Dgl[a][m]);
 			rB += fabs(o->B[a][m]);
 			rI += fabs(o->Binv[a][m]);
 			mD = fmax(mD, fabs(o->Dgl[m][a]));
@@ -230,6 +231,7 @@ inline void derive_fix_ops(int q, int d, TPOps* o)
 			mI = fmax(mI, fabs(o->Binv[a][m]));
 		}
 		sD = fmax(sD, d * rD);
+		sG = fmax(sG, rG);
 		sB = fmax(sB, rB);
 		sI = fmax(sI, rI);
 		sU = fmax(sU, 1.0 + d * (fabs(o->lb[0][a]) + fabs(o->lb[1][a])));
@@ -242,13 +244,15 @@ inline void derive_fix_ops(int q, int d, TPOps* o)
 		sT = fmax(sT, r);
 	}
 	o->sD = fix_shift(sD, mD, 63);
-	o->sT = fix_shift(sT, mL, 63);
+	o->sG = fix_shift(sG, mD, 63);
+	o->sT = fix_shift(sT, mL, 62);   // also a pass (batched faces of a higher order)
 	o->sU = fix_shift(sU, fmax(mL, 1.0), 63);
 	o->sB = fix_shift(sB, mB, 62);
 	o->sBinv = fix_shift(sI, mI, 62);
 	for (int a = 0; a < q; ++a)
 		for (int m = 0; m < q; ++m) {
 			o->fD[a][m] = fix_entry(o->Dgl[m][a], o->sD);
+			o->fG[a][m] = fix_entry(o->Dgl[a][m], o->sG);
 			o->fB[a][m] = fix_entry(o->B[a][m], o->sB);
 			o->fBinv[a][m] = fix_entry(o->Binv[a][m], o->sBinv);
 		}

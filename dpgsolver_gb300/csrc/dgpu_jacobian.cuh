@@ -18,7 +18,7 @@
 namespace dgpu {
 
 // du[w nb + k] = value for the volumes w of one colour.
-__global__ void __launch_bounds__(256) jac_seed_kernel(double* du, const int* __restrict__ members, int n_members,
+static __global__ void __launch_bounds__(256) jac_seed_kernel(double* du, const int* __restrict__ members, int n_members,
                                                       int nb, int k, double value)
 {
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(256) jac_seed_kernel(double* du, const int* __
 
 // Column k of every block (v, w(v, c)): values[(s nb + i) nb + k] = jv[v nb + i], s = slot[v n_colours + c] the block's
 // index in the block-sparse rows (row-major blocks: row i = eq n_vs + node, column k = var n_vs + node).
-__global__ void __launch_bounds__(256) jac_scatter_kernel(const double* __restrict__ jv, const int* __restrict__ slot,
+static __global__ void __launch_bounds__(256) jac_scatter_kernel(const double* __restrict__ jv, const int* __restrict__ slot,
                                                          int n_colours, int c, int n_vol, int nb, int k,
                                                          double* values)
 {

@@ -45,12 +45,13 @@ struct TPOps {
 	double BinvT[kQMax][kQMax]; // Binv^T (adjoint: V^-T)
 	// Fixed-point forms (dgpu_fix.cuh) and their scales: W = w 2^s
 	FixW fD[kQMax][kQMax];      // Dgl^T: fD[a][m] = Dgl[m][a], summed over the D directions
+	FixW fG[kQMax][kQMax];      // Dgl, one direction (Navier-Stokes gradients)
 	FixW fT[2][kQMax];          // lb as the trace operator
 	FixW fU[2][kQMax];          // lb as the lifting operator, summed over the 2D faces and fOne
 	FixW fOne;                  // the volume term's weight 1 in that sum
 	FixW fB[kQMax][kQMax];      // B and B^-1 as 1D passes (sum |W| <= 2^62)
 	FixW fBinv[kQMax][kQMax];
-	int sD, sT, sU, sB, sBinv, pad_;
+	int sD, sT, sU, sB, sBinv, sG;
 	float SBf[kQMax][kQMax];    // SBg rounded to FP32 (positivity pre-filter)
 	float pos_err;              // |FP32 Bezier coefficient - exact| <= pos_err * max_i |x_i| (per variable)
 };
