@@ -68,106 +68,167 @@ __global__ void __launch_bounds__(256) tp_ns_lambda_kernel(const __grid_constant
 	lam[(size_t)P.vol_face[(size_t)v * 2 * D + lf] * NF + t] = s;
 }
 
-// Shared memory per element of the two NS element kernels (doubles): the state and D gradient components.
+// Shared memory per element of the two NS element kernels (doubles): the state and D gradient components, then their
+// block exponents (ints): a change of basis, the state with its spreads, the gradient (or the faces' X and the fluxes).
 template <int D, int Q, int NV>
 struct NsSmem {
-	static constexpr int PER_E = (1 + D) * NV * TPShape<D, Q>::N;
+	static constexpr int WORDS = (1 + D) * NV * TPShape<D, Q>::N;
+	static constexpr int EXP = 2 * TPSmem<D, Q, NV>::AEXP + (D + 1) * NV;
+	static constexpr int PER_E = WORDS + (EXP + 1) / 2;
 };
 
-// GL values of the element into su (from GLL coefficients when GLL_IN), the GL collocation derivatives into sd and
-// the physical volume gradient at this thread's node into g. All threads call it (it synchronises).
-template <int D, int Q, int NV, bool GLL_IN>
-__device__ __forceinline__ void ns_element_gradient(const TPOps* sops, const TPParams& P, int v, int node, bool active,
-                                                    double* su, double* sd, double (*g)[NV])
+// K values of every node staged in an element's buffer (K N words): in block fixed point when the element is in range
+// (returned), as doubles otherwise. eb: the K block exponents. STATE: fix_spread on x[0] and x[K - 1] (K + 2 exponents).
+// All threads of the CTA must call it; synchronises before it returns.
+template <int N, int K, bool STATE>
+__device__ __forceinline__ bool ns_stage(const double* x, int e, int node, bool active, double* buf, int* sx, int stride,
+                                         int* eb)
 {
-	constexpr int N = TPShape<D, Q>::N;
-	if (GLL_IN) {
-		tp_apply<D, Q, NV>(su, sd, sd + NV * N, sops->B, node, active);
-		if (active)
+	constexpr int KX = STATE ? K + 2 : K;
+	int m[KX];
 #pragma unroll
-			for (int k = 0; k < NV; ++k)
-				su[k * N + node] = sd[k * N + node];
-		__syncthreads();
+	for (int k = 0; k < K; ++k)
+		m[k] = active ? fix_exponent(x[k]) : 0;
+	if constexpr (STATE) {
+		m[K] = active ? fix_low(x[0]) : 0;
+		m[K + 1] = active ? fix_low(x[K - 1]) : 0;
 	}
-	if (active)
-#pragma unroll
-		for (int k = 0; k < D; ++k)
-			tp_pass<D, Q, NV>(su, sd + k * NV * N, sops->Dgl, k, node);
+	elem_max<N, KX>(m, e, active, sx, stride);
 	__syncthreads();
+	bool ok = true;
 	if (active) {
-		const double iwJ = P.inv_wJ[(size_t)v * N + node];
-		double gm[D * D];
+		const int* se = sx + e * stride;
+		if constexpr (STATE)
+			ok = fix_spread(se[0], se[K]) && fix_spread(se[K - 1], se[K + 1]);
 #pragma unroll
-		for (int c = 0; c < D * D; ++c)
-			gm[c] = P.gmet[((size_t)v * D * D + c) * N + node];
+		for (int k = 0; k < K; ++k) {
+			ok = ok && fix_in_range(se[k]);
+			eb[k] = fix_block(se[k]);
+		}
 #pragma unroll
-		for (int dir = 0; dir < D; ++dir)
-#pragma unroll
-			for (int var = 0; var < NV; ++var) {
-				double a = 0.0;
-#pragma unroll
-				for (int k = 0; k < D; ++k)
-					a += gm[k * D + dir] * sd[(k * NV + var) * N + node];   // w J dr_k/dx_dir d_r_k u
-				g[dir][var] = iwJ * a;
-			}
+		for (int k = 0; k < K; ++k)
+			if (ok)
+				reinterpret_cast<int2*>(buf)[k * N + node] = fix_pack(x[k], eb[k]);
+			else
+				buf[k * N + node] = x[k];
 	}
 	__syncthreads();
+	return ok;
 }
 
+// The physical volume gradient of a staged state at the node, and the traces' source: three passes of Dgl in fixed point.
+template <int D, int Q, int NV>
+__device__ __forceinline__ void ns_node_gradient(const TPOps* sops, const TPParams& P, int v, int node, const double* su,
+                                                 const int* eb, bool ok, double (*g)[NV])
+{
+	constexpr int N = TPShape<D, Q>::N;
+	double d[D][NV];
+#pragma unroll
+	for (int j = 0; j < D; ++j) {
+		const int stride = (j == 0 ? 1 : (j == 1 ? Q : Q * Q));
+		const int a = node_coord<Q>(node, j);
+		const int b0 = node - a * stride;
+		if (ok) {
+			FixW w[Q];
+#pragma unroll
+			for (int m = 0; m < Q; ++m)
+				w[m] = sops->fG[a][m];
+#pragma unroll
+			for (int k = 0; k < NV; ++k) {
+				FixAcc s = {0, 0};
+#pragma unroll
+				for (int m = 0; m < Q; ++m)
+					fix_mac(s, w[m], reinterpret_cast<const int2*>(su)[k * N + b0 + m * stride]);
+				d[j][k] = fix_to_double(fix_sum(s), fix_scale(eb[k], sops->sG));
+			}
+		} else {
+#pragma unroll
+			for (int k = 0; k < NV; ++k)
+				d[j][k] = 0.0;
+#pragma unroll 1
+			for (int m = 0; m < Q; ++m)
+#pragma unroll
+				for (int k = 0; k < NV; ++k)
+					d[j][k] = fma(sops->Dgl[a][m], su[k * N + b0 + m * stride], d[j][k]);
+		}
+	}
+	const double iwJ = P.inv_wJ[(size_t)v * N + node];
+	double gm[D * D];
+#pragma unroll
+	for (int c = 0; c < D * D; ++c)
+		gm[c] = P.gmet[((size_t)v * D * D + c) * N + node];
+#pragma unroll
+	for (int dir = 0; dir < D; ++dir)
+#pragma unroll
+		for (int var = 0; var < NV; ++var) {
+			double a = mul(gm[dir], d[0][var]);
+#pragma unroll
+			for (int k = 1; k < D; ++k)
+				a = mad(gm[k * D + dir], d[k][var], a);   // w J dr_k/dx_dir d_r_k u
+			g[dir][var] = mul(iwJ, a);
+		}
+}
+
+// Gradients and traces. At q = 4 the derivative (60 products a node) and the traces of the state and its gradient (120)
+// run in block fixed point; the FP64 pipe keeps the metric products (60).
 template <int D, int Q, int NV, bool GLL_IN>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS)
 tp_ns_grad_kernel(const __grid_constant__ TPOps ops, const TPParams P, const double* __restrict__ u)
 {
 	using S = TPShape<D, Q>;
-	constexpr int N = S::N, NF = S::NF, E = S::E, PER_E = NsSmem<D, Q, NV>::PER_E;
+	constexpr int N = S::N, NF = S::NF, E = S::E, PER_E = NsSmem<D, Q, NV>::PER_E, AE = TPSmem<D, Q, NV>::AEXP;
 	extern __shared__ double smem[];
 	TPOps* sops = reinterpret_cast<TPOps*>(smem);
 	double* base = smem + sizeof(TPOps) / 8;
 	load_ops(sops, ops);
 	const int tid = threadIdx.x, v0 = blockIdx.x * E, n_here = min(E, P.n_vol - v0);
-	for (int i = tid; i < n_here * NV * N; i += blockDim.x)
-		base[(i / (NV * N)) * PER_E + i % (NV * N)] = u[(size_t)v0 * NV * N + i];
-	__syncthreads();
 	const int e = tid / N, node = tid % N;
 	const bool active = e < n_here;
 	double* su = base + e * PER_E;
 	double* sd = su + NV * N;
+	int* sx = reinterpret_cast<int*>(base + NsSmem<D, Q, NV>::WORDS);
 	const int v = v0 + e;
-	double g[D][NV];
-	ns_element_gradient<D, Q, NV, GLL_IN>(sops, P, v, node, active, su, sd, g);
-	if (active)
+	double W[NV], g[D][NV];
+	if (active) {
+#pragma unroll
+		for (int k = 0; k < NV; ++k)
+			W[k] = u[((size_t)v * NV + k) * N + node];
+		for (int i = node; i < NsSmem<D, Q, NV>::EXP; i += N)
+			sx[e * 2 * PER_E + i] = 0;
+	}
+	__syncthreads();
+	if (GLL_IN)
+		tp_apply_fix<D, Q, NV, true>(W, su, sd, sops->fB, sops->sB, sops->B, e, node, active, sx, 2 * PER_E);
+	int eb[NV], eg[D * NV];
+	const bool ok = ns_stage<N, NV, true>(W, e, node, active, su, sx + AE, 2 * PER_E, eb);
+	if (active) {
+		ns_node_gradient<D, Q, NV>(sops, P, v, node, su, eb, ok, g);
 #pragma unroll
 		for (int dir = 0; dir < D; ++dir)
 #pragma unroll
-			for (int var = 0; var < NV; ++var) {
-				sd[(dir * NV + var) * N + node] = g[dir][var];
+			for (int var = 0; var < NV; ++var)
 				P.ns_gv[(((size_t)v * D + dir) * NV + var) * N + node] = g[dir][var];
-			}
-	__syncthreads();
+	}
+	const bool okg = ns_stage<N, D * NV, false>(&g[0][0], e, node, active, sd, sx + 2 * AE, 2 * PER_E, eg);
 	if (!active)
 		return;
 	// traces of the state and of the volume gradient on the 2D local faces
 	for (int it = node; it < 2 * D * NF; it += N) {
-		const int lf = it / NF, t = it % NF, nd = lf >> 1, side = lf & 1;
-		int b, stride;
-		face_line<D, Q>(nd, t, &b, &stride);
+		const int lf = it / NF, t = it % NF;
 		const int fs = P.vol_face[(size_t)v * 2 * D + lf];
-		double* ds = P.traces + (size_t)fs * NV * NF;
-		double* dg = P.ns_gtr + (size_t)fs * D * NV * NF;
+		double* ds = P.traces + (size_t)fs * NV * NF + t;
+		double* dg = P.ns_gtr + (size_t)fs * D * NV * NF + t;
+		double out[NV];
+		tp_trace<D, Q, NV>(sops, su, eb, ok, lf, t, out);
 #pragma unroll
-		for (int k = 0; k < NV; ++k) {
-			double s = 0.0;
+		for (int k = 0; k < NV; ++k)
+			ds[k * NF] = out[k];
 #pragma unroll
-			for (int m = 0; m < Q; ++m)
-				s += sops->lb[side][m] * su[k * N + b + m * stride];
-			ds[k * NF + t] = s;
-		}
-		for (int c = 0; c < D * NV; ++c) {
-			double s = 0.0;
+		for (int dir = 0; dir < D; ++dir) {
+			tp_trace<D, Q, NV>(sops, sd + dir * NV * N, eg + dir * NV, okg, lf, t, out);
 #pragma unroll
-			for (int m = 0; m < Q; ++m)
-				s += sops->lb[side][m] * sd[c * N + b + m * stride];
-			dg[c * NF + t] = s;
+			for (int k = 0; k < NV; ++k)
+				dg[(dir * NV + k) * NF] = out[k];
 		}
 	}
 }
@@ -382,94 +443,108 @@ __global__ void __launch_bounds__(128) tp_ns_jvp_face_kernel(const TPParams P, c
 		ns_face_node<D, Q, FLUX, Dual<1>>(P, Pd, gid / NF, gid % NF);
 }
 
+// Volume term. At q = 4 the lifting of the faces' X (90 products a node) and the derivative (60) run in block fixed point;
+// the FP64 pipe keeps the pointwise fluxes.
 template <int D, int Q, int NV, bool GLL_IN>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS)
 tp_ns_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const double* __restrict__ u)
 {
 	using S = TPShape<D, Q>;
-	constexpr int N = S::N, NF = S::NF, E = S::E, PER_E = NsSmem<D, Q, NV>::PER_E;
+	constexpr int N = S::N, NF = S::NF, E = S::E, PER_E = NsSmem<D, Q, NV>::PER_E, AE = TPSmem<D, Q, NV>::AEXP;
+	constexpr int NFT = TPSmem<D, Q, NV>::NFT, NR = (NFT + N - 1) / N;
 	extern __shared__ double smem[];
 	TPOps* sops = reinterpret_cast<TPOps*>(smem);
 	double* base = smem + sizeof(TPOps) / 8;
 	load_ops(sops, ops);
 	const int tid = threadIdx.x, v0 = blockIdx.x * E, n_here = min(E, P.n_vol - v0);
-	for (int i = tid; i < n_here * NV * N; i += blockDim.x)
-		base[(i / (NV * N)) * PER_E + i % (NV * N)] = u[(size_t)v0 * NV * N + i];
-	__syncthreads();
 	const int e = tid / N, node = tid % N;
 	const bool active = e < n_here;
 	double* su = base + e * PER_E;
 	double* sf = su + NV * N;
+	int* sx = reinterpret_cast<int*>(base + NsSmem<D, Q, NV>::WORDS);
 	const int v = v0 + e;
-	if (GLL_IN) {   // GL values of the state
-		tp_apply<D, Q, NV>(su, sf, sf + NV * N, sops->B, node, active);
+	double W[NV];
+	if (active) {
+#pragma unroll
+		for (int k = 0; k < NV; ++k)
+			W[k] = u[((size_t)v * NV + k) * N + node];
+		for (int i = node; i < NsSmem<D, Q, NV>::EXP; i += N)
+			sx[e * 2 * PER_E + i] = 0;
+	}
+	__syncthreads();
+	if (GLL_IN)   // GL values of the state
+		tp_apply_fix<D, Q, NV, true>(W, su, sf, sops->fB, sops->sB, sops->B, e, node, active, sx, 2 * PER_E);
+	double g[D][NV], fr[D][NV];
+	const double iwJ = active ? P.inv_wJ[(size_t)v * N + node] : 0.0;
+#pragma unroll
+	for (int dir = 0; dir < D; ++dir) {
+		// + the lifting of every face's X (BR2 total gradient): inv_wJ lb[side][m] X at this node
+		double fv[NR][NV], L[NV];
+		if (active) {
+#pragma unroll
+			for (int k = 0; k < NV; ++k)
+				L[k] = 0.0;
+#pragma unroll
+			for (int r = 0; r < NR; ++r) {
+				const int it = node + r * N;
+				if (it >= NFT)
+					break;
+				const int lf = it / NF, t = it % NF;
+				const int fs = P.vol_face[(size_t)v * 2 * D + lf], f = fs >> 1;
+				const int tX = ((fs & 1) && P.nc_inv) ? P.nc_inv[(size_t)f * NF + t] : t;
+				const double* X = P.ns_X + ((size_t)f * D + dir) * NV * NF + tX;
+#pragma unroll
+				for (int k = 0; k < NV; ++k)
+					fv[r][k] = X[k * NF];
+			}
+		}
+		tp_lift_sum<D, Q, NV>(sops, fv, L, e, node, active, sf, sx + 2 * AE + dir * NV, 2 * PER_E);
 		if (active)
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
-				su[k * N + node] = sf[k * N + node];
-		__syncthreads();
+				g[dir][k] = mad(iwJ, L[k], P.ns_gv[(((size_t)v * D + dir) * NV + k) * N + node]);
 	}
-	double g[D][NV];
-	if (active)
-#pragma unroll
-		for (int dir = 0; dir < D; ++dir)
-#pragma unroll
-			for (int var = 0; var < NV; ++var)
-				g[dir][var] = P.ns_gv[(((size_t)v * D + dir) * NV + var) * N + node];
-	double fr[D][NV];
 	if (active) {
-		// + the lifting of every face's X (BR2 total gradient): inv_wJ lb[side][m] X at this node
-		const double iwJ = P.inv_wJ[(size_t)v * N + node];
-#pragma unroll
-		for (int lf = 0; lf < 2 * D; ++lf) {
-			const int nd = lf >> 1, side = lf & 1;
-			const int tf = face_node_of<D, Q>(node, nd);
-			const int fs = P.vol_face[(size_t)v * 2 * D + lf], f = fs >> 1;
-			const int tX = ((fs & 1) && P.nc_inv) ? P.nc_inv[(size_t)f * NF + tf] : tf;
-			const double c = iwJ * sops->lb[side][node_coord<Q>(node, nd)];
-			const double* X = P.ns_X + (size_t)f * D * NV * NF + tX;
-#pragma unroll
-			for (int dir = 0; dir < D; ++dir)
-#pragma unroll
-				for (int k = 0; k < NV; ++k)
-					g[dir][k] += c * X[(dir * NV + k) * NF];
-		}
-		double W[NV], gm[D * D];
-#pragma unroll
-		for (int k = 0; k < NV; ++k)
-			W[k] = su[k * N + node];
+		double gm[D * D];
 #pragma unroll
 		for (int c = 0; c < D * D; ++c)
 			gm[c] = P.gmet[((size_t)v * D * D + c) * N + node];
 		ns_flux_ref<D, double>(W, g, gm, P.ns, fr);
 	}
-	__syncthreads();   // everyone is done with sf's derivatives
-	if (active)
+	// the fluxes of one variable are one block, as in tp_stage_volume
+	int eb[2 * NV], m[NV];
+#pragma unroll
+	for (int k = 0; k < NV; ++k) {
+		m[k] = 0;
+		if (active)
+#pragma unroll
+			for (int j = 0; j < D; ++j)
+				m[k] = max(m[k], fix_exponent(fr[j][k]));
+	}
+	elem_max<N, NV>(m, e, active, sx + 2 * AE + D * NV, 2 * PER_E);
+	__syncthreads();   // the lifting's sums are read: sf is free
+	bool ok = true;
+	if (active) {
+		const int* se = sx + e * 2 * PER_E + 2 * AE + D * NV;
+#pragma unroll
+		for (int k = 0; k < NV; ++k) {
+			ok = ok && fix_in_range(se[k]);
+			eb[NV + k] = fix_block(se[k]);
+		}
 #pragma unroll
 		for (int j = 0; j < D; ++j)
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
-				sf[(j * NV + k) * N + node] = fr[j][k];
+				if (ok)
+					reinterpret_cast<int2*>(sf)[(j * NV + k) * N + node] = fix_pack(fr[j][k], eb[NV + k]);
+				else
+					sf[(j * NV + k) * N + node] = fr[j][k];
+	}
 	__syncthreads();
 	if (!active)
 		return;
 	double acc[NV];
-#pragma unroll
-	for (int k = 0; k < NV; ++k)
-		acc[k] = 0.0;
-#pragma unroll
-	for (int j = 0; j < D; ++j) {
-		const int stride = (j == 0 ? 1 : (j == 1 ? Q : Q * Q));
-		const int a = node_coord<Q>(node, j);
-		const int b0 = node - a * stride;
-#pragma unroll
-		for (int m = 0; m < Q; ++m) {
-			const double w = sops->Dgl[m][a];
-#pragma unroll
-			for (int k = 0; k < NV; ++k)
-				acc[k] += w * sf[(j * NV + k) * N + b0 + m * stride];
-		}
-	}
+	tp_derivative<D, Q, NV>(sops, sf, eb, ok, node, acc);
 #pragma unroll
 	for (int k = 0; k < NV; ++k)
 		P.vol_gl[((size_t)v * NV + k) * N + node] = acc[k];
