@@ -256,9 +256,9 @@ cudaError_t launch_face_t(dgpu_ctx* c)
 {
 	using S = TPShape<D, Q>;
 	const long long n = (long long)c->n_face * S::NF;
-	const int blocks = (int)((n + 255) / 256);
+	const int blocks = (int)((n + 127) / 128);
 	record_start(c, "tp_face_kernel");
-	tp_face_kernel<D, Q, NV, PDE, FLUX><<<blocks, 256, 0, c->stream>>>(c->params());
+	tp_face_kernel<D, Q, NV, PDE, FLUX><<<blocks, 128, 0, c->stream>>>(c->params());
 	record_stop(c);
 	c->launches++;
 	return cudaGetLastError();

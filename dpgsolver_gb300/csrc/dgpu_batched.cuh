@@ -336,10 +336,7 @@ __device__ __forceinline__ void bface_node_rt(const BParams& P, int f, int i, in
 	if constexpr (PDE == kEuler) {
 		double nF[NV];
 		if constexpr (FLUX == kRoePike) {
-			num_flux_roe_pike<D>(WL, WR, n, nF);
-#pragma unroll
-			for (int k = 0; k < NV; ++k)
-				nF[k] *= sc;
+			num_flux_roe_pike<D>(WL, WR, n, nF, sc);
 		} else {
 			num_flux_lax_friedrichs<D>(WL, WR, n, nF, sc);
 		}

@@ -246,4 +246,34 @@ __device__ __forceinline__ bool abs_less(double a, double b)
 	return ua < ub && ub <= 0x7ff0000000000000ull;
 }
 
+// a b rounded to nearest even, bit for bit __dmul_rn, for factors that are zero or normal and a product that is zero
+// or normal (the caller knows their magnitudes). About 35 integer instructions, the time of one DMUL, but on a pipe that
+// the pointwise fluxes leave idle: they run their lone products here and their sums and fused products on the FP64 pipe.
+__device__ __forceinline__ double fix_mul(double a, double b)
+{
+	const int ha = __double2hiint(a), hb = __double2hiint(b);
+	const unsigned la = __double2loint(a), lb = __double2loint(b);
+	const unsigned mah = (ha & 0x000fffff) | 0x00100000, bh = (hb & 0x000fffff) | 0x00100000;
+	// (a's mantissa 2^11) x (b's mantissa): 116 or 117 bits, the 53 or 52 leading ones above bit 64
+	const unsigned ah = __funnelshift_l(la, mah, 11), al = la << 11;
+	const unsigned long long t0 = (unsigned long long)al * lb;
+	const unsigned long long t1 = (unsigned long long)ah * lb + (t0 >> 32);
+	const unsigned long long t2 = (unsigned long long)al * bh + (unsigned)t1;
+	unsigned long long hi = (unsigned long long)ah * bh + (t1 >> 32) + (t2 >> 32);
+	unsigned long long lo = (t2 << 32) | (unsigned)t0;
+	int ex = (ha & 0x7ff00000) + (hb & 0x7ff00000) - (1023 << 20);
+	if (!(hi >> 52)) {
+		hi = hi * 2 + (lo >> 63);
+		lo *= 2;
+		ex -= 1 << 20;
+	}
+	const bool up = (lo >> 63) && ((lo << 1) || (hi & 1));
+	hi += up;                                    // the leading bit (and a carry) adds to the exponent field
+	int rh = (int)(hi >> 32) + ex;
+	unsigned rl = (unsigned)hi;
+	if (!((ha & 0x7fffffff) && (hb & 0x7fffffff)))
+		rh = rl = 0;
+	return __hiloint2double(rh | ((ha ^ hb) & 0x80000000), rl);
+}
+
 }  // namespace dgpu

@@ -240,24 +240,19 @@ __device__ __forceinline__ void ns_flux_ref(const T* W, const T (*G)[D + 2], con
                                             T (*fr)[D + 2])
 {
 	constexpr int NV = D + 2;
-	euler_flux_ref<D>(W, gm, fr);
+	if constexpr (std::is_same<T, double>::value)
+		euler_flux_node<D>(W, gm, fr);
+	else
+		euler_flux_ref<D>(W, gm, fr);
 	T Fv[D][NV];
-#pragma unroll
-	for (int i = 0; i < D; ++i)
-#pragma unroll
-		for (int k = 0; k < NV; ++k)
-			Fv[i][k] = T(0.0);
-	ns_viscous_sub<D, T>(W, G, ns, Fv);
+	ns_viscous<D, T>(W, G, ns, Fv);
 #pragma unroll
 	for (int j = 0; j < D; ++j)
 #pragma unroll
-		for (int k = 0; k < NV; ++k) {
-			T a = T(0.0);
+		for (int k = 1; k < NV; ++k)   // the mass equation has no viscous flux
 #pragma unroll
 			for (int i = 0; i < D; ++i)
-				a = a + gm[j * D + i] * Fv[i][k];
-			fr[j][k] = fr[j][k] + a;
-		}
+				fr[j][k] = mad(gm[j * D + i], Fv[i][k], fr[j][k]);
 }
 
 // Scalar helpers of the face and volume bodies below: T = double (the residual) or Dual<1> (the residual and its
@@ -322,10 +317,10 @@ __device__ __forceinline__ void ns_face_flux(int code, const double* ext, int ex
 	for (int dir = 0; dir < D; ++dir)
 #pragma unroll
 		for (int k = 0; k < NV; ++k) {
-			X[dir][k] = (0.5 * sc * n[dir]) * (WR[k] - WL[k]);
-			GL[dir][k] = GtL[dir][k] + (eta * lamL) * X[dir][k];
+			X[dir][k] = mul(mul(0.5 * sc, n[dir]), sub(WR[k], WL[k]));
+			GL[dir][k] = mad(eta * lamL, X[dir][k], GtL[dir][k]);
 			// on a boundary face the exterior gradient is the interior one (grad_from_internal; the walls copy it)
-			GR[dir][k] = !bnd ? GtR[dir][k] + (eta * lamR) * X[dir][k] : GL[dir][k];
+			GR[dir][k] = !bnd ? mad(eta * lamR, X[dir][k], GtR[dir][k]) : GL[dir][k];
 		}
 	T nF[NV];
 	if constexpr (FLUX == kRoePike)
@@ -333,24 +328,20 @@ __device__ __forceinline__ void ns_face_flux(int code, const double* ext, int ex
 	else
 		num_flux_lax_friedrichs<D, T>(WL, WR, n, nF);
 	T FL[D][NV], FR[D][NV];
+	ns_viscous<D, T>(WL, GL, ph, FL);
+	ns_viscous<D, T>(WR, GR, ph, FR);
+	o[0] = nF[0] * sc;   // the mass equation has no viscous flux
 #pragma unroll
-	for (int dir = 0; dir < D; ++dir)
+	for (int k = 1; k < NV; ++k) {
+		T s = mul(n[0], add(FL[0][k], FR[0][k]));
 #pragma unroll
-		for (int k = 0; k < NV; ++k)
-			FL[dir][k] = FR[dir][k] = T(0.0);
-	ns_viscous_sub<D, T>(WL, GL, ph, FL);
-	ns_viscous_sub<D, T>(WR, GR, ph, FR);
-#pragma unroll
-	for (int k = 0; k < NV; ++k) {
-		T s = T(0.0);
-#pragma unroll
-		for (int dir = 0; dir < D; ++dir)
-			s = s + n[dir] * (FL[dir][k] + FR[dir][k]);
+		for (int dir = 1; dir < D; ++dir)
+			s = mad(n[dir], add(FL[dir][k], FR[dir][k]), s);
 		// a static wall sets the total normal energy flux to nf_E: 0 when adiabatic, -mu Cp / Pr dTdn when
 		// diabatic (set_provided_Numerical_Flux_members, numerical_flux_central_T.c:222-231)
 		const bool wall_E = (k == D + 1 && (code == kBcNoSlipAdiabatic || code == kBcNoSlipDiabatic));
 		const double nf_E = code == kBcNoSlipDiabatic ? ph.wall_nf_E * sc : 0.0;
-		o[k] = wall_E ? T(nf_E) : (nF[k] + 0.5 * s) * sc;
+		o[k] = wall_E ? T(nf_E) : mul(mad(0.5, s, nF[k]), sc);
 	}
 }
 
@@ -425,7 +416,7 @@ __device__ __forceinline__ void ns_face_node(const TPParams& P, const TPParams& 
 }
 
 template <int D, int Q, int FLUX>
-__global__ void __launch_bounds__(128) tp_ns_face_kernel(const TPParams P)
+__global__ void __launch_bounds__(128, 3) tp_ns_face_kernel(const TPParams P)
 {
 	constexpr int NF = TPShape<D, Q>::NF;
 	const int gid = blockIdx.x * blockDim.x + threadIdx.x;

@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <math.h>
 
+#include <type_traits>
+
 #include "dgpu_dual.cuh"
 
 namespace dgpu {
@@ -59,6 +61,46 @@ __device__ __forceinline__ auto mul(A a, B b)
 	return a * b;
 }
 __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+// mul on the integer pipe (the same bits) where S: see fix_mul for what the factors must be.
+template <bool S, typename A, typename B>
+__device__ __forceinline__ auto mulx(A a, B b)
+{
+	if constexpr (S && std::is_same<A, double>::value && std::is_same<B, double>::value)
+		return fix_mul(a, b);
+	else
+		return mul(a, b);
+}
+// The range in which mulx<true> may be used inside the flux routines: zero, or a magnitude of 2^-LO to 2^60, LO = 60 for
+// densities, energies, viscosities and scalings, 150 for the components of vectors (momentum, normals, metric terms,
+// gradients), which round-off leaves anywhere near zero. No product of a flux formed from such values leaves the normal
+// range (the smallest, a velocity times a stress, stays above 2^-900).
+template <int LO>
+__device__ __forceinline__ bool mulx_range(double x)
+{
+	const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+	return h - ((1023u - LO) << 20) < ((60u + LO) << 20) || (h | (unsigned)__double2loint(x)) == 0u;
+}
+// A conserved state: density positive, every component in range.
+template <int D>
+__device__ __forceinline__ bool mulx_state(const double* W)
+{
+	bool ok = __double2hiint(W[0]) > 0 && mulx_range<60>(W[0]) && mulx_range<60>(W[D + 1]);
+#pragma unroll
+	for (int k = 0; k < D; ++k)
+		ok = ok && mulx_range<150>(W[1 + k]);
+	return ok;
+}
+template <int N>
+__device__ __forceinline__ bool mulx_vector(const double* x)
+{
+	bool ok = true;
+#pragma unroll
+	for (int k = 0; k < N; ++k)
+		ok = ok && mulx_range<150>(x[k]);
+	return ok;
+}
+__device__ __forceinline__ bool positive(double x) { return __double2hiint(x) > 0 && __double2hiint(x) < 0x7ff00000; }
+
 template <typename T>
 __device__ __forceinline__ T add(const T& a, const T& b)
 {
@@ -96,7 +138,8 @@ __device__ __forceinline__ double larger(double a, double b) { return abs_less(b
 // (compute_rlhs_T.c:71-110). The contraction is regrouped through the contravariant momentum
 // M_j = sum_i g[j*D+i] m_i (the mass flux fr_j[0] itself) and velocity U_j = M_j / rho, and the pressure takes
 // rho |u|^2 as |m|^2 / rho: the same sums with fewer FP64 operations.
-template <int D, typename T = double>
+// S: the lone products that mulx<S> takes off the FP64 pipe (the volume kernels' integer pipe is half full already).
+template <int D, typename T = double, bool S = false>
 __device__ __forceinline__ void euler_flux_ref(const T* W, const double* g, T (*fr)[D + 2])
 {
 	const T rho = W[0], E = W[D + 1];
@@ -105,7 +148,7 @@ __device__ __forceinline__ void euler_flux_ref(const T* W, const double* g, T (*
 #pragma unroll
 	for (int k = 1; k < D; ++k)
 		m2 = mad(W[1 + k], W[1 + k], m2);
-	const T p = mul(kGm1, mad(-0.5, mul(m2, rho_inv), E));
+	const T p = mulx<S>(kGm1, mad(-0.5, mulx<S>(m2, rho_inv), E));
 	const T Ep = add(E, p);
 #pragma unroll
 	for (int j = 0; j < D; ++j) {
@@ -113,32 +156,58 @@ __device__ __forceinline__ void euler_flux_ref(const T* W, const double* g, T (*
 #pragma unroll
 		for (int i = 1; i < D; ++i)
 			M = mad(g[j * D + i], W[1 + i], M);
-		const T U = mul(M, rho_inv);
+		const T U = mulx<S>(M, rho_inv);
 		fr[j][0] = M;
 #pragma unroll
 		for (int m = 0; m < D; ++m)
 			fr[j][1 + m] = mad(W[1 + m], U, mul(p, g[j * D + m]));
-		fr[j][D + 1] = mul(Ep, U);
+		fr[j][D + 1] = mulx<S>(Ep, U);
 	}
+}
+
+// The FP64 form of the Roe-Pike flux, out of line and by value: it is rarely taken, and inlined beside the other form it
+// would raise the registers of every face kernel (124 instead of 108).
+template <int D>
+struct FluxNode {
+	double WL[D + 2], WR[D + 2], n[D], scale;
+};
+template <int D>
+struct FluxValue {
+	double F[D + 2];
+};
+template <int D>
+__device__ __forceinline__ FluxNode<D> flux_node(const double* WL, const double* WR, const double* n, double scale)
+{
+	FluxNode<D> x;
+#pragma unroll
+	for (int k = 0; k < D + 2; ++k) {
+		x.WL[k] = WL[k];
+		x.WR[k] = WR[k];
+	}
+#pragma unroll
+	for (int k = 0; k < D; ++k)
+		x.n[k] = n[k];
+	x.scale = scale;
+	return x;
 }
 
 // One side of a face node for Lax-Friedrichs: m.n, the normal velocity Vn = m.n / rho, the pressure and the wave
 // speed |V| + c, with rho |V|^2 formed as |m|^2 / rho (one reciprocal of the density, no velocity vector).
-template <int D, typename T>
+template <int D, typename T, bool S>
 __device__ __forceinline__ void euler_side_lf(const T* W, const double* n, T& mn, T& Vn, T& p, T& lam)
 {
 	const T rho_inv = recip(W[0]);
-	T m2 = mul(W[1], W[1]);
-	mn = mul(n[0], W[1]);
+	T m2 = mulx<S>(W[1], W[1]);
+	mn = mulx<S>(n[0], W[1]);
 #pragma unroll
 	for (int k = 1; k < D; ++k) {
 		m2 = mad(W[1 + k], W[1 + k], m2);
 		mn = mad(n[k], W[1 + k], mn);
 	}
-	const T q = mul(m2, rho_inv);   // rho |V|^2
-	Vn = mul(mn, rho_inv);
-	p = mul(kGm1, mad(-0.5, q, W[D + 1]));
-	lam = add(root(mul(q, rho_inv)), root(mul(mul(kGamma, p), rho_inv)));
+	const T q = mulx<S>(m2, rho_inv);   // rho |V|^2
+	Vn = mulx<S>(mn, rho_inv);
+	p = mulx<S>(kGm1, mad(-0.5, q, W[D + 1]));
+	lam = add(root(mulx<S>(q, rho_inv)), root(mulx<S>(mulx<S>(kGamma, p), rho_inv)));
 }
 
 // Lax-Friedrichs (compute_Numerical_Flux_T_euler_lax_friedrichs, numerical_flux_euler_T.c:60-327):
@@ -146,76 +215,124 @@ __device__ __forceinline__ void euler_side_lf(const T* W, const double* n, T& mn
 // with n.F = (m.n, m Vn + p n, (E + p) Vn) of each side (compute_Flux_euler_0 contracted with n); the two sides'
 // pressure terms share one product with n. scale (the face node's w J, or 1) is folded into the factor 1/2, which
 // gives the same bits as scaling afterwards (the factor 1/2 is exact).
+// Returns false when a pressure is not positive (S only: the products then meet NaN, which fix_mul does not take).
+template <int D, typename T, bool S>
+__device__ __forceinline__ bool num_flux_lf_impl(const T* WL, const T* WR, const double* n, T* nF, double scale)
+{
+	T mnL, VnL, pL, lamL, mnR, VnR, pR, lamR;
+	euler_side_lf<D, T, S>(WL, n, mnL, VnL, pL, lamL);
+	euler_side_lf<D, T, S>(WR, n, mnR, VnR, pR, lamR);
+	if constexpr (S)
+		if (!positive(pL) || !positive(pR))
+			return false;
+	const T maxV = larger(lamL, lamR);
+	const double h = 0.5 * scale;
+	const T pLR = add(pL, pR);
+	nF[0] = mulx<S>(h, mad(maxV, sub(WL[0], WR[0]), add(mnL, mnR)));
+#pragma unroll
+	for (int k = 0; k < D; ++k)
+		nF[1 + k] = mulx<S>(h, mad(maxV, sub(WL[1 + k], WR[1 + k]),
+		                       mad(WL[1 + k], VnL, mad(WR[1 + k], VnR, mulx<S>(pLR, n[k])))));
+	nF[D + 1] = mulx<S>(h, mad(maxV, sub(WL[D + 1], WR[D + 1]),
+	                       mad(add(WL[D + 1], pL), VnL, mulx<S>(add(WR[D + 1], pR), VnR))));
+	return true;
+}
+
 template <int D, typename T = double>
 __device__ __forceinline__ void num_flux_lax_friedrichs(const T* WL, const T* WR, const double* n, T* nF,
                                                         double scale = 1.0)
 {
-	T mnL, VnL, pL, lamL, mnR, VnR, pR, lamR;
-	euler_side_lf<D>(WL, n, mnL, VnL, pL, lamL);
-	euler_side_lf<D>(WR, n, mnR, VnR, pR, lamR);
-	const T maxV = larger(lamL, lamR);
-	const double h = 0.5 * scale;
-	const T pLR = add(pL, pR);
-	nF[0] = mul(h, mad(maxV, sub(WL[0], WR[0]), add(mnL, mnR)));
-#pragma unroll
-	for (int k = 0; k < D; ++k)
-		nF[1 + k] = mul(h, mad(maxV, sub(WL[1 + k], WR[1 + k]),
-		                       mad(WL[1 + k], VnL, mad(WR[1 + k], VnR, mul(pLR, n[k])))));
-	nF[D + 1] = mul(h, mad(maxV, sub(WL[D + 1], WR[D + 1]),
-	                       mad(add(WL[D + 1], pL), VnL, mul(add(WR[D + 1], pR), VnR))));
+	if constexpr (std::is_same<T, double>::value) {
+		if (mulx_state<D>(WL) && mulx_state<D>(WR) && mulx_vector<D>(n) && mulx_range<60>(scale) &&
+		    num_flux_lf_impl<D, T, true>(WL, WR, n, nF, scale))
+			return;
+	}
+	num_flux_lf_impl<D, T, false>(WL, WR, n, nF, scale);
 }
 
 // Roe-Pike with the entropy fix of Qu et al. 2015 (compute_Numerical_Flux_T_euler_roe_pike,
 // numerical_flux_euler_T.c:470-778).
-template <int D, typename T = double>
-__device__ __forceinline__ void num_flux_roe_pike(const T* WL, const T* WR, const double* n, T* nF)
+// scale (the face node's w J, or 1) is folded into the factor 1/2, which gives the same bits as scaling afterwards. Returns
+// false when the squared speed of sound is not positive (S only).
+template <int D, typename T, bool S>
+__device__ __forceinline__ bool num_flux_roe_impl(const T* WL, const T* WR, const double* n, T* nF, double scale)
 {
 	const T rhoL = WL[0], rhoR = WR[0], EL = WL[D + 1], ER = WR[D + 1];
 	const T rhoL_inv = recip(rhoL), rhoR_inv = recip(rhoR);
 	T uL[D], uR[D], V2L, V2R, VnL, VnR;
 #pragma unroll
 	for (int k = 0; k < D; ++k) {
-		uL[k] = mul(WL[1 + k], rhoL_inv);
-		uR[k] = mul(WR[1 + k], rhoR_inv);
-		V2L = k ? mad(uL[k], uL[k], V2L) : mul(uL[k], uL[k]);
-		V2R = k ? mad(uR[k], uR[k], V2R) : mul(uR[k], uR[k]);
-		VnL = k ? mad(n[k], uL[k], VnL) : mul(n[k], uL[k]);
-		VnR = k ? mad(n[k], uR[k], VnR) : mul(n[k], uR[k]);
+		uL[k] = mulx<S>(WL[1 + k], rhoL_inv);
+		uR[k] = mulx<S>(WR[1 + k], rhoR_inv);
+		V2L = k ? mad(uL[k], uL[k], V2L) : mulx<S>(uL[k], uL[k]);
+		V2R = k ? mad(uR[k], uR[k], V2R) : mulx<S>(uR[k], uR[k]);
+		VnL = k ? mad(n[k], uL[k], VnL) : mulx<S>(n[k], uL[k]);
+		VnR = k ? mad(n[k], uR[k], VnR) : mulx<S>(n[k], uR[k]);
 	}
-	const T pL = mul(kGm1, mad(mul(-0.5, rhoL), V2L, EL)), HL = mul(add(EL, pL), rhoL_inv);
-	const T pR = mul(kGm1, mad(mul(-0.5, rhoR), V2R, ER)), HR = mul(add(ER, pR), rhoR_inv);
+	const T pL = mulx<S>(kGm1, mad(mulx<S>(-0.5, rhoL), V2L, EL)), HL = mulx<S>(add(EL, pL), rhoL_inv);
+	const T pR = mulx<S>(kGm1, mad(mulx<S>(-0.5, rhoR), V2R, ER)), HR = mulx<S>(add(ER, pR), rhoR_inv);
 
 	// Roe averages (divisions by r + 1 through one reciprocal)
-	const T r = root(mul(rhoR, rhoL_inv)), rP1_inv = recip(add(r, T(1.0))), rho = mul(r, rhoL);
+	const T r = root(mulx<S>(rhoR, rhoL_inv)), rP1_inv = recip(add(r, T(1.0))), rho = mulx<S>(r, rhoL);
 	T u[D], Vn, V2;
 #pragma unroll
 	for (int k = 0; k < D; ++k) {
-		u[k] = mul(mad(r, uR[k], uL[k]), rP1_inv);
-		Vn = k ? mad(n[k], u[k], Vn) : mul(n[k], u[k]);
-		V2 = k ? mad(u[k], u[k], V2) : mul(u[k], u[k]);
+		u[k] = mulx<S>(mad(r, uR[k], uL[k]), rP1_inv);
+		Vn = k ? mad(n[k], u[k], Vn) : mulx<S>(n[k], u[k]);
+		V2 = k ? mad(u[k], u[k], V2) : mulx<S>(u[k], u[k]);
 	}
-	const T H = mul(mad(r, HR, HL), rP1_inv), c2 = mul(kGm1, mad(-0.5, V2, H)), c = root(c2), c_inv = recip(c);
+	const T H = mulx<S>(mad(r, HR, HL), rP1_inv), c2 = mulx<S>(kGm1, mad(-0.5, V2, H)), c = root(c2);
+	if constexpr (S)
+		if (!positive(c2))
+			return false;
+	const T c_inv = recip(c);
+	const double h = 0.5 * scale;
 
 	const T l1 = min_abs_real(sub(VnL, c), sub(Vn, c)), l5 = max_abs_real(add(VnR, c), add(Vn, c));
 	const T l234 = abs_real(Vn);
 
 	const T drho = sub(rhoR, rhoL), dE = sub(ER, EL), dp = sub(pR, pL), dVn = sub(VnR, VnL);
-	const T lc1 = mad(0.5, add(l5, l1), -l234), lc2 = mul(0.5, sub(l5, l1));
-	const T lc1_dp = mul(mul(lc1, dp), c_inv), lc2_dp = mul(mul(lc2, dp), c_inv);
-	const T disInter1 = mul(mad(mul(lc2, rho), dVn, lc1_dp), c_inv);
-	const T disInter2 = mad(mul(lc1, rho), dVn, lc2_dp);
+	const T lc1 = mad(0.5, add(l5, l1), -l234), lc2 = mulx<S>(0.5, sub(l5, l1));
+	const T lc1_dp = mulx<S>(mulx<S>(lc1, dp), c_inv), lc2_dp = mulx<S>(mulx<S>(lc2, dp), c_inv);
+	const T disInter1 = mulx<S>(mad(mulx<S>(lc2, rho), dVn, lc1_dp), c_inv);
+	const T disInter2 = mad(mulx<S>(lc1, rho), dVn, lc2_dp);
 
-	const T rhoVnL = mul(rhoL, VnL), rhoVnR = mul(rhoR, VnR), pLR = add(pL, pR);
-	nF[0] = mul(0.5, sub(add(rhoVnL, rhoVnR), mad(l234, drho, disInter1)));
+	const T rhoVnL = mulx<S>(rhoL, VnL), rhoVnR = mulx<S>(rhoR, VnR), pLR = add(pL, pR);
+	nF[0] = mulx<S>(h, sub(add(rhoVnL, rhoVnR), mad(l234, drho, disInter1)));
 #pragma unroll
 	for (int k = 0; k < D; ++k) {
 		const T drhou = sub(WR[1 + k], WL[1 + k]);
-		const T nFk = mad(rhoVnL, uL[k], mad(rhoVnR, uR[k], mul(n[k], pLR)));
-		const T disk = mad(l234, drhou, mad(disInter1, u[k], mul(disInter2, n[k])));
-		nF[1 + k] = mul(0.5, sub(nFk, disk));
+		const T nFk = mad(rhoVnL, uL[k], mad(rhoVnR, uR[k], mulx<S>(n[k], pLR)));
+		const T disk = mad(l234, drhou, mad(disInter1, u[k], mulx<S>(disInter2, n[k])));
+		nF[1 + k] = mulx<S>(h, sub(nFk, disk));
 	}
-	nF[D + 1] = mul(0.5, sub(mad(VnL, add(EL, pL), mul(VnR, add(ER, pR))),
-	                         mad(l234, dE, mad(disInter1, H, mul(disInter2, Vn)))));
+	nF[D + 1] = mulx<S>(h, sub(mad(VnL, add(EL, pL), mulx<S>(VnR, add(ER, pR))),
+	                         mad(l234, dE, mad(disInter1, H, mulx<S>(disInter2, Vn)))));
+	return true;
+}
+
+template <int D>
+__device__ __noinline__ FluxValue<D> num_flux_roe_fp64(FluxNode<D> x)
+{
+	FluxValue<D> r;
+	num_flux_roe_impl<D, double, false>(x.WL, x.WR, x.n, r.F, x.scale);
+	return r;
+}
+
+template <int D, typename T = double>
+__device__ __forceinline__ void num_flux_roe_pike(const T* WL, const T* WR, const double* n, T* nF, double scale = 1.0)
+{
+	if constexpr (std::is_same<T, double>::value) {
+		if (!(mulx_state<D>(WL) && mulx_state<D>(WR) && mulx_vector<D>(n) && mulx_range<60>(scale) &&
+		      num_flux_roe_impl<D, T, true>(WL, WR, n, nF, scale))) {
+			const FluxValue<D> r = num_flux_roe_fp64<D>(flux_node<D>(WL, WR, n, scale));
+#pragma unroll
+			for (int k = 0; k < D + 2; ++k)
+				nF[k] = r.F[k];
+		}
+	} else {
+		num_flux_roe_impl<D, T, false>(WL, WR, n, nF, scale);
+	}
 }
 
 // Upwind advection flux (compute_Numerical_Flux_T_advection_upwind, numerical_flux_advection_T.c:39-75).
@@ -316,9 +433,10 @@ __device__ __forceinline__ void euler_boundary_state(int bc, const T* WL, const 
 		const T cM = t1 - t2, cP = t1 + t2;
 		const T c = (cM > cP ? cM : cP);
 		const T Vn = R_l - (2.0 / kGm1) * c;
-		const T M = Vn / c;
-		const T Tb = bd.t_total / (1.0 + 0.5 * kGm1 * M * M);
-		const T p = bd.p_total * pow(Tb * (1.0 / bd.t_total), kGamma / kGm1);
+		const T M = Vn * recip(c);
+		const T iso = recip(1.0 + 0.5 * kGm1 * M * M);   // T / T_total; p / p_total is its 7/2 power (gamma = 7/5)
+		const T Tb = bd.t_total * iso;
+		const T p = bd.p_total * (iso * iso * iso * root(iso));
 		const T rho = p / (bd.r_s * Tb);
 		T V2 = 0.0;
 		WR[0] = rho;
@@ -366,16 +484,17 @@ __device__ __forceinline__ void euler_boundary_state(int bc, const T* WL, const 
 	}
 	const T p_l = kGm1 * (WL[D + 1] - 0.5 * rho_l * V2_l);
 	const double rho_r = ext[0];
+	const double rho_r_inv = recip(rho_r);
 	double u_r[D], V2_r = 0.0, Vn_r = 0.0;
 #pragma unroll
 	for (int k = 0; k < D; ++k) {
-		u_r[k] = ext[1 + k] / rho_r;
+		u_r[k] = ext[1 + k] * rho_r_inv;
 		V2_r += u_r[k] * u_r[k];
 		Vn_r += n[k] * u_r[k];
 	}
 	const double p_r = kGm1 * (ext[D + 1] - 0.5 * rho_r * V2_r);
 	const T c_l = root(kGamma * p_l * rho_l_inv);
-	const double c_r = root(kGamma * p_r / rho_r);
+	const double c_r = root(kGamma * p_r * rho_r_inv);
 	const T R_l = Vn_l + (2.0 / kGm1) * c_l;   // outgoing
 	const T R_r = Vn_r - (2.0 / kGm1) * c_r;   // incoming
 	const T Vn = 0.5 * (R_l + R_r), cc = 0.25 * kGm1 * (R_l - R_r);
@@ -395,16 +514,19 @@ __device__ __forceinline__ void euler_boundary_state(int bc, const T* WL, const 
 				uvw[k] = u_l[k];
 		}
 	} else {                        // subsonic: entropy and tangential velocity from the upwind side
+		// rho = (c^2 / (gamma s))^(1 / (gamma - 1)) with s = p / rho^gamma of the upwind side: for gamma = 7/5 that is
+		// (c^2 / (gamma p))^(5/2) rho^(7/2), which needs square roots only (a pow is hundreds of FP64 operations, and the
+		// few warps at the boundary were half of a small mesh's face kernel)
 		const T c2g = (1.0 / kGamma) * cc * cc;
 		if (Vn < 0.0) {
-			const double s_r = p_r / ::pow(rho_r, kGamma);
-			rho = pow(c2g / s_r, 1.0 / kGm1);
+			const T t = c2g * recip(p_r);
+			rho = (t * t * root(t)) * (rho_r * rho_r * rho_r * root(rho_r));
 #pragma unroll
 			for (int k = 0; k < D; ++k)
 				uvw[k] = Vn * n[k] + (u_r[k] - Vn_r * n[k]);
 		} else {
-			const T s_l = p_l / pow(rho_l, kGamma);
-			rho = pow(c2g / s_l, 1.0 / kGm1);
+			const T t = c2g * recip(p_l);
+			rho = (t * t * root(t)) * (rho_l * rho_l * rho_l * root(rho_l));
 #pragma unroll
 			for (int k = 0; k < D; ++k)
 				uvw[k] = Vn * n[k] + (u_l[k] - Vn_l * n[k]);
@@ -448,52 +570,122 @@ struct NsPhys {
 	double wall_nf_E;   // BC_NOSLIP_DIABATIC: the wall's normal energy flux -mu Cp / Pr dTdn
 };
 
-template <int D, typename T>
+// S: lone products on the integer pipe. The state and its gradient must then be in range (mulx_state, mulx_range).
+template <int D, typename T, bool S = false>
 __device__ __forceinline__ void ns_viscous_sub(const T* W, const T (*G)[D + 2], const NsPhys& ph, T (*F)[D + 2])
 {
 	const T rho = W[0], E = W[D + 1], rho_inv = recip(rho);
-	T u[D], du[D][D], V2 = 0.0;
+	T u[D], du[D][D];
 #pragma unroll
-	for (int k = 0; k < D; ++k) {
-		u[k] = W[1 + k] * rho_inv;
-		V2 += u[k] * u[k];
-	}
+	for (int k = 0; k < D; ++k)
+		u[k] = mulx<S>(W[1 + k], rho_inv);
 #pragma unroll
 	for (int s = 0; s < D; ++s)
 #pragma unroll
 		for (int x = 0; x < D; ++x)
-			du[s][x] = rho_inv * (G[x][1 + s] - G[x][0] * u[s]);
+			du[s][x] = mulx<S>(rho_inv, mad(-G[x][0], u[s], G[x][1 + s]));
 	T mu = ph.mu;
 	if (ph.viscosity == kViscositySutherland) {
-		const T p = kGm1 * (E - 0.5 * rho * V2), Tt = p / (rho * ph.r_s);
+		T V2 = mul(u[0], u[0]);
+#pragma unroll
+		for (int k = 1; k < D; ++k)
+			V2 = mad(u[k], u[k], V2);
+		const T p = kGm1 * mad(mul(-0.5, rho), V2, E), Tt = p / (rho * ph.r_s);
 		mu = 0.08 * ph.mu / (1.0 + 112.0 / Tt) * root(Tt);
 	}
-	T div = 0.0;
+	T div = du[0][0];
 #pragma unroll
-	for (int k = 0; k < D; ++k)
-		div += du[k][k];
+	for (int k = 1; k < D; ++k)
+		div = add(div, du[k][k]);
 	T tau[D][D];
+	const T mu2 = mul(mu, 2.0);
 #pragma unroll
-	for (int a = 0; a < D; ++a)
+	for (int a = 0; a < D; ++a) {
+		tau[a][a] = mul(mu2, mad(-1.0 / 3.0, div, du[a][a]));
 #pragma unroll
-		for (int b = 0; b < D; ++b)
-			tau[a][b] = (a == b) ? mu * 2.0 * (du[a][a] - div * (1.0 / 3.0)) : mu * (du[b][a] + du[a][b]);
-	const T kappa = (kGamma / ph.Pr) * mu;
+		for (int b = 0; b < a; ++b)
+			tau[a][b] = tau[b][a] = mul(mu, add(du[b][a], du[a][b]));
+	}
+	const T kappa = mul(kGamma / ph.Pr, mu), r2 = mulx<S>(rho_inv, rho_inv);
 #pragma unroll
 	for (int x = 0; x < D; ++x) {
-		const T dE_o_rho = rho_inv * rho_inv * (G[x][D + 1] * rho - E * G[x][0]);
-		T dV2 = 0.0, ut = 0.0;
+		// dTs = grad(E / rho) - 1/2 grad |u|^2
+		T dTs = mulx<S>(r2, mad(G[x][D + 1], rho, -mulx<S>(E, G[x][0])));
+		T ut = mulx<S>(u[0], tau[x][0]);
 #pragma unroll
 		for (int k = 0; k < D; ++k) {
-			dV2 += 2.0 * u[k] * du[k][x];
-			ut += u[k] * tau[x][k];
+			dTs = mad(-u[k], du[k][x], dTs);
+			if (k > 0)
+				ut = mad(u[k], tau[x][k], ut);
 		}
-		const T dTs = dE_o_rho - 0.5 * dV2;
 #pragma unroll
 		for (int k = 0; k < D; ++k)
-			F[x][1 + k] = F[x][1 + k] - tau[k][x];
-		F[x][D + 1] = F[x][D + 1] - (kappa * dTs + ut);
+			F[x][1 + k] = sub(F[x][1 + k], tau[k][x]);
+		F[x][D + 1] = sub(F[x][D + 1], mad(kappa, dTs, ut));
 	}
+}
+
+// Both forms of ns_viscous_sub from zero: -F_v of a node. The FP64 form is out of line, by value: it is rarely taken.
+template <int D>
+struct NsNode {
+	double W[D + 2], G[D][D + 2];
+};
+template <int D>
+struct NsFlux {
+	double F[D][D + 2];
+};
+template <int D>
+__device__ __noinline__ NsFlux<D> ns_viscous_fp64(NsNode<D> x, NsPhys ph)
+{
+	NsFlux<D> r;
+#pragma unroll
+	for (int i = 0; i < D; ++i)
+#pragma unroll
+		for (int k = 0; k < D + 2; ++k)
+			r.F[i][k] = 0.0;
+	ns_viscous_sub<D, double>(x.W, x.G, ph, r.F);
+	return r;
+}
+template <int D, typename T>
+__device__ __forceinline__ void ns_viscous(const T* W, const T (*G)[D + 2], const NsPhys& ph, T (*F)[D + 2])
+{
+	if constexpr (std::is_same<T, double>::value) {
+		// Sutherland's law gives NaN where the pressure is negative: it stays on the FP64 form
+		if (!(mulx_state<D>(W) && mulx_vector<D * (D + 2)>(&G[0][0]) && ph.viscosity == kViscosityConstant &&
+		      mulx_range<60>(ph.mu))) {
+			NsNode<D> x;
+#pragma unroll
+			for (int k = 0; k < D + 2; ++k) {
+				x.W[k] = W[k];
+#pragma unroll
+				for (int i = 0; i < D; ++i)
+					x.G[i][k] = G[i][k];
+			}
+			const NsFlux<D> r = ns_viscous_fp64<D>(x, ph);
+#pragma unroll
+			for (int i = 0; i < D; ++i)
+#pragma unroll
+				for (int k = 0; k < D + 2; ++k)
+					F[i][k] = r.F[i][k];
+			return;
+		}
+	}
+#pragma unroll
+	for (int i = 0; i < D; ++i)
+#pragma unroll
+		for (int k = 0; k < D + 2; ++k)
+			F[i][k] = T(0.0);
+	ns_viscous_sub<D, T, std::is_same<T, double>::value>(W, G, ph, F);
+}
+
+// The contravariant Euler flux of a node, with mulx where its values allow.
+template <int D>
+__device__ __forceinline__ void euler_flux_node(const double* W, const double* g, double (*fr)[D + 2])
+{
+	if (mulx_state<D>(W) && mulx_vector<D * D>(g))
+		euler_flux_ref<D, double, true>(W, g, fr);
+	else
+		euler_flux_ref<D>(W, g, fr);
 }
 
 }  // namespace dgpu

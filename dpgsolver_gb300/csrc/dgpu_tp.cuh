@@ -235,7 +235,7 @@ template <int D, int NV, int PDE>
 __device__ __forceinline__ void tp_flux(const double* b_adv, const double* W, const double* g, double (*fr)[NV])
 {
 	if constexpr (PDE == kEuler) {
-		euler_flux_ref<D>(W, g, fr);
+		euler_flux_node<D>(W, g, fr);
 	} else {
 		// advection: f_i = b_i u ; fr_j = sum_i g[j][i] b_i u
 #pragma unroll
@@ -662,8 +662,12 @@ tp_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const doub
 // ---------------------------------------------------------------------------------------------------------------
 // Face numerical flux
 // ---------------------------------------------------------------------------------------------------------------
+// Roe-Pike: five CTAs an SM (102 registers); the two pipes it uses overlap only across warps.
+template <int FLUX>
+struct FaceOccupancy { static constexpr int value = (FLUX == kRoePike) ? 5 : 6; };
+
 template <int D, int Q, int NV, int PDE, int FLUX>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(128, FaceOccupancy<FLUX>::value)
 tp_face_kernel(const TPParams P)
 {
 	using S = TPShape<D, Q>;
@@ -696,10 +700,7 @@ tp_face_kernel(const TPParams P)
 	if constexpr (PDE == kEuler) {
 		double nF[NV];
 		if constexpr (FLUX == kRoePike) {
-			num_flux_roe_pike<D>(WL, WR, n, nF);
-#pragma unroll
-			for (int k = 0; k < NV; ++k)
-				nF[k] *= sc;
+			num_flux_roe_pike<D>(WL, WR, n, nF, sc);
 		} else {
 			num_flux_lax_friedrichs<D>(WL, WR, n, nF, sc);
 		}
