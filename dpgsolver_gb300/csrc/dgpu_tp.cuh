@@ -642,8 +642,10 @@ __device__ __forceinline__ void tp_volume_body(const TPOps* sops, const TPParams
 	}
 }
 
+// Four CTAs per SM (64 registers, what the shared memory allows at q = 4): the FP64 flux of one CTA then overlaps the
+// integer contractions of the others. HEX 32^3 p3, 5 steps: 9.33 -> 8.97 ms together with the lift's.
 template <int D, int Q, int NV, int PDE, bool GLL_IN>
-__global__ void __launch_bounds__(TPShape<D, Q>::THREADS)
+__global__ void __launch_bounds__(TPShape<D, Q>::THREADS, 4)
 tp_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const double* __restrict__ u)
 {
 	using S = TPShape<D, Q>;
@@ -1010,9 +1012,10 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, const TPParams& 
 	}
 }
 
-// Minimum CTAs per SM of the lift kernel (caps its registers): 3 for the plain RK stage, 2 otherwise.
+// Minimum CTAs per SM of the lift kernel (caps its registers): 4 for the plain RK stage, 3 otherwise (80 registers; at 2
+// CTAs the last stage of a step with max |rhs| took 449 us at HEX 32^3 p3, twice the plain one).
 template <int MODE>
-struct LiftOccupancy { static constexpr int value = (MODE == kModeRkGlNoMax) ? 4 : 2; };   // Out: as RkGl
+struct LiftOccupancy { static constexpr int value = (MODE == kModeRkGlNoMax) ? 4 : 3; };   // Out: as RkGl
 
 template <int D, int Q, int NV, int MODE>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS, LiftOccupancy<MODE>::value)

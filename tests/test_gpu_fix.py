@@ -67,3 +67,46 @@ def test_density_spread(gpu_lib, d, p, scale):
     ok = np.isfinite(ref)
     assert np.array_equal(np.isfinite(r), ok)
     assert np.max(np.abs(np.where(ok, r - ref, 0.0))) <= 1e-12 * max(1.0, 1e-3 / scale) * np.max(np.abs(ref[ok]))
+
+
+@pytest.mark.parametrize("flux", [P.NUM_FLUX_ROE_PIKE, P.NUM_FLUX_LAX_FRIEDRICHS])
+@pytest.mark.parametrize("d", [2, 3])
+@pytest.mark.parametrize("a,b", [(0, 0), (58, 0), (61, 0), (-58, 0), (-61, 0), (0, 29), (0, 31), (0, -29), (0, -90), (-200, 70)])
+def test_scaled_euler(gpu_lib, flux, d, a, b):
+    """Density scaled by 2^a and velocity by 2^b (momentum 2^(a+b), energy 2^(a+2b)): the residual scales exactly on
+    either side of the range in which the fluxes use integer products."""
+    prob = P.euler_vortex_2d(4, 2, num_flux=flux) if d == 2 else P.euler_hex_3d(3, 2, num_flux=flux)
+    r0, _ = oracle.Oracle(prob).compute_rhs(prob.sol)
+    k = np.array([a] + [a + b] * d + [a + 2 * b])[None, :, None]
+    r, _ = _residual(prob, np.ldexp(prob.sol, k))
+    r = np.ldexp(r, -k - b)
+    assert np.max(np.abs(r - r0)) <= 1e-12 * np.max(np.abs(r0))
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("kind", ["types", "tri_quad"])
+def test_non_finite_values_in_dense_groups(gpu_lib, bad, kind):
+    """As test_non_finite_values_stay_in_their_elements, on meshes with dense groups, for one volume of every group."""
+    from dpgsolver_gb300.host.mixed_types import mixed_tri_quad_euler, mixed_types_euler
+    from dpgsolver_gb300.solver import BatchSimulation
+    prob = mixed_types_euler(4, seed=0) if kind == "types" else mixed_tri_quad_euler(6, seed=0)
+    o = oracle.Oracle(prob)
+    with BatchSimulation(prob) as sim:
+        sim.compute_rhs()
+        r0 = sim.rhs
+        for vols in prob.group_vols:
+            if not len(vols):
+                continue
+            sol = prob.sol.copy()
+            sol[prob.state_off[vols[0]]] = bad
+            with np.errstate(all="ignore"):
+                ref, _ = o.compute_rhs(sol)
+            sim.upload_state(sol)
+            sim.compute_rhs()
+            r = sim.rhs
+            off = prob.state_off
+            hit = np.array([not np.all(np.isfinite(ref[off[v]:off[v + 1]])) for v in range(prob.n_volumes)])
+            got = np.array([not np.all(np.isfinite(r[off[v]:off[v + 1]])) for v in range(prob.n_volumes)])
+            assert hit.any() and np.array_equal(got, hit)
+            same = np.repeat(~hit, np.diff(off))
+            assert np.array_equal(r[same], r0[same])
