@@ -172,7 +172,7 @@ __device__ __forceinline__ void ns_node_gradient(const TPOps* sops, const TPPara
 // Gradients and traces. At q = 4 the derivative (60 products a node) and the traces of the state and its gradient (120)
 // run in block fixed point; the FP64 pipe keeps the metric products (60).
 template <int D, int Q, int NV, bool GLL_IN>
-__global__ void __launch_bounds__(TPShape<D, Q>::THREADS)
+__global__ void __launch_bounds__(TPShape<D, Q>::THREADS, 4)
 tp_ns_grad_kernel(const __grid_constant__ TPOps ops, const TPParams P, const double* __restrict__ u)
 {
 	using S = TPShape<D, Q>;
@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(128) tp_ns_jvp_face_kernel(const TPParams P, c
 // Volume term. At q = 4 the lifting of the faces' X (90 products a node) and the derivative (60) run in block fixed point;
 // the FP64 pipe keeps the pointwise fluxes.
 template <int D, int Q, int NV, bool GLL_IN>
-__global__ void __launch_bounds__(TPShape<D, Q>::THREADS)
+__global__ void __launch_bounds__(TPShape<D, Q>::THREADS, 3)
 tp_ns_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const double* __restrict__ u)
 {
 	using S = TPShape<D, Q>;
