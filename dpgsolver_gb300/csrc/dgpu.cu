@@ -432,7 +432,8 @@ template <int D, int Q, int NV>
 size_t jvp_volume_smem_bytes()
 {
 	using S = TPShape<D, Q>;
-	return (sizeof(TPOps) + 7) / 8 * 8 + (size_t)S::E * 2 * TPSmem<D, Q, NV>::VOL * sizeof(double);
+	return sizeof(TPOps) + (size_t)S::E * 2 * (TPSmem<D, Q, NV>::VOL * sizeof(double) +
+	                                           (TPSmem<D, Q, NV>::EXP + TPSmem<D, Q, NV>::AEXP) * sizeof(int));
 }
 
 // R(u) and the directional derivative along jv_du: tangent-carrying volume and face kernels, then the residual-mode

@@ -346,8 +346,8 @@ __device__ __forceinline__ void tp_apply_fix(double* x, double* buf, double* tmp
 // The contractions of the volume term, shared by the uniform and the batched kernels: the node's state W and fluxes fr
 // are staged in su (NV N words) and sf (D NV N words) of its element, in block fixed point when the element is in range
 // (the return value), as doubles otherwise; eb receives the element's block exponents. sx: EXP zeroed ints per element,
-// `stride` ints apart. All threads of the CTA must call it; synchronises before it returns.
-template <int D, int Q, int NV>
+// `stride` ints apart. All threads of the CTA must call it; synchronises before it returns. STATE as in tp_apply_fix.
+template <int D, int Q, int NV, bool STATE = true>
 __device__ __forceinline__ bool tp_stage_volume(const double* W, const double (*fr)[NV], int e, int node, bool active,
                                                 double* su, double* sf, int* sx, int stride, int* eb)
 {
@@ -366,7 +366,7 @@ __device__ __forceinline__ bool tp_stage_volume(const double* W, const double (*
 				m = max(m, fix_exponent(fr[j][k]));
 			x[AE + k] = m;
 		}
-		if constexpr (AE > NV) {
+		if constexpr (STATE && AE > NV) {
 			x[NV] = fix_low(W[0]);
 			x[NV + 1] = fix_low(W[NV - 1]);
 		}
@@ -376,7 +376,7 @@ __device__ __forceinline__ bool tp_stage_volume(const double* W, const double (*
 	bool ok = true;
 	if (active) {
 		const int* se = sx + e * stride;
-		if constexpr (AE > NV)
+		if constexpr (STATE && AE > NV)
 			ok = fix_spread(se[0], se[NV]) && fix_spread(se[NV - 1], se[NV + 1]);
 #pragma unroll
 		for (int k = 0; k < NV; ++k) {
