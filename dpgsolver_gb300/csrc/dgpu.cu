@@ -209,7 +209,8 @@ template <int D, int Q, int NV>
 size_t adj_volume_smem_bytes()
 {
 	using S = TPShape<D, Q>;
-	return (sizeof(TPOps) + 7) / 8 * 8 + (size_t)S::E * (3 * NV * S::N + D * NV * S::N) * sizeof(double);
+	return sizeof(TPOps) + (size_t)S::E * (AdjSmem<D, Q, NV>::WORDS * sizeof(double) +
+	                                       AdjSmem<D, Q, NV>::EXP * sizeof(int));
 }
 
 template <int D, int Q, int NV>
@@ -389,7 +390,7 @@ cudaError_t launch_adjoint_t(dgpu_ctx* c, const double* u, const double* rbar, d
 	if ((e = cudaGetLastError()) != cudaSuccess)
 		return e;
 	record_start(c, "tp_adj_lift_kernel");
-	tp_adj_lift_kernel<D, Q, NV><<<blocks, S::THREADS, convert_smem_bytes<D, Q, NV>(), c->stream>>>(
+	tp_adj_lift_kernel<D, Q, NV><<<blocks, S::THREADS, lift_smem_bytes<D, Q, NV>(), c->stream>>>(
 		c->ops, c->params(), A);
 	record_stop(c);
 	c->launches += 3;
@@ -422,7 +423,7 @@ cudaError_t launch_objective_t(dgpu_ctx* c, double* ubar)
 	A.atraces = c->atraces;
 	A.wbar = c->wbar;
 	const int blocks = (c->n_vol + S::E - 1) / S::E;
-	tp_adj_lift_kernel<D, Q, NV><<<blocks, S::THREADS, convert_smem_bytes<D, Q, NV>(), c->stream>>>(
+	tp_adj_lift_kernel<D, Q, NV><<<blocks, S::THREADS, lift_smem_bytes<D, Q, NV>(), c->stream>>>(
 		c->ops, c->params(), A);
 	c->launches++;
 	return cudaGetLastError();
@@ -521,7 +522,7 @@ cudaError_t bind(dgpu_ctx* c)
 		return e;
 	if ((e = cudaFuncSetAttribute(tp_adj_volume_kernel<D, Q, NV, PDE>, smem, (int)adj_volume_smem_bytes<D, Q, NV>())))
 		return e;
-	if ((e = cudaFuncSetAttribute(tp_adj_lift_kernel<D, Q, NV>, smem, (int)convert_smem_bytes<D, Q, NV>())))
+	if ((e = cudaFuncSetAttribute(tp_adj_lift_kernel<D, Q, NV>, smem, (int)lift_smem_bytes<D, Q, NV>())))
 		return e;
 	if ((e = cudaFuncSetAttribute(tp_mass_kernel<D, Q, NV>, smem, (int)lift_smem_bytes<D, Q, NV>())))
 		return e;

@@ -307,127 +307,99 @@ __device__ __forceinline__ void num_flux_vjp_boundary(const TPParams& P, int b, 
 }
 
 // ---------------------------------------------------------------------------------------------------------------
+// Shared memory of tp_adj_volume_kernel per element (doubles) and its block exponents (ints): V u with its spreads, V^-T rbar,
+// and the same two again as staged for the traces and the derivative.
+template <int D, int Q, int NV>
+struct AdjSmem {
+	static constexpr int WORDS = 3 * NV * TPShape<D, Q>::N;
+	static constexpr int EXP = 2 * (TPSmem<D, Q, NV>::AEXP + NV);
+};
+
+// The changes of basis, the traces of both fields and Dgl_j xbar contract in block fixed point (at q = 4: 240 products a
+// node off the FP64 pipe, which keeps the flux's reverse mode). With the lift's, the adjoint of a HEX 12^3 p3 march of four
+// steps went from 3.50 to 3.01 ms.
 template <int D, int Q, int NV, int PDE>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS)
 tp_adj_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const AdjArgs A)
 {
 	using S = TPShape<D, Q>;
 	constexpr int N = S::N, NF = S::NF, E = S::E;
+	constexpr int AE = TPSmem<D, Q, NV>::AEXP, XE = AdjSmem<D, Q, NV>::EXP, PER_E = AdjSmem<D, Q, NV>::WORDS;
 	extern __shared__ double smem[];
 	TPOps* sops = reinterpret_cast<TPOps*>(smem);
 	double* base = smem + sizeof(TPOps) / 8;
-	// per element: su (ug), st (tmp), sr (xbar), sf (D blocks: Dgl_j xbar)
-	constexpr int PER_E = NV * N * 3 + D * NV * N;
-
-	const int tid = threadIdx.x;
+	int* sx = reinterpret_cast<int*>(base + E * PER_E);
 	load_ops(sops, ops);
-	const int v0 = blockIdx.x * E;
-	const int n_here = min(E, P.n_vol - v0);
-	for (int i = tid; i < n_here * NV * N; i += blockDim.x) {
-		const int e = i / (NV * N), r = i % (NV * N);
-		base[e * PER_E + r] = A.u[(size_t)v0 * NV * N + i];                    // su <- u
-		base[e * PER_E + 2 * NV * N + r] = A.rbar[(size_t)v0 * NV * N + i];    // sr <- rbar
-	}
-	__syncthreads();
-
-	const int e = tid / N, node = tid % N;
+	const int tid = threadIdx.x, v0 = blockIdx.x * E, n_here = min(E, P.n_vol - v0);
+	const int e = tid / N, node = tid % N, v = v0 + e;
 	const bool active = e < n_here;
-	const int v = v0 + e;
+	for (int i = tid; i < E * XE; i += blockDim.x)
+		sx[i] = 0;
+	double W[NV], X[NV];
+	if (active)
+#pragma unroll
+		for (int k = 0; k < NV; ++k) {
+			W[k] = A.u[((size_t)v * NV + k) * N + node];
+			X[k] = A.rbar[((size_t)v * NV + k) * N + node];
+		}
+	__syncthreads();
 	double* su = base + e * PER_E;
 	double* st = su + NV * N;
 	double* sr = st + NV * N;
-	double* sf = sr + NV * N;
-
-	// ug = V u (into st, then su)
-	tp_apply<D, Q, NV>(su, st, sf, sops->B, node, active);
-	if (active)
-#pragma unroll
-		for (int k = 0; k < NV; ++k)
-			su[k * N + node] = st[k * N + node];
-	__syncthreads();
-	// xbar = diag(1/(wJ)) V^-T rbar (into st, scaled into sr)
-	tp_apply<D, Q, NV>(sr, st, sf, sops->BinvT, node, active);
-	if (active) {
+	tp_apply_fix<D, Q, NV, true>(W, su, st, sops->fB, sops->sB, sops->B, e, node, active, sx, XE);   // ug = V u
+	tp_apply_fix<D, Q, NV, false>(X, sr, st, sops->fBinvT, sops->sBinvT, sops->BinvT, e, node, active, sx + AE, XE);
+	if (active) {   // xbar = diag(1/(wJ)) V^-T rbar
 		const double iw = P.inv_wJ[(size_t)v * N + node];
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
-			sr[k * N + node] = st[k * N + node] * iw;
+			X[k] = mul(X[k], iw);
 	}
-	__syncthreads();
+	int eb[NV], ex[NV];
+	const bool ok = tp_stage<N, NV, (NV > 1)>(W, e, node, active, su, sx + AE + NV, XE, eb);
+	const bool okx = tp_stage<N, NV, false>(X, e, node, active, sr, sx + 2 * AE + NV, XE, ex);
+	if (!active)
+		return;
 
-	if (active) {
-		// forward traces of ug and adjoint traces of xbar on the 2D local faces
-		for (int it = node; it < 2 * D * NF; it += N) {
-			const int lf = it / NF, t = it % NF;
-			const int nd = lf >> 1, side = lf & 1;
-			int t0, t1;
-			if (D == 2) {
-				t0 = t; t1 = 0;
-			} else {
-				t0 = t % Q; t1 = t / Q;
-			}
-			int stride_n, base_n;
-			if (D == 2) {
-				stride_n = (nd == 0 ? 1 : Q);
-				base_n = (nd == 0 ? t0 * Q : t0);
-			} else {
-				stride_n = (nd == 0 ? 1 : (nd == 1 ? Q : Q * Q));
-				base_n = (nd == 0 ? t0 * Q + t1 * Q * Q : (nd == 1 ? t0 + t1 * Q * Q : t0 + t1 * Q));
-			}
-			const int fs = P.vol_face[(size_t)v * 2 * D + lf];
-			double* dst = P.traces + (size_t)fs * NV * NF;
-			double* adst = A.atraces + (size_t)fs * NV * NF;
-#pragma unroll
-			for (int k = 0; k < NV; ++k) {
-				double s = 0.0, sa = 0.0;
-#pragma unroll
-				for (int m = 0; m < Q; ++m) {
-					s += sops->lb[side][m] * su[k * N + base_n + m * stride_n];
-					sa += sops->lb[side][m] * sr[k * N + base_n + m * stride_n];
-				}
-				dst[k * NF + t] = s;
-				adst[k * NF + t] = sa;
-			}
-		}
-		// Dgl_j xbar for each direction j
-#pragma unroll
-		for (int j = 0; j < D; ++j)
-			tp_pass<D, Q, NV>(sr, sf + j * NV * N, sops->Dgl, j, node);
-	}
-	__syncthreads();
-
-	if (active) {
-		double W[NV], Wb[NV], g[D * D];
-#pragma unroll
-		for (int k = 0; k < NV; ++k) {
-			W[k] = su[k * N + node];
-			Wb[k] = 0.0;
-		}
-#pragma unroll
-		for (int c = 0; c < D * D; ++c)
-			g[c] = P.gmet[((size_t)v * D * D + c) * N + node];
-		if constexpr (PDE == kEuler) {
-			double sb[D][D + 2];
-#pragma unroll
-			for (int j = 0; j < D; ++j)
-#pragma unroll
-				for (int k = 0; k < NV; ++k)
-					sb[j][k] = sf[(j * NV + k) * N + node];
-			euler_flux_ref_vjp<D>(W, g, sb, Wb);
-		} else {
-#pragma unroll
-			for (int j = 0; j < D; ++j) {
-				double gb = 0.0;
-#pragma unroll
-				for (int i = 0; i < D; ++i)
-					gb += g[j * D + i] * P.b_adv[i];
-				Wb[0] += gb * sf[j * N + node];
-			}
-		}
+	// forward traces of ug and adjoint traces of xbar on the 2D local faces
+	for (int it = node; it < 2 * D * NF; it += N) {
+		const int lf = it / NF, t = it % NF;
+		const int fs = P.vol_face[(size_t)v * 2 * D + lf];
+		double* dst = P.traces + (size_t)fs * NV * NF + t;
+		double* adst = A.atraces + (size_t)fs * NV * NF + t;
+		double out[NV];
+		tp_trace<D, Q, NV>(sops, su, eb, ok, lf, t, out);
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
-			P.vol_gl[((size_t)v * NV + k) * N + node] = Wb[k];
+			dst[k * NF] = out[k];
+		tp_trace<D, Q, NV>(sops, sr, ex, okx, lf, t, out);
+#pragma unroll
+		for (int k = 0; k < NV; ++k)
+			adst[k * NF] = out[k];
 	}
+	double sb[D][NV];
+	tp_gradient<D, Q, NV>(sops, sr, ex, okx, node, sb);   // Dgl_j xbar for each direction j
+	double Wb[NV], g[D * D];
+#pragma unroll
+	for (int k = 0; k < NV; ++k)
+		Wb[k] = 0.0;
+#pragma unroll
+	for (int c = 0; c < D * D; ++c)
+		g[c] = P.gmet[((size_t)v * D * D + c) * N + node];
+	if constexpr (PDE == kEuler) {
+		euler_flux_ref_vjp<D>(W, g, sb, Wb);
+	} else {
+#pragma unroll
+		for (int j = 0; j < D; ++j) {
+			double gb = 0.0;
+#pragma unroll
+			for (int i = 0; i < D; ++i)
+				gb += g[j * D + i] * P.b_adv[i];
+			Wb[0] += gb * sb[j][0];
+		}
+	}
+#pragma unroll
+	for (int k = 0; k < NV; ++k)
+		P.vol_gl[((size_t)v * NV + k) * N + node] = Wb[k];
 }
 
 // FP64-bound by the flux. Reverse mode took the adjoint of a HEX 12^3 p3 Lax-Friedrichs march of four steps from 4.76 to
@@ -505,60 +477,50 @@ tp_adj_face_kernel(const TPParams P, const AdjArgs A)
 	}
 }
 
+// The lifting of the face cotangents and V^T in block fixed point, as in the residual's lift.
 template <int D, int Q, int NV>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS)
 tp_adj_lift_kernel(const __grid_constant__ TPOps ops, const TPParams P, const AdjArgs A)
 {
 	using S = TPShape<D, Q>;
-	constexpr int N = S::N, NF = S::NF, E = S::E;
+	constexpr int N = S::N, NF = S::NF, E = S::E, PER_E = TPSmem<D, Q, NV>::LIFT;
+	constexpr int NFT = TPSmem<D, Q, NV>::NFT, NR = (NFT + N - 1) / N;
 	extern __shared__ double smem[];
 	TPOps* sops = reinterpret_cast<TPOps*>(smem);
 	double* base = smem + sizeof(TPOps) / 8;
-	constexpr int PER_E = 3 * NV * N;
-	const int tid = threadIdx.x;
+	int* sx = reinterpret_cast<int*>(base + E * PER_E);   // 2 NV per element, of LEXP
 	load_ops(sops, ops);
-	const int v0 = blockIdx.x * E;
-	const int n_here = min(E, P.n_vol - v0);
-	const int e = tid / N, node = tid % N;
+	const int tid = threadIdx.x, v0 = blockIdx.x * E, n_here = min(E, P.n_vol - v0);
+	const int e = tid / N, node = tid % N, v = v0 + e;
 	const bool active = e < n_here;
-	const int v = v0 + e;
 	double* sa = base + e * PER_E;
 	double* sb = sa + NV * N;
-	double* sc = sb + NV * N;
-	__syncthreads();
+	for (int i = tid; i < E * 2 * NV; i += blockDim.x)
+		sx[i] = 0;
+	double fv[NR][NV], ub[NV];
 	if (active) {
-		double ub[NV];
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
 			ub[k] = P.vol_gl[((size_t)v * NV + k) * N + node];
 #pragma unroll
-		for (int lf = 0; lf < 2 * D; ++lf) {
-			const int fs = P.vol_face[(size_t)v * 2 * D + lf];
-			const int nd = lf >> 1;
-			const int a = node_coord<Q>(node, nd);
-			int t;
-			if (D == 2) {
-				t = (nd == 0 ? node_coord<Q>(node, 1) : node_coord<Q>(node, 0));
-			} else {
-				const int c0 = node_coord<Q>(node, 0), c1 = node_coord<Q>(node, 1), c2 = node_coord<Q>(node, 2);
-				t = (nd == 0 ? c1 + Q * c2 : (nd == 1 ? c0 + Q * c2 : c0 + Q * c1));
-			}
-			const double l = sops->lb[lf & 1][a];
-			const double* src = A.wbar + (size_t)fs * NV * NF;   // this side's own node order
+		for (int r = 0; r < NR; ++r) {
+			const int it = node + r * N;
+			if (it >= NFT)
+				break;
+			const int lf = it / NF, t = it % NF;
+			const double* src = A.wbar + (size_t)P.vol_face[(size_t)v * 2 * D + lf] * NV * NF;   // this side's own node order
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
-				ub[k] += l * src[k * NF + t];
+				fv[r][k] = src[k * NF + t];
 		}
-#pragma unroll
-		for (int k = 0; k < NV; ++k)
-			sa[k * N + node] = ub[k];
 	}
 	__syncthreads();
-	tp_apply<D, Q, NV>(sa, sb, sc, sops->BT, node, active);   // ubar = V^T ubar_g
-	if (active)
+	tp_lift_sum<D, Q, NV>(sops, fv, ub, e, node, active, sa, sx, NV);
+	tp_apply_fix<D, Q, NV, false>(ub, sa, sb, sops->fBT, sops->sBT, sops->BT, e, node, active, sx + E * NV, NV);
+	if (active)   // ubar = V^T ubar_g
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
-			A.ubar[((size_t)v * NV + k) * N + node] = sb[k * N + node];
+			A.ubar[((size_t)v * NV + k) * N + node] = ub[k];
 }
 
 }  // namespace dgpu

@@ -219,13 +219,16 @@ inline FixW fix_entry(double w, int s)
 inline void derive_fix_ops(int q, int d, TPOps* o)
 {
 	double sD = 0.0, sG = 0.0, mD = 0.0, sT = 0.0, sU = 0.0, mL = 0.0, sB = 0.0, mB = 0.0, sI = 0.0, mI = 0.0;
+	double sBT = 0.0, sIT = 0.0;
 	for (int a = 0; a < q; ++a) {
-		double rD = 0.0, rG = 0.0, rB = 0.0, rI = 0.0;
+		double rD = 0.0, rG = 0.0, rB = 0.0, rI = 0.0, rBT = 0.0, rIT = 0.0;
 		for (int m = 0; m < q; ++m) {
 			rD += fabs(o->Dgl[m][a]);
 			rG += fabs(o->Dgl[a][m]);
 			rB += fabs(o->B[a][m]);
 			rI += fabs(o->Binv[a][m]);
+			rBT += fabs(o->B[m][a]);
+			rIT += fabs(o->Binv[m][a]);
 			mD = fmax(mD, fabs(o->Dgl[m][a]));
 			mB = fmax(mB, fabs(o->B[a][m]));
 			mI = fmax(mI, fabs(o->Binv[a][m]));
@@ -234,6 +237,8 @@ inline void derive_fix_ops(int q, int d, TPOps* o)
 		sG = fmax(sG, rG);
 		sB = fmax(sB, rB);
 		sI = fmax(sI, rI);
+		sBT = fmax(sBT, rBT);
+		sIT = fmax(sIT, rIT);
 		sU = fmax(sU, 1.0 + d * (fabs(o->lb[0][a]) + fabs(o->lb[1][a])));
 		mL = fmax(mL, fmax(fabs(o->lb[0][a]), fabs(o->lb[1][a])));
 	}
@@ -249,12 +254,16 @@ inline void derive_fix_ops(int q, int d, TPOps* o)
 	o->sU = fix_shift(sU, fmax(mL, 1.0), 63);
 	o->sB = fix_shift(sB, mB, 62);
 	o->sBinv = fix_shift(sI, mI, 62);
+	o->sBT = fix_shift(sBT, mB, 62);
+	o->sBinvT = fix_shift(sIT, mI, 62);
 	for (int a = 0; a < q; ++a)
 		for (int m = 0; m < q; ++m) {
 			o->fD[a][m] = fix_entry(o->Dgl[m][a], o->sD);
 			o->fG[a][m] = fix_entry(o->Dgl[a][m], o->sG);
 			o->fB[a][m] = fix_entry(o->B[a][m], o->sB);
 			o->fBinv[a][m] = fix_entry(o->Binv[a][m], o->sBinv);
+			o->fBT[a][m] = fix_entry(o->B[m][a], o->sBT);
+			o->fBinvT[a][m] = fix_entry(o->Binv[m][a], o->sBinvT);
 		}
 	for (int s = 0; s < 2; ++s)
 		for (int m = 0; m < q; ++m) {

@@ -77,45 +77,6 @@ struct NsSmem {
 	static constexpr int PER_E = WORDS + (EXP + 1) / 2;
 };
 
-// K values of every node staged in an element's buffer (K N words): in block fixed point when the element is in range
-// (returned), as doubles otherwise. eb: the K block exponents. STATE: fix_spread on x[0] and x[K - 1] (K + 2 exponents).
-// All threads of the CTA must call it; synchronises before it returns.
-template <int N, int K, bool STATE>
-__device__ __forceinline__ bool ns_stage(const double* x, int e, int node, bool active, double* buf, int* sx, int stride,
-                                         int* eb)
-{
-	constexpr int KX = STATE ? K + 2 : K;
-	int m[KX];
-#pragma unroll
-	for (int k = 0; k < K; ++k)
-		m[k] = active ? fix_exponent(x[k]) : 0;
-	if constexpr (STATE) {
-		m[K] = active ? fix_low(x[0]) : 0;
-		m[K + 1] = active ? fix_low(x[K - 1]) : 0;
-	}
-	elem_max<N, KX>(m, e, active, sx, stride);
-	__syncthreads();
-	bool ok = true;
-	if (active) {
-		const int* se = sx + e * stride;
-		if constexpr (STATE)
-			ok = fix_spread(se[0], se[K]) && fix_spread(se[K - 1], se[K + 1]);
-#pragma unroll
-		for (int k = 0; k < K; ++k) {
-			ok = ok && fix_in_range(se[k]);
-			eb[k] = fix_block(se[k]);
-		}
-#pragma unroll
-		for (int k = 0; k < K; ++k)
-			if (ok)
-				reinterpret_cast<int2*>(buf)[k * N + node] = fix_pack(x[k], eb[k]);
-			else
-				buf[k * N + node] = x[k];
-	}
-	__syncthreads();
-	return ok;
-}
-
 // The physical volume gradient of a staged state at the node, and the traces' source: three passes of Dgl in fixed point.
 template <int D, int Q, int NV>
 __device__ __forceinline__ void ns_node_gradient(const TPOps* sops, const TPParams& P, int v, int node, const double* su,
@@ -123,35 +84,7 @@ __device__ __forceinline__ void ns_node_gradient(const TPOps* sops, const TPPara
 {
 	constexpr int N = TPShape<D, Q>::N;
 	double d[D][NV];
-#pragma unroll
-	for (int j = 0; j < D; ++j) {
-		const int stride = (j == 0 ? 1 : (j == 1 ? Q : Q * Q));
-		const int a = node_coord<Q>(node, j);
-		const int b0 = node - a * stride;
-		if (ok) {
-			FixW w[Q];
-#pragma unroll
-			for (int m = 0; m < Q; ++m)
-				w[m] = sops->fG[a][m];
-#pragma unroll
-			for (int k = 0; k < NV; ++k) {
-				FixAcc s = {0, 0};
-#pragma unroll
-				for (int m = 0; m < Q; ++m)
-					fix_mac(s, w[m], reinterpret_cast<const int2*>(su)[k * N + b0 + m * stride]);
-				d[j][k] = fix_to_double(fix_sum(s), fix_scale(eb[k], sops->sG));
-			}
-		} else {
-#pragma unroll
-			for (int k = 0; k < NV; ++k)
-				d[j][k] = 0.0;
-#pragma unroll 1
-			for (int m = 0; m < Q; ++m)
-#pragma unroll
-				for (int k = 0; k < NV; ++k)
-					d[j][k] = fma(sops->Dgl[a][m], su[k * N + b0 + m * stride], d[j][k]);
-		}
-	}
+	tp_gradient<D, Q, NV>(sops, su, eb, ok, node, d);
 	const double iwJ = P.inv_wJ[(size_t)v * N + node];
 	double gm[D * D];
 #pragma unroll
@@ -200,7 +133,7 @@ tp_ns_grad_kernel(const __grid_constant__ TPOps ops, const TPParams P, const dou
 	if (GLL_IN)
 		tp_apply_fix<D, Q, NV, true>(W, su, sd, sops->fB, sops->sB, sops->B, e, node, active, sx, 2 * PER_E);
 	int eb[NV], eg[D * NV];
-	const bool ok = ns_stage<N, NV, true>(W, e, node, active, su, sx + AE, 2 * PER_E, eb);
+	const bool ok = tp_stage<N, NV, true>(W, e, node, active, su, sx + AE, 2 * PER_E, eb);
 	if (active) {
 		ns_node_gradient<D, Q, NV>(sops, P, v, node, su, eb, ok, g);
 #pragma unroll
@@ -209,7 +142,7 @@ tp_ns_grad_kernel(const __grid_constant__ TPOps ops, const TPParams P, const dou
 			for (int var = 0; var < NV; ++var)
 				P.ns_gv[(((size_t)v * D + dir) * NV + var) * N + node] = g[dir][var];
 	}
-	const bool okg = ns_stage<N, D * NV, false>(&g[0][0], e, node, active, sd, sx + 2 * AE, 2 * PER_E, eg);
+	const bool okg = tp_stage<N, D * NV, false>(&g[0][0], e, node, active, sd, sx + 2 * AE, 2 * PER_E, eg);
 	if (!active)
 		return;
 	// traces of the state and of the volume gradient on the 2D local faces

@@ -51,7 +51,9 @@ struct TPOps {
 	FixW fOne;                  // the volume term's weight 1 in that sum
 	FixW fB[kQMax][kQMax];      // B and B^-1 as 1D passes (sum |W| <= 2^62)
 	FixW fBinv[kQMax][kQMax];
-	int sD, sT, sU, sB, sBinv, sG;
+	FixW fBT[kQMax][kQMax];     // their transposes (adjoint)
+	FixW fBinvT[kQMax][kQMax];
+	int sD, sT, sU, sB, sBinv, sG, sBT, sBinvT;
 	float SBf[kQMax][kQMax];    // SBg rounded to FP32 (positivity pre-filter)
 	float pos_err;              // |FP32 Bezier coefficient - exact| <= pos_err * max_i |x_i| (per variable)
 };
@@ -450,6 +452,82 @@ __device__ __forceinline__ void tp_derivative(const TPOps* sops, const double* s
 #pragma unroll
 				for (int k = 0; k < NV; ++k)
 					out[k] = fma(sops->Dgl[m][a], f[k * N + m * stride], out[k]);
+		}
+	}
+}
+
+// K values of every node staged in an element's buffer (K N words): in block fixed point when the element is in range
+// (returned), as doubles otherwise. eb: the K block exponents. STATE: fix_spread on x[0] and x[K - 1] (K + 2 exponents).
+// All threads of the CTA must call it; synchronises before it returns.
+template <int N, int K, bool STATE>
+__device__ __forceinline__ bool tp_stage(const double* x, int e, int node, bool active, double* buf, int* sx, int stride,
+                                         int* eb)
+{
+	constexpr int KX = STATE ? K + 2 : K;
+	int m[KX];
+#pragma unroll
+	for (int k = 0; k < K; ++k)
+		m[k] = active ? fix_exponent(x[k]) : 0;
+	if constexpr (STATE) {
+		m[K] = active ? fix_low(x[0]) : 0;
+		m[K + 1] = active ? fix_low(x[K - 1]) : 0;
+	}
+	elem_max<N, KX>(m, e, active, sx, stride);
+	__syncthreads();
+	bool ok = true;
+	if (active) {
+		const int* se = sx + e * stride;
+		if constexpr (STATE)
+			ok = fix_spread(se[0], se[K]) && fix_spread(se[K - 1], se[K + 1]);
+#pragma unroll
+		for (int k = 0; k < K; ++k) {
+			ok = ok && fix_in_range(se[k]);
+			eb[k] = fix_block(se[k]);
+		}
+#pragma unroll
+		for (int k = 0; k < K; ++k)
+			if (ok)
+				reinterpret_cast<int2*>(buf)[k * N + node] = fix_pack(x[k], eb[k]);
+			else
+				buf[k * N + node] = x[k];
+	}
+	__syncthreads();
+	return ok;
+}
+
+// d[j][k] = sum_m Dgl[a][m] x of the staged values, the reference derivative in direction j at the node.
+template <int D, int Q, int NV>
+__device__ __forceinline__ void tp_gradient(const TPOps* sops, const double* su, const int* eb, bool ok, int node,
+                                            double (*d)[NV])
+{
+	constexpr int N = TPShape<D, Q>::N;
+#pragma unroll
+	for (int j = 0; j < D; ++j) {
+		const int stride = (j == 0 ? 1 : (j == 1 ? Q : Q * Q));
+		const int a = node_coord<Q>(node, j);
+		const int b0 = node - a * stride;
+		if (ok) {
+			FixW w[Q];
+#pragma unroll
+			for (int m = 0; m < Q; ++m)
+				w[m] = sops->fG[a][m];
+#pragma unroll
+			for (int k = 0; k < NV; ++k) {
+				FixAcc s = {0, 0};
+#pragma unroll
+				for (int m = 0; m < Q; ++m)
+					fix_mac(s, w[m], reinterpret_cast<const int2*>(su)[k * N + b0 + m * stride]);
+				d[j][k] = fix_to_double(fix_sum(s), fix_scale(eb[k], sops->sG));
+			}
+		} else {
+#pragma unroll
+			for (int k = 0; k < NV; ++k)
+				d[j][k] = 0.0;
+#pragma unroll 1
+			for (int m = 0; m < Q; ++m)
+#pragma unroll
+				for (int k = 0; k < NV; ++k)
+					d[j][k] = fma(sops->Dgl[a][m], su[k * N + b0 + m * stride], d[j][k]);
 		}
 	}
 }
