@@ -485,7 +485,7 @@ __device__ void blift_body(const BParams& P, const BatchOps* sops, const BGroup&
 		const double iw = P.inv_wJ[G.wj_off + (long long)(e0 + e) * N + node];
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
-			Rg[k] = mul(Rg[k], iw);
+			Rg[k] = mul_int(Rg[k], iw);
 		if (P.source) {
 			const double* sv = P.source + G.state_off + (long long)(e0 + e) * NV * N + node;
 #pragma unroll

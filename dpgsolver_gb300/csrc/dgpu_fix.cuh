@@ -276,4 +276,14 @@ __device__ __forceinline__ double fix_mul(double a, double b)
 	return __hiloint2double(rh | ((ha ^ hb) & 0x80000000), rl);
 }
 
+// a b with the bits of __dmul_rn for any factors: fix_mul when they are zero or normal and the product stays normal, the FP64
+// operation otherwise.
+__device__ __forceinline__ double mul_int(double a, double b)
+{
+	const int ea = (__double2hiint(a) >> 20) & 0x7ff, eb = (__double2hiint(b) >> 20) & 0x7ff;
+	if ((unsigned)(ea - 1) < 2046u && (unsigned)(eb - 1) < 2046u && (unsigned)(ea + eb - 1025) < 2042u)
+		return fix_mul(a, b);
+	return __dmul_rn(a, b);
+}
+
 }  // namespace dgpu

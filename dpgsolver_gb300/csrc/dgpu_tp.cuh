@@ -645,14 +645,14 @@ __device__ __forceinline__ void tp_lift_sum(const TPOps* sops, const double (*fv
 	}
 }
 
-// One SSP-RK3 stage of a value (solve_explicit.c:277-295), rounding written out.
+// One SSP-RK3 stage of a value (solve_explicit.c:277-295), rounding written out; the lone products on the integer pipe.
 __device__ __forceinline__ double rk_update(int stage, double s, double s0, double dt, double R)
 {
 	if (stage == 0)
 		return mad(dt, R, s);
 	if (stage == 1)
-		return mul(0.25, mad(dt, R, mad(3.0, s0, s)));
-	return mul(1.0 / 3.0, mad(2.0, mad(dt, R, s), s0));
+		return mul_int(0.25, mad(dt, R, mad(3.0, s0, s)));
+	return mul_int(1.0 / 3.0, mad(2.0, mad(dt, R, s), s0));
 }
 
 // Volume term of the CTA's E elements; per element PER_E doubles at base (su, st, sf at the start), sx the block
@@ -953,7 +953,7 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, const TPParams& 
 		const double iw = P.inv_wJ[(size_t)v * N + node];
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
-			Rg[k] = mul(Rg[k], iw);
+			Rg[k] = mul_int(Rg[k], iw);
 		if (P.source)
 #pragma unroll
 			for (int k = 0; k < NV; ++k)

@@ -110,3 +110,21 @@ def test_non_finite_values_in_dense_groups(gpu_lib, bad, kind):
             assert hit.any() and np.array_equal(got, hit)
             same = np.repeat(~hit, np.diff(off))
             assert np.array_equal(r[same], r0[same])
+
+
+@pytest.mark.parametrize("p", [1, 3, 4])
+@pytest.mark.parametrize("power", [-1000, -900, 0, 900, 990])
+def test_scaled_advection_steps(gpu_lib, p, power):
+    """Two SSP-RK3 steps of the linear equation scale exactly with the state: the stage's products near both ends of the
+    exponent range, where they go back to the FP64 pipe."""
+    from dpgsolver_gb300.solver import Simulation
+    prob = P.advection_2d(5, p)
+    o = oracle.Oracle(prob)
+    ref = prob.sol
+    for _ in range(2):
+        ref, _, _ = o.ssp_rk3_step(ref, prob.dt)
+    with Simulation(prob) as sim:
+        sim.upload_state(np.ldexp(prob.sol, power))
+        sim.ssp_rk3_steps(prob.dt, 2)
+        got = np.ldexp(sim.sol_coef, -power)
+    assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
