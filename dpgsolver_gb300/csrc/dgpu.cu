@@ -459,7 +459,7 @@ cudaError_t launch_jvp_t(dgpu_ctx* c)
 	tp_jvp_volume_kernel<D, Q, NV, PDE><<<blocks, S::THREADS, jvp_volume_smem_bytes<D, Q, NV>(), c->stream>>>(
 		c->ops, P, Pd, c->u, c->jv_du);
 	const long long nf = (long long)c->n_face * S::NF;
-	tp_jvp_face_kernel<D, Q, NV, PDE, FLUX><<<(unsigned)((nf + 255) / 256), 256, 0, c->stream>>>(P, Pd);
+	tp_jvp_face_kernel<D, Q, NV, PDE, FLUX><<<(unsigned)((nf + 127) / 128), 128, 0, c->stream>>>(P, Pd);
 	RkArgs rk;
 	rk.u = c->u;
 	rk.u0 = c->u0;

@@ -165,4 +165,33 @@ __device__ __forceinline__ Dual<K> recip(const Dual<K>& a)
 	return r;
 }
 
+// The value, for range checks; and the product with the value's product on the integer pipe (fix_mul).
+__device__ __forceinline__ double value(double a) { return a; }
+template <int K>
+__device__ __forceinline__ double value(const Dual<K>& a) { return a.v; }
+
+__device__ __forceinline__ double mul_fix(double a, double b) { return fix_mul(a, b); }
+template <int K>
+__device__ __forceinline__ Dual<K> mul_fix(const Dual<K>& a, const Dual<K>& b)
+{
+	Dual<K> r;
+	r.v = fix_mul(a.v, b.v);
+#pragma unroll
+	for (int k = 0; k < K; ++k)
+		r.d[k] = a.d[k] * b.v + a.v * b.d[k];
+	return r;
+}
+template <int K>
+__device__ __forceinline__ Dual<K> mul_fix(double a, const Dual<K>& b)
+{
+	Dual<K> r;
+	r.v = fix_mul(a, b.v);
+#pragma unroll
+	for (int k = 0; k < K; ++k)
+		r.d[k] = a * b.d[k];
+	return r;
+}
+template <int K>
+__device__ __forceinline__ Dual<K> mul_fix(const Dual<K>& a, double b) { return mul_fix(b, a); }
+
 }  // namespace dgpu

@@ -65,8 +65,8 @@ __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, 
 template <bool S, typename A, typename B>
 __device__ __forceinline__ auto mulx(A a, B b)
 {
-	if constexpr (S && std::is_same<A, double>::value && std::is_same<B, double>::value)
-		return fix_mul(a, b);
+	if constexpr (S)
+		return mul_fix(a, b);
 	else
 		return mul(a, b);
 }
@@ -81,13 +81,13 @@ __device__ __forceinline__ bool mulx_range(double x)
 	return h - ((1023u - LO) << 20) < ((60u + LO) << 20) || (h | (unsigned)__double2loint(x)) == 0u;
 }
 // A conserved state: density positive, every component in range.
-template <int D>
-__device__ __forceinline__ bool mulx_state(const double* W)
+template <int D, typename T>
+__device__ __forceinline__ bool mulx_state(const T* W)
 {
-	bool ok = __double2hiint(W[0]) > 0 && mulx_range<60>(W[0]) && mulx_range<60>(W[D + 1]);
+	bool ok = __double2hiint(value(W[0])) > 0 && mulx_range<60>(value(W[0])) && mulx_range<60>(value(W[D + 1]));
 #pragma unroll
 	for (int k = 0; k < D; ++k)
-		ok = ok && mulx_range<150>(W[1 + k]);
+		ok = ok && mulx_range<150>(value(W[1 + k]));
 	return ok;
 }
 template <int N>
@@ -223,7 +223,7 @@ __device__ __forceinline__ bool num_flux_lf_impl(const T* WL, const T* WR, const
 	euler_side_lf<D, T, S>(WL, n, mnL, VnL, pL, lamL);
 	euler_side_lf<D, T, S>(WR, n, mnR, VnR, pR, lamR);
 	if constexpr (S)
-		if (!positive(pL) || !positive(pR))
+		if (!positive(value(pL)) || !positive(value(pR)))
 			return false;
 	const T maxV = larger(lamL, lamR);
 	const double h = 0.5 * scale;
@@ -242,11 +242,9 @@ template <int D, typename T = double>
 __device__ __forceinline__ void num_flux_lax_friedrichs(const T* WL, const T* WR, const double* n, T* nF,
                                                         double scale = 1.0)
 {
-	if constexpr (std::is_same<T, double>::value) {
-		if (mulx_state<D>(WL) && mulx_state<D>(WR) && mulx_vector<D>(n) && mulx_range<60>(scale) &&
-		    num_flux_lf_impl<D, T, true>(WL, WR, n, nF, scale))
-			return;
-	}
+	if (mulx_state<D>(WL) && mulx_state<D>(WR) && mulx_vector<D>(n) && mulx_range<60>(scale) &&
+	    num_flux_lf_impl<D, T, true>(WL, WR, n, nF, scale))
+		return;
 	num_flux_lf_impl<D, T, false>(WL, WR, n, nF, scale);
 }
 
@@ -283,7 +281,7 @@ __device__ __forceinline__ bool num_flux_roe_impl(const T* WL, const T* WR, cons
 	}
 	const T H = mulx<S>(mad(r, HR, HL), rP1_inv), c2 = mulx<S>(kGm1, mad(-0.5, V2, H)), c = root(c2);
 	if constexpr (S)
-		if (!positive(c2))
+		if (!positive(value(c2)))
 			return false;
 	const T c_inv = recip(c);
 	const double h = 0.5 * scale;
@@ -330,7 +328,8 @@ __device__ __forceinline__ void num_flux_roe_pike(const T* WL, const T* WR, cons
 			for (int k = 0; k < D + 2; ++k)
 				nF[k] = r.F[k];
 		}
-	} else {
+	} else if (!(mulx_state<D>(WL) && mulx_state<D>(WR) && mulx_vector<D>(n) &&
+	             num_flux_roe_impl<D, T, true>(WL, WR, n, nF, scale))) {
 		num_flux_roe_impl<D, T, false>(WL, WR, n, nF, scale);
 	}
 }
