@@ -188,8 +188,13 @@ size_t bconv_smem(int E) { return sizeof(BatchOps) + (size_t)E * 3 * NV * TPShap
 [[maybe_unused]] size_t dvol_smem(int, const DGroup& G, int E) { return (size_t)E * G.vol_per_e * sizeof(double); }
 [[maybe_unused]] size_t dlift_smem(int, const DGroup& G, int E) { return (size_t)E * G.lift_per_e * sizeof(double); }
 
-// Whole warps, and at least four: the faces' interpolation between orders takes every thread of the CTA.
-[[maybe_unused]] int threads_for(int E, int N) { return std::max(((E * N + 31) / 32) * 32, 128); }
+// Whole warps, and at least four (eight in 3D, where a face has q times the columns): the faces' interpolation between
+// orders takes every thread of the CTA. 3D from four to eight: mixed types 18^3, 4 steps, 13.07 -> 12.73 ms.
+template <int D>
+int threads_for(int E, int N)
+{
+	return std::max(((E * N + 31) / 32) * 32, D == 3 ? 256 : 128);
+}
 
 [[maybe_unused]] RkArgs rk_args(const dgpu_batch* c, double dt, int stage, int want_max)
 {
@@ -212,7 +217,7 @@ cudaError_t launch_bvol(dgpu_batch* c, int g, bool gll_in)
 	const BGroup& G = c->hgroups[t];
 	if (G.n_vol == 0)
 		return cudaSuccess;
-	const int blocks = (G.n_vol + G.E - 1) / G.E, thr = threads_for(G.E, TPShape<D, Q>::N);
+	const int blocks = (G.n_vol + G.E - 1) / G.E, thr = threads_for<D>(G.E, TPShape<D, Q>::N);
 	if (gll_in)
 		bvol_group_kernel<D, Q, NV, PDE, true><<<blocks, thr, bvol_smem<D, Q, NV>(G.E), c->stream>>>(c->params(), t, c->u);
 	else
@@ -228,7 +233,7 @@ cudaError_t launch_blift(dgpu_batch* c, int g, int mode, double dt, int stage, i
 	const BGroup& G = c->hgroups[t];
 	if (G.n_vol == 0)
 		return cudaSuccess;
-	const int blocks = (G.n_vol + G.E - 1) / G.E, thr = threads_for(G.E, TPShape<D, Q>::N);
+	const int blocks = (G.n_vol + G.E - 1) / G.E, thr = threads_for<D>(G.E, TPShape<D, Q>::N);
 	const RkArgs rk = rk_args(c, dt, stage, want_max);
 	if (mode == kModeRhs)
 		blift_group_kernel<D, Q, NV, kModeRhs><<<blocks, thr, blift_smem<D, Q, NV>(G.E), c->stream>>>(c->params(), t, rk);
@@ -248,7 +253,7 @@ cudaError_t launch_bconv(dgpu_batch* c, int g, bool to_gl)
 	const BGroup& G = c->hgroups[t];
 	if (G.n_vol == 0)
 		return cudaSuccess;
-	const int blocks = (G.n_vol + G.E - 1) / G.E, thr = threads_for(G.E, TPShape<D, Q>::N);
+	const int blocks = (G.n_vol + G.E - 1) / G.E, thr = threads_for<D>(G.E, TPShape<D, Q>::N);
 	if (to_gl)
 		bconvert_group_kernel<D, Q, NV, true><<<blocks, thr, bconv_smem<D, Q, NV>(G.E), c->stream>>>(c->params(), t, c->u, c->ug);
 	else
@@ -517,7 +522,7 @@ cudaError_t launch_bns(dgpu_batch* c, int g, bool gll_in, bool volume)
 	const BGroup& G = c->hgroups[t];
 	if (G.n_vol == 0)
 		return cudaSuccess;
-	const int blocks = (G.n_vol + G.E_ns - 1) / G.E_ns, thr = threads_for(G.E_ns, TPShape<D, Q>::N);
+	const int blocks = (G.n_vol + G.E_ns - 1) / G.E_ns, thr = threads_for<D>(G.E_ns, TPShape<D, Q>::N);
 	const size_t sm = bns_smem<D, Q, NV>(G.E_ns);
 	const double* u = gll_in ? c->u : c->ug;
 	if (volume) {

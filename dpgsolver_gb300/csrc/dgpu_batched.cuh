@@ -608,7 +608,7 @@ __device__ __forceinline__ void load_batch_ops(BatchOps* sops, const BatchOps* g
 }
 
 template <int D, int Q, int NV, int PDE, bool GLL_IN>
-__global__ void __launch_bounds__(256, 3) bvol_group_kernel(const BParams P, int g, const double* __restrict__ u)
+__global__ void __launch_bounds__(256) bvol_group_kernel(const BParams P, int g, const double* __restrict__ u)
 {
 	extern __shared__ double smem[];
 	BatchOps* sops = reinterpret_cast<BatchOps*>(smem);
@@ -623,7 +623,7 @@ __global__ void __launch_bounds__(256, 3) bvol_group_kernel(const BParams P, int
 // Minimum CTAs per SM of the per-group lift (caps its registers): 4 for the RK stages that reduce no max |rhs|
 // (64 registers: twice the resident warps of the 128-register build), 2 otherwise.
 template <int MODE>
-struct BLiftOccupancy { static constexpr int value = (MODE == kModeRkGlNoMax) ? 4 : 3; };
+struct BLiftOccupancy { static constexpr int value = (MODE == kModeRkGlNoMax) ? 4 : 2; };
 
 template <int D, int Q, int NV, int MODE>
 __global__ void __launch_bounds__(256, BLiftOccupancy<MODE>::value) blift_group_kernel(const BParams P, int g,

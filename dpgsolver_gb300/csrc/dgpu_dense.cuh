@@ -1038,7 +1038,7 @@ bstage_kernel(const BParams P, const BTile* __restrict__ tiles, int n_tiles, con
 
 // Face numerical flux at every node of the faces in [node_lo, node_hi) of the q_f-sorted face node list.
 template <int D, int NV, int PDE, int FLUX>
-__global__ void __launch_bounds__(256, 2) bface_nodes_kernel(const BParams P, const int* __restrict__ node_face,
+__global__ void __launch_bounds__(256) bface_nodes_kernel(const BParams P, const int* __restrict__ node_face,
                                                            long long node_lo, long long node_hi)
 {
 	for (long long gid = node_lo + (long long)blockIdx.x * blockDim.x + threadIdx.x; gid < node_hi;
