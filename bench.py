@@ -145,8 +145,9 @@ def hbm_peak():
 
 
 def flops_per_element(d, q, nv, flux, coef_io):
-    """FP64 flops of one residual per element, counted from the kernels (FMA = 2 flops; a division or square root
-    counted as 1 flop; the instruction sequences behind them take more FP64 issue slots). coef_io: the residual
+    """Flops of one residual per element, counted from the sum-factorised formulation (FMA = 2 flops; a division or square
+    root counted as 1 flop). The kernels run the contractions, reciprocals, roots and lone products on the integer pipe,
+    so this is the work done, not the FP64 instructions issued. coef_io: the residual
     reads and writes the reference's GLL coefficients (compute_rhs_dg: + V u and V^-1 R); otherwise it is the RK
     stage on GL nodal values (+ the stage update)."""
     N = q ** d
@@ -170,9 +171,9 @@ def flops_per_element(d, q, nv, flux, coef_io):
 
 
 # FP64 thread-instructions (DFMA + DMUL + DADD) per element of one RK stage, from ncu
-# (sm__sass_thread_inst_executed_op_{dfma,dmul,dadd}_pred_on of the volume, face and lift kernels on the 24^3 p3
-# Lax-Friedrichs case, the --set full capture of one stage): 8.64 k + 4.85 k + 2.94 k.
-FP64_INSTR_PER_ELEMENT = {(3, 3, "lf"): 16432}
+# (smsp__sass_thread_inst_executed_op_{dfma,dmul,dadd}_pred_on.sum of the volume, face and lift kernels of one step on the
+# 32^3 p3 Lax-Friedrichs case): 2,048 + 1,728 + 1,013 (the mean of the three stages' lifts).
+FP64_INSTR_PER_ELEMENT = {(3, 3, "lf"): 4789}
 
 
 def ranks_barrier(torch, world):
@@ -200,23 +201,19 @@ def fp64_issue(prob, w, stage_ms, peak_tflops):
         return {}
     rate = n * prob.n_volumes / (stage_ms * 1e-3)
     return {"instr_per_element": n, "issue_frac": rate / (peak_tflops * 1e12 / 2.0),
-            "issue_source": "ncu FP64 instruction counts per element (the --set full capture of one 24^3 p3 stage) x "
-                            "elements / live stage time, against the DFMA probe's instruction rate"}
+            "issue_source": "ncu FP64 instruction counts per element (one 32^3 p3 step) x elements / live stage time, "
+                            "against the DFMA probe's instruction rate"}
 
 
 def _batching_bound(prob, w, plain_stage_ms, peak_tflops):
-    """How much faster any launch form can make a stage than the plain per-kernel launches: the plain form already
-    fills this fraction of the FP64 pipe's issue slots, and every form issues the same FP64 instructions."""
+    """How much faster the FP64 pipe would let any launch form make a stage than the plain per-kernel launches: the plain
+    form fills this fraction of the pipe's issue slots, and every form issues the same FP64 instructions."""
     iss = fp64_issue(prob, w, plain_stage_ms, peak_tflops)
     if not iss:
         return None
     return {"plain_fp64_issue_frac": iss["issue_frac"], "max_speedup_vs_plain": 1.0 / iss["issue_frac"],
-            "mixed_order_hex": {"plain_fp64_pipe_frac": 0.717, "max_speedup_vs_plain": 1.39,
-                                "source": "time-weighted FP64 pipe (elapsed) of the plain per-group stage's kernels in "
-                                          "the ncu --set full capture of the 36^3 mixed-order HEX mesh"},
-            "note": "a 3x batched-vs-plain speed-up exceeds these bounds: the plain form is FP64-issue "
-                    "bound already, so batching can only recover the idle issue slots (launch gaps, tails, low "
-                    "occupancy of the lifts)"}
+            "note": "the FP64 pipe alone; the integer contractions fill issue slots beside it, so a form can recover "
+                    "less than this (launch gaps, tails, low occupancy)"}
 
 
 def algorithmic_bytes(prob, kernel):
@@ -239,7 +236,7 @@ def algorithmic_bytes(prob, kernel):
 # DRAM bytes per element of one tp_volume_kernel launch (GL state in) measured by ncu on curved HEX 24^3, p = 3,
 # 5 variables: 99.5 MB read + 42.7 MB written over 13,824 elements (writes stay below the algorithmic vol_gl +
 # traces because L2 holds part of them until the face kernel reads them).
-_VOLUME_DRAM_BYTES_PER_ELEMENT_HEX_P3 = (99.5e6 + 42.7e6) / 13824
+_VOLUME_DRAM_BYTES_PER_ELEMENT_HEX_P3 = (235.7e6 + 167.4e6) / 32768
 
 
 def volume_traffic(prob, kernel):
@@ -426,7 +423,7 @@ def run_ours(args, rank, world, local_rank):
         "roofline": {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": volume_traffic(prob, dom),
                      "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of tp_volume_kernel on the "
-                                       "24^3 p3 case (the --set full capture of one stage), scaled per element",
+                                       "32^3 p3 case, scaled per element",
                      "peak_source": f"{peak_kind} (MEASURED_PEAKS hbm_gbs)",
                      "algorithmic_bytes_per_launch": ab, "kernel_ms": kt},
         "fp64_pipe": {"achieved_tflops": stage_flops / (stage_ms * 1e-3) / 1e12,
@@ -436,8 +433,9 @@ def run_ours(args, rank, world, local_rank):
                       **fp64_issue(prob, w, stage_ms, fp64_peak.value),
                       "dmma_tflops": mma_peak.value,
                       "dmma_source": "measured (dgpu_probe_fp64_mma: mma.sync m8n8k4 f64 loop)",
-                      "note": "binding roof: FP64 issue rate, not HBM; the FP64 tensor cores (dmma_tflops) run at "
-                              "the DFMA rate on this part, so the contractions stay on DFMA"},
+                      "note": "flops of the formulation against the FP64 pipe: the contractions run in integer arithmetic "
+                              "beside it, so frac may exceed 1; issue_frac is the pipe's own load. The FP64 tensor "
+                              "cores (dmma_tflops) run at the DFMA rate on this part"},
         "batching_bound": _batching_bound(prob, w, ms_plain / (3.0 * n_plain), fp64_peak.value),
         "eval_hbm": {"bytes_per_eval": eval_bytes(prob),
                      "achieved_gbs": eval_bytes(prob) / (ms_per_step / 3 * 1e-3) / 1e9,
@@ -825,8 +823,8 @@ def mixed_measurements(torch, stream, args, kind="types"):
         "autotune": {"form": tuned_form, "report": report},
         "fp64_pipe": {"flops_per_stage": flops, "achieved_tflops": flops / stage_s / 1e12,
                       "peak_tflops": fp64_peak.value, "frac": flops / stage_s / 1e12 / fp64_peak.value,
-                      "form": best, "note": "flops counted per volume at its own order (face interpolation to "
-                                            "p_f not counted)"},
+                      "form": best, "note": "flops of the formulation (its contractions run on the integer pipe), per volume "
+                                            "at its own order (face interpolation to p_f not counted)"},
         "eval_hbm": {"bytes_per_eval": bytes_eval, "achieved_gbs": bytes_eval / stage_s / 1e9,
                      "frac": bytes_eval / stage_s / 1e9 / peak, "peak_source": peak_kind},
         "setup_s": setup_s,

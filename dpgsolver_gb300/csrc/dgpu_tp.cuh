@@ -269,7 +269,8 @@ __device__ __noinline__ void tp_pass_rolled(const double* in, double* out, const
 }
 
 // M (x) .. (x) M applied to the CTA's elements in block fixed point (FP64 passes for an element out of range): x holds
-// the node's values on entry and exit; buf and tmp NV N words per element, sx AEXP zeroed ints per element, stride_x ints apart. STATE: x is
+// the node's values on entry and exit; buf and tmp NV N words per element, sx AEXP zeroed ints per element, stride_x ints
+// apart. STATE: x is
 // a conserved state (fix_spread). All threads of the CTA must call it; buf is free again after the next barrier.
 template <int D, int Q, int NV, bool STATE>
 __device__ __forceinline__ void tp_apply_fix(double* x, double* buf, double* tmp, const FixW (*F)[kQMax], int sF,
@@ -657,7 +658,8 @@ __device__ __forceinline__ double rk_update(int stage, double s, double s0, doub
 
 // Volume term of the CTA's E elements; per element PER_E doubles at base (su, st, sf at the start), sx the block
 // exponents. The flux is FP64; the derivative and the traces contract in block fixed point (dgpu_fix.cuh): 90 of the
-// 138 FP64 operations per node at q = 4 leave the FP64 pipe, which bounds the kernel.
+// 138 FP64 operations per node at q = 4 leave the FP64 pipe, which bounded the kernel. HEX 32^3 p3: 488 -> 218 us, the FP64
+// pipe at 50 % and the issue slots at 57 %.
 template <int D, int Q, int NV, int PDE, bool GLL_IN, int PER_E>
 __device__ __forceinline__ void tp_volume_body(const TPOps* sops, const TPParams& P, const double* __restrict__ u,
                                                int v0, int n_here, double* base, int* sx)
@@ -742,6 +744,8 @@ tp_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const doub
 // ---------------------------------------------------------------------------------------------------------------
 // Face numerical flux
 // ---------------------------------------------------------------------------------------------------------------
+// Bound by the FP64 pipe's sums and fused products (76 %); reciprocals, roots and lone products run on the integer pipe.
+// Lax-Friedrichs at HEX 32^3 p3: 295 -> 123 us.
 // Roe-Pike: five CTAs an SM (102 registers); the two pipes it uses overlap only across warps.
 template <int FLUX>
 struct FaceOccupancy { static constexpr int value = (FLUX == kRoePike) ? 5 : 6; };
@@ -1092,6 +1096,7 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, const TPParams& 
 
 // Minimum CTAs per SM of the lift kernel (caps its registers): 4 for the plain RK stage, 3 otherwise (80 registers; at 2
 // CTAs the last stage of a step with max |rhs| took 449 us at HEX 32^3 p3, twice the plain one).
+// Plain stages at HEX 32^3 p3: 244 us with FP64 products in the stage update, 187 to 212 with integer ones; both pipes at half.
 template <int MODE>
 struct LiftOccupancy { static constexpr int value = (MODE == kModeRkGlNoMax) ? 4 : 3; };   // Out: as RkGl
 
