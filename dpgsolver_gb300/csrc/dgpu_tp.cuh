@@ -270,8 +270,8 @@ __device__ __noinline__ void tp_pass_rolled(const double* in, double* out, const
 
 // M (x) .. (x) M applied to the CTA's elements in block fixed point (FP64 passes for an element out of range): x holds
 // the node's values on entry and exit; buf and tmp NV N words per element, sx AEXP zeroed ints per element, stride_x ints
-// apart. STATE: x is
-// a conserved state (fix_spread). All threads of the CTA must call it; buf is free again after the next barrier.
+// apart. STATE: x is a conserved state (fix_spread). All threads of the CTA must call it; buf is free again after the next
+// barrier.
 template <int D, int Q, int NV, bool STATE>
 __device__ __forceinline__ void tp_apply_fix(double* x, double* buf, double* tmp, const FixW (*F)[kQMax], int sF,
                                              const double (*M)[kQMax], int e, int node, bool active, int* sx,
