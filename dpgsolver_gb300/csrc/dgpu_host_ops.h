@@ -278,7 +278,7 @@ inline bool derive_tp_ops(const dgpu_tp_operators* ops, int d, TPOps* out)
 {
 	const int q = ops->p + 1;
 	memset(out, 0, sizeof *out);
-	double Bm[kQMax * kQMax], Bi[kQMax * kQMax];
+	double Bm[kQMax * kQMax], Bi[kQMax * kQMax], SB[kQMax][kQMax] = {}, BS[kQMax][kQMax] = {};   // ccSB0, ccBS0
 	for (int i = 0; i < q * q; ++i)
 		Bm[i] = ops->cv0_vs_vc[i];
 	if (!host_invert_small(q, Bm, Bi))
@@ -291,8 +291,8 @@ inline bool derive_tp_ops(const dgpu_tp_operators* ops, int d, TPOps* out)
 			for (int k = 0; k < q; ++k)
 				s += ops->cv1_vs_vc[a * q + k] * Bi[k * q + m];
 			out->Dgl[a][m] = s;
-			if (ops->ccSB0_vs_vs) out->SB[a][m] = ops->ccSB0_vs_vs[a * q + m];
-			if (ops->ccBS0_vs_vs) out->BS[a][m] = ops->ccBS0_vs_vs[a * q + m];
+			if (ops->ccSB0_vs_vs) SB[a][m] = ops->ccSB0_vs_vs[a * q + m];
+			if (ops->ccBS0_vs_vs) BS[a][m] = ops->ccBS0_vs_vs[a * q + m];
 		}
 	for (int s = 0; s < 2; ++s)
 		for (int m = 0; m < q; ++m) {
@@ -307,8 +307,8 @@ inline bool derive_tp_ops(const dgpu_tp_operators* ops, int d, TPOps* out)
 		for (int m = 0; m < q; ++m) {
 			double sbg = 0.0, bsg = 0.0;
 			for (int k = 0; k < q; ++k) {
-				sbg += out->SB[a][k] * Bi[k * q + m];
-				bsg += Bm[a * q + k] * out->BS[k][m];
+				sbg += SB[a][k] * Bi[k * q + m];
+				bsg += Bm[a * q + k] * BS[k][m];
 			}
 			out->SBg[a][m] = sbg;
 			out->BSg[a][m] = bsg;

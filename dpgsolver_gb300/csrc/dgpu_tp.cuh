@@ -37,9 +37,7 @@ struct TPOps {
 	double Binv[kQMax][kQMax];  // GL -> GLL                 Binv[a][m]
 	double Dgl[kQMax][kQMax];   // GL collocation derivative Dgl[m][k] = l_k'(x_m)
 	double lb[2][kQMax];        // GL Lagrange basis at r = -1 / +1
-	double SB[kQMax][kQMax];    // ccSB0 1D (Lagrange -> Bezier)
-	double BS[kQMax][kQMax];    // ccBS0 1D (Bezier -> Lagrange)
-	double SBg[kQMax][kQMax];   // ccSB0 B^-1: GL nodal values -> Bezier coefficients
+	double SBg[kQMax][kQMax];   // ccSB0 B^-1: GL nodal values -> Bezier coefficients (ccSB0: Lagrange -> Bezier, 1D)
 	double BSg[kQMax][kQMax];   // B ccBS0:   Bezier coefficients -> GL nodal values
 	double BT[kQMax][kQMax];    // B^T    (adjoint: V^T)
 	double BinvT[kQMax][kQMax]; // Binv^T (adjoint: V^-T)
