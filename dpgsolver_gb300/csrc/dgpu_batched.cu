@@ -1003,7 +1003,7 @@ dgpu_status create_impl(const dgpu_physics* phys, const std::vector<GroupIn>& gi
 	c->n_vol = mesh->n_volumes;
 	c->n_face = mesh->n_faces;
 	const int nv = c->nv, nV = c->n_vol, nF = c->n_face, nG = (int)gin.size();
-	auto reject = [&](dgpu_status st, const std::string& m) {
+	auto reject = [&](dgpu_status st, std::string m) {   // by value: m may be the context's own message
 		free_batch(c);
 		delete c;
 		return bfail(nullptr, st, m);
