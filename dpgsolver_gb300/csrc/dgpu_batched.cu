@@ -876,11 +876,21 @@ double abs_sum(const double* w, int rows, int cols, bool by_col, double* mx)
 // Scale of an operator of fix_dot: |W| < 2^61 and sum |W| <= 2^66.
 int dense_shift(double sum, double mx) { return fix_shift(sum, 2.0 * mx, 66); }
 
-// The fixed-point operators of a dense group (dgpu_fix.cuh), each at the largest scale its sums allow.
+// The fixed-point operators of a dense group (dgpu_fix.cuh), each at the largest scale its sums allow; none if one of them
+// has no such form.
 cudaError_t upload_fix_ops(dgpu_batch* c, const dgpu_dense_operators* op, int d, const std::vector<double>& Minv,
                            const std::vector<double>& fops, const std::vector<long long>& foff, DGroup* G)
 {
 	const int nvs = op->n_vs, nvc = op->n_vc;
+	const size_t nl = (size_t)G->n_lvc * G->n_lvs, nt = (size_t)G->n_tvc * G->n_tvs;
+	G->fix = fix_usable(op->cv0_vs_vc, (size_t)nvc * nvs) && fix_usable(op->cv1_vs_vc, (size_t)d * nvc * nvs) &&
+	         fix_usable(Minv.data(), Minv.size()) && fix_usable(fops.data(), fops.size()) &&
+	         fix_even_basis(op->cv0_vs_vc, nvc, nvs, nvs);
+	if (G->prism)
+		G->fix = G->fix && fix_usable(op->tri_cv0, nt) && fix_usable(op->tri_cv1, 2 * nt) &&
+		         fix_usable(op->line_cv0, nl) && fix_usable(op->line_cv1, nl);
+	if (!G->fix)
+		return cudaSuccess;
 	cudaError_t e;
 	double m = 0.0;
 	G->s_cv0 = dense_shift(abs_sum(op->cv0_vs_vc, nvc, nvs, false, &m), m);

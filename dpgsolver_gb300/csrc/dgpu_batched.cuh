@@ -71,6 +71,7 @@ struct DGroup {
 	const FixW *xt0, *xt0T, *xt1, *xl0, *xl1;   // WEDGE factors: tri0 [rt][t] and [t][rt], tri1, line0, line1
 	int s_cv0, s_cv1, s_f, s_minv, s_t0, s_l0, s_t1;   // s_l1 = s_t1 + s_l0 - s_t0 (one sum)
 	int nff_max;                // face nodes of the group's largest face
+	int fix;                    // 0: the operators have no fixed-point form (fix_usable): every volume keeps the FP64 loops
 };
 
 struct BParams {
@@ -179,7 +180,7 @@ __device__ void bvol_body(const BParams& P, const BatchOps* sops, const BGroup& 
 	}
 	__syncthreads();
 	if (GLL_IN)
-		tp_apply_fix<D, Q, NV, true>(W, su, st, sops->t.fB, sops->t.sB, sops->t.B, e, node, active, sx + XE, 2 * PER_E);
+		tp_apply_fix<D, Q, NV, true>(W, su, st, sops->t.fB, sops->t.sB, sops->t.B, sops->t.fix, e, node, active, sx + XE, 2 * PER_E);
 	double fr[D][NV];
 	if (active) {
 		double g[D * D];
@@ -190,7 +191,7 @@ __device__ void bvol_body(const BParams& P, const BatchOps* sops, const BGroup& 
 		tp_flux<D, NV, PDE>(P.b_adv, W, g, fr);
 	}
 	int eb[2 * NV];
-	const bool ok = tp_stage_volume<D, Q, NV>(W, fr, e, node, active, su, sf, sx, 2 * PER_E, eb);
+	const bool ok = tp_stage_volume<D, Q, NV>(W, fr, sops->t.fix, e, node, active, su, sf, sx, 2 * PER_E, eb);
 	if (active) {
 		// traces at this element's own GL points: written out where the face has them (q_f == Q), kept as limbs (or as
 		// doubles out of range) where the face's order is higher
@@ -502,7 +503,7 @@ __device__ void blift_body(const BParams& P, const BatchOps* sops, const BGroup&
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
 			R[k] = Rg[k];
-		tp_apply_fix<D, Q, NV, false>(R, sa, sb, sops->t.fBinv, sops->t.sBinv, sops->t.Binv, e, node, active,
+		tp_apply_fix<D, Q, NV, false>(R, sa, sb, sops->t.fBinv, sops->t.sBinv, sops->t.Binv, sops->t.fix, e, node, active,
 		                              sx + 2 * NV, SX);
 		if (active) {
 #pragma unroll
@@ -663,7 +664,7 @@ __global__ void __launch_bounds__(256) bconvert_group_kernel(const BParams P, in
 	}
 	__syncthreads();
 	tp_apply_fix<D, Q, NV, true>(x, base + e * PER_E, base + e * PER_E + NV * N, TO_GL ? sops->t.fB : sops->t.fBinv,
-	                             TO_GL ? sops->t.sB : sops->t.sBinv, TO_GL ? sops->t.B : sops->t.Binv, e, node, active,
+	                             TO_GL ? sops->t.sB : sops->t.sBinv, TO_GL ? sops->t.B : sops->t.Binv, sops->t.fix, e, node, active,
 	                             sx, 2 * PER_E);
 	if (active)
 #pragma unroll

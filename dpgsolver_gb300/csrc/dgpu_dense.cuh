@@ -62,15 +62,15 @@ __device__ __forceinline__ bool blk_ok(const double* smem, int PER_E, int e, int
 	return reinterpret_cast<const int*>(smem + e * PER_E + xo)[2 * NV + (slot ? 1 : 0)] != 0;
 }
 
-// The values packed in place, for the elements in range, and the flags of blk_ok.
+// The values packed in place, for the elements in range (none unless fix: DGroup::fix), and the flags of blk_ok.
 template <int NV>
-__device__ __forceinline__ void blk_pack(double* smem, int PER_E, int n_here, int off, int len, int xo, int slot)
+__device__ __forceinline__ void blk_pack(double* smem, int PER_E, int n_here, bool fix, int off, int len, int xo, int slot)
 {
 	const int lane = threadIdx.x & 31;
 	for (int p = threadIdx.x >> 5; p < n_here * NV; p += blockDim.x >> 5) {
 		const int e = p / NV, k = p % NV;
 		int* xe = reinterpret_cast<int*>(smem + e * PER_E + xo);
-		bool ok = true;
+		bool ok = fix;
 #pragma unroll
 		for (int j = 0; j < NV; ++j)
 			ok = ok && fix_in_range(xe[slot + j]);
@@ -267,7 +267,7 @@ __device__ void dvol_prism_phases(const BParams& P, const DGroup& G, int e0, int
 	__syncthreads();
 	blk_max<NV>(smem, PER_E, n_here, so, D * nvc, xo, NV);
 	__syncthreads();
-	blk_pack<NV>(smem, PER_E, n_here, so, D * nvc, xo, NV);
+	blk_pack<NV>(smem, PER_E, n_here, G.fix, so, D * nvc, xo, NV);
 	__syncthreads();
 	// 2a: gx, gy[k][c][rt] = sum_rz L0[rz][c] f_x,y[k][rz][rt];  h[k][rz][t] = sum_rt T0[rt][t] f_z[k][rz][rt]
 	const int gsz = NV * nlv * ntc;
@@ -363,7 +363,7 @@ __device__ void dvol_body(const BParams& P, const DGroup& G, int e0, int E, cons
 	__syncthreads();
 	blk_max<NV>(smem, PER_E, n_here, 0, nvs, xo, 0);
 	__syncthreads();
-	blk_pack<NV>(smem, PER_E, n_here, 0, nvs, xo, 0);
+	blk_pack<NV>(smem, PER_E, n_here, G.fix, 0, nvs, xo, 0);
 	__syncthreads();
 	if (G.prism) {
 		dvol_prism_phases<D, NV, PDE>(P, G, e0, n_here, smem, PER_E, xo);
@@ -392,7 +392,7 @@ __device__ void dvol_body(const BParams& P, const DGroup& G, int e0, int E, cons
 		__syncthreads();
 		blk_max<NV>(smem, PER_E, n_here, so, D * nvc, xo, NV);
 		__syncthreads();
-		blk_pack<NV>(smem, PER_E, n_here, so, D * nvc, xo, NV);
+		blk_pack<NV>(smem, PER_E, n_here, G.fix, so, D * nvc, xo, NV);
 		__syncthreads();
 		// phase 2: rhs_vol[k][m] = sum_j sum_r cv1_j[r][m] sf[k][j][r]
 		const int n2 = n_here * nvs, s2 = fix_split_for(n2, D * nvc);
@@ -633,7 +633,7 @@ __device__ void dlift_body(const BParams& P, const DGroup& G, int e0, int E, con
 			reinterpret_cast<int*>(smem + e * PER_E + xo)[k] = m;
 	}
 	__syncthreads();
-	blk_pack<NV>(smem, PER_E, n_here, fo, nft, xo, 0);
+	blk_pack<NV>(smem, PER_E, n_here, G.fix, fo, nft, xo, 0);
 	__syncthreads();
 	const int n1 = n_here * nvs, s1 = fix_split_for(n1, nfm);
 	for (int t0 = threadIdx.x & ~31; t0 < n1 * s1; t0 += blockDim.x) {   // whole warps: fix_join is a warp operation
@@ -683,7 +683,7 @@ __device__ void dlift_body(const BParams& P, const DGroup& G, int e0, int E, con
 	if (dense_m) {
 		blk_max<NV>(smem, PER_E, n_here, 0, nvs, xo, NV);
 		__syncthreads();
-		blk_pack<NV>(smem, PER_E, n_here, 0, nvs, xo, NV);
+		blk_pack<NV>(smem, PER_E, n_here, G.fix, 0, nvs, xo, NV);
 		__syncthreads();
 	}
 	unsigned long long mx = 0ull;

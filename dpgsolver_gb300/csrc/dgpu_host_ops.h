@@ -4,6 +4,9 @@
 #include <math.h>
 #include <string.h>
 
+#include <cmath>
+#include <initializer_list>
+
 #include "../../include/dgpu.h"
 #include "dgpu_tp.cuh"
 
@@ -194,12 +197,40 @@ inline void gauss_lobatto_nodes(int q, double* x)
 		x[q / 2] = 0.0;
 }
 
+// Whether an operator of dgpu_fix.cuh has a fixed-point form: finite, and of a magnitude between 2^-24 and 2^24, far inside
+// what the scales and the results' exponents allow. Callers' operators outside (NaN among them) stay in FP64 arithmetic,
+// which carries them through as it finds them.
+inline bool fix_usable(const double* w, size_t n)
+{
+	double mx = 0.0;
+	bool finite = true;
+	for (size_t i = 0; i < n; ++i) {
+		finite = finite && std::isfinite(w[i]);
+		mx = fmax(mx, fabs(w[i]));
+	}
+	return finite && mx >= ldexp(1.0, -24) && mx <= ldexp(1.0, 24);
+}
+
+// Whether the basis functions (columns) of an interpolation are of one magnitude: a function scaled down against the others
+// has its coefficients scaled up, and they would set the block exponent of all. The orthonormal and the nodal bases in
+// use stay within 2^3.4.
+inline bool fix_even_basis(const double* w, int rows, int cols, int ld)
+{
+	double lo = INFINITY, hi = 0.0;
+	for (int j = 0; j < cols; ++j) {
+		double m = 0.0;
+		for (int i = 0; i < rows; ++i)
+			m = fmax(m, fabs(w[(size_t)i * ld + j]));
+		lo = fmin(lo, m);
+		hi = fmax(hi, m);
+	}
+	return hi <= 64.0 * lo;
+}
+
 // Scale of a fixed-point operator (dgpu_fix.cuh): the largest s with sum 2^s <= 2^bits and max 2^s < 2^62, where sum
-// bounds sum |w| over every sum the operator enters and max its entries.
+// bounds sum |w| over every sum the operator enters and max its entries (both positive: fix_usable).
 inline int fix_shift(double sum, double mx, int bits)
 {
-	if (!(sum > 0.0) || !(sum < 1e30))
-		return 0;
 	int a, b;
 	frexp(sum * (1.0 + 1e-9), &a);   // sum < 2^a
 	frexp(mx, &b);
@@ -215,9 +246,15 @@ inline FixW fix_entry(double w, int s)
 	return f;
 }
 
-// The fixed-point operators of TPOps from its FP64 ones.
+// The fixed-point operators of TPOps from its FP64 ones, if they have such a form.
 inline void derive_fix_ops(int q, int d, TPOps* o)
 {
+	bool ok = fix_usable(&o->lb[0][0], 2 * kQMax);
+	for (const auto* M : {&o->B, &o->Binv, &o->Dgl})
+		ok = ok && fix_usable(&(*M)[0][0], kQMax * kQMax);   // zeros beyond q
+	o->fix = ok && fix_even_basis(&o->B[0][0], q, q, kQMax);
+	if (!o->fix)
+		return;
 	double sD = 0.0, sG = 0.0, mD = 0.0, sT = 0.0, sU = 0.0, mL = 0.0, sB = 0.0, mB = 0.0, sI = 0.0, mI = 0.0;
 	double sBT = 0.0, sIT = 0.0;
 	for (int a = 0; a < q; ++a) {

@@ -52,6 +52,8 @@ struct TPOps {
 	FixW fBT[kQMax][kQMax];     // their transposes (adjoint)
 	FixW fBinvT[kQMax][kQMax];
 	int sD, sT, sU, sB, sBinv, sG, sBT, sBinvT;
+	int fix;                    // 0: the operators have no fixed-point form (fix_usable): every element keeps the FP64 loops
+	int pad;
 	float SBf[kQMax][kQMax];    // SBg rounded to FP32 (positivity pre-filter)
 	float pos_err;              // |FP32 Bezier coefficient - exact| <= pos_err * max_i |x_i| (per variable)
 };
@@ -268,11 +270,11 @@ __device__ __noinline__ void tp_pass_rolled(const double* in, double* out, const
 
 // M (x) .. (x) M applied to the CTA's elements in block fixed point (FP64 passes for an element out of range): x holds
 // the node's values on entry and exit; buf and tmp NV N words per element, sx AEXP zeroed ints per element, stride_x ints
-// apart. STATE: x is a conserved state (fix_spread). All threads of the CTA must call it; buf is free again after the next
+// apart. STATE: x is a conserved state (fix_spread); fix: TPOps::fix. All threads of the CTA must call it; buf is free again after the next
 // barrier.
 template <int D, int Q, int NV, bool STATE>
 __device__ __forceinline__ void tp_apply_fix(double* x, double* buf, double* tmp, const FixW (*F)[kQMax], int sF,
-                                             const double (*M)[kQMax], int e, int node, bool active, int* sx,
+                                             const double (*M)[kQMax], bool fix, int e, int node, bool active, int* sx,
                                              int stride_x)
 {
 	constexpr int N = TPShape<D, Q>::N, K = STATE ? TPSmem<D, Q, NV>::AEXP : NV;
@@ -286,11 +288,11 @@ __device__ __forceinline__ void tp_apply_fix(double* x, double* buf, double* tmp
 	}
 	elem_max<N, K>(eb, e, active, sx, stride_x);
 	__syncthreads();
-	bool ok = true;
+	bool ok = fix;
 	if (active) {
 		const int* se = sx + e * stride_x;
 		if constexpr (K > NV)
-			ok = fix_spread(se[0], se[NV]) && fix_spread(se[NV - 1], se[NV + 1]);
+			ok = ok && fix_spread(se[0], se[NV]) && fix_spread(se[NV - 1], se[NV + 1]);
 #pragma unroll
 		for (int k = 0; k < NV; ++k) {
 			ok = ok && fix_in_range(se[k]);
@@ -349,7 +351,7 @@ __device__ __forceinline__ void tp_apply_fix(double* x, double* buf, double* tmp
 // (the return value), as doubles otherwise; eb receives the element's block exponents. sx: EXP zeroed ints per element,
 // `stride` ints apart. All threads of the CTA must call it; synchronises before it returns. STATE as in tp_apply_fix.
 template <int D, int Q, int NV, bool STATE = true>
-__device__ __forceinline__ bool tp_stage_volume(const double* W, const double (*fr)[NV], int e, int node, bool active,
+__device__ __forceinline__ bool tp_stage_volume(const double* W, const double (*fr)[NV], bool fix, int e, int node, bool active,
                                                 double* su, double* sf, int* sx, int stride, int* eb)
 {
 	constexpr int N = TPShape<D, Q>::N, XE = TPSmem<D, Q, NV>::EXP, AE = TPSmem<D, Q, NV>::AEXP;
@@ -374,11 +376,11 @@ __device__ __forceinline__ bool tp_stage_volume(const double* W, const double (*
 	}
 	elem_max<N, XE>(x, e, active, sx, stride);
 	__syncthreads();
-	bool ok = true;
+	bool ok = fix;
 	if (active) {
 		const int* se = sx + e * stride;
 		if constexpr (STATE && AE > NV)
-			ok = fix_spread(se[0], se[NV]) && fix_spread(se[NV - 1], se[NV + 1]);
+			ok = ok && fix_spread(se[0], se[NV]) && fix_spread(se[NV - 1], se[NV + 1]);
 #pragma unroll
 		for (int k = 0; k < NV; ++k) {
 			ok = ok && fix_in_range(se[k]) && fix_in_range(se[AE + k]);
@@ -459,7 +461,7 @@ __device__ __forceinline__ void tp_derivative(const TPOps* sops, const double* s
 // (returned), as doubles otherwise. eb: the K block exponents. STATE: fix_spread on x[0] and x[K - 1] (K + 2 exponents).
 // All threads of the CTA must call it; synchronises before it returns.
 template <int N, int K, bool STATE>
-__device__ __forceinline__ bool tp_stage(const double* x, int e, int node, bool active, double* buf, int* sx, int stride,
+__device__ __forceinline__ bool tp_stage(const double* x, bool fix, int e, int node, bool active, double* buf, int* sx, int stride,
                                          int* eb)
 {
 	constexpr int KX = STATE ? K + 2 : K;
@@ -473,11 +475,11 @@ __device__ __forceinline__ bool tp_stage(const double* x, int e, int node, bool 
 	}
 	elem_max<N, KX>(m, e, active, sx, stride);
 	__syncthreads();
-	bool ok = true;
+	bool ok = fix;
 	if (active) {
 		const int* se = sx + e * stride;
 		if constexpr (STATE)
-			ok = fix_spread(se[0], se[K]) && fix_spread(se[K - 1], se[K + 1]);
+			ok = ok && fix_spread(se[0], se[K]) && fix_spread(se[K - 1], se[K + 1]);
 #pragma unroll
 		for (int k = 0; k < K; ++k) {
 			ok = ok && fix_in_range(se[k]);
@@ -590,7 +592,7 @@ __device__ __forceinline__ void tp_lift_sum(const TPOps* sops, const double (*fv
 	}
 	elem_max<N, NV>(eb, e, active, sx, stride);
 	__syncthreads();
-	bool ok = true;
+	bool ok = sops->fix;
 	if (active) {
 #pragma unroll
 		for (int k = 0; k < NV; ++k) {
@@ -684,7 +686,7 @@ __device__ __forceinline__ void tp_volume_body(const TPOps* sops, const TPParams
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
 				P.keep_coef[((size_t)v * NV + k) * N + node] = W[k];
-		tp_apply_fix<D, Q, NV, true>(W, su, st, sops->fB, sops->sB, sops->B, e, node, active, sx + S::E * XE, AE);   // V u
+		tp_apply_fix<D, Q, NV, true>(W, su, st, sops->fB, sops->sB, sops->B, sops->fix, e, node, active, sx + S::E * XE, AE);   // V u
 		if (active && P.keep_gl)
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
@@ -700,7 +702,7 @@ __device__ __forceinline__ void tp_volume_body(const TPOps* sops, const TPParams
 		tp_flux<D, NV, PDE>(P.b_adv, W, g, fr);
 	}
 	int eb[2 * NV];
-	const bool ok = tp_stage_volume<D, Q, NV>(W, fr, e, node, active, su, sf, sx, XE, eb);
+	const bool ok = tp_stage_volume<D, Q, NV>(W, fr, sops->fix, e, node, active, su, sf, sx, XE, eb);
 	if (!active)
 		return;
 	double out[NV];
@@ -971,7 +973,7 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, const TPParams& 
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
 			R[k] = Rg[k];
-		tp_apply_fix<D, Q, NV, false>(R, sa, sb, sops->fBinv, sops->sBinv, sops->Binv, e, node, active,
+		tp_apply_fix<D, Q, NV, false>(R, sa, sb, sops->fBinv, sops->sBinv, sops->Binv, sops->fix, e, node, active,
 		                              sx + 2 * S::E * NV, AE);
 		if (active) {
 #pragma unroll
@@ -1078,7 +1080,7 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, const TPParams& 
 		if constexpr (MODE == kModeRkGlOut) {
 			// the new state's GLL coefficients: V^-1 of the GL values (D passes of Binv)
 			__syncthreads();   // sa/sb/sc are free again
-			tp_apply_fix<D, Q, NV, true>(snew, sa, sb, sops->fBinv, sops->sBinv, sops->Binv, e, node, active,
+			tp_apply_fix<D, Q, NV, true>(snew, sa, sb, sops->fBinv, sops->sBinv, sops->Binv, sops->fix, e, node, active,
 			                             sx + S::E * (2 * NV + AE), AE);
 			if (active)
 #pragma unroll
@@ -1148,7 +1150,7 @@ tp_convert_kernel(const __grid_constant__ TPOps ops, int n_vol, const double* __
 		sx[i] = 0;
 	__syncthreads();
 	tp_apply_fix<D, Q, NV, true>(x, base + e * PER_E, base + e * PER_E + NV * N, TO_GL ? sops->fB : sops->fBinv,
-	                       TO_GL ? sops->sB : sops->sBinv, TO_GL ? sops->B : sops->Binv, e, node, active, sx,
+	                       TO_GL ? sops->sB : sops->sBinv, TO_GL ? sops->B : sops->Binv, sops->fix, e, node, active, sx,
 	                             TPSmem<D, Q, NV>::AEXP);
 	if (active)
 #pragma unroll
