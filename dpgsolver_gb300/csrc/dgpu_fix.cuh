@@ -180,51 +180,90 @@ __device__ __forceinline__ void fix_pass(const int2* __restrict__ in, int2* __re
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Reciprocal, square root and magnitude comparison of doubles on the integer pipe
+// Reciprocal, quotient, square root and magnitude comparison of doubles on the integer pipe
 // ---------------------------------------------------------------------------------------------------------------
-// 1/x and sqrt(x) in FP64 arithmetic take 8 to 10 operations of 64 cycles; a comparison takes one. Newton's iteration
+// 1/x, sqrt(x) and a/b in FP64 arithmetic take 8 to 10 operations of 64 cycles; a comparison takes one. Newton's iteration
 // (Newton-Raphson for 1/x, the binomial series of sqrt(s0^2 + r) for the root) on integers, started from the FP32
-// approximations of the special function unit, needs about 50 to 70 cycles. Residuals are formed exactly, the result
-// carries an error of a few 2^-60 before its single rounding to nearest (at most 0.508 and 0.501 ulp over 2^30 random
-// arguments each, powers of two exact). Zeros, denormals, Inf, NaN, negative roots and reciprocals
-// that would be denormal take the FP64 operation.
-__device__ __forceinline__ double fix_rcp(double x)
+// approximations of the special function unit, needs about 50 to 70 cycles. It gives 63 bits that are at most 0.5 above and 2.4
+// below the value (over 2^30 arguments, with seeds up to two units off). One in 256 lies so near to the middle of two
+// doubles that this does not tell which way to round: those go by the remainder, which is exact in 64 bits. Every bit is
+// then the one of the FP64 operation. (No quotient, reciprocal or root of 53-bit numbers that is not one itself lies in the
+// middle.) The remainder for all of them cost 7 % of the Lax-Friedrichs face kernel, this 1 %. Zeros, denormals, Inf, NaN, negative roots and results that would be denormal take the FP64 operation.
+
+// 2^63 / d for a mantissa d in [1, 2), given by the low 20 bits of hi and lo. The seed y is in
+// [1/2, 1] for every leading mantissa (rcp.approx is within one unit, and no 1/f rounds below 1/2).
+__device__ __forceinline__ unsigned long long fix_rcp63(int hi, int lo)
 {
-	const int hi = __double2hiint(x), lo = __double2loint(x);
-	const int ex = (hi >> 20) & 0x7ff;
-	if ((unsigned)(ex - 1) >= 2044u)   // 0, denormal, Inf, NaN, or a denormal result
-		return 1.0 / x;
 	const float f = __int_as_float((__funnelshift_l(lo, hi, 3) & 0x007fffff) | 0x3f800000);   // [1, 2)
 	float y;
 	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(f));
 	const unsigned M = (min(__float_as_uint(y), 0x3f7fffffu) & 0x007fffff) | 0x00800000;      // y 2^24
 	const unsigned dh = (hi & 0x000fffff) | 0x00100000;                                        // 1.m 2^52
-	// e = 1 - d y in units of 2^-76, exactly: |e| < 2^54, so the low 64 bits suffice
-	const long long e = -(long long)((unsigned long long)(unsigned)lo * M + ((unsigned long long)(dh * M) << 32));
+	// e = d y - 1 in units of 2^-76, exactly: |e| < 2^54, so the low 64 bits suffice
+	const long long e = (long long)((unsigned long long)(unsigned)lo * M + ((unsigned long long)(dh * M) << 32));
 	const int eh = (int)(e >> 32);
-	// y (1 + e + e^2) in units of 2^-60
+	// y (1 - e + e^2) in units of 2^-63
 	const long long t = (long long)eh * (int)M + (long long)(((unsigned long long)(unsigned)e * M) >> 32);
-	const unsigned sq = (unsigned)(((long long)eh * eh) >> 20);
-	const unsigned long long R = ((unsigned long long)M << 36) + (t >> 8) + __umulhi(sq, M);
-	const unsigned long long q = (R + 64) >> 7;   // 53 bits, leading bit 52 (or 2^53)
+	const unsigned sq = (unsigned)(((long long)eh * eh) >> 17);
+	return ((unsigned long long)M << 39) + ~(t >> 5) + __umulhi(sq, M);   // ~: the next one below
+}
+// Whether a value of 63 bits is that near to the middle of two of 53, which adding 513 makes a multiple of 2^10.
+__device__ __forceinline__ bool fix_middle(unsigned long long R) { return (((unsigned)R + 515) & 1023) < 4; }
+__device__ __forceinline__ unsigned long long fix_mantissa(int hi, int lo)
+{
+	return ((unsigned long long)((hi & 0x000fffff) | 0x00100000) << 32) | (unsigned)lo;
+}
+
+// ANY: false where the caller knows that argument and result are normal numbers (a root's argument positive).
+template <bool ANY = true>
+__device__ __forceinline__ double fix_rcp(double x)
+{
+	const int hi = __double2hiint(x), lo = __double2loint(x);
+	const int ex = (hi >> 20) & 0x7ff;
+	const unsigned long long R = fix_rcp63(hi, lo);
+	unsigned long long q = (R + 513) >> 10;   // 53 bits, leading bit 52 (or 2^53)
+	const bool normal = !ANY || (unsigned)(ex - 1) < 2044u;   // not 0, denormal, Inf, NaN; and so is the result
+	if (fix_middle(R) || !normal) {                   // one branch for both
+		if (!normal)
+			return 1.0 / x;
+		const unsigned long long d = fix_mantissa(hi, lo);
+		q = (R - 16) >> 10;                           // the integer below
+		const unsigned long long rem = 0ull - d * q;  // 2^105 - d q
+		q += 2 * rem > d;
+	}
 	const int rh = (int)(q >> 32) + ((2044 - ex) << 20);
 	return __hiloint2double(rh | (hi & 0x80000000), (int)q);
 }
 
+__device__ __forceinline__ double fix_div(double a, double b)
+{
+	const int ha = __double2hiint(a), hb = __double2hiint(b);
+	const int ea = (ha >> 20) & 0x7ff, eb = (hb >> 20) & 0x7ff;
+	unsigned long long A = fix_mantissa(ha, __double2loint(a));
+	const unsigned long long d = fix_mantissa(hb, __double2loint(b));
+	const int s = A < d, ex = ea - eb + 1022 - s;   // exponent of the result, less the leading bit's one
+	if ((unsigned)(ea - 1) >= 2046u || (unsigned)(eb - 1) >= 2046u || (unsigned)ex >= 2045u)
+		return a / b;
+	A <<= s;
+	// q = A 2^52 / d, 53 bits: taken 3/16 to 21/16 low from 2^63 / d, then by the remainder
+	unsigned long long q = (__umul64hi(A << 5, fix_rcp63(hb, __double2loint(b))) - 4) >> 4;
+	const unsigned long long rem = (A << 52) - q * d;
+	q += 2 * rem > d;
+	return __hiloint2double(((int)(q >> 32) + (ex << 20)) | ((ha ^ hb) & 0x80000000), (int)q);
+}
+
+template <bool ANY = true>
 __device__ __forceinline__ double fix_sqrt(double x)
 {
 	const int hi = __double2hiint(x), lo = __double2loint(x);
 	const int ex = hi >> 20;   // negative for a negative argument
-	if ((unsigned)(ex - 1) >= 2046u)
-		return ::sqrt(x);
+	const bool normal = !ANY || (unsigned)(ex - 1) < 2046u;
 	const int t = (ex + 1) & 1;   // x = f 4^k, f = 1.m 2^t in [1, 4)
 	const float f = __int_as_float((__funnelshift_l(lo, hi, 3) & 0x007fffff) | (0x3f800000 + (t << 23)));
 	float y;
 	asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(f));
-	const unsigned M = (min(__float_as_uint(y), 0x3f7fffffu) & 0x007fffff) | 0x00800000;      // y 2^24, y in (1/2, 1]
-	const unsigned mh = (hi & 0x000fffff) | 0x00100000;
-	const unsigned long long X =
-		((((unsigned long long)mh) << 32) | (unsigned)lo) << (8 + t);                            // f 2^60
+	const unsigned M = (min(__float_as_uint(y), 0x3f7fffffu) & 0x007fffff) | 0x00800000;      // y 2^24, y in [1/2, 1]
+	const unsigned long long X = fix_mantissa(hi, lo) << (8 + t);                                // f 2^60
 	const unsigned S0 = (unsigned)(((unsigned long long)(unsigned)(X >> 32) * M) >> 22);         // s0 = f y, 2^30
 	const long long r = (long long)(X - (unsigned long long)S0 * S0);                           // f - s0^2, 2^60
 	const int d = (int)(((1ll << 54) - (long long)((unsigned long long)S0 * M)) >> 4);           // 1 - s0 y, 2^50
@@ -233,7 +272,15 @@ __device__ __forceinline__ double fix_sqrt(double x)
 	const int U = (int)(u >> 12);                                                               // 2^50
 	const int z = d - (int)(((long long)U * (int)M) >> 25);
 	const long long v = ((long long)U * z) >> 38;
-	const unsigned long long q = (((unsigned long long)S0 << 32) + u + v + 512) >> 10;
+	const unsigned long long V = ((unsigned long long)S0 << 32) + u + v;                         // sqrt(f) 2^62
+	unsigned long long q = (V + 513) >> 10;
+	if (fix_middle(V) || !normal) {
+		if (!normal)
+			return ::sqrt(x);
+		q = (V - 16) >> 10;                                                                     // the integer below
+		const unsigned long long rem = ((unsigned long long)((unsigned)lo << (20 + t)) << 32) - q * q;   // f 2^104 - q^2
+		q += rem > q;                                                                          // f 2^104 > (q + 1/2)^2
+	}
 	const int rh = (int)(q >> 32) + ((((ex - 1023 - t) >> 1) + 1022) << 20);
 	return __hiloint2double(rh, (int)q);
 }

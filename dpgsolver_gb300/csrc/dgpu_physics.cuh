@@ -24,6 +24,24 @@ using ::pow;
 __device__ __forceinline__ double recip(double x) { return fix_rcp(x); }
 __device__ __forceinline__ double root(double x) { return fix_sqrt(x); }
 
+// The same where S: the argument is known to be a positive normal number with a normal result.
+template <bool S, typename T>
+__device__ __forceinline__ T recipx(const T& x)
+{
+	if constexpr (S && std::is_same<T, double>::value)
+		return fix_rcp<false>(x);
+	else
+		return recip(x);
+}
+template <bool S, typename T>
+__device__ __forceinline__ T rootx(const T& x)
+{
+	if constexpr (S && std::is_same<T, double>::value)
+		return fix_sqrt<false>(x);
+	else
+		return root(x);
+}
+
 constexpr double kGamma = 1.4;          // definitions_physics.h:23
 constexpr double kGm1 = 0.4;            // definitions_physics.h:24
 constexpr double kEpsPhys = 1.0e-13;    // definitions_physics.h:30
@@ -143,7 +161,7 @@ template <int D, typename T = double, bool S = false>
 __device__ __forceinline__ void euler_flux_ref(const T* W, const double* g, T (*fr)[D + 2])
 {
 	const T rho = W[0], E = W[D + 1];
-	const T rho_inv = recip(rho);
+	const T rho_inv = recipx<S>(rho);
 	T m2 = mul(W[1], W[1]);
 #pragma unroll
 	for (int k = 1; k < D; ++k)
@@ -196,7 +214,7 @@ __device__ __forceinline__ FluxNode<D> flux_node(const double* WL, const double*
 template <int D, typename T, bool S>
 __device__ __forceinline__ void euler_side_lf(const T* W, const double* n, T& mn, T& Vn, T& p, T& lam)
 {
-	const T rho_inv = recip(W[0]);
+	const T rho_inv = recipx<S>(W[0]);
 	T m2 = mulx<S>(W[1], W[1]);
 	mn = mulx<S>(n[0], W[1]);
 #pragma unroll
@@ -207,7 +225,7 @@ __device__ __forceinline__ void euler_side_lf(const T* W, const double* n, T& mn
 	const T q = mulx<S>(m2, rho_inv);   // rho |V|^2
 	Vn = mulx<S>(mn, rho_inv);
 	p = mulx<S>(kGm1, mad(-0.5, q, W[D + 1]));
-	lam = add(root(mulx<S>(q, rho_inv)), root(mulx<S>(mulx<S>(kGamma, p), rho_inv)));
+	lam = add(root(mulx<S>(q, rho_inv)), rootx<S>(mulx<S>(mulx<S>(kGamma, p), rho_inv)));   // p > 0: see below
 }
 
 // Lax-Friedrichs (compute_Numerical_Flux_T_euler_lax_friedrichs, numerical_flux_euler_T.c:60-327):
@@ -215,7 +233,8 @@ __device__ __forceinline__ void euler_side_lf(const T* W, const double* n, T& mn
 // with n.F = (m.n, m Vn + p n, (E + p) Vn) of each side (compute_Flux_euler_0 contracted with n); the two sides'
 // pressure terms share one product with n. scale (the face node's w J, or 1) is folded into the factor 1/2, which
 // gives the same bits as scaling afterwards (the factor 1/2 is exact).
-// Returns false when a pressure is not positive (S only: the products then meet NaN, which fix_mul does not take).
+// Returns false when a pressure is not positive (S only: the products then meet NaN, which fix_mul does not take, and the
+// speed of sound was formed without a check).
 template <int D, typename T, bool S>
 __device__ __forceinline__ bool num_flux_lf_impl(const T* WL, const T* WR, const double* n, T* nF, double scale)
 {
@@ -256,7 +275,7 @@ template <int D, typename T, bool S>
 __device__ __forceinline__ bool num_flux_roe_impl(const T* WL, const T* WR, const double* n, T* nF, double scale)
 {
 	const T rhoL = WL[0], rhoR = WR[0], EL = WL[D + 1], ER = WR[D + 1];
-	const T rhoL_inv = recip(rhoL), rhoR_inv = recip(rhoR);
+	const T rhoL_inv = recipx<S>(rhoL), rhoR_inv = recipx<S>(rhoR);
 	T uL[D], uR[D], V2L, V2R, VnL, VnR;
 #pragma unroll
 	for (int k = 0; k < D; ++k) {
@@ -271,7 +290,7 @@ __device__ __forceinline__ bool num_flux_roe_impl(const T* WL, const T* WR, cons
 	const T pR = mulx<S>(kGm1, mad(mulx<S>(-0.5, rhoR), V2R, ER)), HR = mulx<S>(add(ER, pR), rhoR_inv);
 
 	// Roe averages (divisions by r + 1 through one reciprocal)
-	const T r = root(mulx<S>(rhoR, rhoL_inv)), rP1_inv = recip(add(r, T(1.0))), rho = mulx<S>(r, rhoL);
+	const T r = rootx<S>(mulx<S>(rhoR, rhoL_inv)), rP1_inv = recipx<S>(add(r, T(1.0))), rho = mulx<S>(r, rhoL);
 	T u[D], Vn, V2;
 #pragma unroll
 	for (int k = 0; k < D; ++k) {
@@ -279,11 +298,11 @@ __device__ __forceinline__ bool num_flux_roe_impl(const T* WL, const T* WR, cons
 		Vn = k ? mad(n[k], u[k], Vn) : mulx<S>(n[k], u[k]);
 		V2 = k ? mad(u[k], u[k], V2) : mulx<S>(u[k], u[k]);
 	}
-	const T H = mulx<S>(mad(r, HR, HL), rP1_inv), c2 = mulx<S>(kGm1, mad(-0.5, V2, H)), c = root(c2);
+	const T H = mulx<S>(mad(r, HR, HL), rP1_inv), c2 = mulx<S>(kGm1, mad(-0.5, V2, H)), c = rootx<S>(c2);   // c2 > 0, or returned below
 	if constexpr (S)
 		if (!positive(value(c2)))
 			return false;
-	const T c_inv = recip(c);
+	const T c_inv = recipx<S>(c);
 	const double h = 0.5 * scale;
 
 	const T l1 = min_abs_real(sub(VnL, c), sub(Vn, c)), l5 = max_abs_real(add(VnR, c), add(Vn, c));
