@@ -346,8 +346,8 @@ tp_adj_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const 
 	double* su = base + e * PER_E;
 	double* st = su + NV * N;
 	double* sr = st + NV * N;
-	tp_apply_fix<D, Q, NV, true>(W, su, st, sops->fB, sops->sB, sops->B, sops->fix, e, node, active, sx, XE);   // ug = V u
-	tp_apply_fix<D, Q, NV, false>(X, sr, st, sops->fBinvT, sops->sBinvT, sops->BinvT, sops->fix, e, node, active, sx + AE, XE);
+	tp_apply_fix<D, Q, NV, true>(W, su, st, sops->fB, sops->sB, sops->B, ops.fix, e, node, active, sx, XE);   // ug = V u
+	tp_apply_fix<D, Q, NV, false>(X, sr, st, sops->fBinvT, sops->sBinvT, sops->BinvT, ops.fix, e, node, active, sx + AE, XE);
 	if (active) {   // xbar = diag(1/(wJ)) V^-T rbar
 		const double iw = P.inv_wJ[(size_t)v * N + node];
 #pragma unroll
@@ -355,8 +355,8 @@ tp_adj_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const 
 			X[k] = mul(X[k], iw);
 	}
 	int eb[NV], ex[NV];
-	const bool ok = tp_stage<N, NV, (NV > 1)>(W, sops->fix, e, node, active, su, sx + AE + NV, XE, eb);
-	const bool okx = tp_stage<N, NV, false>(X, sops->fix, e, node, active, sr, sx + 2 * AE + NV, XE, ex);
+	const bool ok = tp_stage<N, NV, (NV > 1)>(W, ops.fix, e, node, active, su, sx + AE + NV, XE, eb);
+	const bool okx = tp_stage<N, NV, false>(X, ops.fix, e, node, active, sr, sx + 2 * AE + NV, XE, ex);
 	if (!active)
 		return;
 
@@ -515,8 +515,8 @@ tp_adj_lift_kernel(const __grid_constant__ TPOps ops, const TPParams P, const Ad
 		}
 	}
 	__syncthreads();
-	tp_lift_sum<D, Q, NV>(sops, fv, ub, e, node, active, sa, sx, NV);
-	tp_apply_fix<D, Q, NV, false>(ub, sa, sb, sops->fBT, sops->sBT, sops->BT, sops->fix, e, node, active, sx + E * NV, NV);
+	tp_lift_sum<D, Q, NV>(sops, ops.fix, fv, ub, e, node, active, sa, sx, NV);
+	tp_apply_fix<D, Q, NV, false>(ub, sa, sb, sops->fBT, sops->sBT, sops->BT, ops.fix, e, node, active, sx + E * NV, NV);
 	if (active)   // ubar = V^T ubar_g
 #pragma unroll
 		for (int k = 0; k < NV; ++k)

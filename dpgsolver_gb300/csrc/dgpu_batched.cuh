@@ -327,7 +327,7 @@ __device__ __forceinline__ void bface_node_rt(const BParams& P, int f, int i, in
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
 				e[k] = ext[k * nff];
-			euler_boundary_state<D, double>(code, WL, e, n, WR, P.bc_data);
+			euler_boundary<D, double>(code, WL, e, n, WR, P.bc_data);
 		} else {
 			WR[0] = advection_boundary_value<D, double>(WL[0], ext[0], n, P.b_adv);
 		}
@@ -481,7 +481,7 @@ __device__ void blift_body(const BParams& P, const BatchOps* sops, const BGroup&
 				fv[r][k] = sg[((it / NFQ) * NV + k) * NFQ + it % NFQ];
 		}
 	}
-	tp_lift_sum<D, Q, NV>(&sops->t, fv, Rg, e, node, active, sa, sx, SX);
+	tp_lift_sum<D, Q, NV>(&sops->t, sops->t.fix, fv, Rg, e, node, active, sa, sx, SX);
 	if (active) {
 		const double iw = P.inv_wJ[G.wj_off + (long long)(e0 + e) * N + node];
 #pragma unroll

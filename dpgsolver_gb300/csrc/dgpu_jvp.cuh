@@ -51,8 +51,8 @@ tp_jvp_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const 
 	double* dst = dsu + NV * N;
 	double* dsf = dst + NV * N;
 	int* dsx = sx + E * (XE + AE);
-	tp_apply_fix<D, Q, NV, true>(W, su, st, sops->fB, sops->sB, sops->B, sops->fix, e, node, active, sx + E * XE, AE);
-	tp_apply_fix<D, Q, NV, false>(dW, dsu, dst, sops->fB, sops->sB, sops->B, sops->fix, e, node, active, dsx + E * XE, AE);
+	tp_apply_fix<D, Q, NV, true>(W, su, st, sops->fB, sops->sB, sops->B, ops.fix, e, node, active, sx + E * XE, AE);
+	tp_apply_fix<D, Q, NV, false>(dW, dsu, dst, sops->fB, sops->sB, sops->B, ops.fix, e, node, active, dsx + E * XE, AE);
 	double fr[D][NV], dfr[D][NV];
 	if (active) {
 		double g[D * D];
@@ -80,8 +80,8 @@ tp_jvp_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const 
 		}
 	}
 	int eb[2 * NV], deb[2 * NV];
-	const bool ok = tp_stage_volume<D, Q, NV>(W, fr, sops->fix, e, node, active, su, sf, sx, XE, eb);
-	const bool dok = tp_stage_volume<D, Q, NV, false>(dW, dfr, sops->fix, e, node, active, dsu, dsf, dsx, XE, deb);
+	const bool ok = tp_stage_volume<D, Q, NV>(W, fr, ops.fix, e, node, active, su, sf, sx, XE, eb);
+	const bool dok = tp_stage_volume<D, Q, NV, false>(dW, dfr, ops.fix, e, node, active, dsu, dsf, dsx, XE, deb);
 	if (!active)
 		return;
 	double out[NV];

@@ -133,9 +133,9 @@ tp_ns_grad_kernel(const __grid_constant__ TPOps ops, const TPParams P, const dou
 	}
 	__syncthreads();
 	if (GLL_IN)
-		tp_apply_fix<D, Q, NV, true>(W, su, sd, sops->fB, sops->sB, sops->B, sops->fix, e, node, active, sx, 2 * PER_E);
+		tp_apply_fix<D, Q, NV, true>(W, su, sd, sops->fB, sops->sB, sops->B, ops.fix, e, node, active, sx, 2 * PER_E);
 	int eb[NV], eg[D * NV];
-	const bool ok = tp_stage<N, NV, true>(W, sops->fix, e, node, active, su, sx + AE, 2 * PER_E, eb);
+	const bool ok = tp_stage<N, NV, true>(W, ops.fix, e, node, active, su, sx + AE, 2 * PER_E, eb);
 	if (active) {
 		ns_node_gradient<D, Q, NV>(sops, P, v, node, su, eb, ok, g);
 #pragma unroll
@@ -144,7 +144,7 @@ tp_ns_grad_kernel(const __grid_constant__ TPOps ops, const TPParams P, const dou
 			for (int var = 0; var < NV; ++var)
 				P.ns_gv[(((size_t)v * D + dir) * NV + var) * N + node] = g[dir][var];
 	}
-	const bool okg = tp_stage<N, D * NV, false>(&g[0][0], sops->fix, e, node, active, sd, sx + 2 * AE, 2 * PER_E, eg);
+	const bool okg = tp_stage<N, D * NV, false>(&g[0][0], ops.fix, e, node, active, sd, sx + 2 * AE, 2 * PER_E, eg);
 	if (!active)
 		return;
 	// traces of the state and of the volume gradient on the 2D local faces
@@ -228,7 +228,7 @@ __device__ __forceinline__ void ns_boundary_state(int code, const T* WL, const d
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
 			e[k] = ext[k * ext_stride];
-		euler_boundary_state<D, T>(code, WL, e, n, WR, bcd);
+		euler_boundary<D, T>(code, WL, e, n, WR, bcd);
 	}
 }
 
@@ -399,7 +399,7 @@ tp_ns_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const d
 	}
 	__syncthreads();
 	if (GLL_IN)   // GL values of the state
-		tp_apply_fix<D, Q, NV, true>(W, su, sf, sops->fB, sops->sB, sops->B, sops->fix, e, node, active, sx, 2 * PER_E);
+		tp_apply_fix<D, Q, NV, true>(W, su, sf, sops->fB, sops->sB, sops->B, ops.fix, e, node, active, sx, 2 * PER_E);
 	double g[D][NV], fr[D][NV];
 	const double iwJ = active ? P.inv_wJ[(size_t)v * N + node] : 0.0;
 #pragma unroll
@@ -424,7 +424,7 @@ tp_ns_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const d
 					fv[r][k] = X[k * NF];
 			}
 		}
-		tp_lift_sum<D, Q, NV>(sops, fv, L, e, node, active, sf, sx + 2 * AE + dir * NV, 2 * PER_E);
+		tp_lift_sum<D, Q, NV>(sops, ops.fix, fv, L, e, node, active, sf, sx + 2 * AE + dir * NV, 2 * PER_E);
 		if (active)
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
@@ -449,7 +449,7 @@ tp_ns_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const d
 	}
 	elem_max<N, NV>(m, e, active, sx + 2 * AE + D * NV, 2 * PER_E);
 	__syncthreads();   // the lifting's sums are read: sf is free
-	bool ok = sops->fix;
+	bool ok = ops.fix;
 	if (active) {
 		const int* se = sx + e * 2 * PER_E + 2 * AE + D * NV;
 #pragma unroll

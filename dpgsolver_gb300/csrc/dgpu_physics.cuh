@@ -19,10 +19,16 @@ namespace dgpu {
 using ::fabs;
 using ::pow;
 
-// 1/x, sqrt(x) and the comparison of magnitudes of the flux routines' scalar type: doubles on the integer pipe
+// 1/x, sqrt(x), a/b and the comparison of magnitudes of the flux routines' scalar type: doubles on the integer pipe
 // (dgpu_fix.cuh), Dual in dgpu_dual.cuh.
 __device__ __forceinline__ double recip(double x) { return fix_rcp(x); }
 __device__ __forceinline__ double root(double x) { return fix_sqrt(x); }
+__device__ __forceinline__ double quot(double a, double b) { return fix_div(a, b); }
+template <typename A, typename B>
+__device__ __forceinline__ auto quot(const A& a, const B& b)
+{
+	return a / b;
+}
 
 // The same where S: the argument is known to be a positive normal number with a normal result.
 template <bool S, typename T>
@@ -451,11 +457,11 @@ __device__ __forceinline__ void euler_boundary_state(int bc, const T* WL, const 
 		const T cM = t1 - t2, cP = t1 + t2;
 		const T c = (cM > cP ? cM : cP);
 		const T Vn = R_l - (2.0 / kGm1) * c;
-		const T M = Vn * recip(c);
-		const T iso = recip(1.0 + 0.5 * kGm1 * M * M);   // T / T_total; p / p_total is its 7/2 power (gamma = 7/5)
-		const T Tb = bd.t_total * iso;
+		const T M = quot(Vn, c);
+		const T Tb = quot(bd.t_total, 1.0 + 0.5 * kGm1 * M * M);
+		const T iso = Tb * recip(bd.t_total);   // p / p_total is its 7/2 power (gamma = 7/5)
 		const T p = bd.p_total * (iso * iso * iso * root(iso));
-		const T rho = p / (bd.r_s * Tb);
+		const T rho = quot(p, bd.r_s * Tb);
 		T V2 = 0.0;
 		WR[0] = rho;
 #pragma unroll
@@ -502,17 +508,16 @@ __device__ __forceinline__ void euler_boundary_state(int bc, const T* WL, const 
 	}
 	const T p_l = kGm1 * (WL[D + 1] - 0.5 * rho_l * V2_l);
 	const double rho_r = ext[0];
-	const double rho_r_inv = recip(rho_r);
 	double u_r[D], V2_r = 0.0, Vn_r = 0.0;
 #pragma unroll
 	for (int k = 0; k < D; ++k) {
-		u_r[k] = ext[1 + k] * rho_r_inv;
+		u_r[k] = quot(ext[1 + k], rho_r);
 		V2_r += u_r[k] * u_r[k];
 		Vn_r += n[k] * u_r[k];
 	}
 	const double p_r = kGm1 * (ext[D + 1] - 0.5 * rho_r * V2_r);
 	const T c_l = root(kGamma * p_l * rho_l_inv);
-	const double c_r = root(kGamma * p_r * rho_r_inv);
+	const double c_r = root(quot(kGamma * p_r, rho_r));
 	const T R_l = Vn_l + (2.0 / kGm1) * c_l;   // outgoing
 	const T R_r = Vn_r - (2.0 / kGm1) * c_r;   // incoming
 	const T Vn = 0.5 * (R_l + R_r), cc = 0.25 * kGm1 * (R_l - R_r);
@@ -533,18 +538,19 @@ __device__ __forceinline__ void euler_boundary_state(int bc, const T* WL, const 
 		}
 	} else {                        // subsonic: entropy and tangential velocity from the upwind side
 		// rho = (c^2 / (gamma s))^(1 / (gamma - 1)) with s = p / rho^gamma of the upwind side: for gamma = 7/5 that is
-		// (c^2 / (gamma p))^(5/2) rho^(7/2), which needs square roots only (a pow is hundreds of FP64 operations, and the
-		// few warps at the boundary were half of a small mesh's face kernel)
+		// rho x^(5/2), x = c^2 rho / (gamma p) the ratio of the squared speeds of sound, which needs square roots only (a
+		// pow is hundreds of FP64 operations, and the few warps at the boundary were half of a small mesh's face kernel).
+		// The root of x is taken factor by factor: a negative pressure or density gives NaN, as its power does.
 		const T c2g = (1.0 / kGamma) * cc * cc;
 		if (Vn < 0.0) {
-			const T t = c2g * recip(p_r);
-			rho = (t * t * root(t)) * (rho_r * rho_r * rho_r * root(rho_r));
+			const T t = quot(c2g, p_r), x = t * rho_r;
+			rho = x * x * (root(t) * root(rho_r)) * rho_r;
 #pragma unroll
 			for (int k = 0; k < D; ++k)
 				uvw[k] = Vn * n[k] + (u_r[k] - Vn_r * n[k]);
 		} else {
-			const T t = c2g * recip(p_l);
-			rho = (t * t * root(t)) * (rho_l * rho_l * rho_l * root(rho_l));
+			const T t = quot(c2g, p_l), x = t * rho_l;
+			rho = x * x * (root(t) * root(rho_l)) * rho_l;
 #pragma unroll
 			for (int k = 0; k < D; ++k)
 				uvw[k] = Vn * n[k] + (u_l[k] - Vn_l * n[k]);
@@ -560,6 +566,29 @@ __device__ __forceinline__ void euler_boundary_state(int bc, const T* WL, const 
 	for (int k = 0; k < D; ++k)
 		WR[1 + k] = rho * uvw[k];
 	WR[D + 1] = p * (1.0 / kGm1) + 0.5 * rho * V2;
+}
+
+// The boundary state out of line and by value (the exterior state in x.WR): few nodes take it, and its quotients and
+// roots inlined beside a flux cost the interior nodes 4 % (Lax-Friedrichs face kernel at HEX 32^3 p3, which has no boundary:
+// 127.7 us with it inlined before its quotients were rounded, 133.3 after, 122.4 out of line).
+template <int D>
+__device__ __noinline__ FluxValue<D> euler_boundary_call(int bc, FluxNode<D> x, BcData bd)
+{
+	FluxValue<D> r;
+	euler_boundary_state<D, double>(bc, x.WL, x.WR, x.n, r.F, bd);
+	return r;
+}
+template <int D, typename T>
+__device__ __forceinline__ void euler_boundary(int bc, const T* WL, const double* ext, const double* n, T* WR, const BcData& bd)
+{
+	if constexpr (std::is_same<T, double>::value) {
+		const FluxValue<D> r = euler_boundary_call<D>(bc, flux_node<D>(WL, ext, n, 0.0), bd);
+#pragma unroll
+		for (int k = 0; k < D + 2; ++k)
+			WR[k] = r.F[k];
+	} else {
+		euler_boundary_state<D, T>(bc, WL, ext, n, WR, bd);
+	}
 }
 
 // Exterior value of an advection boundary node (constructor_Boundary_Value_T_advection_upwind,

@@ -108,7 +108,7 @@ __device__ __forceinline__ void boundary_value(const TPParams& P, int b, int i, 
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
 			e[k] = ext[k * NF + i];
-		euler_boundary_state<D, T>(P.bc_code[b], WL, e, n, WR, P.bc_data);
+		euler_boundary<D, T>(P.bc_code[b], WL, e, n, WR, P.bc_data);
 	} else {
 		WR[0] = advection_boundary_value<D, T>(WL[0], ext[i], n, P.b_adv);
 	}
@@ -572,7 +572,7 @@ __device__ __forceinline__ void tp_trace(const TPOps* sops, const double* su, co
 // words of the element, sx: NV zeroed ints per element. All threads of the CTA must call it; sa must not be written
 // before the next barrier.
 template <int D, int Q, int NV>
-__device__ __forceinline__ void tp_lift_sum(const TPOps* sops, const double (*fv)[NV], double* Rg, int e, int node,
+__device__ __forceinline__ void tp_lift_sum(const TPOps* sops, bool fix, const double (*fv)[NV], double* Rg, int e, int node,
                                             bool active, double* sa, int* sx, int stride)
 {
 	constexpr int N = TPShape<D, Q>::N, NF = TPShape<D, Q>::NF, NFT = TPSmem<D, Q, NV>::NFT, NR = (NFT + N - 1) / N;
@@ -592,7 +592,7 @@ __device__ __forceinline__ void tp_lift_sum(const TPOps* sops, const double (*fv
 	}
 	elem_max<N, NV>(eb, e, active, sx, stride);
 	__syncthreads();
-	bool ok = sops->fix;
+	bool ok = fix;
 	if (active) {
 #pragma unroll
 		for (int k = 0; k < NV; ++k) {
@@ -661,7 +661,7 @@ __device__ __forceinline__ double rk_update(int stage, double s, double s0, doub
 // 138 FP64 operations per node at q = 4 leave the FP64 pipe, which bounded the kernel. HEX 32^3 p3: 488 -> 218 us, the FP64
 // pipe at 50 % and the issue slots at 57 %.
 template <int D, int Q, int NV, int PDE, bool GLL_IN, int PER_E>
-__device__ __forceinline__ void tp_volume_body(const TPOps* sops, const TPParams& P, const double* __restrict__ u,
+__device__ __forceinline__ void tp_volume_body(const TPOps* sops, bool fix, const TPParams& P, const double* __restrict__ u,
                                                int v0, int n_here, double* base, int* sx)
 {
 	using S = TPShape<D, Q>;
@@ -686,7 +686,7 @@ __device__ __forceinline__ void tp_volume_body(const TPOps* sops, const TPParams
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
 				P.keep_coef[((size_t)v * NV + k) * N + node] = W[k];
-		tp_apply_fix<D, Q, NV, true>(W, su, st, sops->fB, sops->sB, sops->B, sops->fix, e, node, active, sx + S::E * XE, AE);   // V u
+		tp_apply_fix<D, Q, NV, true>(W, su, st, sops->fB, sops->sB, sops->B, fix, e, node, active, sx + S::E * XE, AE);   // V u
 		if (active && P.keep_gl)
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
@@ -702,7 +702,7 @@ __device__ __forceinline__ void tp_volume_body(const TPOps* sops, const TPParams
 		tp_flux<D, NV, PDE>(P.b_adv, W, g, fr);
 	}
 	int eb[2 * NV];
-	const bool ok = tp_stage_volume<D, Q, NV>(W, fr, sops->fix, e, node, active, su, sf, sx, XE, eb);
+	const bool ok = tp_stage_volume<D, Q, NV>(W, fr, fix, e, node, active, su, sf, sx, XE, eb);
 	if (!active)
 		return;
 	double out[NV];
@@ -737,7 +737,7 @@ tp_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const doub
 		*P.max_bits = 0ull;
 	double* base = smem + sizeof(TPOps) / 8;
 	constexpr int VOL = TPSmem<D, Q, NV>::VOL;
-	tp_volume_body<D, Q, NV, PDE, GLL_IN, VOL>(sops, P, u, v0, min(S::E, P.n_vol - v0), base,
+	tp_volume_body<D, Q, NV, PDE, GLL_IN, VOL>(sops, ops.fix, P, u, v0, min(S::E, P.n_vol - v0), base,
 	                                           reinterpret_cast<int*>(base + S::E * VOL));
 }
 
@@ -911,7 +911,7 @@ __device__ __noinline__ bool tp_positivity_exact(const double (*toB)[kQMax], con
 // Lift, 1/(wJ), then the residual (V^-1, max|rhs|) or the RK stage + positivity, for the CTA's E elements; per
 // element PER_E doubles at base.
 template <int D, int Q, int NV, int MODE, int PER_E>
-__device__ __forceinline__ void tp_lift_body(const TPOps* sops, const TPParams& P, const RkArgs& rk, int v0,
+__device__ __forceinline__ void tp_lift_body(const TPOps* sops, bool fix, const TPParams& P, const RkArgs& rk, int v0,
                                              int n_here, double* base, int* sx)
 {
 	using S = TPShape<D, Q>;
@@ -952,7 +952,7 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, const TPParams& 
 		}
 	}
 	__syncthreads();   // sx is zero; sops is written by other warps
-	tp_lift_sum<D, Q, NV>(sops, fv, Rg, e, node, active, sa, sx, NV);
+	tp_lift_sum<D, Q, NV>(sops, fix, fv, Rg, e, node, active, sa, sx, NV);
 	if (active) {
 		const double iw = P.inv_wJ[(size_t)v * N + node];
 #pragma unroll
@@ -973,7 +973,7 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, const TPParams& 
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
 			R[k] = Rg[k];
-		tp_apply_fix<D, Q, NV, false>(R, sa, sb, sops->fBinv, sops->sBinv, sops->Binv, sops->fix, e, node, active,
+		tp_apply_fix<D, Q, NV, false>(R, sa, sb, sops->fBinv, sops->sBinv, sops->Binv, fix, e, node, active,
 		                              sx + 2 * S::E * NV, AE);
 		if (active) {
 #pragma unroll
@@ -1080,7 +1080,7 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, const TPParams& 
 		if constexpr (MODE == kModeRkGlOut) {
 			// the new state's GLL coefficients: V^-1 of the GL values (D passes of Binv)
 			__syncthreads();   // sa/sb/sc are free again
-			tp_apply_fix<D, Q, NV, true>(snew, sa, sb, sops->fBinv, sops->sBinv, sops->Binv, sops->fix, e, node, active,
+			tp_apply_fix<D, Q, NV, true>(snew, sa, sb, sops->fBinv, sops->sBinv, sops->Binv, fix, e, node, active,
 			                             sx + S::E * (2 * NV + AE), AE);
 			if (active)
 #pragma unroll
@@ -1111,7 +1111,7 @@ tp_lift_kernel(const __grid_constant__ TPOps ops, const TPParams P, const RkArgs
 	const int v0 = blockIdx.x * S::E;
 	constexpr int LIFT = TPSmem<D, Q, NV>::LIFT;
 	double* base = smem + sizeof(TPOps) / 8;
-	tp_lift_body<D, Q, NV, MODE, LIFT>(sops, P, rk, v0, min(S::E, P.n_vol - v0), base,
+	tp_lift_body<D, Q, NV, MODE, LIFT>(sops, ops.fix, P, rk, v0, min(S::E, P.n_vol - v0), base,
 	                                   reinterpret_cast<int*>(base + S::E * LIFT));
 }
 
@@ -1150,7 +1150,7 @@ tp_convert_kernel(const __grid_constant__ TPOps ops, int n_vol, const double* __
 		sx[i] = 0;
 	__syncthreads();
 	tp_apply_fix<D, Q, NV, true>(x, base + e * PER_E, base + e * PER_E + NV * N, TO_GL ? sops->fB : sops->fBinv,
-	                       TO_GL ? sops->sB : sops->sBinv, TO_GL ? sops->B : sops->Binv, sops->fix, e, node, active, sx,
+	                       TO_GL ? sops->sB : sops->sBinv, TO_GL ? sops->B : sops->Binv, ops.fix, e, node, active, sx,
 	                             TPSmem<D, Q, NV>::AEXP);
 	if (active)
 #pragma unroll
