@@ -329,7 +329,7 @@ tp_adj_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const 
 	TPOps* sops = reinterpret_cast<TPOps*>(smem);
 	double* base = smem + sizeof(TPOps) / 8;
 	int* sx = reinterpret_cast<int*>(base + E * PER_E);
-	load_ops(sops, ops);
+	load_ops<kFixed<NV>>(sops, ops);
 	const int tid = threadIdx.x, v0 = blockIdx.x * E, n_here = min(E, P.n_vol - v0);
 	const int e = tid / N, node = tid % N, v = v0 + e;
 	const bool active = e < n_here;
@@ -489,7 +489,7 @@ tp_adj_lift_kernel(const __grid_constant__ TPOps ops, const TPParams P, const Ad
 	TPOps* sops = reinterpret_cast<TPOps*>(smem);
 	double* base = smem + sizeof(TPOps) / 8;
 	int* sx = reinterpret_cast<int*>(base + E * PER_E);   // 2 NV per element, of LEXP
-	load_ops(sops, ops);
+	load_ops<kFixed<NV>>(sops, ops);
 	const int tid = threadIdx.x, v0 = blockIdx.x * E, n_here = min(E, P.n_vol - v0);
 	const int e = tid / N, node = tid % N, v = v0 + e;
 	const bool active = e < n_here;

@@ -204,7 +204,7 @@ __device__ void bvol_body(const BParams& P, const BatchOps* sops, const BGroup& 
 #pragma unroll
 				for (int k = 0; k < NV; ++k)
 					dst[k * NFQ + t] = out[k];
-			} else if (ok) {
+			} else if (kFixed<NV> && ok) {
 				int stride, b0;
 				tp_face_line<D, Q>(lf, t, b0, stride);
 				const int2* xu = reinterpret_cast<const int2*>(su) + b0;
@@ -245,7 +245,7 @@ __device__ void bvol_body(const BParams& P, const BatchOps* sops, const BGroup& 
 			const int lf = it / (NV * kQMax), k = it / kQMax % NV, i0 = it % kQMax, qf = tab[lf].qf;
 			if (qf == Q || i0 >= qf)
 				continue;
-			const bool ok = sx[e * 2 * PER_E + XE] != 0;
+			const bool ok = kFixed<NV> && sx[e * 2 * PER_E + XE] != 0;
 			const int nff = (D == 2 ? qf : qf * qf);
 			double* dst = P.traces + 2 * NV * tab[lf].base + (long long)tab[lf].side * NV * nff + k * nff + i0;
 			if (ok) {
@@ -413,7 +413,7 @@ __device__ void blift_body(const BParams& P, const BatchOps* sops, const BGroup&
 					if (i0 < qf && (D == 2 || i1 < qf))
 						xe = max(xe, (reinterpret_cast<const int*>(src)[2 * (ci ? ci[i] : i) + 1] >> 20) & 0x7ff);
 				}
-			if (fix_in_range(xe)) {
+			if (kFixed<NV> && fix_in_range(xe)) {
 				const int eb = fix_block(xe), sI = sops->sI[qf];
 				int2 r[N1];
 #pragma unroll

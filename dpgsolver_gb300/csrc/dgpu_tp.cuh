@@ -22,6 +22,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #include "dgpu_fix.cuh"
@@ -41,7 +42,9 @@ struct TPOps {
 	double BSg[kQMax][kQMax];   // B ccBS0:   Bezier coefficients -> GL nodal values
 	double BT[kQMax][kQMax];    // B^T    (adjoint: V^T)
 	double BinvT[kQMax][kQMax]; // Binv^T (adjoint: V^-T)
-	// Fixed-point forms (dgpu_fix.cuh) and their scales: W = w 2^s
+	float SBf[kQMax][kQMax];    // SBg rounded to FP32 (positivity pre-filter)
+	float pos_err;              // |FP32 Bezier coefficient - exact| <= pos_err * max_i |x_i| (per variable)
+	// Fixed-point forms (dgpu_fix.cuh) and their scales: W = w 2^s. Last: load_ops leaves them out where they are not used
 	FixW fD[kQMax][kQMax];      // Dgl^T: fD[a][m] = Dgl[m][a], summed over the D directions
 	FixW fG[kQMax][kQMax];      // Dgl, one direction (Navier-Stokes gradients)
 	FixW fT[2][kQMax];          // lb as the trace operator
@@ -54,10 +57,16 @@ struct TPOps {
 	int sD, sT, sU, sB, sBinv, sG, sBT, sBinvT;
 	int fix;                    // 0: the operators have no fixed-point form (fix_usable): every element keeps the FP64 loops
 	int pad;
-	float SBf[kQMax][kQMax];    // SBg rounded to FP32 (positivity pre-filter)
-	float pos_err;              // |FP32 Bezier coefficient - exact| <= pos_err * max_i |x_i| (per variable)
 };
-static_assert(sizeof(TPOps) % 8 == 0, "TPOps is copied to shared memory as doubles");
+static_assert(sizeof(TPOps) % 8 == 0 && offsetof(TPOps, fD) % 8 == 0, "TPOps is copied to shared memory as doubles");
+
+// Whether the contractions of NV variables run in block fixed point. The advected scalar stays in FP64: its flux couples a
+// line of nodes to no other one when the velocity lies along it, and a line far below its element's largest value would
+// keep fewer bits than FP64 gives it. (The variables of the Euler equations are coupled by every numerical flux: see
+// dgpu_fix.cuh.) On QUAD 16^2 p2 an RK step takes 22.9 us so, 26.9 in fixed point, and a residual 41.3 and 41.7; a
+// residual on 128^2 p4 67 and 55.
+template <int NV>
+constexpr bool kFixed = NV > 1;
 
 struct TPParams {
 	int n_vol;
@@ -152,6 +161,23 @@ __device__ __forceinline__ void tp_pass(const T* __restrict__ in, T* __restrict_
 	}
 }
 
+// The pass's result at the node alone, kept in registers.
+template <int D, int Q, int NV>
+__device__ __forceinline__ void tp_pass_value(const double* in, double* x, const double (*M)[kQMax], int dir, int node)
+{
+	constexpr int N = TPShape<D, Q>::N;
+	const int stride = (dir == 0 ? 1 : (dir == 1 ? Q : Q * Q));
+	const int a = node_coord<Q>(node, dir);
+	const int base = node - a * stride;
+#pragma unroll
+	for (int v = 0; v < NV; ++v) {
+		x[v] = 0.0;
+#pragma unroll
+		for (int m = 0; m < Q; ++m)
+			x[v] += M[a][m] * in[v * N + base + m * stride];
+	}
+}
+
 // The D passes of M (x) M (x) M over one element block: in -> out, `tmp` as scratch (in, out, tmp distinct).
 // Every thread of the CTA must call it (it synchronises); `active` selects the threads that compute.
 template <int D, int Q, int NV, typename T, typename TM>
@@ -178,11 +204,12 @@ __device__ __forceinline__ unsigned long long abs_bits(double x)
 
 // Copies the operator set (a __grid_constant__ kernel parameter) into shared memory; the caller synchronises before use.
 // The loads go through the parameter's generic address: indexed by thread, the constant port would serve the 32 addresses
-// of a warp one after the other.
+// of a warp one after the other. FIX: with the fixed-point forms.
+template <bool FIX = true>
 __device__ __forceinline__ void load_ops(TPOps* sops, const TPOps& ops)
 {
 	const double* src = reinterpret_cast<const double*>(&ops);
-	for (int i = threadIdx.x; i < (int)(sizeof(TPOps) / 8); i += blockDim.x) {
+	for (int i = threadIdx.x; i < (int)((FIX ? sizeof(TPOps) : offsetof(TPOps, fD)) / 8); i += blockDim.x) {
 		double x;
 		asm volatile("ld.f64 %0, [%1];" : "=d"(x) : "l"(src + i));
 		reinterpret_cast<double*>(sops)[i] = x;
@@ -270,78 +297,94 @@ __device__ __noinline__ void tp_pass_rolled(const double* in, double* out, const
 
 // M (x) .. (x) M applied to the CTA's elements in block fixed point (FP64 passes for an element out of range): x holds
 // the node's values on entry and exit; buf and tmp NV N words per element, sx AEXP zeroed ints per element, stride_x ints
-// apart. STATE: x is a conserved state (fix_spread); fix: TPOps::fix. All threads of the CTA must call it; buf is free again after the next
-// barrier.
-template <int D, int Q, int NV, bool STATE>
+// apart. STATE: x is a conserved state (fix_spread); fix: TPOps::fix; FIX: false for FP64 passes throughout (sx is not
+// used then). All threads of the CTA must call it; buf is free again after the next barrier.
+template <int D, int Q, int NV, bool STATE, bool FIX = kFixed<NV>>
 __device__ __forceinline__ void tp_apply_fix(double* x, double* buf, double* tmp, const FixW (*F)[kQMax], int sF,
                                              const double (*M)[kQMax], bool fix, int e, int node, bool active, int* sx,
                                              int stride_x)
 {
 	constexpr int N = TPShape<D, Q>::N, K = STATE ? TPSmem<D, Q, NV>::AEXP : NV;
-	int eb[K];
-#pragma unroll
-	for (int k = 0; k < NV; ++k)
-		eb[k] = active ? fix_exponent(x[k]) : 0;
-	if constexpr (K > NV) {
-		eb[NV] = active ? fix_low(x[0]) : 0;
-		eb[NV + 1] = active ? fix_low(x[NV - 1]) : 0;
-	}
-	elem_max<N, K>(eb, e, active, sx, stride_x);
-	__syncthreads();
-	bool ok = fix;
-	if (active) {
-		const int* se = sx + e * stride_x;
-		if constexpr (K > NV)
-			ok = ok && fix_spread(se[0], se[NV]) && fix_spread(se[NV - 1], se[NV + 1]);
-#pragma unroll
-		for (int k = 0; k < NV; ++k) {
-			ok = ok && fix_in_range(se[k]);
-			eb[k] = fix_block(se[k]);
-		}
-#pragma unroll
-		for (int k = 0; k < NV; ++k) {
-			if (ok)
-				reinterpret_cast<int2*>(buf)[k * N + node] = fix_pack(x[k], eb[k]);
-			else
-				buf[k * N + node] = x[k];
-		}
-	}
-	__syncthreads();
-	double *src = buf, *dst = tmp;
-#pragma unroll
-	for (int dir = 0; dir < D - 1; ++dir) {
-		if (active) {
-			if (ok)
-				fix_pass<D, Q, NV>(reinterpret_cast<int2*>(src), reinterpret_cast<int2*>(dst), F, dir, node);
-			else   // Inf, NaN, huge values or a spread state: FP64 for this element
-				tp_pass_rolled<Q, NV>(src, dst, M, node, dir == 0 ? 1 : Q, N);
-		}
-		__syncthreads();
-		double* t = src;
-		src = dst;
-		dst = t;
-	}
-	constexpr int stride = (D == 2 ? Q : Q * Q);
-	if (active) {
-		if (ok) {
-			const int a = node / stride, base = node % stride;
-			FixW w[Q];
-#pragma unroll
-			for (int m = 0; m < Q; ++m)
-				w[m] = F[a][m];
-#pragma unroll
-			for (int k = 0; k < NV; ++k) {
-				FixAcc s = {0, 0};
-#pragma unroll
-				for (int m = 0; m < Q; ++m)
-					fix_mac(s, w[m], reinterpret_cast<const int2*>(src)[k * N + base + m * stride]);
-				x[k] = fix_to_double(fix_sum(s), fix_scale(eb[k] + (D - 1) * (62 - sF), sF));
-			}
-		} else {
-			tp_pass_rolled<Q, NV>(src, dst, M, node, stride, N);
+	if constexpr (!FIX) {
+		__syncthreads();   // buf may still be read, as before the barrier below
+		if (active)
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
-				x[k] = dst[k * N + node];
+				buf[k * N + node] = x[k];
+		__syncthreads();
+		if (active) tp_pass<D, Q, NV>(buf, tmp, M, 0, node);
+		__syncthreads();
+		if constexpr (D == 3) {
+			if (active) tp_pass<D, Q, NV>(tmp, buf, M, 1, node);
+			__syncthreads();
+		}
+		if (active) tp_pass_value<D, Q, NV>(D == 2 ? tmp : buf, x, M, D - 1, node);
+	} else {
+		int eb[K];
+#pragma unroll
+		for (int k = 0; k < NV; ++k)
+			eb[k] = active ? fix_exponent(x[k]) : 0;
+		if constexpr (K > NV) {
+			eb[NV] = active ? fix_low(x[0]) : 0;
+			eb[NV + 1] = active ? fix_low(x[NV - 1]) : 0;
+		}
+		elem_max<N, K>(eb, e, active, sx, stride_x);
+		__syncthreads();
+		bool ok = fix;
+		if (active) {
+			const int* se = sx + e * stride_x;
+			if constexpr (K > NV)
+				ok = ok && fix_spread(se[0], se[NV]) && fix_spread(se[NV - 1], se[NV + 1]);
+#pragma unroll
+			for (int k = 0; k < NV; ++k) {
+				ok = ok && fix_in_range(se[k]);
+				eb[k] = fix_block(se[k]);
+			}
+#pragma unroll
+			for (int k = 0; k < NV; ++k) {
+				if (ok)
+					reinterpret_cast<int2*>(buf)[k * N + node] = fix_pack(x[k], eb[k]);
+				else
+					buf[k * N + node] = x[k];
+			}
+		}
+		__syncthreads();
+		double *src = buf, *dst = tmp;
+#pragma unroll
+		for (int dir = 0; dir < D - 1; ++dir) {
+			if (active) {
+				if (ok)
+					fix_pass<D, Q, NV>(reinterpret_cast<int2*>(src), reinterpret_cast<int2*>(dst), F, dir, node);
+				else   // Inf, NaN, huge values or a spread state: FP64 for this element
+					tp_pass_rolled<Q, NV>(src, dst, M, node, dir == 0 ? 1 : Q, N);
+			}
+			__syncthreads();
+			double* t = src;
+			src = dst;
+			dst = t;
+		}
+		constexpr int stride = (D == 2 ? Q : Q * Q);
+		if (active) {
+			if (ok) {
+				const int a = node / stride, base = node % stride;
+				FixW w[Q];
+#pragma unroll
+				for (int m = 0; m < Q; ++m)
+					w[m] = F[a][m];
+#pragma unroll
+				for (int k = 0; k < NV; ++k) {
+					FixAcc s = {0, 0};
+#pragma unroll
+					for (int m = 0; m < Q; ++m)
+						fix_mac(s, w[m], reinterpret_cast<const int2*>(src)[k * N + base + m * stride]);
+					x[k] = fix_to_double(fix_sum(s), fix_scale(eb[k] + (D - 1) * (62 - sF), sF));
+				}
+			} else {
+				tp_pass_rolled<Q, NV>(src, dst, M, node, stride, N);
+#pragma unroll
+				for (int k = 0; k < NV; ++k)
+					x[k] = dst[k * N + node];
+			}
 		}
 	}
 }
@@ -349,55 +392,16 @@ __device__ __forceinline__ void tp_apply_fix(double* x, double* buf, double* tmp
 // The contractions of the volume term, shared by the uniform and the batched kernels: the node's state W and fluxes fr
 // are staged in su (NV N words) and sf (D NV N words) of its element, in block fixed point when the element is in range
 // (the return value), as doubles otherwise; eb receives the element's block exponents. sx: EXP zeroed ints per element,
-// `stride` ints apart. All threads of the CTA must call it; synchronises before it returns. STATE as in tp_apply_fix.
-template <int D, int Q, int NV, bool STATE = true>
+// `stride` ints apart. All threads of the CTA must call it; synchronises before it returns. STATE, fix and FIX as in
+// tp_apply_fix.
+template <int D, int Q, int NV, bool STATE = true, bool FIX = kFixed<NV>>
 __device__ __forceinline__ bool tp_stage_volume(const double* W, const double (*fr)[NV], bool fix, int e, int node, bool active,
                                                 double* su, double* sf, int* sx, int stride, int* eb)
 {
 	constexpr int N = TPShape<D, Q>::N, XE = TPSmem<D, Q, NV>::EXP, AE = TPSmem<D, Q, NV>::AEXP;
-	int x[XE];
-#pragma unroll
-	for (int k = 0; k < XE; ++k)
-		x[k] = 0;
-	if (active) {
-#pragma unroll
-		for (int k = 0; k < NV; ++k) {
-			x[k] = fix_exponent(W[k]);
-			int m = 0;
-#pragma unroll
-			for (int j = 0; j < D; ++j)
-				m = max(m, fix_exponent(fr[j][k]));
-			x[AE + k] = m;
-		}
-		if constexpr (STATE && AE > NV) {
-			x[NV] = fix_low(W[0]);
-			x[NV + 1] = fix_low(W[NV - 1]);
-		}
-	}
-	elem_max<N, XE>(x, e, active, sx, stride);
-	__syncthreads();
-	bool ok = fix;
-	if (active) {
-		const int* se = sx + e * stride;
-		if constexpr (STATE && AE > NV)
-			ok = ok && fix_spread(se[0], se[NV]) && fix_spread(se[NV - 1], se[NV + 1]);
-#pragma unroll
-		for (int k = 0; k < NV; ++k) {
-			ok = ok && fix_in_range(se[k]) && fix_in_range(se[AE + k]);
-			eb[k] = fix_block(se[k]);
-			eb[NV + k] = fix_block(se[AE + k]);
-		}
-		if (ok) {
-			int2* xu = reinterpret_cast<int2*>(su);
-			int2* xf = reinterpret_cast<int2*>(sf);
-#pragma unroll
-			for (int k = 0; k < NV; ++k) {
-				xu[k * N + node] = fix_pack(W[k], eb[k]);
-#pragma unroll
-				for (int j = 0; j < D; ++j)
-					xf[(j * NV + k) * N + node] = fix_pack(fr[j][k], eb[NV + k]);
-			}
-		} else {
+	if constexpr (!FIX) {
+		__syncthreads();   // su and sf may still be read
+		if (active)
 #pragma unroll
 			for (int k = 0; k < NV; ++k) {
 				su[k * N + node] = W[k];
@@ -405,19 +409,73 @@ __device__ __forceinline__ bool tp_stage_volume(const double* W, const double (*
 				for (int j = 0; j < D; ++j)
 					sf[(j * NV + k) * N + node] = fr[j][k];
 			}
+		__syncthreads();
+		return false;
+	} else {
+		int x[XE];
+#pragma unroll
+		for (int k = 0; k < XE; ++k)
+			x[k] = 0;
+		if (active) {
+#pragma unroll
+			for (int k = 0; k < NV; ++k) {
+				x[k] = fix_exponent(W[k]);
+				int m = 0;
+#pragma unroll
+				for (int j = 0; j < D; ++j)
+					m = max(m, fix_exponent(fr[j][k]));
+				x[AE + k] = m;
+			}
+			if constexpr (STATE && AE > NV) {
+				x[NV] = fix_low(W[0]);
+				x[NV + 1] = fix_low(W[NV - 1]);
+			}
 		}
+		elem_max<N, XE>(x, e, active, sx, stride);
+		__syncthreads();
+		bool ok = fix;
+		if (active) {
+			const int* se = sx + e * stride;
+			if constexpr (STATE && AE > NV)
+				ok = ok && fix_spread(se[0], se[NV]) && fix_spread(se[NV - 1], se[NV + 1]);
+#pragma unroll
+			for (int k = 0; k < NV; ++k) {
+				ok = ok && fix_in_range(se[k]) && fix_in_range(se[AE + k]);
+				eb[k] = fix_block(se[k]);
+				eb[NV + k] = fix_block(se[AE + k]);
+			}
+			if (ok) {
+				int2* xu = reinterpret_cast<int2*>(su);
+				int2* xf = reinterpret_cast<int2*>(sf);
+#pragma unroll
+				for (int k = 0; k < NV; ++k) {
+					xu[k * N + node] = fix_pack(W[k], eb[k]);
+#pragma unroll
+					for (int j = 0; j < D; ++j)
+						xf[(j * NV + k) * N + node] = fix_pack(fr[j][k], eb[NV + k]);
+				}
+			} else {
+#pragma unroll
+				for (int k = 0; k < NV; ++k) {
+					su[k * N + node] = W[k];
+#pragma unroll
+					for (int j = 0; j < D; ++j)
+						sf[(j * NV + k) * N + node] = fr[j][k];
+				}
+			}
+		}
+		__syncthreads();
+		return ok;
 	}
-	__syncthreads();
-	return ok;
 }
 
 // out[k] = sum_j Dgl_j^T (w fr_j) at the node.
-template <int D, int Q, int NV>
+template <int D, int Q, int NV, bool FIX = kFixed<NV>>
 __device__ __forceinline__ void tp_derivative(const TPOps* sops, const double* sf, const int* eb, bool ok, int node,
                                               double* out)
 {
 	constexpr int N = TPShape<D, Q>::N;
-	if (ok) {
+	if (FIX && ok) {
 		const int2* xf = reinterpret_cast<const int2*>(sf);
 		FixAcc acc[NV];
 #pragma unroll
@@ -443,12 +501,12 @@ __device__ __forceinline__ void tp_derivative(const TPOps* sops, const double* s
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
 			out[k] = 0.0;
-#pragma unroll 1
+#pragma unroll(FIX ? 1 : D)
 		for (int j = 0; j < D; ++j) {
 			const int stride = (j == 0 ? 1 : (j == 1 ? Q : Q * Q));
 			const int a = (node / stride) % Q;
 			const double* f = sf + j * NV * N + node - a * stride;
-#pragma unroll 1
+#pragma unroll(FIX ? 1 : Q)
 			for (int m = 0; m < Q; ++m)
 #pragma unroll
 				for (int k = 0; k < NV; ++k)
@@ -460,44 +518,54 @@ __device__ __forceinline__ void tp_derivative(const TPOps* sops, const double* s
 // K values of every node staged in an element's buffer (K N words): in block fixed point when the element is in range
 // (returned), as doubles otherwise. eb: the K block exponents. STATE: fix_spread on x[0] and x[K - 1] (K + 2 exponents).
 // All threads of the CTA must call it; synchronises before it returns.
-template <int N, int K, bool STATE>
+template <int N, int K, bool STATE, bool FIX = kFixed<K>>
 __device__ __forceinline__ bool tp_stage(const double* x, bool fix, int e, int node, bool active, double* buf, int* sx, int stride,
                                          int* eb)
 {
 	constexpr int KX = STATE ? K + 2 : K;
-	int m[KX];
+	if constexpr (!FIX) {
+		__syncthreads();   // buf may still be read
+		if (active)
 #pragma unroll
-	for (int k = 0; k < K; ++k)
-		m[k] = active ? fix_exponent(x[k]) : 0;
-	if constexpr (STATE) {
-		m[K] = active ? fix_low(x[0]) : 0;
-		m[K + 1] = active ? fix_low(x[K - 1]) : 0;
-	}
-	elem_max<N, KX>(m, e, active, sx, stride);
-	__syncthreads();
-	bool ok = fix;
-	if (active) {
-		const int* se = sx + e * stride;
-		if constexpr (STATE)
-			ok = ok && fix_spread(se[0], se[K]) && fix_spread(se[K - 1], se[K + 1]);
-#pragma unroll
-		for (int k = 0; k < K; ++k) {
-			ok = ok && fix_in_range(se[k]);
-			eb[k] = fix_block(se[k]);
-		}
+			for (int k = 0; k < K; ++k)
+				buf[k * N + node] = x[k];
+		__syncthreads();
+		return false;
+	} else {
+		int m[KX];
 #pragma unroll
 		for (int k = 0; k < K; ++k)
-			if (ok)
-				reinterpret_cast<int2*>(buf)[k * N + node] = fix_pack(x[k], eb[k]);
-			else
-				buf[k * N + node] = x[k];
+			m[k] = active ? fix_exponent(x[k]) : 0;
+		if constexpr (STATE) {
+			m[K] = active ? fix_low(x[0]) : 0;
+			m[K + 1] = active ? fix_low(x[K - 1]) : 0;
+		}
+		elem_max<N, KX>(m, e, active, sx, stride);
+		__syncthreads();
+		bool ok = fix;
+		if (active) {
+			const int* se = sx + e * stride;
+			if constexpr (STATE)
+				ok = ok && fix_spread(se[0], se[K]) && fix_spread(se[K - 1], se[K + 1]);
+#pragma unroll
+			for (int k = 0; k < K; ++k) {
+				ok = ok && fix_in_range(se[k]);
+				eb[k] = fix_block(se[k]);
+			}
+#pragma unroll
+			for (int k = 0; k < K; ++k)
+				if (ok)
+					reinterpret_cast<int2*>(buf)[k * N + node] = fix_pack(x[k], eb[k]);
+				else
+					buf[k * N + node] = x[k];
+		}
+		__syncthreads();
+		return ok;
 	}
-	__syncthreads();
-	return ok;
 }
 
 // d[j][k] = sum_m Dgl[a][m] x of the staged values, the reference derivative in direction j at the node.
-template <int D, int Q, int NV>
+template <int D, int Q, int NV, bool FIX = kFixed<NV>>
 __device__ __forceinline__ void tp_gradient(const TPOps* sops, const double* su, const int* eb, bool ok, int node,
                                             double (*d)[NV])
 {
@@ -507,7 +575,7 @@ __device__ __forceinline__ void tp_gradient(const TPOps* sops, const double* su,
 		const int stride = (j == 0 ? 1 : (j == 1 ? Q : Q * Q));
 		const int a = node_coord<Q>(node, j);
 		const int b0 = node - a * stride;
-		if (ok) {
+		if (FIX && ok) {
 			FixW w[Q];
 #pragma unroll
 			for (int m = 0; m < Q; ++m)
@@ -524,7 +592,7 @@ __device__ __forceinline__ void tp_gradient(const TPOps* sops, const double* su,
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
 				d[j][k] = 0.0;
-#pragma unroll 1
+#pragma unroll(FIX ? 1 : Q)
 			for (int m = 0; m < Q; ++m)
 #pragma unroll
 				for (int k = 0; k < NV; ++k)
@@ -534,14 +602,14 @@ __device__ __forceinline__ void tp_gradient(const TPOps* sops, const double* su,
 }
 
 // out[k] = the trace of the staged state at node t of local face lf.
-template <int D, int Q, int NV>
+template <int D, int Q, int NV, bool FIX = kFixed<NV>>
 __device__ __forceinline__ void tp_trace(const TPOps* sops, const double* su, const int* eb, bool ok, int lf, int t,
                                          double* out)
 {
 	constexpr int N = TPShape<D, Q>::N;
 	int stride, base;
 	tp_face_line<D, Q>(lf, t, base, stride);
-	if (ok) {
+	if (FIX && ok) {
 		const int2* xu = reinterpret_cast<const int2*>(su) + base;
 		FixW w[Q];
 #pragma unroll
@@ -559,7 +627,7 @@ __device__ __forceinline__ void tp_trace(const TPOps* sops, const double* su, co
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
 			out[k] = 0.0;
-#pragma unroll 1
+#pragma unroll(FIX ? 1 : Q)
 		for (int m = 0; m < Q; ++m)
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
@@ -569,35 +637,39 @@ __device__ __forceinline__ void tp_trace(const TPOps* sops, const double* su, co
 
 // The lifting, shared likewise: fv holds the signed face terms of the element's face nodes node + r N (node index
 // lf NF + t), Rg the node's volume term; Rg becomes volume term + sum over the faces of E_lf^T (face terms). sa: NV NFT
-// words of the element, sx: NV zeroed ints per element. All threads of the CTA must call it; sa must not be written
-// before the next barrier.
-template <int D, int Q, int NV>
+// words of the element, sx: NV zeroed ints per element (not used unless FIX). All threads of the CTA must call it; sa must
+// not be written before the next barrier.
+template <int D, int Q, int NV, bool FIX = kFixed<NV>>
 __device__ __forceinline__ void tp_lift_sum(const TPOps* sops, bool fix, const double (*fv)[NV], double* Rg, int e, int node,
                                             bool active, double* sa, int* sx, int stride)
 {
 	constexpr int N = TPShape<D, Q>::N, NF = TPShape<D, Q>::NF, NFT = TPSmem<D, Q, NV>::NFT, NR = (NFT + N - 1) / N;
 	int eb[NV];
+	bool ok = FIX && fix;
+	if constexpr (FIX) {
 #pragma unroll
-	for (int k = 0; k < NV; ++k)
-		eb[k] = 0;
-	if (active) {
+		for (int k = 0; k < NV; ++k)
+			eb[k] = 0;
+		if (active) {
 #pragma unroll
-		for (int k = 0; k < NV; ++k) {
-			eb[k] = fix_exponent(Rg[k]);
+			for (int k = 0; k < NV; ++k) {
+				eb[k] = fix_exponent(Rg[k]);
 #pragma unroll
-			for (int r = 0; r < NR; ++r)
-				if (node + r * N < NFT)
-					eb[k] = max(eb[k], fix_exponent(fv[r][k]));
+				for (int r = 0; r < NR; ++r)
+					if (node + r * N < NFT)
+						eb[k] = max(eb[k], fix_exponent(fv[r][k]));
+			}
 		}
+		elem_max<N, NV>(eb, e, active, sx, stride);
 	}
-	elem_max<N, NV>(eb, e, active, sx, stride);
 	__syncthreads();
-	bool ok = fix;
 	if (active) {
+		if constexpr (FIX) {
 #pragma unroll
-		for (int k = 0; k < NV; ++k) {
-			ok = ok && fix_in_range(sx[e * stride + k]);
-			eb[k] = fix_block(sx[e * stride + k]);
+			for (int k = 0; k < NV; ++k) {
+				ok = ok && fix_in_range(sx[e * stride + k]);
+				eb[k] = fix_block(sx[e * stride + k]);
+			}
 		}
 #pragma unroll
 		for (int r = 0; r < NR; ++r) {
@@ -635,7 +707,7 @@ __device__ __forceinline__ void tp_lift_sum(const TPOps* sops, bool fix, const d
 		for (int k = 0; k < NV; ++k)
 			Rg[k] = fix_to_double(fix_sum(acc[k]), fix_scale(eb[k], sops->sU));
 	} else {
-#pragma unroll 1
+#pragma unroll(FIX ? 1 : 2 * D)
 		for (int lf = 0; lf < 2 * D; ++lf) {
 			const double l = sops->lb[lf & 1][node_coord<Q>(node, lf >> 1)];
 			const double* x = sa + lf * NF + tp_face_node<D, Q>(lf, node);
@@ -678,8 +750,9 @@ __device__ __forceinline__ void tp_volume_body(const TPOps* sops, bool fix, cons
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
 			W[k] = u[((size_t)v * NV + k) * N + node];
-	for (int i = tid; i < S::E * XE + (GLL_IN ? S::E * AE : 0); i += blockDim.x)
-		sx[i] = 0;
+	if constexpr (kFixed<NV>)
+		for (int i = tid; i < S::E * XE + (GLL_IN ? S::E * AE : 0); i += blockDim.x)
+			sx[i] = 0;
 	__syncthreads();
 	if (GLL_IN) {
 		if (active && P.keep_coef)
@@ -731,7 +804,7 @@ tp_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const doub
 	using S = TPShape<D, Q>;
 	extern __shared__ double smem[];
 	TPOps* sops = reinterpret_cast<TPOps*>(smem);
-	load_ops(sops, ops);
+	load_ops<kFixed<NV>>(sops, ops);
 	const int v0 = blockIdx.x * S::E;
 	if (blockIdx.x == 0 && threadIdx.x == 0 && P.max_bits)
 		*P.max_bits = 0ull;
@@ -1107,7 +1180,7 @@ tp_lift_kernel(const __grid_constant__ TPOps ops, const TPParams P, const RkArgs
 	using S = TPShape<D, Q>;
 	extern __shared__ double smem[];
 	TPOps* sops = reinterpret_cast<TPOps*>(smem);
-	load_ops(sops, ops);
+	load_ops<kFixed<NV>>(sops, ops);
 	const int v0 = blockIdx.x * S::E;
 	constexpr int LIFT = TPSmem<D, Q, NV>::LIFT;
 	double* base = smem + sizeof(TPOps) / 8;
@@ -1133,7 +1206,7 @@ tp_convert_kernel(const __grid_constant__ TPOps ops, int n_vol, const double* __
 	constexpr int PER_E = 2 * NV * N;
 	int* sx = reinterpret_cast<int*>(base + E * PER_E);
 	const int tid = threadIdx.x;
-	load_ops(sops, ops);
+	load_ops<kFixed<NV>>(sops, ops);
 	const int v0 = blockIdx.x * E;
 	const int e = tid / N, node = tid % N;
 	const bool active = e < min(E, n_vol - v0);
@@ -1146,8 +1219,9 @@ tp_convert_kernel(const __grid_constant__ TPOps ops, int n_vol, const double* __
 			if (in_copy)
 				in_copy[o + (size_t)k * N] = x[k];
 		}
-	for (int i = tid; i < E * TPSmem<D, Q, NV>::AEXP; i += blockDim.x)
-		sx[i] = 0;
+	if constexpr (kFixed<NV>)
+		for (int i = tid; i < E * TPSmem<D, Q, NV>::AEXP; i += blockDim.x)
+			sx[i] = 0;
 	__syncthreads();
 	tp_apply_fix<D, Q, NV, true>(x, base + e * PER_E, base + e * PER_E + NV * N, TO_GL ? sops->fB : sops->fBinv,
 	                       TO_GL ? sops->sB : sops->sBinv, TO_GL ? sops->B : sops->Binv, ops.fix, e, node, active, sx,
