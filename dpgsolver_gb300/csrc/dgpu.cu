@@ -440,11 +440,12 @@ size_t jvp_volume_smem_bytes()
 // R(u) and the directional derivative along jv_du: tangent-carrying volume and face kernels, then the residual-mode
 // lift on the primal buffers and on the tangent buffers (the lift is linear).
 // PRIMAL = false: the derivative only (the primal volume and face quantities are still formed, the primal lift is
-// skipped and rhs is left as it was).
+// skipped and rhs is left as it was), for the columns of a Jacobian: the tangent in FP64 throughout.
 template <int D, int Q, int NV, int PDE, int FLUX, bool PRIMAL>
 cudaError_t launch_jvp_t(dgpu_ctx* c)
 {
 	using S = TPShape<D, Q>;
+	constexpr bool FIXT = PRIMAL && kFixed<NV>;
 	const int blocks = (c->n_vol + S::E - 1) / S::E;
 	const TPParams P = c->params();
 	TPParams Pd = P;
@@ -456,7 +457,7 @@ cudaError_t launch_jvp_t(dgpu_ctx* c)
 	cudaError_t e = PRIMAL ? cudaMemsetAsync(c->max_bits, 0, sizeof(unsigned long long), c->stream) : cudaSuccess;
 	if (e != cudaSuccess)
 		return e;
-	tp_jvp_volume_kernel<D, Q, NV, PDE><<<blocks, S::THREADS, jvp_volume_smem_bytes<D, Q, NV>(), c->stream>>>(
+	tp_jvp_volume_kernel<D, Q, NV, PDE, FIXT><<<blocks, S::THREADS, jvp_volume_smem_bytes<D, Q, NV>(), c->stream>>>(
 		c->ops, P, Pd, c->u, c->jv_du);
 	const long long nf = (long long)c->n_face * S::NF;
 	tp_jvp_face_kernel<D, Q, NV, PDE, FLUX><<<(unsigned)((nf + 127) / 128), 128, 0, c->stream>>>(P, Pd);
@@ -472,7 +473,7 @@ cudaError_t launch_jvp_t(dgpu_ctx* c)
 		tp_lift_kernel<D, Q, NV, kModeRhs><<<blocks, S::THREADS, lift_smem_bytes<D, Q, NV>(), c->stream>>>(c->ops, P,
 		                                                                                                   rk);
 	rk.rhs = c->jv_out;
-	tp_lift_kernel<D, Q, NV, kModeRhs><<<blocks, S::THREADS, lift_smem_bytes<D, Q, NV>(), c->stream>>>(c->ops, Pd, rk);
+	tp_lift_kernel<D, Q, NV, kModeRhs, FIXT><<<blocks, S::THREADS, lift_smem_bytes<D, Q, NV>(), c->stream>>>(c->ops, Pd, rk);
 	c->launches += PRIMAL ? 4 : 3;
 	return cudaGetLastError();
 }
@@ -514,6 +515,8 @@ cudaError_t bind(dgpu_ctx* c)
 		return e;
 	if ((e = cudaFuncSetAttribute(tp_lift_kernel<D, Q, NV, kModeRhs>, smem, (int)lift_smem_bytes<D, Q, NV>())))
 		return e;
+	if ((e = cudaFuncSetAttribute(tp_lift_kernel<D, Q, NV, kModeRhs, false>, smem, (int)lift_smem_bytes<D, Q, NV>())))
+		return e;
 	if ((e = cudaFuncSetAttribute(tp_lift_kernel<D, Q, NV, kModeRkGl>, smem, (int)lift_smem_bytes<D, Q, NV>())))
 		return e;
 	if ((e = cudaFuncSetAttribute(tp_lift_kernel<D, Q, NV, kModeRkGlNoMax>, smem, (int)lift_smem_bytes<D, Q, NV>())))
@@ -525,6 +528,9 @@ cudaError_t bind(dgpu_ctx* c)
 	if ((e = cudaFuncSetAttribute(tp_adj_lift_kernel<D, Q, NV>, smem, (int)lift_smem_bytes<D, Q, NV>())))
 		return e;
 	if ((e = cudaFuncSetAttribute(tp_mass_kernel<D, Q, NV>, smem, (int)lift_smem_bytes<D, Q, NV>())))
+		return e;
+	if ((e = cudaFuncSetAttribute(tp_jvp_volume_kernel<D, Q, NV, PDE, false>, smem,
+	                              (int)jvp_volume_smem_bytes<D, Q, NV>())))
 		return e;
 	if ((e = cudaFuncSetAttribute(tp_jvp_volume_kernel<D, Q, NV, PDE>, smem, (int)jvp_volume_smem_bytes<D, Q, NV>())))
 		return e;
@@ -598,8 +604,8 @@ cudaError_t launch_ns_jvp_t(dgpu_ctx* c)
 	if (e != cudaSuccess)
 		return e;
 	tp_ns_grad_kernel<D, Q, NV, true><<<blocks, S::THREADS, ns_smem_bytes<D, Q, NV>(), c->stream>>>(c->ops, P, c->u);
-	tp_ns_grad_kernel<D, Q, NV, true><<<blocks, S::THREADS, ns_smem_bytes<D, Q, NV>(), c->stream>>>(c->ops, Pd,
-	                                                                                               c->jv_du);
+	tp_ns_grad_kernel<D, Q, NV, true, false><<<blocks, S::THREADS, ns_smem_bytes<D, Q, NV>(), c->stream>>>(c->ops, Pd,
+	                                                                                                      c->jv_du);
 	const long long nf = (long long)c->n_face * S::NF;
 	tp_ns_jvp_face_kernel<D, Q, FLUX><<<(unsigned)((nf + 127) / 128), 128, 0, c->stream>>>(P, Pd);
 	tp_ns_jvp_volume_kernel<D, Q, NV><<<blocks, S::THREADS, ns_jvp_smem_bytes<D, Q, NV>(), c->stream>>>(
@@ -616,7 +622,7 @@ cudaError_t launch_ns_jvp_t(dgpu_ctx* c)
 		tp_lift_kernel<D, Q, NV, kModeRhs><<<blocks, S::THREADS, lift_smem_bytes<D, Q, NV>(), c->stream>>>(c->ops, P,
 		                                                                                                   rk);
 	rk.rhs = c->jv_out;
-	tp_lift_kernel<D, Q, NV, kModeRhs><<<blocks, S::THREADS, lift_smem_bytes<D, Q, NV>(), c->stream>>>(c->ops, Pd, rk);
+	tp_lift_kernel<D, Q, NV, kModeRhs, false><<<blocks, S::THREADS, lift_smem_bytes<D, Q, NV>(), c->stream>>>(c->ops, Pd, rk);
 	c->launches += PRIMAL ? 6 : 5;
 	return cudaGetLastError();
 }
@@ -681,6 +687,7 @@ cudaError_t bind_ns(dgpu_ctx* c)
 		return e;
 	const int bytes = (int)ns_smem_bytes<D, Q, NV>();
 	if ((e = cudaFuncSetAttribute(tp_ns_grad_kernel<D, Q, NV, true>, smem, bytes)) ||
+	    (e = cudaFuncSetAttribute(tp_ns_grad_kernel<D, Q, NV, true, false>, smem, bytes)) ||
 	    (e = cudaFuncSetAttribute(tp_ns_grad_kernel<D, Q, NV, false>, smem, bytes)) ||
 	    (e = cudaFuncSetAttribute(tp_ns_volume_kernel<D, Q, NV, true>, smem, bytes)) ||
 	    (e = cudaFuncSetAttribute(tp_ns_volume_kernel<D, Q, NV, false>, smem, bytes)))

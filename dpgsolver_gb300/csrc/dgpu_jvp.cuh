@@ -18,7 +18,11 @@ namespace dgpu {
 // the traces of each in block fixed point (dgpu_fix.cuh), as in the residual's volume kernel. Per element:
 // 2 x (su, st, sf) in shared memory and the block exponents of both. R and J d on a HEX 17^3 p2 mesh, Roe-Pike, from host
 // buffers and back: 386 -> 353 us.
-template <int D, int Q, int NV, int PDE>
+// FIXT: whether the tangent is in fixed point too. Not for the columns of a Jacobian: a unit direction's values fall by the
+// product of D interpolation weights over an element, and the entries far from it would keep fewer bits (HEX p2,
+// Lax-Friedrichs: median relative error of an entry 3.2e-14 in FP64, 5.9e-14 in fixed point; for directions without such
+// structure there is no difference).
+template <int D, int Q, int NV, int PDE, bool FIXT = kFixed<NV>>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS)
 tp_jvp_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const TPParams Pd, const double* __restrict__ u,
                      const double* __restrict__ du)
@@ -52,7 +56,7 @@ tp_jvp_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const 
 	double* dsf = dst + NV * N;
 	int* dsx = sx + E * (XE + AE);
 	tp_apply_fix<D, Q, NV, true>(W, su, st, sops->fB, sops->sB, sops->B, ops.fix, e, node, active, sx + E * XE, AE);
-	tp_apply_fix<D, Q, NV, false>(dW, dsu, dst, sops->fB, sops->sB, sops->B, ops.fix, e, node, active, dsx + E * XE, AE);
+	tp_apply_fix<D, Q, NV, false, FIXT>(dW, dsu, dst, sops->fB, sops->sB, sops->B, ops.fix, e, node, active, dsx + E * XE, AE);
 	double fr[D][NV], dfr[D][NV];
 	if (active) {
 		double g[D * D];
@@ -81,7 +85,7 @@ tp_jvp_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const 
 	}
 	int eb[2 * NV], deb[2 * NV];
 	const bool ok = tp_stage_volume<D, Q, NV>(W, fr, ops.fix, e, node, active, su, sf, sx, XE, eb);
-	const bool dok = tp_stage_volume<D, Q, NV, false>(dW, dfr, ops.fix, e, node, active, dsu, dsf, dsx, XE, deb);
+	const bool dok = tp_stage_volume<D, Q, NV, false, FIXT>(dW, dfr, ops.fix, e, node, active, dsu, dsf, dsx, XE, deb);
 	if (!active)
 		return;
 	double out[NV];
@@ -89,7 +93,7 @@ tp_jvp_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const 
 #pragma unroll
 	for (int k = 0; k < NV; ++k)
 		P.vol_gl[((size_t)v * NV + k) * N + node] = out[k];
-	tp_derivative<D, Q, NV>(sops, dsf, deb, dok, node, out);
+	tp_derivative<D, Q, NV, FIXT>(sops, dsf, deb, dok, node, out);
 #pragma unroll
 	for (int k = 0; k < NV; ++k)
 		Pd.vol_gl[((size_t)v * NV + k) * N + node] = out[k];
@@ -103,7 +107,7 @@ tp_jvp_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const 
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
 			tp[k * NF + t] = out[k];
-		tp_trace<D, Q, NV>(sops, dsu, deb, dok, lf, t, out);
+		tp_trace<D, Q, NV, FIXT>(sops, dsu, deb, dok, lf, t, out);
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
 			td[k * NF + t] = out[k];

@@ -78,13 +78,13 @@ struct NsSmem {
 };
 
 // The physical volume gradient of a staged state at the node, and the traces' source: three passes of Dgl in fixed point.
-template <int D, int Q, int NV>
+template <int D, int Q, int NV, bool FIX = true>
 __device__ __forceinline__ void ns_node_gradient(const TPOps* sops, const TPParams& P, int v, int node, const double* su,
                                                  const int* eb, bool ok, double (*g)[NV])
 {
 	constexpr int N = TPShape<D, Q>::N;
 	double d[D][NV];
-	tp_gradient<D, Q, NV>(sops, su, eb, ok, node, d);
+	tp_gradient<D, Q, NV, FIX>(sops, su, eb, ok, node, d);
 	const double iwJ = P.inv_wJ[(size_t)v * N + node];
 	double gm[D * D];
 #pragma unroll
@@ -106,7 +106,8 @@ __device__ __forceinline__ void ns_node_gradient(const TPOps* sops, const TPPara
 // run in block fixed point; the FP64 pipe keeps the metric products (60). HEX 24^3 p3:
 // 374 -> 227 us; four CTAs per SM here and three in the volume kernel overlap the FP64 work of one with the integer work of
 // the others: 3 steps 9.82 -> 9.11 ms.
-template <int D, int Q, int NV, bool GLL_IN>
+// FIX: false for FP64 contractions, which the tangent of a directional derivative takes (the rules of a state do not fit it).
+template <int D, int Q, int NV, bool GLL_IN, bool FIX = true>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS, 4)
 tp_ns_grad_kernel(const __grid_constant__ TPOps ops, const TPParams P, const double* __restrict__ u)
 {
@@ -133,18 +134,18 @@ tp_ns_grad_kernel(const __grid_constant__ TPOps ops, const TPParams P, const dou
 	}
 	__syncthreads();
 	if (GLL_IN)
-		tp_apply_fix<D, Q, NV, true>(W, su, sd, sops->fB, sops->sB, sops->B, ops.fix, e, node, active, sx, 2 * PER_E);
+		tp_apply_fix<D, Q, NV, true, FIX>(W, su, sd, sops->fB, sops->sB, sops->B, ops.fix, e, node, active, sx, 2 * PER_E);
 	int eb[NV], eg[D * NV];
-	const bool ok = tp_stage<N, NV, true>(W, ops.fix, e, node, active, su, sx + AE, 2 * PER_E, eb);
+	const bool ok = tp_stage<N, NV, true, FIX>(W, ops.fix, e, node, active, su, sx + AE, 2 * PER_E, eb);
 	if (active) {
-		ns_node_gradient<D, Q, NV>(sops, P, v, node, su, eb, ok, g);
+		ns_node_gradient<D, Q, NV, FIX>(sops, P, v, node, su, eb, ok, g);
 #pragma unroll
 		for (int dir = 0; dir < D; ++dir)
 #pragma unroll
 			for (int var = 0; var < NV; ++var)
 				P.ns_gv[(((size_t)v * D + dir) * NV + var) * N + node] = g[dir][var];
 	}
-	const bool okg = tp_stage<N, D * NV, false>(&g[0][0], ops.fix, e, node, active, sd, sx + 2 * AE, 2 * PER_E, eg);
+	const bool okg = tp_stage<N, D * NV, false, FIX>(&g[0][0], ops.fix, e, node, active, sd, sx + 2 * AE, 2 * PER_E, eg);
 	if (!active)
 		return;
 	// traces of the state and of the volume gradient on the 2D local faces
@@ -154,13 +155,13 @@ tp_ns_grad_kernel(const __grid_constant__ TPOps ops, const TPParams P, const dou
 		double* ds = P.traces + (size_t)fs * NV * NF + t;
 		double* dg = P.ns_gtr + (size_t)fs * D * NV * NF + t;
 		double out[NV];
-		tp_trace<D, Q, NV>(sops, su, eb, ok, lf, t, out);
+		tp_trace<D, Q, NV, FIX>(sops, su, eb, ok, lf, t, out);
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
 			ds[k * NF] = out[k];
 #pragma unroll
 		for (int dir = 0; dir < D; ++dir) {
-			tp_trace<D, Q, NV>(sops, sd + dir * NV * N, eg + dir * NV, okg, lf, t, out);
+			tp_trace<D, Q, NV, FIX>(sops, sd + dir * NV * N, eg + dir * NV, okg, lf, t, out);
 #pragma unroll
 			for (int k = 0; k < NV; ++k)
 				dg[(dir * NV + k) * NF] = out[k];

@@ -982,8 +982,8 @@ __device__ __noinline__ bool tp_positivity_exact(const double (*toB)[kQMax], con
 // the exact check, so the decisions are those of the exact FP64 check.
 
 // Lift, 1/(wJ), then the residual (V^-1, max|rhs|) or the RK stage + positivity, for the CTA's E elements; per
-// element PER_E doubles at base.
-template <int D, int Q, int NV, int MODE, int PER_E>
+// element PER_E doubles at base. FIX: false for FP64 contractions (kModeRhs: tangents).
+template <int D, int Q, int NV, int MODE, int PER_E, bool FIX>
 __device__ __forceinline__ void tp_lift_body(const TPOps* sops, bool fix, const TPParams& P, const RkArgs& rk, int v0,
                                              int n_here, double* base, int* sx)
 {
@@ -1025,7 +1025,7 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, bool fix, const 
 		}
 	}
 	__syncthreads();   // sx is zero; sops is written by other warps
-	tp_lift_sum<D, Q, NV>(sops, fix, fv, Rg, e, node, active, sa, sx, NV);
+	tp_lift_sum<D, Q, NV, FIX>(sops, fix, fv, Rg, e, node, active, sa, sx, NV);
 	if (active) {
 		const double iw = P.inv_wJ[(size_t)v * N + node];
 #pragma unroll
@@ -1046,7 +1046,7 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, bool fix, const 
 #pragma unroll
 		for (int k = 0; k < NV; ++k)
 			R[k] = Rg[k];
-		tp_apply_fix<D, Q, NV, false>(R, sa, sb, sops->fBinv, sops->sBinv, sops->Binv, fix, e, node, active,
+		tp_apply_fix<D, Q, NV, false, FIX>(R, sa, sb, sops->fBinv, sops->sBinv, sops->Binv, fix, e, node, active,
 		                              sx + 2 * S::E * NV, AE);
 		if (active) {
 #pragma unroll
@@ -1173,7 +1173,7 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, bool fix, const 
 template <int MODE>
 struct LiftOccupancy { static constexpr int value = (MODE == kModeRkGlNoMax) ? 4 : 3; };   // Out: as RkGl
 
-template <int D, int Q, int NV, int MODE>
+template <int D, int Q, int NV, int MODE, bool FIX = kFixed<NV>>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS, LiftOccupancy<MODE>::value)
 tp_lift_kernel(const __grid_constant__ TPOps ops, const TPParams P, const RkArgs rk)
 {
@@ -1184,7 +1184,7 @@ tp_lift_kernel(const __grid_constant__ TPOps ops, const TPParams P, const RkArgs
 	const int v0 = blockIdx.x * S::E;
 	constexpr int LIFT = TPSmem<D, Q, NV>::LIFT;
 	double* base = smem + sizeof(TPOps) / 8;
-	tp_lift_body<D, Q, NV, MODE, LIFT>(sops, ops.fix, P, rk, v0, min(S::E, P.n_vol - v0), base,
+	tp_lift_body<D, Q, NV, MODE, LIFT, FIX>(sops, ops.fix, P, rk, v0, min(S::E, P.n_vol - v0), base,
 	                                   reinterpret_cast<int*>(base + S::E * LIFT));
 }
 
