@@ -1177,7 +1177,8 @@ dgpu_status create_impl(const dgpu_physics* phys, const std::vector<GroupIn>& gi
 			while (G.E > 1 && (size_t)G.E * std::max(G.vol_per_e, G.lift_per_e) * 8 > 96 * 1024)
 				G.E /= 2;
 			G.E_fused = G.E;
-			if ((size_t)std::max(G.vol_per_e, G.lift_per_e) * 8 > 200 * 1024)
+			// (without the block exponents; a lift beyond its bound would take faces of a thousand nodes)
+			if ((size_t)(G.vol_per_e - nv - 1) * 8 > 200 * 1024 || (size_t)G.lift_per_e * 8 > 216 * 1024)
 				return reject(DGPU_ERR_UNSUPPORTED, "dense operator set too large for one volume per CTA");
 		}
 	}
