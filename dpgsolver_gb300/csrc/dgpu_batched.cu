@@ -812,10 +812,13 @@ void set_group_E(dgpu_batch* c, int g, int E)
 }
 
 // Elements per CTA of the per-group kernels. A large group fills its CTAs (256 nodes); a group too small to give every
-// SM two of those is split further, down to a warp of a QUAD/HEX group or one dense volume: its kernels are chains
+// one of the device's SMs two of those is split further, down to a warp of a QUAD/HEX group or one dense volume: its kernels are chains
 // of dependent steps, so idle SMs cost more than half-empty CTAs.
 void default_tiles(dgpu_batch* c)
 {
+	int dev = 0, sms = 0;
+	cudaGetDevice(&dev);
+	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
 	for (int g = 0; g < c->n_all; ++g) {
 		const int n_vol = c->group_n_vol(g);
 		int E = c->gl[g].E_max, N = 32;
@@ -823,7 +826,7 @@ void default_tiles(dgpu_batch* c)
 			const int q = c->hgroups[c->gl[g].idx].q;
 			N = c->d == 2 ? q * q : q * q * q;
 		}
-		while (E > 1 && n_vol < E * 2 * 152 && (E / 2) * N >= 32)
+		while (E > 1 && n_vol < E * 2 * sms && (E / 2) * N >= 32)
 			E /= 2;
 		set_group_E(c, g, E);
 	}
@@ -1530,22 +1533,6 @@ dgpu_status create_impl(const dgpu_physics* phys, const std::vector<GroupIn>& gi
 			for (int b = 0; b < nvs; ++b)
 				off_id = std::max(off_id, fabs(M[(size_t)a * nvs + b] - (a == b ? 1.0 : 0.0)));
 		G.minv_identity = off_id <= 1e-13 ? 1 : 0;
-		if (G.prism) {
-			double *d_t0 = nullptr, *d_t1 = nullptr, *d_l0 = nullptr, *d_l1 = nullptr;
-			const size_t nt = (size_t)G.n_tvc * G.n_tvs, nl = (size_t)G.n_lvc * G.n_lvs;
-			B_TRY(upload_vec(&d_t0, std::vector<double>(op->tri_cv0, op->tri_cv0 + nt)));
-			c->dense_bufs.push_back(d_t0);
-			B_TRY(upload_vec(&d_t1, std::vector<double>(op->tri_cv1, op->tri_cv1 + 2 * nt)));
-			c->dense_bufs.push_back(d_t1);
-			B_TRY(upload_vec(&d_l0, std::vector<double>(op->line_cv0, op->line_cv0 + nl)));
-			c->dense_bufs.push_back(d_l0);
-			B_TRY(upload_vec(&d_l1, std::vector<double>(op->line_cv1, op->line_cv1 + nl)));
-			c->dense_bufs.push_back(d_l1);
-			G.tri0 = d_t0;
-			G.tri1 = d_t1;
-			G.line0 = d_l0;
-			G.line1 = d_l1;
-		}
 		std::vector<double> fops;
 		std::vector<long long> foff((size_t)kMaxLf * kMaxOrd * (kQMax + 1), -1);
 		for (int lf = 0; lf < op->n_lf; ++lf)

@@ -54,10 +54,6 @@ struct DGroup {
 	int minv_identity;          // M_ref is the identity to rounding (orthonormal basis): M^-1 = 1/J
 	int prism;                  // WEDGE with TRI x LINE factors: sum-factorised volume term
 	int n_tvs, n_tvc, n_lvs, n_lvc;
-	const double* tri0;         // n_tvc x n_tvs
-	const double* tri1;         // 2 x n_tvc x n_tvs
-	const double* line0;        // n_lvc x n_lvs
-	const double* line1;        // n_lvc x n_lvs
 	const double* ccSB0;        // n_vs x n_vs: coefficients -> Bezier coefficients (positivity), or null
 	const double* ccBS0;        // n_vs x n_vs: Bezier -> coefficients
 	const float* ccSB0f;        // ccSB0 in FP32 (the limiter's pre-filter)
