@@ -128,13 +128,6 @@ __device__ __forceinline__ void bface_get(const BatchOps* sops, int qf, int C, F
 	}
 }
 
-// Start index and stride of the line of volume nodes under own face point t of local face lf.
-template <int D, int Q>
-__device__ __forceinline__ void bface_line(int lf, int t, int* base, int* stride)
-{
-	face_line<D, Q>(lf >> 1, t, base, stride);
-}
-
 // ---- gradient, kept, and the traces of state and gradient at each face's order ----
 template <int D, int Q, int NV, bool GLL_IN>
 __device__ void bns_grad_body(const BParams& P, const BatchOps* sops, const BGroup& G, int e0, int E,
@@ -201,7 +194,7 @@ __device__ void bns_grad_body(const BParams& P, const BatchOps* sops, const BGro
 		for (int it = node; it < 2 * D * NFQ; it += N) {
 			const int lf = it / NFQ, t = it % NFQ, side = lf & 1;
 			int b, stride;
-			bface_line<D, Q>(lf, t, &b, &stride);
+			tp_face_line<D, Q>(lf, t, b, stride);
 			for (int c = 0; c < C; ++c) {
 				const double* src = c < NV ? su + c * N : sd + (c - NV) * N;
 				double s = 0.0;
@@ -333,7 +326,7 @@ __device__ void bns_volume_body(const BParams& P, const BatchOps* sops, const BG
 		for (int lf = 0; lf < 2 * D; ++lf) {
 			const int nd = lf >> 1;
 			const double l = iwJ * sops->t.lb[lf & 1][node_coord<Q>(node, nd)];
-			const double* x = sx + lf * C * NFQ + face_node_of<D, Q>(node, nd);
+			const double* x = sx + lf * C * NFQ + tp_face_node<D, Q>(lf, node);
 #pragma unroll
 			for (int c = 0; c < C; ++c)
 				g[c / NV][c % NV] += l * x[c * NFQ];
@@ -359,7 +352,7 @@ __device__ void bns_volume_body(const BParams& P, const BatchOps* sops, const BG
 		for (int it = node; it < 2 * D * NFQ; it += N) {
 			const int lf = it / NFQ, t = it % NFQ, side = lf & 1;
 			int b, stride;
-			bface_line<D, Q>(lf, t, &b, &stride);
+			tp_face_line<D, Q>(lf, t, b, stride);
 			double lam = 0.0;
 #pragma unroll
 			for (int m = 0; m < Q; ++m) {

@@ -23,30 +23,6 @@
 
 namespace dgpu {
 
-// Start index and stride of the line of volume nodes under face node t of local face lf (normal direction nd).
-template <int D, int Q>
-__device__ __forceinline__ void face_line(int nd, int t, int* base, int* stride)
-{
-	const int t0 = (D == 2 ? t : t % Q), t1 = (D == 2 ? 0 : t / Q);
-	if (D == 2) {
-		*stride = (nd == 0 ? 1 : Q);
-		*base = (nd == 0 ? t0 * Q : t0);
-	} else {
-		*stride = (nd == 0 ? 1 : (nd == 1 ? Q : Q * Q));
-		*base = (nd == 0 ? t0 * Q + t1 * Q * Q : (nd == 1 ? t0 + t1 * Q * Q : t0 + t1 * Q));
-	}
-}
-
-// Face node index of volume node `node` on a face with normal direction nd (tangential directions ascending).
-template <int D, int Q>
-__device__ __forceinline__ int face_node_of(int node, int nd)
-{
-	const int c0 = node_coord<Q>(node, 0), c1 = node_coord<Q>(node, 1), c2 = (D == 3 ? node_coord<Q>(node, 2) : 0);
-	if (D == 2)
-		return nd == 0 ? c1 : c0;
-	return nd == 0 ? c1 + Q * c2 : (nd == 1 ? c0 + Q * c2 : c0 + Q * c1);
-}
-
 // lambda(t) of every face side at its own nodes (setup).
 template <int D, int Q>
 __global__ void __launch_bounds__(256) tp_ns_lambda_kernel(const __grid_constant__ TPOps ops, const TPParams P, double* lam)
@@ -57,9 +33,9 @@ __global__ void __launch_bounds__(256) tp_ns_lambda_kernel(const __grid_constant
 	if (gid >= (long long)P.n_vol * 2 * D * NF)
 		return;
 	const int v = (int)(gid / (2 * D * NF)), r = (int)(gid % (2 * D * NF));
-	const int lf = r / NF, t = r % NF, nd = lf >> 1, side = lf & 1;
+	const int lf = r / NF, t = r % NF, side = lf & 1;
 	int base, stride;
-	face_line<D, Q>(nd, t, &base, &stride);
+	tp_face_line<D, Q>(lf, t, base, stride);
 	double s = 0.0;
 	for (int m = 0; m < Q; ++m) {
 		const double l = ops.lb[side][m];
@@ -535,7 +511,7 @@ tp_ns_jvp_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, con
 #pragma unroll
 		for (int lf = 0; lf < 2 * D; ++lf) {
 			const int nd = lf >> 1, side = lf & 1;
-			const int tf = face_node_of<D, Q>(node, nd);
+			const int tf = tp_face_node<D, Q>(lf, node);
 			const int fs = P.vol_face[(size_t)v * 2 * D + lf], f = fs >> 1;
 			const int tX = ((fs & 1) && P.nc_inv) ? P.nc_inv[(size_t)f * NF + tf] : tf;
 			const double c = iwJ * sops->lb[side][node_coord<Q>(node, nd)];

@@ -123,9 +123,9 @@ tp_ns_adj_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, con
 	if (active) {
 		// E_lf xbar on the local faces: the face flux's cotangent is E_R xbar_R - E_L xbar_L
 		for (int it = node; it < 2 * D * NF; it += N) {
-			const int lf = it / NF, t = it % NF, nd = lf >> 1, side = lf & 1;
+			const int lf = it / NF, t = it % NF, side = lf & 1;
 			int b0, stride;
-			face_line<D, Q>(nd, t, &b0, &stride);
+			tp_face_line<D, Q>(lf, t, b0, stride);
 			const int fs = P.vol_face[(size_t)v * 2 * D + lf];
 			double* adst = A.atraces + (size_t)fs * NV * NF;
 #pragma unroll
@@ -157,7 +157,7 @@ tp_ns_adj_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, con
 #pragma unroll
 		for (int lf = 0; lf < 2 * D; ++lf) {
 			const int nd = lf >> 1, side = lf & 1;
-			const int tf = face_node_of<D, Q>(node, nd);
+			const int tf = tp_face_node<D, Q>(lf, node);
 			const int fs = P.vol_face[(size_t)v * 2 * D + lf], f = fs >> 1;
 			const int tX = ((fs & 1) && P.nc_inv) ? P.nc_inv[(size_t)f * NF + tf] : tf;
 			const double c = iw * sops->lb[side][node_coord<Q>(node, nd)];
@@ -195,9 +195,9 @@ tp_ns_adj_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, con
 	// the liftings' cotangent of X: this volume's lifting of face node t adds 1/(wJ) lb[side][m] X(t) to the
 	// gradient on the line of nodes under t
 	for (int it = node; it < 2 * D * NF; it += N) {
-		const int lf = it / NF, t = it % NF, nd = lf >> 1, side = lf & 1;
+		const int lf = it / NF, t = it % NF, side = lf & 1;
 		int b0, stride;
-		face_line<D, Q>(nd, t, &b0, &stride);
+		tp_face_line<D, Q>(lf, t, b0, stride);
 		const int fs = P.vol_face[(size_t)v * 2 * D + lf];
 		double* xd = B.xbar + (size_t)fs * D * NV * NF;
 		for (int c = 0; c < D * NV; ++c) {
@@ -345,7 +345,7 @@ tp_ns_adj_lift_kernel(const __grid_constant__ TPOps ops, const TPParams P, const
 		for (int lf = 0; lf < 2 * D; ++lf) {
 			const int fs = P.vol_face[(size_t)v * 2 * D + lf];
 			const int nd = lf >> 1;
-			const int t = face_node_of<D, Q>(node, nd);
+			const int t = tp_face_node<D, Q>(lf, node);
 			const double l = sops->lb[lf & 1][node_coord<Q>(node, nd)];
 			const double* ws = A.wbar + (size_t)fs * NV * NF;        // this side's own node order
 			const double* gs = B.gtbar + (size_t)fs * D * NV * NF;
