@@ -233,8 +233,8 @@ def algorithmic_bytes(prob, kernel):
     raise KeyError(kernel)
 
 
-# DRAM bytes per element of one tp_volume_kernel launch (GL state in) measured by ncu on curved HEX 24^3, p = 3,
-# 5 variables: 99.5 MB read + 42.7 MB written over 13,824 elements (writes stay below the algorithmic vol_gl +
+# DRAM bytes per element of one tp_volume_kernel launch (GL state in) measured by ncu on curved HEX 32^3, p = 3,
+# 5 variables: 235.7 MB read + 167.4 MB written over 32,768 elements (writes stay below the algorithmic vol_gl +
 # traces because L2 holds part of them until the face kernel reads them).
 _VOLUME_DRAM_BYTES_PER_ELEMENT_HEX_P3 = (235.7e6 + 167.4e6) / 32768
 

@@ -9,9 +9,10 @@
 // M^-1 = M_ref^-1 / J with M_ref = cv0^T diag(w) cv0 inverted once on the host. A group with a curved volume (J
 // varying over the cubature nodes) keeps every volume's own M^-1 instead (dense_minv_kernel).
 //
-// One CTA handles E volumes of one group; every phase maps one thread to one output row of one volume (all
-// variables per thread), reading the operators through the L1 cache (they are shared by every CTA of the group)
-// and the volume's state and fluxes from shared memory. The state stays in coefficient space between stages.
+// One CTA handles E volumes of one group; every phase maps one output row of one volume (all variables) to one thread, or
+// to up to eight consecutive lanes that share its terms when the CTA has threads to spare (fix_split_for), reading the
+// operators through the L1 cache (they are shared by every CTA of the group) and the volume's state and fluxes from shared
+// memory. The state stays in coefficient space between stages.
 //
 // The contractions run in block fixed point (dgpu_fix.cuh): as FP64 sums they were chains of 35 to 400 operations of 64
 // cycles each, which bounded these kernels at every size. The blocks are one volume's values of one variable. A volume

@@ -16,14 +16,23 @@
 // s is chosen on the host so that sum |W| <= 2^63 over every sum an operator enters (and |W| < 2^62), which bounds
 // a.h by 2^59 and, for at most 32 terms, a.m by 2^62: neither accumulator can overflow.
 //
-// Accuracy. A value is rounded to 2^-59 of its block's largest magnitude, an operator entry to about 2^-60 of its
-// row sum, and the dropped l l products are below 2^-60 of the sum's bound (both l are balanced, so
-// they have no bias): the sum is exact to a few 2^-59 of max |v| sum |w|, where FP64 arithmetic rounds every partial sum
-// to 2^-53. The result is rounded once to FP64, to nearest.
+// Accuracy. fix_pack truncates in its shift and then rounds to a multiple of 4: a value is held to less than 3 units, at most
+// 3 2^-59 of its block's largest magnitude (exactly, where it lies at most 2^5 below it). An operator entry is rounded to 2 units of
+// its own. The dropped l l products are at most 2^62 each, against a sum of up to 2^60 sum |W|: with the operators' rounding,
+// 6 terms of 2^-62 of max |v| sum |w| at worst (2^-55.4 for the 15 terms of a derivative at p = 4), and typically, since both
+// l are balanced and have no bias, a few 2^-60. FP64 arithmetic rounds every partial sum to 2^-53. The result is rounded
+// once to FP64, to nearest.
 //
-// States. A density or an energy far below its element's largest one would keep less than FP64's relative precision,
-// which the divisions by the density feel: an element whose densities or energies spread over more than kFixSpread
-// binary orders stays on the FP64 loops as well (fix_spread), so that each is held to 2^-54 relative.
+// States. What lies far below its block's largest value keeps less than FP64's relative precision. Where that would be felt,
+// an element stays in FP64 arithmetic: a state whose densities or energies spread over more than kFixSpread binary orders
+// (fix_spread; the fluxes divide by the density), which holds both to FP64's own bound on every line of nodes. Its momenta
+// are then at most sqrt(2 rho E), so 2^5 times sqrt(2 rho E) of any node (positive pressure), and held to the bound of
+// that, the scale at which every numerical flux adds them to density differences times the wave speed. The advected scalar has
+// no such coupling, nor has the tangent along a unit direction: both contract in FP64 (kFixed, tp_jvp_volume_kernel).
+// Directions and cotangents of whole meshes lose nothing that the changes of basis at both ends, which mix the values of an
+// element, would have kept.
+//
+// Operators outside fix_usable (not finite, beyond 2^24 or below 2^-24, basis functions of different scales) have no such form.
 //
 // Range. Infinities, NaN, magnitudes of 2^824 and above and non-zero blocks below 2^-823 do not enter: fix_in_range
 // tells, and the caller keeps its FP64 loop for such an element, which propagates them as before. (A block of zeros and

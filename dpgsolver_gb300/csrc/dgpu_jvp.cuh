@@ -116,7 +116,7 @@ tp_jvp_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const 
 
 // Numerical flux at every face node of the primal traces (P) and its derivative along the tangent traces (Pd). FP64-bound
 // (84 %): the value half of the fluxes' lone products runs on the integer pipe. With it, and CTAs of 128 threads for the
-// registers it takes, R and J d on HEX 17^3 p2, Roe-Pike, went from 353 to 337 us.
+// registers it takes (128; Roe-Pike in 3D spills 332 bytes, and three CTAs an SM, which spill none, were slower), R and J d on HEX 17^3 p2, Roe-Pike, went from 353 to 337 us.
 template <int D, int Q, int NV, int PDE, int FLUX>
 __global__ void __launch_bounds__(128, 4) tp_jvp_face_kernel(const TPParams P, const TPParams Pd)
 {

@@ -80,7 +80,7 @@ __device__ __forceinline__ void ns_node_gradient(const TPOps* sops, const TPPara
 
 // Gradients and traces. At q = 4 the derivative (60 products a node) and the traces of the state and its gradient (120)
 // run in block fixed point; the FP64 pipe keeps the metric products (60). HEX 24^3 p3:
-// 374 -> 227 us; four CTAs per SM here and three in the volume kernel overlap the FP64 work of one with the integer work of
+// 374 -> 227 us; four CTAs per SM here (64 registers, 36 bytes spilled) and three in the volume kernel overlap the FP64 work of one with the integer work of
 // the others: 3 steps 9.82 -> 9.11 ms.
 // FIX: false for FP64 contractions, which the tangent of a directional derivative takes (the rules of a state do not fit it).
 template <int D, int Q, int NV, bool GLL_IN, bool FIX = true>
@@ -327,6 +327,7 @@ __device__ __forceinline__ void ns_face_node(const TPParams& P, const TPParams& 
 	}
 }
 
+// FP64-bound (78 %). Three CTAs an SM: 168 registers, 188 bytes spilled with Roe-Pike in 3D.
 template <int D, int Q, int FLUX>
 __global__ void __launch_bounds__(128, 3) tp_ns_face_kernel(const TPParams P)
 {
@@ -347,7 +348,8 @@ __global__ void __launch_bounds__(128) tp_ns_jvp_face_kernel(const TPParams P, c
 }
 
 // Volume term. At q = 4 the lifting of the faces' X (90 products a node) and the derivative (60) run in block fixed point;
-// the FP64 pipe keeps the pointwise fluxes. HEX 24^3 p3: 550 -> 451 us before the bound of three CTAs per SM.
+// the FP64 pipe keeps the pointwise fluxes. HEX 24^3 p3: 550 -> 451 us before the bound of three CTAs per SM, which spills 324
+// bytes (127 registers without) and is faster all the same.
 template <int D, int Q, int NV, bool GLL_IN>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS, 3)
 tp_ns_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const double* __restrict__ u)

@@ -795,7 +795,7 @@ __device__ __forceinline__ void tp_volume_body(const TPOps* sops, bool fix, cons
 	}
 }
 
-// Four CTAs per SM (64 registers, what the shared memory allows at q = 4): the FP64 flux of one CTA then overlaps the
+// Four CTAs per SM (64 registers, 28 bytes spilled at q = 4, whose shared memory allows no more): the FP64 flux of one CTA then overlaps the
 // integer contractions of the others. HEX 32^3 p3, 5 steps: 9.33 -> 8.97 ms together with the lift's.
 template <int D, int Q, int NV, int PDE, bool GLL_IN>
 __global__ void __launch_bounds__(TPShape<D, Q>::THREADS, 4)
@@ -818,8 +818,9 @@ tp_volume_kernel(const __grid_constant__ TPOps ops, const TPParams P, const doub
 // Face numerical flux
 // ---------------------------------------------------------------------------------------------------------------
 // Bound by the FP64 pipe's sums and fused products (76 %); reciprocals, roots and lone products run on the integer pipe.
-// Lax-Friedrichs at HEX 32^3 p3: 295 -> 123 us.
-// Roe-Pike: five CTAs an SM (102 registers); the two pipes it uses overlap only across warps.
+// Lax-Friedrichs at HEX 32^3 p3: 295 -> 122 us.
+// Roe-Pike: five CTAs an SM (96 registers, 56 bytes spilled); the two pipes it uses overlap only across warps. HEX 21^3 p2 with
+// boundaries: 59 us, and 60 at four CTAs (128 registers, no spills).
 template <int FLUX>
 struct FaceOccupancy { static constexpr int value = (FLUX == kRoePike) ? 5 : 6; };
 
@@ -1167,8 +1168,9 @@ __device__ __forceinline__ void tp_lift_body(const TPOps* sops, bool fix, const 
 	}
 }
 
-// Minimum CTAs per SM of the lift kernel (caps its registers): 4 for the plain RK stage, 3 otherwise (80 registers; at 2
-// CTAs the last stage of a step with max |rhs| took 449 us at HEX 32^3 p3, twice the plain one).
+// Minimum CTAs per SM of the lift kernel (caps its registers): 4 for the plain RK stage, 3 otherwise (80 registers; the
+// stages spill some 280 bytes around the positivity check's call; at 2 CTAs the last stage of a step with max |rhs| took
+// 449 us at HEX 32^3 p3, twice the plain one).
 // Plain stages at HEX 32^3 p3: 244 us with FP64 products in the stage update, 187 to 212 with integer ones; both pipes at half.
 template <int MODE>
 struct LiftOccupancy { static constexpr int value = (MODE == kModeRkGlNoMax) ? 4 : 3; };   // Out: as RkGl
