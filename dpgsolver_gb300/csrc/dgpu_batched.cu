@@ -179,6 +179,26 @@ thread_local std::string g_batch_error;
 			return bfail((ctx), DGPU_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));        \
 	} while (0)
 
+// Lets a kernel take `bytes` of dynamic shared memory. The limit belongs to the process, not to a context, so every context
+// sets the same one, all that the device has for the kernel: one of its own size would take it away from a context with
+// larger groups.
+template <typename K>
+cudaError_t allow_smem(K* kernel, size_t bytes)
+{
+	int dev = 0, most = 0;
+	cudaFuncAttributes a;
+	cudaError_t e = cudaGetDevice(&dev);
+	if (e == cudaSuccess)
+		e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+	if (e == cudaSuccess)
+		e = cudaFuncGetAttributes(&a, kernel);
+	if (e != cudaSuccess)
+		return e;
+	most -= (int)a.sharedSizeBytes;
+	return bytes > (size_t)most ? cudaErrorInvalidValue
+	                            : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 template <int D, int Q, int NV>
 size_t bvol_smem(int E) { return sizeof(BatchOps) + (size_t)E * BSmem<D, Q, NV>::VOL * sizeof(double); }
 template <int D, int Q, int NV>
@@ -391,13 +411,12 @@ cudaError_t launch_stage(dgpu_batch* c, bool rhs_mode, double dt, int stage, int
 template <int D, int NV, int PDE, int FLUX>
 cudaError_t bind_stage(dgpu_batch* c, int sms)
 {
-	const cudaFuncAttribute A = cudaFuncAttributeMaxDynamicSharedMemorySize;
 	const size_t smem = std::max(c->fused_vol_smem, c->fused_lift_smem);
 	const void* ks[3] = {(const void*)bstage_kernel<D, NV, PDE, FLUX, kModeRhs, true>,
 	                     (const void*)bstage_kernel<D, NV, PDE, FLUX, kModeRkGl, false>,
 	                     (const void*)bstage_kernel<D, NV, PDE, FLUX, kModeRkGlNoMax, false>};
 	for (int m = 0; m < 3; ++m) {
-		cudaError_t e = cudaFuncSetAttribute(ks[m], A, (int)smem);
+		cudaError_t e = allow_smem(ks[m], smem);
 		if (e != cudaSuccess)
 			return e;
 		int per_sm = 0;
@@ -417,22 +436,21 @@ cudaError_t bind_tp_group(dgpu_batch* c, int g)
 	L.lift = launch_blift<D, Q, NV>;
 	L.conv = launch_bconv<D, Q, NV>;
 	L.E_max = std::max(1, 256 / TPShape<D, Q>::N);
-	const cudaFuncAttribute A = cudaFuncAttributeMaxDynamicSharedMemorySize;
 	const int E = L.E_max;
 	cudaError_t e;
-	if ((e = cudaFuncSetAttribute(bvol_group_kernel<D, Q, NV, PDE, true>, A, (int)bvol_smem<D, Q, NV>(E))))
+	if ((e = allow_smem(bvol_group_kernel<D, Q, NV, PDE, true>, bvol_smem<D, Q, NV>(E))))
 		return e;
-	if ((e = cudaFuncSetAttribute(bvol_group_kernel<D, Q, NV, PDE, false>, A, (int)bvol_smem<D, Q, NV>(E))))
+	if ((e = allow_smem(bvol_group_kernel<D, Q, NV, PDE, false>, bvol_smem<D, Q, NV>(E))))
 		return e;
-	if ((e = cudaFuncSetAttribute(blift_group_kernel<D, Q, NV, kModeRhs>, A, (int)blift_smem<D, Q, NV>(E))))
+	if ((e = allow_smem(blift_group_kernel<D, Q, NV, kModeRhs>, blift_smem<D, Q, NV>(E))))
 		return e;
-	if ((e = cudaFuncSetAttribute(blift_group_kernel<D, Q, NV, kModeRkGl>, A, (int)blift_smem<D, Q, NV>(E))))
+	if ((e = allow_smem(blift_group_kernel<D, Q, NV, kModeRkGl>, blift_smem<D, Q, NV>(E))))
 		return e;
-	if ((e = cudaFuncSetAttribute(blift_group_kernel<D, Q, NV, kModeRkGlNoMax>, A, (int)blift_smem<D, Q, NV>(E))))
+	if ((e = allow_smem(blift_group_kernel<D, Q, NV, kModeRkGlNoMax>, blift_smem<D, Q, NV>(E))))
 		return e;
-	if ((e = cudaFuncSetAttribute(bconvert_group_kernel<D, Q, NV, true>, A, (int)bconv_smem<D, Q, NV>(E))))
+	if ((e = allow_smem(bconvert_group_kernel<D, Q, NV, true>, bconv_smem<D, Q, NV>(E))))
 		return e;
-	if ((e = cudaFuncSetAttribute(bconvert_group_kernel<D, Q, NV, false>, A, (int)bconv_smem<D, Q, NV>(E))))
+	if ((e = allow_smem(bconvert_group_kernel<D, Q, NV, false>, bconv_smem<D, Q, NV>(E))))
 		return e;
 	// the fused kernels need the largest of the groups' shared memory
 	c->fused_vol_smem = std::max(c->fused_vol_smem, bvol_smem<D, Q, NV>(E));
@@ -467,28 +485,27 @@ cudaError_t bind_all(dgpu_batch* c)
 		if (e != cudaSuccess)
 			return e;
 	}
-	const cudaFuncAttribute A = cudaFuncAttributeMaxDynamicSharedMemorySize;
 	cudaError_t e;
 	if (c->n_dense > 0) {
-		if ((e = cudaFuncSetAttribute(dvol_group_kernel<D, NV, PDE>, A, (int)dvol_max)))
+		if ((e = allow_smem(dvol_group_kernel<D, NV, PDE>, dvol_max)))
 			return e;
-		if ((e = cudaFuncSetAttribute(dlift_group_kernel<NV, kModeRhs>, A, (int)dlift_max)))
+		if ((e = allow_smem(dlift_group_kernel<NV, kModeRhs>, dlift_max)))
 			return e;
-		if ((e = cudaFuncSetAttribute(dlift_group_kernel<NV, kModeRkGl>, A, (int)dlift_max)))
+		if ((e = allow_smem(dlift_group_kernel<NV, kModeRkGl>, dlift_max)))
 			return e;
 	}
 	c->fused_vol = launch_fused_vol<D, NV, PDE>;
 	c->fused_lift = launch_fused_lift<D, NV>;
 	c->face_nodes = launch_face_nodes<D, NV, PDE, FLUX>;
-	if ((e = cudaFuncSetAttribute(bvol_fused_kernel<D, NV, PDE, true>, A, (int)c->fused_vol_smem)))
+	if ((e = allow_smem(bvol_fused_kernel<D, NV, PDE, true>, c->fused_vol_smem)))
 		return e;
-	if ((e = cudaFuncSetAttribute(bvol_fused_kernel<D, NV, PDE, false>, A, (int)c->fused_vol_smem)))
+	if ((e = allow_smem(bvol_fused_kernel<D, NV, PDE, false>, c->fused_vol_smem)))
 		return e;
-	if ((e = cudaFuncSetAttribute(blift_fused_kernel<D, NV, kModeRhs>, A, (int)c->fused_lift_smem)))
+	if ((e = allow_smem(blift_fused_kernel<D, NV, kModeRhs>, c->fused_lift_smem)))
 		return e;
-	if ((e = cudaFuncSetAttribute(blift_fused_kernel<D, NV, kModeRkGl>, A, (int)c->fused_lift_smem)))
+	if ((e = allow_smem(blift_fused_kernel<D, NV, kModeRkGl>, c->fused_lift_smem)))
 		return e;
-	if ((e = cudaFuncSetAttribute(blift_fused_kernel<D, NV, kModeRkGlNoMax>, A, (int)c->fused_lift_smem)))
+	if ((e = allow_smem(blift_fused_kernel<D, NV, kModeRkGlNoMax>, c->fused_lift_smem)))
 		return e;
 	// persistent grids: as many CTAs as fit on the device at once
 	int dev = 0, sms = 0, per_sm = 0;
@@ -574,16 +591,15 @@ cudaError_t bind_ns_group(dgpu_batch* c, int g)
 	const int by_smem = (int)((110 * 1024 - sizeof(BatchOps)) / (BnsSmem<D, Q, NV>::MAX * sizeof(double)));
 	const int E = std::max(1, std::min(256 / N, by_smem));
 	c->hgroups[L.idx].E_ns = E;
-	const cudaFuncAttribute A = cudaFuncAttributeMaxDynamicSharedMemorySize;
 	const int sm = (int)bns_smem<D, Q, NV>(E);
 	cudaError_t e;
-	if ((e = cudaFuncSetAttribute(bns_grad_group_kernel<D, Q, NV, true>, A, sm)))
+	if ((e = allow_smem(bns_grad_group_kernel<D, Q, NV, true>, sm)))
 		return e;
-	if ((e = cudaFuncSetAttribute(bns_grad_group_kernel<D, Q, NV, false>, A, sm)))
+	if ((e = allow_smem(bns_grad_group_kernel<D, Q, NV, false>, sm)))
 		return e;
-	if ((e = cudaFuncSetAttribute(bns_volume_group_kernel<D, Q, NV, true>, A, sm)))
+	if ((e = allow_smem(bns_volume_group_kernel<D, Q, NV, true>, sm)))
 		return e;
-	return cudaFuncSetAttribute(bns_volume_group_kernel<D, Q, NV, false>, A, sm);
+	return allow_smem(bns_volume_group_kernel<D, Q, NV, false>, sm);
 }
 
 template <int D, int FLUX>
@@ -1602,7 +1618,7 @@ dgpu_status create_impl(const dgpu_physics* phys, const std::vector<GroupIn>& gi
 			B_TRY(upload_vec(&d_wj, dense_wJ[t]));
 			B_TRY(cudaMalloc((void**)&d_mv, (size_t)G.n_vol * nvs * nvs * sizeof(double)));
 			c->dense_bufs.push_back(d_mv);
-			B_TRY(cudaFuncSetAttribute(dense_minv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+			B_TRY(allow_smem(dense_minv_kernel, smem));
 			dense_minv_kernel<<<G.n_vol, 128, smem, c->stream>>>(d_cv0, d_wj, nvs, nvc, G.n_vol, d_mv);
 			B_TRY(cudaGetLastError());
 			B_TRY(cudaStreamSynchronize(c->stream));

@@ -88,6 +88,12 @@ cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const
 	(void)g;
 	return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, f, b, s);
 }
+cudaError_t cudaFuncGetAttributes(struct cudaFuncAttributes* a, const void* f)
+{
+	(void)f;
+	memset(a, 0, sizeof *a);
+	return call();
+}
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned f)
 {
 	(void)f;
